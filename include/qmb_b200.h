@@ -470,7 +470,9 @@ QMB_API qmb_status qmb_batch_create(const qmb_batch_desc* desc, qmb_batch* out);
 QMB_API qmb_status qmb_batch_destroy(qmb_batch b);
 QMB_API qmb_status qmb_batch_get_info(qmb_batch b, qmb_batch_info* info);
 /* Ground energies of all pairs: E0[set*n_sectors + sector].  c_xy, c_z are
- * host arrays [n_sets]; copied in, solved, E0 copied out. */
+ * host arrays [n_sets]; copied in, solved, E0 copied out.  Of two sectors whose
+ * matrices are complex conjugates (momenta k and -k of a real Hamiltonian) one
+ * is solved and both get its energies; summary counts the products computed. */
 QMB_API qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const double* c_z,
                            const qmb_lanczos_opts* opts, double* E0, qmb_lanczos_result* summary);
 /* One batched y = H x over all pairs on device buffers in the layout of
@@ -494,7 +496,8 @@ QMB_API qmb_status qmb_batch_k1_time(qmb_batch b, int prec, int reps, double* ms
  * a quarter of the complex sectors' rows are stored and solved complex, with
  * zero imaginary parts); each sector is [row][set] with set stride
  * info.set_stride.  offsets[s] is the
- * start of caller sector s in scalars (a complex element counts 2);
+ * start of caller sector s in scalars (a complex element counts 2; the order of
+ * the sectors inside a kind is the library's);
  * offsets[n_sectors] is the total. */
 QMB_API qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets /* [n_sectors+1] */,
                             int* is_complex /* [n_sectors] */);

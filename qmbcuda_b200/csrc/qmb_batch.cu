@@ -95,6 +95,7 @@ struct BatchArgs {
     const int* active;           // [n_sectors]
     int max_tile_entries;        // largest CSR entry count of one work item
     int c_stride;                // couplings of sector s at cxy[s * c_stride + set] (0: shared)
+    int n_tiles;                 // work items of these sectors
 };
 
 // SPL consecutive sets of one row: one 4-, 8- or 16-byte access.
@@ -1101,12 +1102,15 @@ __global__ void k_place_sector(PlaceArgs a, V64* __restrict__ val64, V32* __rest
 
 using namespace qmb;
 
-// One kind (real or complex) of sectors.
+// One kind (real or complex) of sectors.  The sectors a solve runs come first
+// (n_sectors, n_tiles); behind them lie the sectors whose matrices are the
+// complex conjugates of one of those (up to n_all, n_tiles_all), which only the
+// plain product reads.
 struct BKind {
-    int n_sectors = 0;
-    std::vector<int> sec_index;        // positions in the caller's sector list
-    std::vector<int64_t> nrows;        // per sector
-    std::vector<int64_t> sec_elem;     // [n+1]
+    int n_sectors = 0, n_all = 0;
+    std::vector<int> sec_index;        // [n_all] positions in the caller's sector list
+    std::vector<int64_t> nrows;        // [n_all] per sector
+    std::vector<int64_t> sec_elem;     // [n_all+1]
     std::vector<int> tile_sector, tile_row0, sec_tile0, sec_ntiles;
     DevBuf<int> d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active;
     DevBuf<unsigned> d_ctr;      // work queue head + retired blocks
@@ -1120,8 +1124,9 @@ struct BKind {
     std::vector<int64_t> h_row_base, h_row0;  // per sector, as on the device
     DevBuf<uint32_t> d_col;
     DevBuf<unsigned char> val64, val32, dxy64, dxy32, dz64, dz32;
-    int64_t nnz = 0, rows = 0;
-    int n_tiles = 0;
+    int64_t nnz = 0, rows = 0;          // all sectors
+    int64_t nnz_solve = 0, rows_solve = 0;  // the first n_sectors
+    int n_tiles = 0, n_tiles_all = 0;
     int max_tile_entries = 1;
 };
 
@@ -1131,6 +1136,7 @@ struct qmb_batch_s {
     BKind kind[2];  // 0 real, 1 complex
     qmb::WsPool ws;  // temporaries of the solves, reused from one solve to the next
     std::vector<int> sector_kind, sector_pos;
+    std::vector<int> alias;  // caller sector whose solve gives this sector's energies (itself, or its conjugate)
     DevBuf<double> cxy, cz;
 };
 
@@ -1157,6 +1163,7 @@ static BatchArgs make_args(const qmb_batch_s* b, const BKind& k) {
     a.active = k.d_active.p;
     a.max_tile_entries = k.max_tile_entries;
     a.c_stride = 0;
+    a.n_tiles = k.n_tiles;
     return a;
 }
 
@@ -1188,7 +1195,7 @@ static void launch_bhv_v(const BatchArgs& a, BKind& k, const V* x, V* y, V* vrin
         g = std::max(1, per_sm) * sms;
     }
     g_kernels += 1;
-    kern<<<std::min(g, k.n_tiles), kBThreads, smem, st>>>(a, k.n_tiles, k.d_ctr.p, x, y, vring, K, lz, ritz,
+    kern<<<std::min(g, a.n_tiles), kBThreads, smem, st>>>(a, a.n_tiles, k.d_ctr.p, x, y, vring, K, lz, ritz,
                                                           psi, lanczos);
 }
 
@@ -1202,7 +1209,7 @@ static bool bhv_variant_ok(int v, int nsp, int spl) {
 template <class V, int SPL>
 static void launch_bhv(int variant, const BatchArgs& a, BKind& k, const V* x, V* y, V* vring, int K,
                        BLz lz, const double* ritz, void* psi, int lanczos, cudaStream_t st) {
-    if (k.n_tiles == 0) return;
+    if (a.n_tiles == 0) return;
     QMB_REQUIRE(variant >= 0 && variant < kBVariants && bhv_variant_ok<V>(variant, a.nsp, SPL),
                 QMB_ERR_UNSUPPORTED, "k_bhv variant does not fit this batch's set count");
     switch (variant) {
@@ -1288,7 +1295,8 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     // a batch of the same shape tuned before in this process reuses the choice
     int dev = 0;
     QMB_CUDA_TRY(cudaGetDevice(&dev));
-    const TuneKey key{dev, (int)sizeof(V), a.nsp, k.n_sectors, k.n_tiles, k.max_tile_entries, k.rows, k.nnz};
+    const TuneKey key{dev, (int)sizeof(V), a.nsp, k.n_sectors, k.n_tiles, k.max_tile_entries, k.rows_solve,
+                      k.nnz_solve};
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         auto it = g_tune_cache.find(key);
@@ -1308,6 +1316,8 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     std::vector<int> ones(k.n_sectors, 1);
     act.upload(ones.data(), k.n_sectors, st);
     BatchArgs at = a;
+    at.n_sectors = k.n_sectors;
+    at.n_tiles = k.n_tiles;
     at.active = act.p;  // every sector, whatever the caller's phase has active
     BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_sec_tile0.p, k.d_sec_ntiles.p};
     k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(at, tot, 0, 2212456ull, nullptr, w.p);
@@ -1706,6 +1716,7 @@ static int run_compacted(qmb_batch_s* b, BKind& k, std::unique_ptr<BKind>& holde
     BatchArgs ac = a_base;  // matrix arrays of the base kind
     ac.n_sectors = nv;
     ac.nsp = NC;
+    ac.n_tiles = ck.n_tiles;
     ac.tile_sector = ck.d_tile_sector.p;
     ac.tile_row0 = ck.d_tile_row0.p;
     ac.sec_elem = ck.d_sec_elem.p;
@@ -2061,6 +2072,134 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
 
 }  // namespace qmb
 
+// ------------------------------------------------------ conjugate sectors
+namespace qmb {
+
+// One sector's matrices during assembly.
+struct BatchPart {
+    std::vector<int64_t> row_ptr;      // host copy, for the tile tables
+    DevBuf<int64_t> rp;                // [n+1] entry offsets within the sector
+    DevBuf<uint32_t> col;              // [nnz]
+    DevBuf<double2> val, dxy, dz;      // [nnz], [n], [n]
+};
+
+// Weighted sums of a sector's values, with weights in [1, 2) hashed from the
+// entry's place and column: out[0] = sum w Re, out[1] = sum w Im, out[2] =
+// sum w |v|, over the off-diagonal entries and both diagonals.  Two conjugate
+// matrices have equal out[0] and opposite out[1].
+__device__ __forceinline__ double hash_weight(uint64_t k) {
+    return 1.0 + (double)(mf_hash_slot(k + 0x9E3779B97F4A7C15ull, ~0ull) >> 11) * 0x1p-53;
+}
+__global__ void k_part_print(int64_t n, int64_t nnz, const uint32_t* __restrict__ col,
+                             const double2* __restrict__ val, const double2* __restrict__ dxy,
+                             const double2* __restrict__ dz, double* __restrict__ out) {
+    __shared__ double red[32];
+    double re = 0.0, im = 0.0, ab = 0.0;
+    auto add = [&](double w, double2 v) {
+        re += w * v.x;
+        im += w * v.y;
+        ab += w * (fabs(v.x) + fabs(v.y));
+    };
+    const int64_t m = n > nnz ? n : nnz;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i < nnz) add(hash_weight(((uint64_t)i << 24) ^ col[i]), val[i]);
+        if (i < n) {
+            add(hash_weight(~(uint64_t)(2 * i)), dxy[i]);
+            add(hash_weight(~(uint64_t)(2 * i + 1)), dz[i]);
+        }
+    }
+    re = block_sum(re, red);
+    im = block_sum(im, red);
+    ab = block_sum(ab, red);
+    if (threadIdx.x == 0) {
+        atomicAdd(out, re);
+        atomicAdd(out + 1, im);
+        atomicAdd(out + 2, ab);
+    }
+}
+
+// Clears *same unless the two sectors' entries have equal places and values
+// conjugate to within tol.
+__global__ void k_part_conj(int64_t n, int64_t nnz, const int64_t* __restrict__ rp1, const int64_t* __restrict__ rp2,
+                            const uint32_t* __restrict__ col1, const uint32_t* __restrict__ col2,
+                            const double2* __restrict__ v1, const double2* __restrict__ v2,
+                            const double2* __restrict__ x1, const double2* __restrict__ x2,
+                            const double2* __restrict__ z1, const double2* __restrict__ z2, double tol,
+                            int* __restrict__ same) {
+    auto conj_eq = [&](double2 a, double2 b) { return fabs(a.x - b.x) <= tol && fabs(a.y + b.y) <= tol; };
+    bool ok = true;
+    const int64_t m = n + 1 > nnz ? n + 1 : nnz;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i <= n) ok = ok && rp1[i] == rp2[i];
+        if (i < nnz) ok = ok && col1[i] == col2[i] && conj_eq(v1[i], v2[i]);
+        if (i < n) ok = ok && conj_eq(x1[i], x2[i]) && conj_eq(z1[i], z2[i]);
+    }
+    if (!ok) *same = 0;
+}
+
+// Pairs of sectors with conjugate matrices (momenta k and -k of a real
+// Hamiltonian) have the same spectrum for every coupling set, so a solve runs
+// one of the two: alias[s] is the sector that is solved for s.  A rotation's
+// characters are rounded at about 5e-16 times their phase, 2e-14 at 20 sites
+// and 5e-14 at 48, which moves an energy far less than the solves' tolerance;
+// 2.5e-13 of the mean entry is accepted.  The L=20 batch of all 20 momenta
+// solves 11 sectors (128 sets, mixed: 55.8 -> 35.6 ms a solve).
+constexpr double kConjTol = 2.5e-13;
+static void find_conjugates(const std::vector<BatchPart>& parts, const std::vector<int>& kind,
+                            std::vector<int>& alias) {
+    const int S = (int)parts.size();
+    alias.resize(S);
+    for (int s = 0; s < S; ++s) alias[s] = s;
+    if (S < 2) return;
+    auto rows = [&](int s) { return (int64_t)parts[s].row_ptr.size() - 1; };
+    auto ents = [&](int s) { return parts[s].row_ptr.back(); };
+    DevBuf<double> pr(3 * (size_t)S);
+    pr.zero();
+    for (int s = 0; s < S; ++s) {
+        const BatchPart& P = parts[s];
+        if (rows(s) == 0) continue;
+        k_part_print<<<std::min(grid_for(std::max(rows(s), ents(s)), 256), 592), 256>>>(
+            rows(s), ents(s), P.col.p, P.val.p, P.dxy.p, P.dz.p, pr.p + 3 * s);
+    }
+    check_launch("k_part_print");
+    std::vector<double> h(3 * (size_t)S);
+    pr.download(h.data(), h.size());
+    QMB_CUDA_TRY(cudaStreamSynchronize(0));
+    // candidates: the first earlier sector with equal sizes and matching sums
+    std::multimap<std::pair<int64_t, int64_t>, int> by_size;
+    std::vector<int> cand(S, -1);
+    DevBuf<int> same(S);
+    QMB_CUDA_TRY(cudaMemset(same.p, 1, sizeof(int) * S));
+    for (int s = 0; s < S; ++s) {
+        const std::pair<int64_t, int64_t> key(rows(s), ents(s));
+        auto range = by_size.equal_range(key);
+        for (auto it = range.first; it != range.second && cand[s] < 0; ++it) {
+            const int t = it->second;
+            const double tol = 1e-11 * std::max(h[3 * s + 2], h[3 * t + 2]);
+            if (kind[s] == kind[t] && rows(s) > 0 && std::fabs(h[3 * s] - h[3 * t]) <= tol &&
+                std::fabs(h[3 * s + 1] + h[3 * t + 1]) <= tol)
+                cand[s] = t;
+        }
+        if (cand[s] < 0) {
+            by_size.emplace(key, s);
+            continue;
+        }
+        const BatchPart &P = parts[cand[s]], &Q = parts[s];
+        const double mean = h[3 * s + 2] / std::max<double>(1.0, 1.5 * (double)(ents(s) + 2 * rows(s)));
+        k_part_conj<<<grid_for(std::max(rows(s) + 1, ents(s)), 256), 256>>>(
+            rows(s), ents(s), P.rp.p, Q.rp.p, P.col.p, Q.col.p, P.val.p, Q.val.p, P.dxy.p, Q.dxy.p, P.dz.p, Q.dz.p,
+            kConjTol * mean, same.p + s);
+    }
+    check_launch("k_part_conj");
+    std::vector<int> hs(S);
+    same.download(hs.data(), S);
+    QMB_CUDA_TRY(cudaStreamSynchronize(0));
+    for (int s = 0; s < S; ++s)
+        if (cand[s] >= 0 && hs[s]) alias[s] = cand[s];
+}
+
+}  // namespace qmb
+
 // ------------------------------------------------------------------ C ABI
 extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) {
     return guarded([&] {
@@ -2082,13 +2221,7 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
         b->sector_pos.resize(d->n_sectors);
         // per-sector matrices through the single-sector builder, turned into
         // CSR on the device (the sector's SELL table never leaves HBM)
-        struct Part {
-            std::vector<int64_t> row_ptr;      // host copy, for the tile tables
-            DevBuf<int64_t> rp;                // [n+1] entry offsets within the sector
-            DevBuf<uint32_t> col;              // [nnz]
-            DevBuf<double2> val, dxy, dz;      // [nnz], [n], [n]
-        };
-        std::vector<Part> parts(d->n_sectors);
+        std::vector<BatchPart> parts(d->n_sectors);
         const auto t_create = std::chrono::steady_clock::now();
         double ms_build = 0.0, ms_csr = 0.0;
         auto ms_since = [](std::chrono::steady_clock::time_point t) {
@@ -2113,7 +2246,7 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             t_part = std::chrono::steady_clock::now();
             const int64_t n = hx->n;
             b->sector_kind[s] = (hx->cplx || hz->cplx) ? 1 : 0;
-            Part& P = parts[s];
+            BatchPart& P = parts[s];
             P.rp.alloc(n + 1);
             P.row_ptr.assign(n + 1, 0);
             if (n == 0) P.rp.zero();
@@ -2175,21 +2308,32 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
                 for (int s = 0; s < d->n_sectors; ++s) b->sector_kind[s] = 1;
         }
         const auto t_assemble = std::chrono::steady_clock::now();
+        find_conjugates(parts, b->sector_kind, b->alias);
         // assemble the two kinds: host tile tables, device placement of the parts
         for (int kd = 0; kd < 2; ++kd) {
             BKind& K = b->kind[kd];
             std::vector<int64_t> row_base, row0, ent0;
             int64_t n_rp = 0, n_ent = 0, n_rows = 0;
             K.sec_elem.assign(1, 0);
-            for (int s = 0; s < d->n_sectors; ++s) {
-                if (b->sector_kind[s] != kd) continue;
-                Part& P = parts[s];
-                int ks = K.n_sectors++;
+            std::vector<int> order;  // the sectors to solve, then the conjugates of some of them
+            for (int s = 0; s < d->n_sectors; ++s)
+                if (b->sector_kind[s] == kd && b->alias[s] == s) order.push_back(s);
+            K.n_sectors = (int)order.size();
+            for (int s = 0; s < d->n_sectors; ++s)
+                if (b->sector_kind[s] == kd && b->alias[s] != s) order.push_back(s);
+            K.n_all = (int)order.size();
+            for (int ks = 0; ks < K.n_all; ++ks) {
+                const int s = order[ks];
+                BatchPart& P = parts[s];
                 b->sector_pos[s] = ks;
                 K.sec_index.push_back(s);
                 int64_t n = (int64_t)P.row_ptr.size() - 1;
                 K.nrows.push_back(n);
                 K.rows += n;
+                if (ks < K.n_sectors) {
+                    K.rows_solve += n;
+                    K.nnz_solve += P.row_ptr[n];
+                }
                 K.sec_elem.push_back(K.sec_elem.back() + n * b->nsp);
                 row_base.push_back(n_rp);
                 row0.push_back(n_rows);
@@ -2207,12 +2351,13 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
                     K.max_tile_entries = std::max<int>(K.max_tile_entries,
                                                        (int)(P.row_ptr[re] - P.row_ptr[(int64_t)t * kBTile]));
                 }
+                if (ks < K.n_sectors) K.n_tiles = (int)K.tile_sector.size();
             }
-            if (!K.n_sectors) continue;
+            if (!K.n_all) continue;
             K.nnz = n_ent;
-            K.n_tiles = (int)K.tile_sector.size();
-            std::vector<int> tiles(K.n_tiles);
-            for (int t = 0; t < K.n_tiles; ++t) tiles[t] = t;
+            K.n_tiles_all = (int)K.tile_sector.size();
+            std::vector<int> tiles(K.n_tiles_all);
+            for (int t = 0; t < K.n_tiles_all; ++t) tiles[t] = t;
             auto up_i = [](DevBuf<int>& dbuf, const std::vector<int>& v) { dbuf.alloc(std::max<size_t>(1, v.size())); if (!v.empty()) dbuf.upload(v.data(), v.size()); };
             auto up_l = [](DevBuf<int64_t>& dbuf, const std::vector<int64_t>& v) { dbuf.alloc(std::max<size_t>(1, v.size())); if (!v.empty()) dbuf.upload(v.data(), v.size()); };
             up_i(K.d_tile_sector, K.tile_sector);
@@ -2220,10 +2365,10 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             up_i(K.d_sec_tile0, K.sec_tile0);
             up_i(K.d_sec_ntiles, K.sec_ntiles);
             up_i(K.d_tiles, tiles);
-            K.d_active.alloc(K.n_sectors);
+            K.d_active.alloc(K.n_all);
             K.d_ctr.alloc(2);
             K.d_ctr.zero();
-            K.d_sec_ctr.alloc(K.n_sectors);
+            K.d_sec_ctr.alloc(K.n_all);
             K.d_sec_ctr.zero();
             up_l(K.d_sec_elem, K.sec_elem);
             up_l(K.d_nrows, K.nrows);
@@ -2241,8 +2386,8 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             K.dxy32.alloc(std::max<int64_t>(1, n_rows) * sf);
             K.dz64.alloc(std::max<int64_t>(1, n_rows) * sv);
             K.dz32.alloc(std::max<int64_t>(1, n_rows) * sf);
-            for (int ks = 0; ks < K.n_sectors; ++ks) {
-                Part& P = parts[K.sec_index[ks]];
+            for (int ks = 0; ks < K.n_all; ++ks) {
+                BatchPart& P = parts[K.sec_index[ks]];
                 const int64_t n = K.nrows[ks], ne = P.row_ptr[n];
                 const int gb = grid_for(std::max<int64_t>(n + 1, ne), 256);
                 PlaceArgs pa{n, ne, ent0[ks], P.rp.p, P.col.p, P.val.p, P.dxy.p, P.dz.p,
@@ -2281,13 +2426,15 @@ extern "C" qmb_status qmb_batch_destroy(qmb_batch b) {
     });
 }
 
-static double batch_bytes(const qmb_batch_s* b, bool f64) {
+// Algorithmic bytes of one product over all sectors, or over those a solve runs.
+static double batch_bytes(const qmb_batch_s* b, bool f64, bool solve = false) {
     double tot = 0;
     for (int kd = 0; kd < 2; ++kd) {
         const BKind& k = b->kind[kd];
+        const double rows = (double)(solve ? k.rows_solve : k.rows), nnz = (double)(solve ? k.nnz_solve : k.nnz);
         double vs = (f64 ? 8.0 : 4.0) * (kd ? 2 : 1);
         // x read once + y written once per (row, set); shared tables once
-        tot += (double)k.rows * b->n_sets * 2 * vs + (double)k.nnz * (4 + vs) + (double)k.rows * 2 * vs;
+        tot += rows * b->n_sets * 2 * vs + nnz * (4 + vs) + rows * 2 * vs;
     }
     return tot;
 }
@@ -2312,7 +2459,7 @@ extern "C" qmb_status qmb_batch_get_info(qmb_batch b, qmb_batch_info* info) {
         info->nnz_total = b->kind[0].nnz + b->kind[1].nnz;
         for (int kd = 0; kd < 2; ++kd) {
             const BKind& k = b->kind[kd];
-            const size_t vb = (size_t)k.sec_elem.back() * (kd ? sizeof(float2) : sizeof(float));
+            const size_t vb = k.n_sectors ? (size_t)k.sec_elem[k.n_sectors] * (kd ? sizeof(float2) : sizeof(float)) : 0;
             info->ring_slots[kd] = (k.n_sectors && vb) ? (int)(k.ws_ring.n / vb) : 0;
         }
     });
@@ -2323,7 +2470,7 @@ extern "C" qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets, int* is_co
         QMB_REQUIRE(b && offsets, QMB_ERR_INVALID, "null argument");
         // real sectors first, then complex ones; each [row][set] with set
         // stride info.set_stride; offsets count scalars (complex = 2)
-        const int64_t r_elems = b->kind[0].n_sectors ? b->kind[0].sec_elem[b->kind[0].n_sectors] : 0;
+        const int64_t r_elems = b->kind[0].n_all ? b->kind[0].sec_elem[b->kind[0].n_all] : 0;
         int64_t end = r_elems;
         for (int s = 0; s < b->n_sectors; ++s) {
             int kd = b->sector_kind[s];
@@ -2332,7 +2479,7 @@ extern "C" qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets, int* is_co
             offsets[s] = kd ? r_elems + 2 * k.sec_elem[ks] : k.sec_elem[ks];
             if (is_complex) is_complex[s] = kd;
         }
-        if (b->kind[1].n_sectors) end = r_elems + 2 * b->kind[1].sec_elem[b->kind[1].n_sectors];
+        if (b->kind[1].n_all) end = r_elems + 2 * b->kind[1].sec_elem[b->kind[1].n_all];
         offsets[b->n_sectors] = end;
     });
 }
@@ -2341,8 +2488,10 @@ extern "C" qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets, int* is_co
 namespace qmb {
 template <class V>
 static void batch_hv_kind(qmb_batch_s* b, BKind& k, bool f64, const V* x, V* y, cudaStream_t st) {
-    if (!k.n_sectors) return;
+    if (!k.n_all) return;
     BatchArgs a = make_args(b, k);
+    a.n_sectors = k.n_all;
+    a.n_tiles = k.n_tiles_all;
     a.val = f64 ? k.val64.p : k.val32.p;
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
@@ -2367,7 +2516,7 @@ extern "C" qmb_status qmb_batch_hv(qmb_batch b, int prec, const void* x_dev, voi
         bool f64 = prec == QMB_PREC_FP64;
         // internal layout: real kind block first, then complex kind block,
         // both padded to nsp sets (see qmb_batch_internal_elems)
-        const int64_t r_elems = b->kind[0].n_sectors ? b->kind[0].sec_elem[b->kind[0].n_sectors] : 0;
+        const int64_t r_elems = b->kind[0].n_all ? b->kind[0].sec_elem[b->kind[0].n_all] : 0;
         const char* xc = (const char*)x_dev;
         char* yc = (char*)y_dev;
         size_t rs = f64 ? 8 : 4;
@@ -2453,9 +2602,9 @@ extern "C" qmb_status qmb_batch_k1_time(qmb_batch b, int prec, int reps, double*
         // the product's bytes, plus v_{j-1} read and v_j written per (row, set)
         double extra = 0.0;
         for (int kd = 0; kd < 2; ++kd)
-            extra += 2.0 * (double)b->kind[kd].rows * b->n_sets * (f64 ? 8.0 : 4.0) * (kd ? 2 : 1);
+            extra += 2.0 * (double)b->kind[kd].rows_solve * b->n_sets * (f64 ? 8.0 : 4.0) * (kd ? 2 : 1);
         *ms = t;
-        *bytes = batch_bytes(b, f64) + extra;
+        *bytes = batch_bytes(b, f64, true) + extra;
     });
 }
 
@@ -2675,6 +2824,14 @@ extern "C" qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const dou
                 }
             (void)n_prob;
         }
+        // a conjugate sector has its partner's energies
+        for (int s = 0; s < b->n_sectors; ++s)
+            if (b->alias[s] != s)
+                for (int set = 0; set < b->n_sets; ++set) {
+                    const size_t row = (size_t)set * b->n_sectors;
+                    result[row + s] = result[row + b->alias[s]];
+                    low[row + s] = low[row + b->alias[s]];
+                }
         QMB_CUDA_TRY(cudaEventRecord(e1, st));
         QMB_CUDA_TRY(cudaEventSynchronize(e1));
         std::memcpy(E0, result.data(), sizeof(double) * result.size());
