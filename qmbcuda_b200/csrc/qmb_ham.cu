@@ -130,45 +130,78 @@ __global__ void k_ell_count(RowGen rg, int64_t n, int* __restrict__ cnt) {
     }
 }
 
-__global__ void k_slice_width(const int* __restrict__ cnt, int64_t n, int64_t n_slices,
-                              int* __restrict__ width, int64_t* __restrict__ slots) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_slices;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        int w = 0;
-        for (int i = 0; i < 32; ++i) {
-            int64_t r = s * 32 + i;
-            if (r < n) w = max(w, cnt[r]);
+// Entry totals of a table, summed on the device.
+struct EllStats {
+    unsigned long long nnz;
+    int max_row;
+};
+
+// Width and slot count of every slice (a warp reads the 32 rows of a slice
+// in one load) and the table's entry total and longest row.
+__global__ void __launch_bounds__(256) k_slice_width(const int* __restrict__ cnt, int64_t n, int64_t n_slices,
+                                                     int* __restrict__ width, int64_t* __restrict__ slots,
+                                                     EllStats* __restrict__ st) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    unsigned long long sum = 0;
+    int top = 0;
+    for (int64_t s = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); s < n_slices; s += warps) {
+        const int64_t r = s * 32 + lane;
+        const int c = r < n ? cnt[r] : 0;
+        sum += c;
+        const int w = __reduce_max_sync(0xffffffffu, c);
+        top = max(top, w);
+        if (lane == 0) {
+            width[s] = w;
+            slots[s] = (int64_t)w * 32;
         }
-        width[s] = w;
-        slots[s] = (int64_t)w * 32;
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && sum) {
+        atomicAdd(&st->nnz, sum);
+        atomicMax(&st->max_row, top);
     }
 }
 
-template <class M>
+// Columns and values of the rows, each value computed in FP64 and stored in
+// every precision kept (val64 / val32 may be null), so that no second pass
+// reads the FP64 table to narrow it.  Lanes past the last row write padding.
+template <class M64, class M32>
 __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off,
                            const int* __restrict__ width, uint32_t* __restrict__ col,
-                           M* __restrict__ val, M* __restrict__ diag) {
+                           M64* __restrict__ val64, M32* __restrict__ val32, M64* __restrict__ diag64,
+                           M32* __restrict__ diag32) {
     QMB_LOAD_GEN(rg);
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n;
+    const int64_t n_pad = (n + 31) & ~(int64_t)31;
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n_pad;
          r += (int64_t)gridDim.x * blockDim.x) {
-        int64_t o = rg.orbit_of_row[r];
-        uint64_t src = apply_elem(rg.g, gs, 0, rg.rt.reps[o]);
         int64_t s = r >> 5;
         int64_t base = off[s] + (r & 31);
         int w = width[s];
         int j = 0;
-        double2 d = gen_row(rg, gs, ts, src, rg.norms[o], [&](int64_t ot, double2 v) {
-            if (j < w) {
-                col[base + (int64_t)j * 32] = (uint32_t)rg.row_of_orbit[ot];
-                val[base + (int64_t)j * 32] = Sc<M>::from(v);
-            }
-            ++j;
-        });
-        for (; j < w; ++j) {
-            col[base + (int64_t)j * 32] = (uint32_t)r;
-            val[base + (int64_t)j * 32] = Sc<M>::zero();
+        if (r < n) {
+            int64_t o = rg.orbit_of_row[r];
+            uint64_t src = apply_elem(rg.g, gs, 0, rg.rt.reps[o]);
+            double2 d = gen_row(rg, gs, ts, src, rg.norms[o], [&](int64_t ot, double2 v) {
+                if (j < w) {
+                    const int64_t at = base + (int64_t)j * 32;
+                    col[at] = (uint32_t)rg.row_of_orbit[ot];
+                    const M64 v64 = Sc<M64>::from(v);
+                    if (val64) val64[at] = v64;
+                    if (val32) val32[at] = cvt<M32>(v64);
+                }
+                ++j;
+            });
+            const M64 d64 = Sc<M64>::from(d);
+            diag64[r] = d64;
+            if (diag32) diag32[r] = cvt<M32>(d64);
         }
-        diag[r] = Sc<M>::from(d);
+        for (; j < w; ++j) {
+            const int64_t at = base + (int64_t)j * 32;
+            col[at] = r < n ? (uint32_t)r : 0u;
+            if (val64) val64[at] = Sc<M64>::zero();
+            if (val32) val32[at] = Sc<M32>::zero();
+        }
     }
 }
 
@@ -227,13 +260,6 @@ __global__ void __launch_bounds__(256, 5) k_hv_mfw(MfOp<M> op, const V* __restri
     }
 }
 
-template <class M32, class M64>
-__global__ void k_narrow(const M64* __restrict__ a, M32* __restrict__ b, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        b[i] = cvt<M32>(a[i]);
-}
-
 // ------------------------------------------------------------- helpers
 template <class Op, class V>
 void launch_hv(const Op& op, const V* x, V* y, cudaStream_t st, size_t smem) {
@@ -256,8 +282,10 @@ void build_sell(qmb_ham_s* h) {
     h->slice_w.alloc(h->n_slices);
     DevBuf<int64_t> slots(h->n_slices + 1);
     QMB_CUDA_TRY(cudaMemset(slots.p + h->n_slices, 0, sizeof(int64_t)));
-    k_slice_width<<<grid_for(h->n_slices, 256), 256>>>(cnt.p, n, h->n_slices, h->slice_w.p,
-                                                       slots.p);
+    DevBuf<EllStats> stats(1);
+    stats.zero();
+    k_slice_width<<<std::min(grid_for(h->n_slices * 32, 256), 1184), 256>>>(cnt.p, n, h->n_slices, h->slice_w.p,
+                                                                           slots.p, stats.p);
     check_launch("k_slice_width");
     h->slice_off.alloc(h->n_slices + 1);
     size_t tb = 0;
@@ -266,57 +294,36 @@ void build_sell(qmb_ham_s* h) {
     cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.p, h->slice_off.p, h->n_slices + 1);
     QMB_CUDA_TRY(cudaMemcpy(&h->padded, h->slice_off.p + h->n_slices, sizeof(int64_t),
                             cudaMemcpyDeviceToHost));
-    // statistics
-    std::vector<int> hc(n);
-    cnt.download(hc.data(), n);
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
-    h->nnz = 0;
-    h->max_row = 0;
-    for (int64_t i = 0; i < n; ++i) {
-        h->nnz += hc[i];
-        h->max_row = std::max(h->max_row, hc[i]);
-    }
+    EllStats hs;
+    QMB_CUDA_TRY(cudaMemcpy(&hs, stats.p, sizeof(hs), cudaMemcpyDeviceToHost));
+    h->nnz = (int64_t)hs.nnz;
+    h->max_row = hs.max_row;
     int err = 0;
     QMB_CUDA_TRY(cudaMemcpy(&err, h->err.p, sizeof(int), cudaMemcpyDeviceToHost));
     QMB_REQUIRE(err == 0, QMB_ERR_INVALID,
                 err == 1 ? "a term changes the number of up spins (not an XXZ-type term)"
                          : "a target string has no representative (inconsistent group)");
 
-    size_t es = h->cplx ? sizeof(double2) : sizeof(double);
-    h->col.alloc(std::max<int64_t>(h->padded, 1));
-    h->val64.alloc(std::max<int64_t>(h->padded, 1) * es);
+    const size_t es = h->cplx ? sizeof(double2) : sizeof(double), e32 = es / 2;
+    const int64_t slots_n = std::max<int64_t>(h->padded, 1);
+    h->col.alloc(slots_n);
     h->diag64.alloc(n * es);
-    QMB_CUDA_TRY(cudaMemset(h->col.p, 0, sizeof(uint32_t) * h->col.n));
-    QMB_CUDA_TRY(cudaMemset(h->val64.p, 0, h->val64.n));
-    if (h->cplx) {
-        set_group_smem_attr((const void*)k_ell_fill<double2>, sm);
-        k_ell_fill<double2><<<grid_for(n, 128), 128, sm>>>(
-            rg, n, h->slice_off.p, h->slice_w.p, h->col.p, (double2*)h->val64.p,
-            (double2*)h->diag64.p);
-    } else {
-        set_group_smem_attr((const void*)k_ell_fill<double>, sm);
-        k_ell_fill<double><<<grid_for(n, 128), 128, sm>>>(rg, n, h->slice_off.p, h->slice_w.p,
-                                                           h->col.p, (double*)h->val64.p,
-                                                           (double*)h->diag64.p);
-    }
-    check_launch("k_ell_fill");
+    if (h->prec & QMB_PREC_FP64) h->val64.alloc(slots_n * es);
     if (h->prec & QMB_PREC_FP32) {
-        size_t e32 = h->cplx ? sizeof(float2) : sizeof(float);
-        h->val32.alloc(std::max<int64_t>(h->padded, 1) * e32);
+        h->val32.alloc(slots_n * e32);
         h->diag32.alloc(n * e32);
-        if (h->cplx) {
-            k_narrow<float2, double2><<<grid_for(h->padded, 256), 256>>>(
-                (double2*)h->val64.p, (float2*)h->val32.p, h->padded);
-            k_narrow<float2, double2><<<grid_for(n, 256), 256>>>((double2*)h->diag64.p,
-                                                                (float2*)h->diag32.p, n);
-        } else {
-            k_narrow<float, double><<<grid_for(h->padded, 256), 256>>>(
-                (double*)h->val64.p, (float*)h->val32.p, h->padded);
-            k_narrow<float, double><<<grid_for(n, 256), 256>>>((double*)h->diag64.p,
-                                                              (float*)h->diag32.p, n);
-        }
-        check_launch("k_narrow");
     }
+    auto fill = [&](auto m64, auto m32) {
+        using M64 = decltype(m64);
+        using M32 = decltype(m32);
+        auto kern = k_ell_fill<M64, M32>;
+        set_group_smem_attr((const void*)kern, sm);
+        kern<<<grid_for(n, 128), 128, sm>>>(rg, n, h->slice_off.p, h->slice_w.p, h->col.p, (M64*)h->val64.p,
+                                            (M32*)h->val32.p, (M64*)h->diag64.p, (M32*)h->diag32.p);
+    };
+    if (h->cplx) fill(double2{}, float2{});
+    else fill(0.0, 0.0f);
+    check_launch("k_ell_fill");
     QMB_CUDA_TRY(cudaDeviceSynchronize());
 }
 
@@ -339,15 +346,48 @@ __device__ __forceinline__ bool val_zero(double v) { return v == 0.0; }
 __device__ __forceinline__ bool val_zero(float2 v) { return v.x == 0.0f && v.y == 0.0f; }
 __device__ __forceinline__ bool val_zero(double2 v) { return v.x == 0.0 && v.y == 0.0; }
 
-// Every stride-th slot of the sliced ELL's FP32 values (dictionary sample).
+// Inserts a nonzero key into an open-addressing set of kCbMissCap keys (empty
+// slots hold ~0): 1 when the key is new, 0 when it was there, -1 when full.
+__device__ __forceinline__ int key_insert(unsigned long long* tab, uint64_t key) {
+    const uint32_t h = (uint32_t)(key ^ (key >> 29)) * 0x9e3779b1u;
+    for (int probe = 0; probe < kCbMissCap; ++probe) {
+        unsigned long long* at = tab + ((h + (uint32_t)probe) & (uint32_t)(kCbMissCap - 1));
+        unsigned long long prev = *(volatile unsigned long long*)at;
+        if (prev == ~0ull) prev = atomicCAS(at, ~0ull, (unsigned long long)key);
+        if (prev == ~0ull) return 1;
+        if (prev == key) return 0;
+    }
+    return -1;
+}
+
+// The distinct nonzero values among every stride-th slot of the sliced ELL,
+// into the set keys [kCbMissCap]; full[0] counts insertions that found no
+// room.  A block collects in shared memory first (a matrix has some tens of
+// values, so almost every probe is one shared-memory read) and adds its set to
+// the global one at the end.
 template <class M>
-__global__ void k_cb_sample(const M* __restrict__ val, int64_t padded, int64_t stride, int64_t n_out,
-                            uint64_t* __restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_out;
+__global__ void __launch_bounds__(256) k_cb_sample(const M* __restrict__ val, int64_t padded, int64_t stride,
+                                                   int64_t n_samp, unsigned long long* __restrict__ keys,
+                                                   int* __restrict__ full) {
+    __shared__ unsigned long long tab[kCbMissCap];
+    for (int i = threadIdx.x; i < kCbMissCap; i += blockDim.x) tab[i] = ~0ull;
+    __syncthreads();
+    int bad = 0;
+    uint64_t last = ~0ull;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_samp;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t k = i * stride;
-        out[i] = k < padded ? val_key(val[k]) : 0ull;
+        if (k >= padded) break;
+        const M v = val[k];
+        const uint64_t key = val_key(v);
+        if (val_zero(v) || key == last) continue;
+        last = key;
+        bad |= key_insert(tab, key) < 0;
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kCbMissCap; i += blockDim.x)
+        if (tab[i] != ~0ull) bad |= key_insert(keys, tab[i]) < 0;
+    if (bad) atomicAdd(full, 1);
 }
 
 // Entries of row r (nonzero values) per column block: cnt[b * n + r].
@@ -418,15 +458,9 @@ __global__ void k_cb_fill(SellOp<M> a, int shift, int nb, const int64_t* __restr
                 else hi = mid;
             }
             if (lo == n_keys || sk[lo] != key) {
-                uint32_t hsh = (uint32_t)(key ^ (key >> 29)) * 0x9e3779b1u;
-                int probe = 0;
-                for (; probe < kCbMissCap; ++probe) {
-                    const int at = (int)((hsh + (uint32_t)probe) & (uint32_t)(kCbMissCap - 1));
-                    const unsigned long long prev = atomicCAS(miss_keys + at, ~0ull, (unsigned long long)key);
-                    if (prev == ~0ull) atomicAdd(miss, 1);
-                    if (prev == ~0ull || prev == key) break;
-                }
-                if (probe == kCbMissCap) atomicAdd(miss + 1, 1);
+                const int ins = key_insert(miss_keys, key);
+                if (ins > 0) atomicAdd(miss, 1);
+                else if (ins < 0) atomicAdd(miss + 1, 1);
                 continue;
             }
             const uint32_t c = a.col[k];
@@ -464,26 +498,29 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
         return;
     }
     SellOp<M> a = h->sell<M>(f64);
-    // dictionary from a strided sample of the values
+    // dictionary from a strided sample of the values, reduced to its distinct
+    // nonzero keys on the device (copying the 2^20 samples out and sorting them
+    // on the host was most of a 28-site matrix's build: 28.4 -> 12.8 ms with the fill below)
     const int64_t n_samp = std::min<int64_t>(h->padded, (int64_t)1 << 20);
-    const int64_t stride = std::max<int64_t>(1, h->padded / n_samp);
+    const int64_t stride = std::max<int64_t>(1, h->padded / std::max<int64_t>(1, n_samp));
     std::vector<uint64_t> keys;
+    DevBuf<int> miss(2);
+    DevBuf<unsigned long long> mkeys(kCbMissCap);
+    std::vector<unsigned long long> extra(kCbMissCap);
     {
-        DevBuf<uint64_t> smp(n_samp);
-        k_cb_sample<M><<<grid_for(n_samp, 256), 256>>>(a.val, h->padded, stride, n_samp, smp.p);
+        miss.zero();
+        QMB_CUDA_TRY(cudaMemset(mkeys.p, 0xff, sizeof(unsigned long long) * kCbMissCap));
+        k_cb_sample<M><<<std::min(grid_for(n_samp, 256), 592), 256>>>(a.val, h->padded, stride, n_samp, mkeys.p,
+                                                                      miss.p);
         check_launch("k_cb_sample");
-        std::vector<uint64_t> hs(n_samp);
-        smp.download(hs.data(), n_samp);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
-        std::sort(hs.begin(), hs.end());
-        hs.erase(std::unique(hs.begin(), hs.end()), hs.end());
-        for (uint64_t k : hs) {
-            // +-0 in every component
-            const bool zero = f64 ? (k << 1) == 0
-                                  : es == 4 ? ((uint32_t)k << 1) == 0
-                                            : (((uint32_t)k << 1) == 0 && ((uint32_t)(k >> 32) << 1) == 0);
-            if (!zero) keys.push_back(k);
-        }
+        int full = 0;
+        QMB_CUDA_TRY(cudaMemcpy(extra.data(), mkeys.p, sizeof(unsigned long long) * kCbMissCap,
+                                cudaMemcpyDeviceToHost));
+        QMB_CUDA_TRY(cudaMemcpy(&full, miss.p, sizeof(int), cudaMemcpyDeviceToHost));
+        for (unsigned long long k : extra)
+            if (k != ~0ull) keys.push_back(k);
+        std::sort(keys.begin(), keys.end());
+        if (full) keys.clear();
     }
     if (keys.empty() || keys.size() > 255) {
         cb_skip("no values, or more than 255 distinct values in the sample");
@@ -520,8 +557,6 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
     }
     DevBuf<uint32_t> packed(std::max<int64_t>(total, 1));
     QMB_CUDA_TRY(cudaMemset(packed.p, 0, sizeof(uint32_t) * packed.n));
-    DevBuf<int> miss(2);
-    DevBuf<unsigned long long> mkeys(kCbMissCap);
     // values the sample missed join the dictionary and the pass repeats (it
     // rewrites every entry in place)
     for (int round = 0;; ++round) {
@@ -539,7 +574,6 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
             cb_skip("more distinct values than the dictionary holds");
             return;
         }
-        std::vector<unsigned long long> extra(kCbMissCap);
         QMB_CUDA_TRY(cudaMemcpy(extra.data(), mkeys.p, sizeof(unsigned long long) * kCbMissCap,
                                 cudaMemcpyDeviceToHost));
         for (unsigned long long k : extra)
@@ -866,18 +900,13 @@ extern "C" qmb_status qmb_ham_create(qmb_sector s, const qmb_terms* terms, int p
         h->device = s->device;
         h->n = s->n_active;
         h->irrep_gen = s->irrep_gen;
-        h->prec = prec | QMB_PREC_FP64;  // FP64 values are always built first
+        h->prec = prec;
         h->cplx = !s->is_real || terms_complex(terms);
         upload_terms(h.get(), terms, s->L);
         h->err.alloc(1);
         h->err.zero();
         build_sell(h.get());
         build_cb(h.get());
-        if (!(prec & QMB_PREC_FP64)) {
-            // keep FP64 values only when asked for; the matrix-free path needs none
-            h->val64.release();
-            h->prec = prec;
-        }
         *out = h.release();
     });
 }
