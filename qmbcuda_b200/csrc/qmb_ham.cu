@@ -205,6 +205,207 @@ __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off
     }
 }
 
+// ------------------------------------------------- packed slot order
+// A product's gathers are bound by the L1 sectors a warp's load of one slot
+// touches.  The 32 rows of a slice have neighbouring representatives, so the
+// entries that one term generates in them have neighbouring columns: placing
+// a term's entries in one slot lets a load share sectors.  With the entries of
+// each row simply in term order, 32 of them touch 17 sectors of 32 bytes on a
+// 26-site J1-J2 sector (FP32) and 12 lines of 128; packed they touch 12 and 8.5,
+// at the same slice widths.  An SM looks up about one line a cycle, so the 8.5
+// lines of a load bound the L=32 J1-J2 product at 0.30 ms.  Measured: that
+// product 383 -> 360 us (FP32), the L=30 one 256 -> 210 us (FP64, with the coded
+// operator's six blocks an SM).
+//
+// Two passes, a warp a slice.  k_ell_masks tests every term on the 32 rows and
+// keeps a ballot of the rows in which it has an entry (mobile terms only, those
+// with an S+ or S-), the diagonal and the slice's width.  When every orbit is
+// active an entry exists wherever the term does not annihilate the string, and
+// no orbit search is needed.  k_ell_pack places the masks, larger ones first,
+// each in the first slot where none of its rows is taken; a mask that fits
+// nowhere is split over the rows' free slots.  Every lane then walks its own
+// terms, so that the orbit searches of a warp run together instead of at the
+// term where each lane finds an entry.  Slices wider than 64 keep term order.
+constexpr int kPackMaxTerms = 1024;  // mobile terms (7 bytes of shared memory a warp each)
+constexpr int kPackWarps = 4;        // warps a block
+
+struct PackArgs {
+    const int16_t* midx;  // [n_terms] position among the mobile terms, or -1
+    const uint16_t* mob;  // [n_mob] their term indices
+    int n_mob;
+    int exact;            // every orbit is active
+    uint32_t* masks;      // [n_slices][n_mob]
+};
+
+template <class M64, class M32>
+__global__ void __launch_bounds__(32 * kPackWarps) k_ell_masks(RowGen rg, PackArgs pk, int64_t n, int64_t n_slices,
+                                                              int* __restrict__ width, int64_t* __restrict__ slots,
+                                                              M64* __restrict__ diag64, M32* __restrict__ diag32,
+                                                              EllStats* __restrict__ st) {
+    QMB_LOAD_GEN(rg);
+    const int lane = threadIdx.x & 31;
+    unsigned long long sum = 0;
+    int top = 0;
+    for (int64_t s = blockIdx.x * (int64_t)kPackWarps + (threadIdx.x >> 5); s < n_slices;
+         s += (int64_t)gridDim.x * kPackWarps) {
+        const int64_t r = s * 32 + lane;
+        const bool act = r < n;
+        const int64_t o = act ? rg.orbit_of_row[r] : 0;
+        const uint64_t src = act ? apply_elem(rg.g, gs, 0, rg.rt.reps[o]) : 0ull;
+        uint32_t* mk = pk.masks + s * pk.n_mob;
+        double2 d = make_double2(0.0, 0.0);
+        int c = 0;
+        for (int hi = 0; hi < ts.n_terms; ++hi) {
+            uint64_t t = src;
+            double2 coef;
+            const bool some = act && apply_term(ts, hi, src, &t, &coef);
+            bool live = some && t != src;
+            if (some && !live) {
+                d.x += coef.x;
+                d.y += coef.y;
+            }
+            const int m = pk.midx[hi];
+            if (m < 0) continue;
+            if (live && __popcll(t) != rg.n_up) {
+                *rg.err = 1;
+                live = false;
+            }
+            if (!pk.exact && live) {
+                int e;
+                const int64_t ot = find_rep(rg.rt, orbit_min(rg.g, gs, t, &e));
+                if (ot < 0) *rg.err = 2;
+                live = ot >= 0 && !(rg.norms[ot] < rg.tol);
+            }
+            const uint32_t b = __ballot_sync(0xffffffffu, live);
+            if (lane == 0) mk[m] = b;
+            c += live ? 1 : 0;
+        }
+        if (act) {
+            const M64 d64 = Sc<M64>::from(d);
+            diag64[r] = d64;
+            if (diag32) diag32[r] = cvt<M32>(d64);
+        }
+        sum += c;
+        const int w = __reduce_max_sync(0xffffffffu, c);
+        top = max(top, w);
+        if (lane == 0) {
+            width[s] = w;
+            slots[s] = (int64_t)w * 32;
+        }
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0 && sum) {
+        atomicAdd(&st->nnz, sum);
+        atomicMax(&st->max_row, top);
+    }
+}
+
+template <class M64, class M32>
+__global__ void __launch_bounds__(32 * kPackWarps) k_ell_pack(RowGen rg, PackArgs pk, int64_t n, int64_t n_slices,
+                                                             const int64_t* __restrict__ off,
+                                                             const int* __restrict__ width, uint32_t* __restrict__ col,
+                                                             M64* __restrict__ val64, M32* __restrict__ val32) {
+    QMB_LOAD_GEN(rg);
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nm = pk.n_mob;
+    const uint32_t lmask = (1u << lane) - 1u;
+    unsigned char* sp = smem + align16(align16(group_smem_bytes(rg.g)) + terms_smem_bytes(rg.terms));
+    uint32_t* s_mask = reinterpret_cast<uint32_t*>(sp) + wib * nm;
+    uint16_t* s_ord = reinterpret_cast<uint16_t*>(sp + 4 * (size_t)nm * kPackWarps) + wib * nm;
+    uint8_t* s_slot = sp + 6 * (size_t)nm * kPackWarps + wib * nm;
+    for (int64_t s = blockIdx.x * (int64_t)kPackWarps + wib; s < n_slices; s += (int64_t)gridDim.x * kPackWarps) {
+        const int w = width[s];
+        const int64_t base = off[s] + lane;
+        const int64_t r = s * 32 + lane;
+        const bool act = r < n;
+        __syncwarp();
+        for (int i = lane; i < nm; i += 32) s_mask[i] = pk.masks[s * nm + i];
+        __syncwarp();
+        uint64_t free = 0;  // this row's slots that no placed mask takes
+        if (w <= 64) {
+            // the terms with entries, in classes of decreasing size
+            int cnt = 0;
+#pragma unroll
+            for (int cl = 3; cl >= 0; --cl)
+                for (int i0 = 0; i0 < nm; i0 += 32) {
+                    const int i = i0 + lane;
+                    const int c = i < nm ? __popc(s_mask[i]) : 0;
+                    const bool in = c > 0 && (c - 1) >> 3 == cl;
+                    const uint32_t b = __ballot_sync(0xffffffffu, in);
+                    if (in) s_ord[cnt + __popc(b & lmask)] = (uint16_t)i;
+                    cnt += __popc(b);
+                }
+            __syncwarp();
+            uint32_t occ0 = lane < w ? 0u : ~0u, occ1 = lane + 32 < w ? 0u : ~0u;  // rows taken of slots lane, lane + 32
+            for (int k = 0; k < cnt; ++k) {
+                const int i = s_ord[k];
+                const uint32_t m = s_mask[i];
+                const uint32_t b0 = __ballot_sync(0xffffffffu, (occ0 & m) == 0u);
+                const uint32_t b1 = w > 32 ? __ballot_sync(0xffffffffu, (occ1 & m) == 0u) : 0u;
+                const int at = b0 ? __ffs(b0) - 1 : (b1 ? 31 + __ffs(b1) : 255);
+                if (at == lane) occ0 |= m;
+                else if (at == lane + 32) occ1 |= m;
+                if (lane == 0) s_slot[i] = (uint8_t)at;
+            }
+            for (int k = 0; k < w; ++k) {
+                const uint32_t o = __shfl_sync(0xffffffffu, k < 32 ? occ0 : occ1, k & 31);
+                if (!((o >> lane) & 1u)) free |= 1ull << k;
+            }
+            __syncwarp();
+        }
+        if (act) {
+            const int64_t o = rg.orbit_of_row[r];
+            const uint64_t src = apply_elem(rg.g, gs, 0, rg.rt.reps[o]);
+            const double ns = rg.norms[o];
+            int j = 0;
+            for (int i = 0;; ++i) {
+                while (i < nm && !((s_mask[i] >> lane) & 1u)) ++i;
+                if (i >= nm) break;
+                const int hi = pk.mob[i];
+                int at = j;
+                if (w <= 64) {
+                    at = s_slot[i];
+                    if (at == 255) {
+                        at = __ffsll((long long)free) - 1;
+                        free &= free - 1;
+                    }
+                }
+                ++j;
+                gen_row_range(rg, gs, ts, hi, hi + 1, src, ns, [&](int64_t ot, double2 v) {
+                    const int64_t p = base + (int64_t)at * 32;
+                    col[p] = (uint32_t)rg.row_of_orbit[ot];
+                    const M64 v64 = Sc<M64>::from(v);
+                    if (val64) val64[p] = v64;
+                    if (val32) val32[p] = cvt<M32>(v64);
+                });
+            }
+            if (w > 64)
+                for (; j < w; ++j) {
+                    const int64_t p = base + (int64_t)j * 32;
+                    col[p] = (uint32_t)r;
+                    if (val64) val64[p] = Sc<M64>::zero();
+                    if (val32) val32[p] = Sc<M32>::zero();
+                }
+        } else {
+            free = w < 64 ? (1ull << w) - 1 : ~0ull;
+            if (w > 64)
+                for (int k = 64; k < w; ++k) {
+                    const int64_t p = base + (int64_t)k * 32;
+                    col[p] = 0u;
+                    if (val64) val64[p] = Sc<M64>::zero();
+                    if (val32) val32[p] = Sc<M32>::zero();
+                }
+        }
+        // padding: the row itself (0 past the last row) with a zero value
+        while (free) {
+            const int64_t p = base + (int64_t)(__ffsll((long long)free) - 1) * 32;
+            free &= free - 1;
+            col[p] = act ? (uint32_t)r : 0u;
+            if (val64) val64[p] = Sc<M64>::zero();
+            if (val32) val32[p] = Sc<M32>::zero();
+        }
+    }
+}
+
 // Reference row-major layout over all orbits (null rows: track 0, ind[row*W] = row).
 __global__ void k_ell_ref(RowGen rg, int64_t R, int W, uint32_t* __restrict__ ind,
                           double2* __restrict__ val, int16_t* __restrict__ track,
@@ -270,23 +471,75 @@ void launch_hv(const Op& op, const V* x, V* y, cudaStream_t st, size_t smem) {
     check_launch("k_hv");
 }
 
-void build_sell(qmb_ham_s* h) {
+// Builds the sliced ELL.  Tables of at most kPackMaxTerms mobile terms whose
+// masks fit an eighth of the free memory get the packed slot order; the others
+// (thousands of couplings) are counted and filled row by row in term order.
+void build_sell(qmb_ham_s* h, const qmb_terms* t) {
     RowGen rg = h->row_gen();
-    size_t sm = gen_smem(rg);
+    const size_t sm = gen_smem(rg);
     int64_t n = h->n;
-    DevBuf<int> cnt(n);
-    set_group_smem_attr((const void*)k_ell_count, sm);
-    k_ell_count<<<grid_for(n, 128), 128, sm>>>(rg, n, cnt.p);
-    check_launch("k_ell_count");
+    const size_t es = h->cplx ? sizeof(double2) : sizeof(double), e32 = es / 2;
     h->n_slices = (n + 31) / 32;
     h->slice_w.alloc(h->n_slices);
     DevBuf<int64_t> slots(h->n_slices + 1);
     QMB_CUDA_TRY(cudaMemset(slots.p + h->n_slices, 0, sizeof(int64_t)));
     DevBuf<EllStats> stats(1);
     stats.zero();
-    k_slice_width<<<std::min(grid_for(h->n_slices * 32, 256), 1184), 256>>>(cnt.p, n, h->n_slices, h->slice_w.p,
-                                                                           slots.p, stats.p);
-    check_launch("k_slice_width");
+    h->diag64.alloc(n * es);
+    if (h->prec & QMB_PREC_FP32) h->diag32.alloc(n * e32);
+
+    std::vector<int16_t> midx(std::max(1, t->n_terms), -1);
+    std::vector<uint16_t> mob;
+    for (int i = 0; i < t->n_terms; ++i)
+        for (int j = 0; j < t->n_ops[i]; ++j) {
+            const int c = t->op_code[i * t->n_col + j];
+            if (c != QMB_OP_SP && c != QMB_OP_SM) continue;
+            midx[i] = (int16_t)mob.size();
+            mob.push_back((uint16_t)i);
+            break;
+        }
+    const size_t sm_pack = align16(sm) + 7 * (size_t)kPackWarps * mob.size();
+    size_t fr = 0, tot = 0;
+    QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    const size_t mask_bytes = sizeof(uint32_t) * (size_t)h->n_slices * std::max<size_t>(1, mob.size());
+    const bool packed = mob.size() <= (size_t)kPackMaxTerms && mask_bytes <= fr / 8 && sm_pack <= 200 * 1024;
+    PackArgs pk{nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0, nullptr};
+    DevBuf<int16_t> d_midx;
+    DevBuf<uint16_t> d_mob;
+    DevBuf<uint32_t> masks;
+    DevBuf<int> cnt;
+    auto typed = [&](auto&& f) {
+        if (h->cplx) f(double2{}, float2{});
+        else f(0.0, 0.0f);
+    };
+    const int pack_grid = grid_for(h->n_slices, kPackWarps);
+    if (packed) {
+        d_midx.alloc(midx.size());
+        d_midx.upload(midx.data(), midx.size());
+        d_mob.alloc(std::max<size_t>(1, mob.size()));
+        if (!mob.empty()) d_mob.upload(mob.data(), mob.size());
+        masks.alloc(mask_bytes / sizeof(uint32_t));
+        pk.midx = d_midx.p;
+        pk.mob = d_mob.p;
+        pk.masks = masks.p;
+        typed([&](auto m64, auto m32) {
+            using M64 = decltype(m64);
+            using M32 = decltype(m32);
+            auto kern = k_ell_masks<M64, M32>;
+            set_group_smem_attr((const void*)kern, sm);
+            kern<<<pack_grid, 32 * kPackWarps, sm>>>(rg, pk, n, h->n_slices, h->slice_w.p, slots.p, (M64*)h->diag64.p,
+                                                     (M32*)h->diag32.p, stats.p);
+        });
+        check_launch("k_ell_masks");
+    } else {
+        cnt.alloc(n);
+        set_group_smem_attr((const void*)k_ell_count, sm);
+        k_ell_count<<<grid_for(n, 128), 128, sm>>>(rg, n, cnt.p);
+        check_launch("k_ell_count");
+        k_slice_width<<<std::min(grid_for(h->n_slices * 32, 256), 1184), 256>>>(cnt.p, n, h->n_slices, h->slice_w.p,
+                                                                               slots.p, stats.p);
+        check_launch("k_slice_width");
+    }
     h->slice_off.alloc(h->n_slices + 1);
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, slots.p, h->slice_off.p, h->n_slices + 1);
@@ -298,33 +551,36 @@ void build_sell(qmb_ham_s* h) {
     QMB_CUDA_TRY(cudaMemcpy(&hs, stats.p, sizeof(hs), cudaMemcpyDeviceToHost));
     h->nnz = (int64_t)hs.nnz;
     h->max_row = hs.max_row;
-    int err = 0;
-    QMB_CUDA_TRY(cudaMemcpy(&err, h->err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    QMB_REQUIRE(err == 0, QMB_ERR_INVALID,
-                err == 1 ? "a term changes the number of up spins (not an XXZ-type term)"
-                         : "a target string has no representative (inconsistent group)");
+    auto check_err = [&]() {
+        int err = 0;
+        QMB_CUDA_TRY(cudaMemcpy(&err, h->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+        QMB_REQUIRE(err == 0, QMB_ERR_INVALID,
+                    err == 1 ? "a term changes the number of up spins (not an XXZ-type term)"
+                             : "a target string has no representative (inconsistent group)");
+    };
+    check_err();
 
-    const size_t es = h->cplx ? sizeof(double2) : sizeof(double), e32 = es / 2;
     const int64_t slots_n = std::max<int64_t>(h->padded, 1);
     h->col.alloc(slots_n);
-    h->diag64.alloc(n * es);
     if (h->prec & QMB_PREC_FP64) h->val64.alloc(slots_n * es);
-    if (h->prec & QMB_PREC_FP32) {
-        h->val32.alloc(slots_n * e32);
-        h->diag32.alloc(n * e32);
-    }
-    auto fill = [&](auto m64, auto m32) {
+    if (h->prec & QMB_PREC_FP32) h->val32.alloc(slots_n * e32);
+    typed([&](auto m64, auto m32) {
         using M64 = decltype(m64);
         using M32 = decltype(m32);
-        auto kern = k_ell_fill<M64, M32>;
-        set_group_smem_attr((const void*)kern, sm);
-        kern<<<grid_for(n, 128), 128, sm>>>(rg, n, h->slice_off.p, h->slice_w.p, h->col.p, (M64*)h->val64.p,
-                                            (M32*)h->val32.p, (M64*)h->diag64.p, (M32*)h->diag32.p);
-    };
-    if (h->cplx) fill(double2{}, float2{});
-    else fill(0.0, 0.0f);
+        if (packed) {
+            auto kern = k_ell_pack<M64, M32>;
+            set_group_smem_attr((const void*)kern, sm_pack);
+            kern<<<pack_grid, 32 * kPackWarps, sm_pack>>>(rg, pk, n, h->n_slices, h->slice_off.p, h->slice_w.p,
+                                                          h->col.p, (M64*)h->val64.p, (M32*)h->val32.p);
+        } else {
+            auto kern = k_ell_fill<M64, M32>;
+            set_group_smem_attr((const void*)kern, sm);
+            kern<<<grid_for(n, 128), 128, sm>>>(rg, n, h->slice_off.p, h->slice_w.p, h->col.p, (M64*)h->val64.p,
+                                                (M32*)h->val32.p, (M64*)h->diag64.p, (M32*)h->diag32.p);
+        }
+    });
     check_launch("k_ell_fill");
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    check_err();
 }
 
 // ------------------------------------------ column-blocked coded layout
@@ -464,6 +720,10 @@ __global__ void k_cb_fill(SellOp<M> a, int shift, int nb, const int64_t* __restr
                 continue;
             }
             const uint32_t c = a.col[k];
+            if (nb == 1) {  // the plain layout's slots, which may be in packed order
+                packed[k] = ((uint32_t)(lo + 1) << 24) | c;
+                continue;
+            }
             const int b = (int)(c >> shift);
             packed[off[(int64_t)b * n_slices + s] + (int64_t)pos[b] * 32 + lane] =
                 ((uint32_t)(lo + 1) << 24) | (c & lmask);
@@ -526,29 +786,35 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
         cb_skip("no values, or more than 255 distinct values in the sample");
         return;
     }
-    // per-block widths and offsets
+    // per-block widths and offsets; a single block keeps the plain layout's
     const int64_t ns = h->n_slices;
     size_t fr = 0, tot = 0;
-    QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-    if ((size_t)nb * n + 2 * n * 16 > fr / 2) {
-        cb_skip("not enough free memory for the counts");
-        return;
-    }
-    DevBuf<uint8_t> cnt((size_t)nb * n);
-    k_cb_count<M><<<grid_for(n, 256), 256>>>(a, shift, nb, cnt.p);
-    check_launch("k_cb_count");
     DevBuf<int> width((size_t)nb * ns);
-    DevBuf<int64_t> slots((size_t)nb * ns + 1), off((size_t)nb * ns + 1);
-    QMB_CUDA_TRY(cudaMemset(slots.p + (size_t)nb * ns, 0, sizeof(int64_t)));
-    k_cb_width<<<grid_for((int64_t)nb * ns, 256), 256>>>(cnt.p, n, ns, nb, width.p, slots.p);
-    check_launch("k_cb_width");
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, slots.p, off.p, (int64_t)nb * ns + 1);
-    DevBuf<unsigned char> tmp(tb);
-    cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.p, off.p, (int64_t)nb * ns + 1);
+    DevBuf<int64_t> off((size_t)nb * ns + 1);
     int64_t total = 0;
-    QMB_CUDA_TRY(cudaMemcpy(&total, off.p + (size_t)nb * ns, sizeof(int64_t), cudaMemcpyDeviceToHost));
-    cnt.release();
+    if (nb == 1) {
+        total = h->padded;
+        QMB_CUDA_TRY(cudaMemcpyAsync(width.p, h->slice_w.p, sizeof(int) * ns, cudaMemcpyDeviceToDevice, 0));
+        QMB_CUDA_TRY(cudaMemcpyAsync(off.p, h->slice_off.p, sizeof(int64_t) * (ns + 1), cudaMemcpyDeviceToDevice, 0));
+    } else {
+        QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        if ((size_t)nb * n + 2 * n * 16 > fr / 2) {
+            cb_skip("not enough free memory for the counts");
+            return;
+        }
+        DevBuf<uint8_t> cnt((size_t)nb * n);
+        k_cb_count<M><<<grid_for(n, 256), 256>>>(a, shift, nb, cnt.p);
+        check_launch("k_cb_count");
+        DevBuf<int64_t> slots((size_t)nb * ns + 1);
+        QMB_CUDA_TRY(cudaMemset(slots.p + (size_t)nb * ns, 0, sizeof(int64_t)));
+        k_cb_width<<<grid_for((int64_t)nb * ns, 256), 256>>>(cnt.p, n, ns, nb, width.p, slots.p);
+        check_launch("k_cb_width");
+        size_t tb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tb, slots.p, off.p, (int64_t)nb * ns + 1);
+        DevBuf<unsigned char> tmp(tb);
+        cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.p, off.p, (int64_t)nb * ns + 1);
+        QMB_CUDA_TRY(cudaMemcpy(&total, off.p + (size_t)nb * ns, sizeof(int64_t), cudaMemcpyDeviceToHost));
+    }
     QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
     const size_t need = (size_t)total * 4 + (size_t)n * (h->cplx ? 16 : 8);
     if (need > fr / 10 * 9) {
@@ -905,7 +1171,7 @@ extern "C" qmb_status qmb_ham_create(qmb_sector s, const qmb_terms* terms, int p
         upload_terms(h.get(), terms, s->L);
         h->err.alloc(1);
         h->err.zero();
-        build_sell(h.get());
+        build_sell(h.get(), terms);
         build_cb(h.get());
         *out = h.release();
     });
