@@ -1128,6 +1128,13 @@ struct BKind {
     int64_t nnz_solve = 0, rows_solve = 0;  // the first n_sectors
     int n_tiles = 0, n_tiles_all = 0;
     int max_tile_entries = 1;
+
+    void mark_idle() {
+        qmb::mark_idle(d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active, d_ctr, d_sec_ctr, ws_ring,
+                       ws_w, d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0, d_col, val64, val32, dxy64, dxy32, dz64,
+                       dz32);
+        if (compact) compact->mark_idle();
+    }
 };
 
 struct qmb_batch_s {
@@ -1138,6 +1145,15 @@ struct qmb_batch_s {
     std::vector<int> sector_kind, sector_pos;
     std::vector<int> alias;  // caller sector whose solve gives this sector's energies (itself, or its conjugate)
     DevBuf<double> cxy, cz;
+
+    // freeing cxy waits for the device; the rest is idle then
+    ~qmb_batch_s() {
+        if (!cxy.p) return;
+        cxy.release();
+        cz.mark_idle();
+        for (BKind& k : kind) k.mark_idle();
+        for (auto& b : ws.bufs) b->mark_idle();
+    }
 };
 
 namespace qmb {
@@ -1413,7 +1429,7 @@ static int ring_start() {
 // device memory (at most want); 0 when fewer than 16 fit.
 static int krylov_slots(size_t vec_bytes, int want, size_t cached = 0) {
     size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return 0;
+    if (!dev_mem_info(&fr, &tot)) return 0;
     fr += cached;
     size_t n = (size_t)(0.5 * (double)fr) / std::max<size_t>(vec_bytes, 1);
     if (n < 16) return 0;
@@ -1928,18 +1944,20 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             // slots copied over (slot i holds v_i while no slot was reused);
             // without the memory the ring stays and wraps from here on
             const int K2 = std::min(K_full, 2 * K);
-            void* np = nullptr;
-            if (cudaMalloc(&np, (size_t)K2 * vec_bytes) != cudaSuccess) {
+            DevBuf<unsigned char> grown;
+            try {
+                grown.alloc((size_t)K2 * vec_bytes);
+            } catch (const Error& e) {
+                if (e.code != QMB_ERR_NOMEM) throw;
                 (void)cudaGetLastError();
                 K_full = K;
                 continue;
             }
-            QMB_CUDA_TRY(cudaMemcpyAsync(np, vring.p, (size_t)j0 * vec_bytes, cudaMemcpyDeviceToDevice, st));
+            QMB_CUDA_TRY(cudaMemcpyAsync(grown.p, vring.p, (size_t)j0 * vec_bytes, cudaMemcpyDeviceToDevice, st));
             QMB_CUDA_TRY(cudaStreamSynchronize(st));
-            k.ws_ring.release();
-            k.ws_ring.p = reinterpret_cast<unsigned char*>(np);
-            k.ws_ring.n = (size_t)K2 * vec_bytes;
-            vring.p = reinterpret_cast<V*>(np);
+            k.ws_ring.swap(grown);
+            grown.release();
+            vring.p = reinterpret_cast<V*>(k.ws_ring.p);
             K = K2;
             if (trace_on()) std::fprintf(stderr, "[qmb batch] ring grown to %d slots at step %d\n", K, j0);
         }
@@ -2194,6 +2212,7 @@ static void find_conjugates(const std::vector<BatchPart>& parts, const std::vect
     std::vector<int> hs(S);
     same.download(hs.data(), S);
     QMB_CUDA_TRY(cudaStreamSynchronize(0));
+    mark_idle(pr, same);
     for (int s = 0; s < S; ++s)
         if (cand[s] >= 0 && hs[s]) alias[s] = cand[s];
 }
@@ -2410,6 +2429,8 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
         b->cxy.zero();
         b->cz.zero();
         QMB_CUDA_TRY(cudaDeviceSynchronize());
+        for (BatchPart& P : parts) mark_idle(P.rp, P.col, P.val, P.dxy, P.dz);
+        mark_idle(scan_tmp, row_cnt);
         if (trace_on())
             std::fprintf(stderr, "[qmb batch] create: sector matrices %.1f ms, device CSR %.1f ms, "
                          "assembly %.1f ms, total %.1f ms\n", ms_build, ms_csr,

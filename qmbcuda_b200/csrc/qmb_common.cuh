@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "qmb_b200.h"
@@ -47,6 +48,12 @@ qmb_status guarded(F&& f) {
 }
 
 // ------------------------------------------------------------ device memory
+// qmb_mem.cu: device memory, with freed idle buffers kept for reuse.
+void* dev_alloc(size_t bytes, size_t* got, int* dev);
+void dev_free(void* p, size_t bytes, int dev, bool idle);
+void dev_trim();  // frees what is kept on the current device
+bool dev_mem_info(size_t* free_bytes, size_t* total);  // cudaMemGetInfo, kept buffers counted as free
+
 template <class T>
 struct DevBuf {
     T* p = nullptr;
@@ -55,22 +62,32 @@ struct DevBuf {
     explicit DevBuf(size_t count) { alloc(count); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+    DevBuf(DevBuf&& o) noexcept { swap(o); }
     DevBuf& operator=(DevBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+        if (this != &o) { release(); swap(o); }
         return *this;
     }
     ~DevBuf() { release(); }
     void alloc(size_t count) {
         release();
         if (count == 0) count = 1;
-        QMB_CUDA_TRY(cudaMalloc(&p, count * sizeof(T)));
+        p = static_cast<T*>(dev_alloc(count * sizeof(T), &bytes_, &dev_));
         n = count;
     }
     void release() {
-        if (p) cudaFree(p);
+        dev_free(p, bytes_, dev_, idle_);
         p = nullptr;
         n = 0;
+        idle_ = false;
+    }
+    // No work on any stream uses the buffer any more: release() may keep it.
+    void mark_idle() { idle_ = p != nullptr; }
+    void swap(DevBuf& o) noexcept {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(bytes_, o.bytes_);
+        std::swap(dev_, o.dev_);
+        std::swap(idle_, o.idle_);
     }
     void zero(cudaStream_t st = 0) { QMB_CUDA_TRY(cudaMemsetAsync(p, 0, n * sizeof(T), st)); }
     void upload(const T* h, size_t count, cudaStream_t st = 0) {
@@ -79,7 +96,16 @@ struct DevBuf {
     void download(T* h, size_t count, cudaStream_t st = 0) const {
         QMB_CUDA_TRY(cudaMemcpyAsync(h, p, count * sizeof(T), cudaMemcpyDeviceToHost, st));
     }
+
+private:
+    size_t bytes_ = 0;   // as allocated
+    int dev_ = -1;
+    bool idle_ = false;
 };
+// mark_idle() on several buffers
+template <class... B>
+void mark_idle(B&... b) { (b.mark_idle(), ...); }
+
 
 struct DeviceGuard {
     int prev = -1;

@@ -421,6 +421,7 @@ void run_expval(qmb_ham_s* h, const V* psi, const std::vector<AvgTerms>& ops, do
         }
         std::vector<unsigned char> res(res_bytes);
         QMB_CUDA_TRY(cudaMemcpy(res.data(), seg_d, res_bytes, cudaMemcpyDeviceToHost));
+        blk.mark_idle();
         const double2* hs = reinterpret_cast<const double2*>(res.data());
         const double* hn = reinterpret_cast<const double*>(hs + seg_h.size());
         for (int i = 0; i < n_seg; ++i) {
@@ -434,7 +435,8 @@ void run_expval(qmb_ham_s* h, const V* psi, const std::vector<AvgTerms>& ops, do
         pos = end;
     } while (pos < items.size());
     int herr = 0;
-    err.download(&herr, 1);
+    QMB_CUDA_TRY(cudaMemcpy(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    err.mark_idle();
     QMB_REQUIRE(herr == 0, QMB_ERR_INVALID, "expval: a term left the sector's representative table");
     QMB_REQUIRE(norm2 > 0.0, QMB_ERR_INVALID, "expval: psi is zero");
     for (size_t k = 0; k < ops.size(); ++k) out[2 * k] = out[2 * k + 1] = 0.0;

@@ -500,7 +500,7 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
         }
     const size_t sm_pack = align16(sm) + 7 * (size_t)kPackWarps * mob.size();
     size_t fr = 0, tot = 0;
-    QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    dev_mem_info(&fr, &tot);
     const size_t mask_bytes = sizeof(uint32_t) * (size_t)h->n_slices * std::max<size_t>(1, mob.size());
     const bool packed = mob.size() <= (size_t)kPackMaxTerms && mask_bytes <= fr / 8 && sm_pack <= 200 * 1024;
     PackArgs pk{nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0, nullptr};
@@ -580,7 +580,8 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
         }
     });
     check_launch("k_ell_fill");
-    check_err();
+    check_err();  // waits for the fill
+    mark_idle(slots, stats, d_midx, d_mob, masks, cnt, tmp);
 }
 
 // ------------------------------------------ column-blocked coded layout
@@ -797,7 +798,7 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
         QMB_CUDA_TRY(cudaMemcpyAsync(width.p, h->slice_w.p, sizeof(int) * ns, cudaMemcpyDeviceToDevice, 0));
         QMB_CUDA_TRY(cudaMemcpyAsync(off.p, h->slice_off.p, sizeof(int64_t) * (ns + 1), cudaMemcpyDeviceToDevice, 0));
     } else {
-        QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        dev_mem_info(&fr, &tot);
         if ((size_t)nb * n + 2 * n * 16 > fr / 2) {
             cb_skip("not enough free memory for the counts");
             return;
@@ -815,7 +816,7 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
         cub::DeviceScan::ExclusiveSum(tmp.p, tb, slots.p, off.p, (int64_t)nb * ns + 1);
         QMB_CUDA_TRY(cudaMemcpy(&total, off.p + (size_t)nb * ns, sizeof(int64_t), cudaMemcpyDeviceToHost));
     }
-    QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    dev_mem_info(&fr, &tot);
     const size_t need = (size_t)total * 4 + (size_t)n * (h->cplx ? 16 : 8);
     if (need > fr / 10 * 9) {
         cb_skip("not enough free memory for the packed entries");
@@ -835,6 +836,7 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
         check_launch("k_cb_fill");
         int hm[2] = {0, 0};
         QMB_CUDA_TRY(cudaMemcpy(hm, miss.p, sizeof(hm), cudaMemcpyDeviceToHost));
+        dkeys.mark_idle();
         if (hm[0] == 0 && hm[1] == 0) break;
         if (hm[1] > 0 || round == 2) {
             cb_skip("more distinct values than the dictionary holds");
@@ -865,6 +867,7 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
     L.shift = shift;
     L.n_codes = (int)keys.size();
     QMB_CUDA_TRY(cudaDeviceSynchronize());
+    mark_idle(miss, mkeys);
 }
 
 // The FP64 values of a matrix whose FP32 values are coded: when every FP32
@@ -951,7 +954,7 @@ static void share_cb64_t(qmb_ham_s* h) {
         if (hb[(size_t)c * W] != kDictEmpty) std::memcpy(&dict[c], &hb[(size_t)c * W], sizeof(M64));
     if (L32.nb > 1) {
         size_t fr = 0, tot = 0;
-        QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+        dev_mem_info(&fr, &tot);
         if ((size_t)h->n * sizeof(M64) > fr / 4) {
             cb_skip("not enough free memory for the FP64 partial sums");
             return;
@@ -1109,7 +1112,7 @@ void mf_tables(qmb_ham_s* h) {
     uint64_t slots = 1;
     while (slots < 2 * (uint64_t)n) slots <<= 1;
     size_t fr = 0, tot = 0;
-    QMB_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+    dev_mem_info(&fr, &tot);
     // the table is an accelerator: without room for it (a quarter of the
     // free memory) the bucket search serves alone
     if (!r32 && (force_hash || (double)n * 8 >= kMfHashMinBytes) && bits + ibits <= 63 &&
@@ -1240,6 +1243,7 @@ extern "C" qmb_status qmb_ham_export_ref(qmb_sector s, const qmb_terms* terms, i
         dv.download(reinterpret_cast<double2*>(val), (size_t)R * W);
         dt.download(track, R);
         QMB_CUDA_TRY(cudaDeviceSynchronize());
+        mark_idle(di, dv, dt, ov);
     });
 }
 

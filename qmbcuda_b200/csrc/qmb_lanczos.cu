@@ -389,6 +389,8 @@ struct LzState {
         d.cpart = cpart.p;
         d.scratch = scratch.p;
     }
+    // after the wait that ends a solve
+    void mark_idle() { qmb::mark_idle(alpha, beta, partials, cpart, scratch, iter, counter, coefs); }
 };
 
 struct PhaseOut {
@@ -464,10 +466,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
     const size_t reserve = 6 * (size_t)n * sizeof(P) + ((size_t)256 << 20);
     auto free_bytes = [&]() {
         size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return (size_t)0;
-        }
+        dev_mem_info(&fr, &tot);
         return fr;
     };
     K = store ? std::min(K_full, std::max({hint, 2 + every_steps, 32})) : 2;
@@ -555,8 +554,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
                 QMB_CUDA_TRY(cudaMemcpyAsync(grown.p, vring.p, (size_t)done * n * sizeof(V),
                                              cudaMemcpyDeviceToDevice, s));
                 QMB_CUDA_TRY(cudaStreamSynchronize(s));
-                std::swap(vring.bytes->p, grown.p);
-                std::swap(vring.bytes->n, grown.n);
+                vring.bytes->swap(grown);
                 vring.p = reinterpret_cast<V*>(vring.bytes->p);
                 K = K2;
                 capture();
@@ -668,6 +666,7 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
         k_ritz<V, P><<<grid_for(n, 256), 256, 0, s>>>(n, vring.p, ph.m, ritz.p, psi);
         check_launch("k_ritz");
         QMB_CUDA_TRY(cudaStreamSynchronize(s));
+        ritz.mark_idle();
         return;
     }
     // regenerate v_0..v_{m-1} with the same start; kernels are deterministic
@@ -683,6 +682,7 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
     }
     check_launch("regenerate");
     QMB_CUDA_TRY(cudaStreamSynchronize(s));
+    ritz.mark_idle();
 }
 
 template <class Op, class P>
@@ -702,7 +702,7 @@ double residual_norm(const Op& op, size_t op_smem, const P* psi, double theta, L
 
 bool fits_device(size_t bytes) {
     size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
+    if (!dev_mem_info(&fr, &tot)) return false;
     return bytes < fr * 0.6;
 }
 
@@ -733,7 +733,8 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
     po.check_every = o.check_every > 0 ? o.check_every : 10;
     const int cap = std::max(1, o.max_iter);
     int n_hv = 0;
-    DevBuf<V64> psi(n);
+    DevBuf<unsigned char> psi_bytes(sizeof(V64) * n);
+    struct { V64* p; } psi{reinterpret_cast<V64*>(psi_bytes.p)};
     double theta = 0.0;
     int iters = 0;
     bool conv = false;
@@ -811,6 +812,7 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
             iters += ph2.m;
             conv = ph2.converged;
             last = ph2;
+            start.mark_idle();  // ritz_vector waited for the stream
         }
     }
     double pn2 = 0;
@@ -843,11 +845,15 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
     if (coeffs) {
         for (int64_t i = 0; i < n_coeffs; ++i) coeffs[i] = i < (int64_t)last.s.size() ? last.s[i] : 0.0;
     }
+    // (the wait for e1 above left nothing of this solve in flight)
     if (o.want_vector) {
-        h->psi.alloc(sizeof(V64) * n);
-        QMB_CUDA_TRY(cudaMemcpy(h->psi.p, psi.p, sizeof(V64) * n, cudaMemcpyDeviceToDevice));
+        QMB_CUDA_TRY(cudaStreamSynchronize(0));  // work on the kept vector, ordered before its replacement
+        h->psi.swap(psi_bytes);
+        h->psi.n = sizeof(V64) * n;
         h->psi_n = n;
     }
+    psi_bytes.mark_idle();
+    st.mark_idle();
 }
 
 }  // namespace qmb
@@ -1025,6 +1031,7 @@ extern "C" qmb_status qmb_lanczos_ref_ell(float* E, int n_iter, int nobv, int ma
             RefEllOp<float> op{nobv, max_terms, ind_dev, (const float*)val_dev, track_dev};
             solve<RefEllOp<float>, RefEllOp<float>, float, double>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter);
         }
+        mark_idle(dummy.lz_ring, dummy.lz_wbuf);  // the solve ended with a wait
         *E = (float)r.E0;
         if (krylov_out)
             for (int i = 0; i < n_iter; ++i) krylov_out[i] = i < o.max_iter ? (float)cf[i] : 0.0f;

@@ -427,7 +427,8 @@ extern "C" qmb_status qmb_sector_create(const qmb_sector_desc* d, qmb_sector* ou
         k_rep_write<<<grid_for((int64_t)n_words, 256), 256>>>(L, s->n_up, n_words, words.p,
                                                               offsets.p, s->reps.p);
         check_launch("k_rep_write");
-        sector_buckets(s);
+        sector_buckets(s);  // waits for the device
+        mark_idle(words, counts, offsets, tmp);
         *out = own.release();
     });
 }
@@ -491,6 +492,7 @@ void sector_select_irrep(qmb_sector_s* s, const double* chars, double tol_norm) 
                                                 s->orbit_of_row.p);
     check_launch("k_active_maps");
     QMB_CUDA_TRY(cudaDeviceSynchronize());
+    mark_idle(active, pos, tmp);
     s->has_irrep = true;
     ++s->irrep_gen;
 }
@@ -551,6 +553,7 @@ extern "C" qmb_status qmb_sector_orbit_map(qmb_sector s, uint32_t* orbit_indices
         check_launch("k_orbit_map");
         out.download(orbit_indices, 2 * s->n_states);
         QMB_CUDA_TRY(cudaDeviceSynchronize());
+        out.mark_idle();
     });
 }
 
@@ -572,5 +575,6 @@ extern "C" qmb_status qmb_sector_lookup(qmb_sector s, const uint64_t* t, int64_t
         o.download(orbit, n);
         e.download(element, n);
         QMB_CUDA_TRY(cudaDeviceSynchronize());
+        mark_idle(in, o, e);
     });
 }
