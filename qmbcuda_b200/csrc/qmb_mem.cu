@@ -19,7 +19,9 @@
 // an earlier context are forgotten.
 #include <cuda.h>
 
+#include <iterator>
 #include <list>
+#include <map>
 #include <mutex>
 
 #include "qmb_common.cuh"
@@ -35,8 +37,10 @@ struct Kept {
     void* p;
     size_t bytes;
 };
+using KeptList = std::list<Kept>;
 struct DeviceCache {
-    std::list<Kept> kept;  // oldest first
+    KeptList kept;                                      // oldest first
+    std::multimap<size_t, KeptList::iterator> by_size;  // newest last among equals
     size_t total = 0;
     unsigned long long ctx = 0;
 };
@@ -74,17 +78,29 @@ DeviceCache* current(int dev) {
     DeviceCache& c = caches()[dev];
     if (c.ctx != id) {
         c.kept.clear();
+        c.by_size.clear();
         c.total = 0;
         c.ctx = id;
     }
     return &c;
 }
 
+void* take(DeviceCache& c, std::multimap<size_t, KeptList::iterator>::iterator at) {
+    void* p = at->second->p;
+    c.total -= at->first;
+    c.kept.erase(at->second);
+    c.by_size.erase(at);
+    return p;
+}
+
 void drop(DeviceCache& c, size_t keep) {
     while (c.total > keep && !c.kept.empty()) {
-        cudaFree(c.kept.front().p);
-        c.total -= c.kept.front().bytes;
-        c.kept.pop_front();
+        auto range = c.by_size.equal_range(c.kept.front().bytes);
+        for (auto it = range.first; it != range.second; ++it)
+            if (it->second == c.kept.begin()) {
+                cudaFree(take(c, it));
+                break;
+            }
     }
 }
 
@@ -104,16 +120,10 @@ void* dev_alloc(size_t bytes, size_t* got, int* dev_out) {
     {
         std::lock_guard<std::mutex> lock(g_mu);
         if (DeviceCache* c = want <= kMaxBlock ? current(dev) : nullptr) {
-            auto best = c->kept.end();
-            for (auto it = c->kept.begin(); it != c->kept.end(); ++it)
-                if (it->bytes >= want && it->bytes <= want + want / 8 && (best == c->kept.end() || it->bytes < best->bytes))
-                    best = it;
-            if (best != c->kept.end()) {
-                void* p = best->p;
-                *got = best->bytes;
-                c->total -= best->bytes;
-                c->kept.erase(best);
-                return p;
+            auto it = c->by_size.lower_bound(want);
+            if (it != c->by_size.end() && it->first <= want + want / 8) {
+                *got = it->first;
+                return take(*c, it);
             }
         }
     }
@@ -137,6 +147,7 @@ void dev_free(void* p, size_t bytes, int dev, bool idle) {
         std::lock_guard<std::mutex> lock(g_mu);
         if (DeviceCache* c = current(dev)) {
             c->kept.push_back(Kept{p, bytes});
+            c->by_size.emplace(bytes, std::prev(c->kept.end()));
             c->total += bytes;
             drop(*c, kMaxTotal);
             return;
