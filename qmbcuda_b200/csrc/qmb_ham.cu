@@ -225,7 +225,10 @@ __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off
 // each in the first slot where none of its rows is taken; a mask that fits
 // nowhere is split over the rows' free slots.  Every lane then walks its own
 // terms, so that the orbit searches of a warp run together instead of at the
-// term where each lane finds an entry.  Slices wider than 64 keep term order.
+// term where each lane finds an entry.  Slices wider than 64 keep term order, and
+// so do sectors without a group: their levels are often degenerate (momenta k and
+// -k, dimer pairs), and which vector of such a level a long solve returns depends
+// on the rounding of its sums.
 constexpr int kPackMaxTerms = 1024;  // mobile terms (7 bytes of shared memory a warp each)
 constexpr int kPackWarps = 4;        // warps a block
 
@@ -234,6 +237,7 @@ struct PackArgs {
     const uint16_t* mob;  // [n_mob] their term indices
     int n_mob;
     int exact;            // every orbit is active
+    int pack;             // 0: slots in term order
     uint32_t* masks;      // [n_slices][n_mob]
 };
 
@@ -321,7 +325,8 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_ell_pack(RowGen rg, PackArg
         for (int i = lane; i < nm; i += 32) s_mask[i] = pk.masks[s * nm + i];
         __syncwarp();
         uint64_t free = 0;  // this row's slots that no placed mask takes
-        if (w <= 64) {
+        const bool place = pk.pack && w <= 64;
+        if (place) {
             // the terms with entries, in classes of decreasing size
             int cnt = 0;
 #pragma unroll
@@ -362,7 +367,7 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_ell_pack(RowGen rg, PackArg
                 if (i >= nm) break;
                 const int hi = pk.mob[i];
                 int at = j;
-                if (w <= 64) {
+                if (place) {
                     at = s_slot[i];
                     if (at == 255) {
                         at = __ffsll((long long)free) - 1;
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_ell_pack(RowGen rg, PackArg
                     if (val32) val32[p] = cvt<M32>(v64);
                 });
             }
-            if (w > 64)
+            if (!place)
                 for (; j < w; ++j) {
                     const int64_t p = base + (int64_t)j * 32;
                     col[p] = (uint32_t)r;
@@ -432,15 +437,11 @@ __global__ void k_ell_ref(RowGen rg, int64_t R, int W, uint32_t* __restrict__ in
     }
 }
 
-template <class Op, class V>
+template <class Op, class V, int S>
 __global__ void __launch_bounds__(256, OpMinBlocks<Op>::value) k_hv(Op op, const V* __restrict__ x, V* __restrict__ y) {
     extern __shared__ __align__(16) unsigned char smem_hv[];
     op.init(smem_hv);
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < op.n;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        V xr;
-        y[r] = op.row(r, x, xr);
-    }
+    for_rows<S>(op, x, [&](int64_t r, V hx, V) { y[r] = hx; });
 }
 
 // The matrix-free product with the warp-cooperative lookup (hop form): the
@@ -464,10 +465,12 @@ __global__ void __launch_bounds__(256, 5) k_hv_mfw(MfOp<M> op, const V* __restri
 // ------------------------------------------------------------- helpers
 template <class Op, class V>
 void launch_hv(const Op& op, const V* x, V* y, cudaStream_t st, size_t smem) {
-    const void* fn = (const void*)k_hv<Op, V>;
-    set_group_smem_attr(fn, smem);
     op.pre(x, (const int*)nullptr, st);  // column-block passes or the matrix-free scaling, if any
-    k_hv<Op, V><<<grid_for(op.n, 256), 256, smem, st>>>(op, x, y);
+    with_split(op, [&](auto sp) {
+        constexpr int S = decltype(sp)::value;
+        set_group_smem_attr((const void*)k_hv<Op, V, S>, smem);
+        k_hv<Op, V, S><<<grid_for(op.n, 256 / S), 256, smem, st>>>(op, x, y);
+    });
     check_launch("k_hv");
 }
 
@@ -499,13 +502,16 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
             break;
         }
     const size_t sm_pack = align16(sm) + 7 * (size_t)kPackWarps * mob.size();
-    size_t fr = 0, tot = 0;
-    dev_mem_info(&fr, &tot);
     const size_t mask_bytes = sizeof(uint32_t) * (size_t)h->n_slices * std::max<size_t>(1, mob.size());
-    const bool packed = mob.size() <= (size_t)kPackMaxTerms && mask_bytes <= fr / 8 && sm_pack <= 200 * 1024;
-    PackArgs pk{nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0, nullptr};
+    bool packed = mob.size() <= (size_t)kPackMaxTerms && sm_pack <= 200 * 1024;
+    if (packed && mask_bytes > ((size_t)64 << 20)) {  // (the query takes 0.2 ms)
+        size_t fr = 0, tot = 0;
+        dev_mem_info(&fr, &tot);
+        packed = mask_bytes <= fr / 8;
+    }
+    PackArgs pk{nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0,
+                h->sector->n_ext > 1 ? 1 : 0, nullptr};
     DevBuf<int16_t> d_midx;
-    DevBuf<uint16_t> d_mob;
     DevBuf<uint32_t> masks;
     DevBuf<int> cnt;
     auto typed = [&](auto&& f) {
@@ -514,13 +520,13 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
     };
     const int pack_grid = grid_for(h->n_slices, kPackWarps);
     if (packed) {
-        d_midx.alloc(midx.size());
-        d_midx.upload(midx.data(), midx.size());
-        d_mob.alloc(std::max<size_t>(1, mob.size()));
-        if (!mob.empty()) d_mob.upload(mob.data(), mob.size());
+        std::vector<int16_t> both(midx);  // midx, then mob
+        for (uint16_t m : mob) both.push_back((int16_t)m);
+        d_midx.alloc(both.size());
+        d_midx.upload(both.data(), both.size());
         masks.alloc(mask_bytes / sizeof(uint32_t));
         pk.midx = d_midx.p;
-        pk.mob = d_mob.p;
+        pk.mob = reinterpret_cast<const uint16_t*>(d_midx.p + midx.size());
         pk.masks = masks.p;
         typed([&](auto m64, auto m32) {
             using M64 = decltype(m64);
@@ -581,7 +587,7 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
     });
     check_launch("k_ell_fill");
     check_err();  // waits for the fill
-    mark_idle(slots, stats, d_midx, d_mob, masks, cnt, tmp);
+    mark_idle(slots, stats, d_midx, masks, cnt, tmp);
 }
 
 // ------------------------------------------ column-blocked coded layout

@@ -1,6 +1,7 @@
 // qmb_ham.cuh -- Hamiltonian storage and the row operators used by H*v.
 #pragma once
 #include <cstdlib>
+#include <type_traits>
 
 #include "qmb_scalar.cuh"
 #include "qmb_sector.cuh"
@@ -198,38 +199,45 @@ struct SellOp {
     __device__ void init(unsigned char*) {}
     template <class V>
     void pre(const V*, const int*, cudaStream_t) const {}
-    // (H x)_r * scale; x_r is returned through xr.
-    template <class V>
-    __device__ __forceinline__ V row(int64_t r, const V* __restrict__ x, V& xr) const {
-        int64_t s = r >> 5;
-        int lane = (int)(r & 31);
-        const uint32_t* c = col + off[s] + lane;
-        const M* v = val + off[s] + lane;
-        int w = width[s];
-        V acc = Sc<V>::zero();
-        xr = x[r];
-        acc = Sc<V>::mul(cvt<V>(diag[r]), xr);
-        int j = 0;
-        for (; j + 4 <= w; j += 4) {
-            uint32_t c0 = __ldg(c + 0 * 32), c1 = __ldg(c + 1 * 32), c2 = __ldg(c + 2 * 32),
-                     c3 = __ldg(c + 3 * 32);
-            M v0 = __ldg(v + 0 * 32), v1 = __ldg(v + 1 * 32), v2 = __ldg(v + 2 * 32),
-              v3 = __ldg(v + 3 * 32);
-            V x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-            acc = Sc<V>::fma(cvt<V>(v0), x0, acc);
-            acc = Sc<V>::fma(cvt<V>(v1), x1, acc);
-            acc = Sc<V>::fma(cvt<V>(v2), x2, acc);
-            acc = Sc<V>::fma(cvt<V>(v3), x3, acc);
-            c += 4 * 32;
-            v += 4 * 32;
+    // Part p of S of (H x)_r: the slots j = p, p + S, ..., four loads of a
+    // column, a value and an x element in flight; part 0 holds the diagonal.
+    template <int S, class V>
+    __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
+        const int64_t s = r >> 5;
+        const int lane = (int)(r & 31);
+        const int w = width[s];
+        const uint32_t* c = col + off[s] + lane + (int64_t)p * 32;
+        const M* v = val + off[s] + lane + (int64_t)p * 32;
+        V acc = p == 0 ? Sc<V>::mul(cvt<V>(diag[r]), x[r]) : Sc<V>::zero();
+        int j = p;
+        for (; j + 3 * S < w; j += 4 * S) {
+            uint32_t cc[4];
+            M vv[4];
+            V xx[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                cc[u] = __ldg(c + u * S * 32);
+                vv[u] = __ldg(v + u * S * 32);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xx[u] = __ldg(x + cc[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc = Sc<V>::fma(cvt<V>(vv[u]), xx[u], acc);
+            c += 4 * S * 32;
+            v += 4 * S * 32;
         }
-        for (; j < w; ++j) {
-            uint32_t c0 = __ldg(c);
-            M v0 = __ldg(v);
-            acc = Sc<V>::fma(cvt<V>(v0), __ldg(x + c0), acc);
-            c += 32;
-            v += 32;
-        }
+        // the last one to three together
+        uint32_t cc[3];
+        M vv[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (j + u * S < w) {
+                cc[u] = __ldg(c + u * S * 32);
+                vv[u] = __ldg(v + u * S * 32);
+            }
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (j + u * S < w) acc = Sc<V>::fma(cvt<V>(vv[u]), __ldg(x + cc[u]), acc);
         return acc;
     }
 };
@@ -293,11 +301,12 @@ struct CbSellOp {
         }
         return acc;
     }
-    // the last pass: (H x)_r from the partial sums of the earlier passes
-    template <class V>
-    __device__ __forceinline__ V row(int64_t r, const V* __restrict__ x, V& xr) const {
-        xr = x[r];
-        const V acc = nb > 1 ? reinterpret_cast<const V*>(ytmp)[r] : Sc<V>::mul(cvt<V>(diag[r]), xr);
+    // the last pass: (H x)_r from the partial sums of the earlier passes (rows
+    // are not split: the layout serves matrices of millions of rows)
+    template <int S, class V>
+    __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int) const {
+        static_assert(S == 1, "coded rows are not split");
+        const V acc = nb > 1 ? reinterpret_cast<const V*>(ytmp)[r] : Sc<V>::mul(cvt<V>(diag[r]), x[r]);
         return block_sum(nb - 1, r, x, acc);
     }
     template <class V>
@@ -342,13 +351,22 @@ struct RefEllOp {
     __device__ void init(unsigned char*) {}
     template <class V>
     void pre(const V*, const int*, cudaStream_t) const {}
-    template <class V>
-    __device__ __forceinline__ V row(int64_t r, const V* __restrict__ x, V& xr) const {
-        xr = x[r];
+    // Part p of S of (H x)_r: S neighbouring lanes read neighbouring slots of
+    // the row-major table, two slots each in flight.
+    template <int S, class V>
+    __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
         V acc = Sc<V>::zero();
-        int nt = track[r];
-        for (int i = 0; i < nt; ++i)
-            acc = Sc<V>::fma(cvt<V>(val[r * W + i]), x[ind[r * W + i]], acc);
+        const int nt = track[r];
+        const uint32_t* c = ind + r * W;
+        const M* v = val + r * W;
+        for (int i = p; i < nt; i += 2 * S) {
+            const bool two = i + S < nt;
+            const uint32_t c0 = __ldg(c + i), c1 = two ? __ldg(c + i + S) : 0u;
+            const M v0 = __ldg(v + i), v1 = two ? __ldg(v + i + S) : Sc<M>::zero();
+            const V x0 = x[c0], x1 = two ? x[c1] : Sc<V>::zero();
+            acc = Sc<V>::fma(cvt<V>(v0), x0, acc);
+            if (two) acc = Sc<V>::fma(cvt<V>(v1), x1, acc);
+        }
         return acc;
     }
 };
@@ -592,13 +610,13 @@ struct MfOp {
     template <class V>
     void pre(const V* x0, const int* iter, cudaStream_t s) const;
     // sum over the hop entries of the row of src (strings beyond 32 sites)
-    template <class V>
-    __device__ __forceinline__ V hop_sum64(uint64_t src, const V* __restrict__ xsv) const {
+    template <int S, class V>
+    __device__ __forceinline__ V hop_sum64(uint64_t src, const V* __restrict__ xsv, int p) const {
         V acc = Sc<V>::zero();
         for (int base = 0; base < n_hops; base += 64) {
             const int nb = min(64, n_hops - base);
             uint64_t live = 0;
-            for (int b = 0; b < nb; ++b) live |= (uint64_t)(__popcll(src & s_hops[base + b].pair) & 1) << b;
+            for (int b = p; b < nb; b += S) live |= (uint64_t)(__popcll(src & s_hops[base + b].pair) & 1) << b;
             while (live) {
                 const int b = base + __ffsll((long long)live) - 1;
                 live &= live - 1;
@@ -624,13 +642,13 @@ struct MfOp {
     // the same up to 32 sites (reps32 set) in 32-bit arithmetic, taking the
     // row's entries two at a time: both orbit minima, then both lookups in
     // lockstep, then both gathers
-    template <class V>
-    __device__ __forceinline__ V hop_sum32x2(uint32_t src, const V* __restrict__ xsv) const {
+    template <int S, class V>
+    __device__ __forceinline__ V hop_sum32x2(uint32_t src, const V* __restrict__ xsv, int p) const {
         V acc = Sc<V>::zero();
         for (int base = 0; base < n_hops; base += 64) {
             const int nb = min(64, n_hops - base);
             uint64_t live = 0;
-            for (int b = 0; b < nb; ++b) live |= (uint64_t)(__popc(src & s_pair32[base + b]) & 1) << b;
+            for (int b = p; b < nb; b += S) live |= (uint64_t)(__popc(src & s_pair32[base + b]) & 1) << b;
             while (live) {
                 const int b1 = base + __ffsll((long long)live) - 1;
                 live &= live - 1;
@@ -722,27 +740,28 @@ struct MfOp {
         acc = Sc<V>::scale(acc, 1.0 / nrow[r]);
         return Sc<V>::fma(Sc<V>::from(d), xr, acc);
     }
-    template <class V>
-    __device__ __forceinline__ V row(int64_t r, const V* __restrict__ x, V& xr) const {
+    // Part p of S of (H x)_r: the hops (or a range of the general terms) p of S;
+    // with a hop table part 0 holds the diagonal.
+    template <int S, class V>
+    __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
         const uint64_t rep = look.reps32 ? (uint64_t)look.reps32[r] : look.reps64[r];
         const uint64_t src = apply_elem(rg.g, gs, 0, rep);
         const V* __restrict__ xsv = reinterpret_cast<const V*>(xs);
-        xr = x[r];
         V acc;
-        double2 d;
+        double2 d = make_double2(0.0, 0.0);
         if (n_hops) {
-            acc = look.reps32 ? hop_sum32x2<V>((uint32_t)src, xsv) : hop_sum64<V>(src, xsv);
-            d = cplx ? reinterpret_cast<const double2*>(diag)[r]
-                     : make_double2(reinterpret_cast<const double*>(diag)[r], 0.0);
+            acc = look.reps32 ? hop_sum32x2<S, V>((uint32_t)src, xsv, p) : hop_sum64<S, V>(src, xsv, p);
+            if (p == 0)
+                d = cplx ? reinterpret_cast<const double2*>(diag)[r]
+                         : make_double2(reinterpret_cast<const double*>(diag)[r], 0.0);
         } else {
             acc = Sc<V>::zero();
-            d = gen_row_look(rg, gs, ts, 0, ts.n_terms, src, look, [&](int64_t c, double2 v) {
-                acc = Sc<V>::fma(Sc<V>::from(v), __ldg(xsv + c), acc);
-            });
+            d = gen_row_look(rg, gs, ts, ts.n_terms * p / S, ts.n_terms * (p + 1) / S, src, look,
+                             [&](int64_t c, double2 v) { acc = Sc<V>::fma(Sc<V>::from(v), __ldg(xsv + c), acc); });
         }
         acc = Sc<V>::scale(acc, 1.0 / nrow[r]);
-        acc = Sc<V>::fma(Sc<V>::from(d), xr, acc);
-        return acc;
+        if (n_hops && p) return acc;
+        return Sc<V>::fma(Sc<V>::from(d), x[r], acc);
     }
 };
 
@@ -756,6 +775,93 @@ template <class M> struct OpMinBlocks<MfOp<M>> { static constexpr int value = 5;
 // and leave the FP32 one (L=32: 318 against 322 us) as it is.  Deeper unrolling
 // or loading the next entries ahead changed neither.
 template <class M> struct OpMinBlocks<CbSellOp<M>> { static constexpr int value = 6; };
+
+// How a product's rows are spread over threads.  One thread a row leaves most
+// of the chip idle below some 10^5 rows, and each thread then walks its row's
+// dependent loads (column, then x) alone.  With S > 1 a row's entries are
+// dealt to S threads: S warps of a block take the same 32 rows and add up
+// through shared memory (sliced ELL, matrix-free), or S neighbouring lanes take
+// one row and add up by shuffles (the caller's row-major ELL, whose slots they
+// then read side by side).  Sums are in a fixed order, so results are
+// reproducible and a regenerated Lanczos vector equals the stored one.
+//
+// The lines lie where the two sides were measured equal (us a product, S = 1
+// against the split): sliced ELL 9,225 rows 4.6 / 4.5 (S = 4), 112,640 10.3 / 8.2
+// and 208,012 10.3 / 8.2 (S = 2), 400,023 complex FP64 49.2 / 34.3 but FP32 real
+// 22.4 / 23.5; matrix-free 2,703 rows 26.2 / 14.0 (S = 8), 32,065 34.8 / 22.5 and
+// 112,632 112 / 96 (S = 4), 208,012 190 / 162 (S = 2), 716,728 369 / 379; row-major
+// ELL, 50 steps of 9,252 rows 2.00 / 1.79 ms and of 112,720 rows 2.42 / 2.29 (S = 4).
+template <class Op> struct OpSplit { static constexpr bool lanes = false; static int of(const Op&) { return 1; } };
+template <class M> struct OpSplit<SellOp<M>> {
+    static constexpr bool lanes = false;
+    static int of(const SellOp<M>& op) { return op.n < 16384 ? 4 : op.n < (sizeof(M) == 16 ? 640000 : 300000) ? 2 : 1; }
+};
+template <class M> struct OpSplit<MfOp<M>> {
+    static constexpr bool lanes = false;
+    static int of(const MfOp<M>& op) { return op.n < 16384 ? 8 : op.n < 131072 ? 4 : op.n < 400000 ? 2 : 1; }
+};
+template <class M> struct OpSplit<RefEllOp<M>> {
+    static constexpr bool lanes = true;
+    static int of(const RefEllOp<M>&) { return 4; }
+};
+template <class Op> struct OpMaxSplit { static constexpr int value = 1; };
+template <class M> struct OpMaxSplit<SellOp<M>> { static constexpr int value = 4; };
+template <class M> struct OpMaxSplit<MfOp<M>> { static constexpr int value = 8; };
+template <class M> struct OpMaxSplit<RefEllOp<M>> { static constexpr int value = 4; };
+
+// f(std::integral_constant<int, S>) for the split of op's rows; S = 1 when the
+// caller wants the rows whole.
+template <class Op, class F>
+inline void with_split(const Op& op, F&& f, bool whole = false) {
+    constexpr int top = OpMaxSplit<Op>::value;
+    const int S = whole ? 1 : OpSplit<Op>::of(op);
+    if constexpr (OpSplit<Op>::lanes) {
+        f(std::integral_constant<int, top>{});
+        return;
+    }
+    if constexpr (top >= 8)
+        if (S == 8) return f(std::integral_constant<int, 8>{});
+    if constexpr (top >= 4)
+        if (S == 4) return f(std::integral_constant<int, 4>{});
+    if constexpr (top >= 2)
+        if (S == 2) return f(std::integral_constant<int, 2>{});
+    f(std::integral_constant<int, 1>{});
+}
+
+// f(r, (H x)_r, x_r) for every row, by one thread of the row's S.  Every thread
+// of a block of 256 calls it.
+template <int S, class Op, class V, class F>
+__device__ __forceinline__ void for_rows(const Op& op, const V* __restrict__ x, F&& f) {
+    const int64_t n = op.n;
+    if constexpr (S == 1) {
+        for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+            f(r, op.template part<1, V>(r, x, 0), x[r]);
+    } else if constexpr (OpSplit<Op>::lanes) {
+        const int p = threadIdx.x % S;
+        for (int64_t base = blockIdx.x * (int64_t)(256 / S); base < n; base += (int64_t)gridDim.x * (256 / S)) {
+            const int64_t r = base + threadIdx.x / S;
+            V a = r < n ? op.template part<S, V>(r, x, p) : Sc<V>::zero();
+#pragma unroll
+            for (int o = S / 2; o; o >>= 1) a = Sc<V>::add(a, Sc<V>::shfl_xor(a, o));
+            if (r < n && p == 0) f(r, a, x[r]);
+        }
+    } else {
+        __shared__ V part[256];
+        const int warp = threadIdx.x >> 5, p = warp % S;
+        for (int64_t base = blockIdx.x * (int64_t)(256 / S); base < n; base += (int64_t)gridDim.x * (256 / S)) {
+            const int64_t r = base + (warp / S) * 32 + (threadIdx.x & 31);
+            if (r < n) part[threadIdx.x] = op.template part<S, V>(r, x, p);
+            __syncthreads();
+            if (r < n && p == 0) {
+                V a = part[threadIdx.x];
+#pragma unroll
+                for (int q = 1; q < S; ++q) a = Sc<V>::add(a, part[threadIdx.x + 32 * q]);
+                f(r, a, x[r]);
+            }
+            __syncthreads();
+        }
+    }
+}
 
 // xs = n(c) x_c for the matrix-free operator, where x = x0, or with iter the
 // half of the Lanczos work buffer x0 that step *iter reads.

@@ -98,7 +98,7 @@ __global__ void k_lz_start(int64_t n, int mode, uint64_t seed, const P* __restri
 
 // K1: y = H w_j / beta_j - beta_j v_{j-1}; v_j = w_j / beta_j; alpha_j = Re <v_j, y>.
 // Optionally psi += c_j v_j (eigenvector regeneration).
-template <class Op, class V, class P>
+template <class Op, class V, class P, int S>
 __global__ void __launch_bounds__(kLzBlock, OpMinBlocks<Op>::value) k_lz_hv(Op op, V* __restrict__ wbuf, V* __restrict__ vring,
                                                     int K, LzDev d, const double* __restrict__ ritz,
                                                     P* __restrict__ psi) {
@@ -115,10 +115,7 @@ __global__ void __launch_bounds__(kLzBlock, OpMinBlocks<Op>::value) k_lz_hv(Op o
     const double inv = 1.0 / bj;
     const double c = ritz ? ritz[j] : 0.0;
     double acc = 0.0;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        V xr;
-        V hx = op.row(r, X, xr);
+    for_rows<S>(op, X, [&](int64_t r, V hx, V xr) {
         V vj = Sc<V>::scale(xr, inv);
         V y = Sc<V>::scale(hx, inv);
         if (j > 0) y = Sc<V>::sub(y, Sc<V>::scale(Vp[r], bj));
@@ -126,7 +123,7 @@ __global__ void __launch_bounds__(kLzBlock, OpMinBlocks<Op>::value) k_lz_hv(Op o
         Y[r] = y;
         acc += Sc<V>::re_conj_mul(vj, y);
         if (psi) psi[r] = Sc<P>::add(psi[r], Sc<P>::scale(cvt<P>(vj), c));
-    }
+    });
     double tot;
     if (grid_reduce(acc, d.partials, d.counter, red, &tot) && threadIdx.x == 0) d.alpha[j] = tot;
 }
@@ -316,20 +313,17 @@ __global__ void k_ritz(int64_t n, const V* __restrict__ vring, int m,
 }
 
 // scratch[0] = ||H psi - theta psi||^2, scratch[1] = ||psi||^2.
-template <class Op, class P>
-__global__ void k_residual(Op op, const P* __restrict__ psi, double theta, LzDev d) {
+template <class Op, class P, int S>
+__global__ void __launch_bounds__(kLzBlock) k_residual(Op op, const P* __restrict__ psi, double theta, LzDev d) {
     extern __shared__ __align__(16) unsigned char smem_rs[];
     __shared__ double red[32];
     op.init(smem_rs);
     double a = 0.0, b = 0.0;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < op.n;
-         r += (int64_t)gridDim.x * blockDim.x) {
-        P xr;
-        P hx = op.row(r, psi, xr);
+    for_rows<S>(op, psi, [&](int64_t, P hx, P xr) {
         P res = Sc<P>::sub(hx, Sc<P>::scale(xr, theta));
         a += Sc<P>::abs2(res);
         b += Sc<P>::abs2(xr);
-    }
+    });
     double ta, tb;
     bool la = grid_reduce(a, d.partials, d.counter, red, &ta);
     if (la && threadIdx.x == 0) d.scratch[0] = ta;
@@ -339,6 +333,25 @@ __global__ void k_residual(Op op, const P* __restrict__ psi, double theta, LzDev
 }
 
 // ------------------------------------------------------------------- host
+// K1 and the residual with the operator's row split.
+template <class Op, class V, class P>
+void launch_lz_hv(const Op& op, size_t smem, int nb, V* wbuf, V* vring, int K, const LzDev& d, const double* ritz,
+                  P* psi, cudaStream_t s, bool whole = false) {
+    with_split(op, [&](auto sp) {
+        constexpr int S = decltype(sp)::value;
+        set_group_smem_attr((const void*)k_lz_hv<Op, V, P, S>, smem);
+        k_lz_hv<Op, V, P, S><<<nb, kLzBlock, smem, s>>>(op, wbuf, vring, K, d, ritz, psi);
+    }, whole);
+}
+template <class Op, class P>
+void launch_residual(const Op& op, size_t smem, int nb, const P* psi, double theta, const LzDev& d, cudaStream_t s) {
+    with_split(op, [&](auto sp) {
+        constexpr int S = decltype(sp)::value;
+        set_group_smem_attr((const void*)k_residual<Op, P, S>, smem);
+        k_residual<Op, P, S><<<nb, kLzBlock, smem, s>>>(op, psi, theta, d);
+    });
+}
+
 // QMB_REORTH_ALWAYS=1: with two passes requested, always run the second one
 // (by default it runs only when the Kahan-Parlett criterion asks for it).
 static bool reorth_selective() {
@@ -496,15 +509,12 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, start_mode, seed, from, wbuf.p, st.d);
     check_launch("k_lz_start");
 
-    const void* f1 = (const void*)k_lz_hv<Op, V, P>;
-    set_group_smem_attr(f1, op_smem);
     size_t ro_smem = sizeof(double2) * (size_t)(cap + 2);
     if (po.reorth) set_group_smem_attr((const void*)k_reorth_update<V>, ro_smem);
 
     auto step = [&](cudaStream_t ss) {
         op.pre((const V*)wbuf.p, st.d.iter, ss);  // column-block passes or the matrix-free scaling, if any
-        k_lz_hv<Op, V, P><<<nb, kLzBlock, op_smem, ss>>>(op, wbuf.p, vring.p, K, st.d, nullptr,
-                                                         (P*)nullptr);
+        launch_lz_hv<Op, V, P>(op, op_smem, nb, wbuf.p, vring.p, K, st.d, nullptr, nullptr, ss, po.reorth > 0);
         k_lz_update<V><<<nb, kLzBlock, 0, ss>>>(n, wbuf.p, vring.p, K, st.d, po.reorth ? 0 : 1);
         for (int p = 0; p < po.reorth; ++p) {
             k_reorth_dots<V><<<nb, kLzBlock, 0, ss>>>(n, wbuf.p, vring.p, st.d, p);
@@ -676,7 +686,7 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, start_mode, seed, from, wbuf.p, st.d);
     for (int j = 0; j < ph.m; ++j) {
         op.pre((const V*)wbuf.p, st.d.iter, s);
-        k_lz_hv<Op, V, P><<<nb, kLzBlock, op_smem, s>>>(op, wbuf.p, vring.p, K, st.d, ritz.p, psi);
+        launch_lz_hv<Op, V, P>(op, op_smem, nb, wbuf.p, vring.p, K, st.d, ritz.p, psi, s);
         if (j + 1 < ph.m) k_lz_update<V><<<nb, kLzBlock, 0, s>>>(n, wbuf.p, vring.p, K, st.d, 1);
         ++n_hv;
     }
@@ -688,10 +698,9 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
 template <class Op, class P>
 double residual_norm(const Op& op, size_t op_smem, const P* psi, double theta, LzState& st,
                      cudaStream_t s, double* psi_norm2) {
-    set_group_smem_attr((const void*)k_residual<Op, P>, op_smem);
     g_lz_kernels += 1;
     op.pre(psi, (const int*)nullptr, s);
-    k_residual<Op, P><<<st.nb, kLzBlock, op_smem, s>>>(op, psi, theta, st.d);
+    launch_residual<Op, P>(op, op_smem, st.nb, psi, theta, st.d, s);
     check_launch("k_residual");
     double h[2];
     QMB_CUDA_TRY(cudaMemcpyAsync(h, st.scratch.p, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -1117,7 +1126,7 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
 
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, 1, seed, (const P*)nullptr, wbuf, d);
     for (int j = 0; j < n_iter; ++j) {
-        k_lz_hv<RefEllOp<V>, V, P><<<nb, kLzBlock, 0, s>>>(op, wbuf, vring, K, d, nullptr, (P*)nullptr);
+        launch_lz_hv<RefEllOp<V>, V, P>(op, 0, nb, wbuf, vring, K, d, nullptr, nullptr, s);
         k_lz_update<V><<<nb, kLzBlock, 0, s>>>(n, wbuf, vring, K, d, 1);
     }
     check_launch("noalloc lanczos steps");
@@ -1147,10 +1156,10 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
     QMB_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(P) * n, s));
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, 1, seed, (const P*)nullptr, wbuf, d);
     for (int j = 0; j < m; ++j) {
-        k_lz_hv<RefEllOp<V>, V, P><<<nb, kLzBlock, 0, s>>>(op, wbuf, vring, K, d, ritz, psi);
+        launch_lz_hv<RefEllOp<V>, V, P>(op, 0, nb, wbuf, vring, K, d, ritz, psi, s);
         if (j + 1 < m) k_lz_update<V><<<nb, kLzBlock, 0, s>>>(n, wbuf, vring, K, d, 1);
     }
-    k_residual<RefEllOp<V>, P><<<nb, kLzBlock, 0, s>>>(op, psi, theta, d);
+    launch_residual<RefEllOp<V>, P>(op, 0, nb, psi, theta, d, s);
     check_launch("noalloc residual");
     double h[2];
     QMB_CUDA_TRY(cudaMemcpyAsync(h, d.scratch, sizeof(h), cudaMemcpyDeviceToHost, s));
