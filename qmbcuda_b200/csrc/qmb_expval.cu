@@ -20,22 +20,28 @@
 //
 // The reference applies the operator to every member of every orbit (|G|
 // applications per term and row) and finds the target orbit through a table
-// over the whole Sz sector.  Here the group average is formed once on the
-// host, identical terms are merged, terms that change Sz are dropped (they
-// have zero expectation in a fixed-Sz sector), and each row applies the
-// averaged terms to its representative only.  Many operators share one
-// launch: their terms sit back to back in shared memory, one segment per
-// operator (or per part of an operator when it does not fit), and every
-// segment reduces separately.
+// over the whole Sz sector.  Here each row applies averaged terms to its
+// representative only, and a term is evaluated once however many operators hold
+// it: <psi|T|psi> is the same for all images of T under the group (up to the
+// sign of an odd number of Sz under inversion), so the terms of all operators
+// are sorted into classes, one value per class is computed on the device, and an
+// operator is the sum of its scalars times its classes' values.  The structure
+// factor at all 24 momenta of a 24-site chain with the 24 correlators has 27,672
+// terms in 13 classes.  Terms that change Sz are dropped (zero expectation in a
+// fixed-Sz sector).
+//
+// Products of Sz are signs: a class's value is a sum over its distinct images m
+// of Q(m) = sum_r |psi_r|^2 (-1)^popc(m & down_r), and k_ev_diag computes all Q
+// in one launch.  Other classes go through the Hamiltonian's row rule, their
+// averaged terms back to back in shared memory, one segment per class, each
+// reduced separately.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <complex>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
-#include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "qmb_ham.cuh"
@@ -46,118 +52,187 @@ namespace {
 
 constexpr int kEvBlock = 256;
 constexpr size_t kEvSmemCap = 200 * 1024;  // dynamic shared memory per block
+constexpr int64_t kEvSlab = (int64_t)1 << 23;  // rows of one pass of the sign sums
 
-// Group average of one operator table: the distinct terms (op words
-// code << 8 | site, in application order) with their summed scalars, in
-// order of first appearance.
-struct AvgTerms {
-    std::vector<std::vector<uint16_t>> keys;
-    std::vector<std::complex<double>> sc;
+using cplx = std::complex<double>;
+
+// A product of operators: up to 8 words code << 8 | site in application order.
+struct TermKey {
+    uint64_t a = 0, b = 0;
+    int n = 0;
+    bool operator==(const TermKey& o) const { return a == o.a && b == o.b && n == o.n; }
 };
+struct TermKeyHash {
+    size_t operator()(const TermKey& k) const {
+        uint64_t h = k.a * 0x9E3779B97F4A7C15ull ^ (k.b + 0x632BE59BD9B4E019ull + (uint64_t)k.n) * 0xC2B2AE3D27D4EB4Full;
+        return (size_t)(h ^ (h >> 29));
+    }
+};
+TermKey make_key(const uint16_t* w, int n) {
+    TermKey k;
+    k.n = n;
+    for (int i = 0; i < n; ++i) (i < 4 ? k.a : k.b) |= (uint64_t)w[i] << (16 * (i & 3));
+    return k;
+}
+void key_words(const TermKey& k, uint16_t* w) {
+    for (int i = 0; i < k.n; ++i) w[i] = (uint16_t)((i < 4 ? k.a : k.b) >> (16 * (i & 3)));
+}
 
-// Open-addressing table over terms packed into 128 bits (up to 8 factors of
-// 16 bits) plus the factor count.
-class TermTable {
-public:
-    explicit TermTable(size_t n_insert) {
-        size_t cap = 16;
-        while (cap < 2 * n_insert) cap <<= 1;
-        slots_.assign(cap, Slot{});
-        mask_ = cap - 1;
-    }
-    void add(const uint16_t* w, int n, std::complex<double> v) {
-        uint64_t a = 0, b = 0;
-        for (int i = 0; i < n && i < 4; ++i) a |= (uint64_t)w[i] << (16 * i);
-        for (int i = 4; i < n; ++i) b |= (uint64_t)w[i] << (16 * (i - 4));
-        uint64_t h = a * 0x9E3779B97F4A7C15ull ^ (b + 0x632BE59BD9B4E019ull + (uint64_t)n) * 0xC2B2AE3D27D4EB4Full;
-        h ^= h >> 29;
-        for (size_t i = h & mask_;; i = (i + 1) & mask_) {
-            Slot& s = slots_[i];
-            if (!s.used) {
-                s = Slot{a, b, n, true, v};
-                order_.push_back(i);
-                return;
-            }
-            if (s.a == a && s.b == b && s.n == n) {
-                s.v += v;
-                return;
-            }
-        }
-    }
-    void emit(AvgTerms& out) const {
-        for (size_t i : order_) {
-            const Slot& s = slots_[i];
-            if (s.v == 0.0) continue;
-            std::vector<uint16_t> k(s.n);
-            for (int j = 0; j < s.n; ++j) k[j] = (uint16_t)((j < 4 ? s.a >> (16 * j) : s.b >> (16 * (j - 4))) & 0xffff);
-            out.keys.push_back(std::move(k));
-            out.sc.push_back(s.v);
-        }
-    }
-
-private:
-    struct Slot {
-        uint64_t a = 0, b = 0;
-        int n = 0;
-        bool used = false;
-        std::complex<double> v = 0.0;
+// The classes of the operators' terms.
+struct Classes {
+    const qmb_sector_s* s;
+    int n = 0;                                  // classes
+    // products of Sz, by the XOR of their sites (a site taken twice is 1/4, no sign)
+    std::unordered_map<uint64_t, int> of_mask;
+    std::vector<int> pair_class;                // [L][L] classes of masks of one or two sites, -1: not seen
+    std::vector<uint64_t> masks;                // images of all diagonal classes
+    std::vector<double> mask_w;                 // their weights
+    std::vector<int> mask_class;
+    // other terms
+    struct At {
+        int cls;
+        double sign;
     };
-    std::vector<Slot> slots_;
-    std::vector<size_t> order_;
-    size_t mask_ = 0;
+    std::unordered_map<TermKey, At, TermKeyHash> of_key;
+    std::vector<TermKey> gen_key;               // averaged terms, class by class
+    std::vector<double> gen_w;
+    std::vector<int> gen_class;
+
+    explicit Classes(const qmb_sector_s* sec) : s(sec), pair_class(sec->L * sec->L, -1) {}
+
+    // Class of a product of Sz, or -1 where the average vanishes.
+    int diag_class(uint64_t m) {
+        const auto it = of_mask.find(m);
+        if (it != of_mask.end()) return it->second;
+        const bool zero = s->flip && (__builtin_popcountll(m) & 1);  // inversion takes it to its negative
+        const int c = zero ? -1 : n++;
+        const size_t first = masks.size();
+        for (int g = 0; g < s->G; ++g) {
+            const uint32_t* p = s->perm.data() + (size_t)g * s->L;
+            uint64_t y = 0;
+            for (uint64_t b = m; b; b &= b - 1) y |= 1ull << p[__builtin_ctzll(b)];
+            if (of_mask.emplace(y, c).second) {
+                if (zero) continue;
+                masks.push_back(y);
+                mask_w.push_back(1.0 / s->G);
+                mask_class.push_back(c);
+            } else if (!zero) {
+                for (size_t k = first; k < masks.size(); ++k)
+                    if (masks[k] == y) mask_w[k] += 1.0 / s->G;
+            }
+        }
+        of_mask.emplace(m, c);  // (among its images already when the group has the identity)
+        return c;
+    }
+
+    // Class of a term with S+ and S-, and the sign of its value.
+    At gen_class_of(const uint16_t* w, int nw, int n_z) {
+        uint16_t img[kMaxCol];
+        auto image = [&](int e) {
+            const uint32_t* p = s->perm.data() + (size_t)(e % s->G) * s->L;
+            const bool z = e >= s->G;
+            for (int j = 0; j < nw; ++j) {
+                int c = w[j] >> 8;
+                if (z && c != QMB_OP_SZ) c = c == QMB_OP_SP ? QMB_OP_SM : QMB_OP_SP;
+                img[j] = (uint16_t)(c << 8 | (int)p[w[j] & 0xff]);
+            }
+            // factors on distinct sites commute: order them by site
+            bool distinct = true;
+            for (int a = 0; a < nw && distinct; ++a)
+                for (int b = a + 1; b < nw; ++b)
+                    if ((img[a] & 0xff) == (img[b] & 0xff)) {
+                        distinct = false;
+                        break;
+                    }
+            if (distinct)
+                std::sort(img, img + nw, [](uint16_t x, uint16_t y) { return (x & 0xff) < (y & 0xff); });
+            return make_key(img, nw);
+        };
+        // (element 0 may be any element: look the term itself up in image order)
+        const TermKey k0 = image(0);
+        const auto it = of_key.find(k0);
+        if (it != of_key.end()) return it->second;
+        const int c = n++;
+        const size_t first = gen_key.size();
+        for (int e = 0; e < s->n_ext; ++e) {
+            const TermKey k = image(e);
+            const double sign = (e >= s->G && (n_z & 1)) ? -1.0 : 1.0;
+            if (of_key.emplace(k, At{c, sign}).second) {
+                gen_key.push_back(k);
+                gen_w.push_back(sign / s->n_ext);
+                gen_class.push_back(c);
+            } else {
+                for (size_t q = first; q < gen_key.size(); ++q)
+                    if (gen_key[q] == k) gen_w[q] += sign / s->n_ext;
+            }
+        }
+        return of_key.find(k0)->second;
+    }
 };
 
-void average_terms(const qmb_sector_s* s, const qmb_terms& A, AvgTerms& out) {
+// Adds the terms of one operator: (class, scalar) pairs, one per class.
+void sort_terms(const qmb_terms& A, Classes& cls, std::vector<int>& last_op, std::vector<size_t>& last_at, int op,
+                std::vector<std::pair<int, cplx>>& out) {
     QMB_REQUIRE(A.n_terms >= 0, QMB_ERR_INVALID, "expval: n_terms must be >= 0");
     if (A.n_terms == 0) return;
     QMB_REQUIRE(A.n_ops && A.op_code && A.op_site && A.scalar, QMB_ERR_INVALID,
                 "expval: null table");
     QMB_REQUIRE(A.n_col >= 1 && A.n_col <= kMaxCol, QMB_ERR_INVALID, "expval: n_col must be in 1..8");
-    const int L = s->L, G = s->G, ne = s->n_ext;
-    TermTable tab((size_t)A.n_terms * ne);
-    uint16_t base[kMaxCol], img[kMaxCol];
+    const int L = cls.s->L;
+    auto add = [&](int c, cplx v) {
+        if (c < 0) return;
+        if ((int)last_op.size() < cls.n) {
+            last_op.resize(2 * cls.n + 16, -1);
+            last_at.resize(last_op.size(), 0);
+        }
+        if (last_op[c] != op) {
+            last_op[c] = op;
+            last_at[c] = out.size();
+            out.emplace_back(c, v);
+        } else {
+            out[last_at[c]].second += v;
+        }
+    };
     for (int i = 0; i < A.n_terms; ++i) {
-        QMB_REQUIRE(A.n_ops[i] >= 0 && A.n_ops[i] <= A.n_col, QMB_ERR_INVALID,
-                    "expval: n_ops out of range");
-        const std::complex<double> sc(A.scalar[2 * i], A.scalar[2 * i + 1]);
+        const int no = A.n_ops[i];
+        QMB_REQUIRE(no >= 0 && no <= A.n_col, QMB_ERR_INVALID, "expval: n_ops out of range");
+        const cplx sc(A.scalar[2 * i], A.scalar[2 * i + 1]);
         QMB_REQUIRE(std::isfinite(sc.real()) && std::isfinite(sc.imag()), QMB_ERR_INVALID,
                     "expval: non-finite scalar");
+        const int *code = A.op_code + (size_t)i * A.n_col, *site = A.op_site + (size_t)i * A.n_col;
+        uint16_t w[kMaxCol];
         int nb = 0, n_p = 0, n_m = 0, n_z = 0;
-        for (int j = 0; j < A.n_ops[i]; ++j) {
-            const int c = A.op_code[i * A.n_col + j], q = A.op_site[i * A.n_col + j];
+        uint64_t m = 0;
+        double f = 1.0;
+        for (int j = 0; j < no; ++j) {
+            const int c = code[j], q = site[j];
             QMB_REQUIRE(c == QMB_OP_SZ || c == QMB_OP_SP || c == QMB_OP_SM || c == QMB_OP_I,
                         QMB_ERR_INVALID, "expval: operator codes must be Sz, Sp, Sm or I");
             QMB_REQUIRE(q >= 0 && q < L, QMB_ERR_INVALID, "expval: site out of range");
             if (c == QMB_OP_I) continue;
             n_p += c == QMB_OP_SP;
             n_m += c == QMB_OP_SM;
-            n_z += c == QMB_OP_SZ;
-            base[nb++] = (uint16_t)(c << 8 | q);
+            if (c == QMB_OP_SZ) {
+                ++n_z;
+                m ^= 1ull << q;
+                f *= 0.5;
+            }
+            w[nb++] = (uint16_t)(c << 8 | q);
         }
         if (n_p != n_m || sc == 0.0) continue;  // leaves the Sz sector, or zero
-        for (int e = 0; e < ne; ++e) {
-            const uint32_t* p = s->perm.data() + (size_t)(e % G) * L;
-            const bool z = e >= G;
-            for (int j = 0; j < nb; ++j) {
-                int c = base[j] >> 8, q = base[j] & 0xff;
-                if (z && c != QMB_OP_SZ) c = c == QMB_OP_SP ? QMB_OP_SM : QMB_OP_SP;
-                img[j] = (uint16_t)(c << 8 | (int)p[q]);
+        if (n_p == 0) {
+            if (nb == 2 && m) {  // two sites, the common product: no hash lookup
+                int& pc = cls.pair_class[(w[0] & 0xff) * L + (w[1] & 0xff)];
+                if (pc == -1) pc = cls.diag_class(m) + 1 ? cls.diag_class(m) : -2;
+                add(pc, sc * f);
+            } else {
+                add(cls.diag_class(m), sc * f);
             }
-            // factors on distinct sites commute: order them by site
-            bool distinct = true;
-            for (int a = 0; a < nb && distinct; ++a)
-                for (int b = a + 1; b < nb; ++b)
-                    if ((img[a] & 0xff) == (img[b] & 0xff)) {
-                        distinct = false;
-                        break;
-                    }
-            if (distinct)
-                std::sort(img, img + nb, [](uint16_t x, uint16_t y) { return (x & 0xff) < (y & 0xff); });
-            const double sign = (z && (n_z & 1)) ? -1.0 : 1.0;
-            tab.add(img, nb, sc * (sign / ne));
+        } else {
+            const Classes::At at = cls.gen_class_of(w, nb, n_z);
+            add(at.cls, sc * at.sign);
         }
     }
-    tab.emit(out);
 }
 
 bool trace_on() {
@@ -187,60 +262,108 @@ __device__ __forceinline__ double2 block_sum2(double x, double y, double2* red) 
     return t;
 }
 
-// One launch: every block strides over the rows for each segment sg and
-// writes its partial sum of conj(psi_r) (Abar_sg psi)_r to part[sg][block];
-// npart[block] receives the block's partial of <psi|psi>.  Segment sg =
-// (d0, d1, g0, g1): diagonal terms d0..d1-1 and general terms g0..g1-1.
-// A diagonal term (a product of Sz only) has the value
-//     sc * (-1)^popc(mask & ~t)
-// on the string t, with sc = scalar * 2^-k for k factors and mask the XOR of
-// the factors' site bits (a site taken twice gives (+-1/2)^2 = 1/4, no sign).
-// One block per SM fits the shared memory, so registers are not the limit.
+// Rows r0 .. r0 + n - 1 for the sign sums: down_r, the string's down spins, and
+// |psi_r|^2, with the block partials of <psi|psi> added to npart.
 template <class V>
-__global__ void __launch_bounds__(kEvBlock, 1) k_expval(RowGen rg, int64_t n, const V* __restrict__ psi,
-                                                        int n_seg, const int4* __restrict__ seg, int n_diag,
-                                                        const uint64_t* __restrict__ dmask,
-                                                        const double2* __restrict__ dsc,
-                                                        double2* __restrict__ part, double* __restrict__ npart) {
+__global__ void __launch_bounds__(kEvBlock) k_ev_rows(RowGen rg, int64_t r0, int64_t n, const V* __restrict__ psi,
+                                                      uint64_t* __restrict__ down64, uint32_t* __restrict__ down32,
+                                                      double* __restrict__ p2, double* __restrict__ npart) {
+    extern __shared__ __align__(16) unsigned char smem_er[];
+    __shared__ double2 red[kEvBlock / 32];
+    const GroupSmem gs = load_group(rg.g, smem_er);
+    double nn = 0.0;
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+        const double p = Sc<V>::abs2(psi[r0 + r]);
+        nn += p;
+        if (p2) {
+            const uint64_t d = ~apply_elem(rg.g, gs, 0, rg.rt.reps[rg.orbit_of_row[r0 + r]]);
+            p2[r] = p;
+            if (down32) down32[r] = (uint32_t)d;
+            else down64[r] = d;
+        }
+    }
+    const double2 t = block_sum2(nn, 0.0, red);
+    if (threadIdx.x == 0) npart[blockIdx.x] += t.x;
+}
+
+// part[chunk][m] = sum over the chunk's rows of p2_r (-1)^popc(mask_m & down_r).
+// A warp takes 8 masks over one chunk of rows, lanes over rows, so that a row's
+// 12 bytes serve 8 masks from registers: an AND, a population count, a sign flip
+// (the parity moved to the sign bit) and an FP64 addition each.  13 classes of a
+// 24-site chain are 300 masks over 112,720 rows: all values with their copies take
+// 75 us (640 us for one kernel over the 7,764 averaged terms of the operators).
+// The population counts bound it (16 a cycle and SM).
+constexpr int kEvMasks = 8;
+template <class U>
+__global__ void __launch_bounds__(kEvBlock) k_ev_diag(int64_t n, const U* __restrict__ down,
+                                                      const double* __restrict__ p2, const U* __restrict__ mask,
+                                                      int n_mask, int n_groups, int n_chunks, int64_t chunk,
+                                                      double* __restrict__ part) {
+    const int lane = threadIdx.x & 31;
+    const int item = blockIdx.x * (kEvBlock / 32) + (threadIdx.x >> 5);
+    if (item >= n_groups * n_chunks) return;
+    const int g = item % n_groups, c = item / n_groups, m0 = g * kEvMasks;
+    U mk[kEvMasks];
+    double acc[kEvMasks];
+#pragma unroll
+    for (int k = 0; k < kEvMasks; ++k) {
+        mk[k] = m0 + k < n_mask ? mask[m0 + k] : (U)0;
+        acc[k] = 0.0;
+    }
+    const int64_t r1 = min(n, (c + 1) * chunk);
+#pragma unroll 2
+    for (int64_t r = c * chunk + lane; r < r1; r += 32) {
+        const U d = down[r];
+        const double p = p2[r];
+        const int hi = __double2hiint(p), lo = __double2loint(p);
+#pragma unroll
+        for (int k = 0; k < kEvMasks; ++k) {
+            const int par = sizeof(U) == 8 ? __popcll((unsigned long long)(mk[k] & d)) : __popc((unsigned)(mk[k] & d));
+            acc[k] += __hiloint2double(hi ^ (int)((unsigned)par << 31), lo);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kEvMasks; ++k) {
+        for (int o = 16; o; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+        if (lane == 0 && m0 + k < n_mask) part[(int64_t)c * n_mask + m0 + k] = acc[k];
+    }
+}
+
+// q[m] += the chunks' part[chunk][m], added up in chunk order.
+__global__ void k_ev_diag_sum(const double* __restrict__ part, int n_mask, int n_chunks, double* __restrict__ q) {
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n_mask; m += gridDim.x * blockDim.x) {
+        double t = 0.0;
+        for (int c = 0; c < n_chunks; ++c) t += part[(int64_t)c * n_mask + m];
+        q[m] += t;
+    }
+}
+
+// One launch over the other terms: every block strides over the rows for each
+// segment sg and writes its partial sum of conj(psi_r) (Abar_sg psi)_r to
+// part[sg][block].  Segment sg holds terms seg[sg].x .. seg[sg].y - 1.
+template <class V>
+__global__ void __launch_bounds__(kEvBlock) k_expval(RowGen rg, int64_t n, const V* __restrict__ psi, int n_seg,
+                                                     const int2* __restrict__ seg, double2* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smem_ev[];
     __shared__ double2 red[kEvBlock / 32];
     const size_t gb = align16(group_smem_bytes(rg.g));
     const GroupSmem gs = load_group(rg.g, smem_ev);
     const TermsSmem ts = load_terms(rg.terms, smem_ev + gb);
-    double2* s_sc = reinterpret_cast<double2*>(smem_ev + gb + terms_smem_bytes(rg.terms));
-    uint64_t* s_mask = reinterpret_cast<uint64_t*>(s_sc + n_diag);
-    for (int i = threadIdx.x; i < n_diag; i += blockDim.x) {
-        s_sc[i] = dsc[i];
-        s_mask[i] = dmask[i];
-    }
-    __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int sg = 0; sg < n_seg; ++sg) {
-        const int4 sd = seg[sg];
+        const int2 sd = seg[sg];
         double ax = 0.0, ay = 0.0;
         for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += stride) {
             const int64_t o = rg.orbit_of_row[r];
             const uint64_t src = apply_elem(rg.g, gs, 0, rg.rt.reps[o]);
-            const uint64_t down = ~src;
-            // complex row sum even for a real psi: scalars may be complex
+            // complex row sum even for a real psi: characters may be complex
             const double2 pr = Sc<V>::to2(psi[r]);
             double2 y = make_double2(0.0, 0.0);
-            double2 d = make_double2(0.0, 0.0);
-            for (int t = sd.x; t < sd.y; ++t) {
-                const double2 c = s_sc[t];
-                const double f = (__popcll(s_mask[t] & down) & 1) ? -1.0 : 1.0;
-                d.x = fma(f, c.x, d.x);
-                d.y = fma(f, c.y, d.y);
-            }
-            if (sd.z < sd.w) {
-                const double2 g = gen_row_range(rg, gs, ts, sd.z, sd.w, src, rg.norms[o], [&](int64_t ot, double2 v) {
-                    const double2 x = Sc<V>::to2(__ldg(psi + rg.row_of_orbit[ot]));
-                    y.x += v.x * x.x - v.y * x.y;
-                    y.y += v.x * x.y + v.y * x.x;
-                });
-                d.x += g.x;
-                d.y += g.y;
-            }
+            const double2 d = gen_row_range(rg, gs, ts, sd.x, sd.y, src, rg.norms[o], [&](int64_t ot, double2 v) {
+                const double2 x = Sc<V>::to2(__ldg(psi + rg.row_of_orbit[ot]));
+                y.x += v.x * x.x - v.y * x.y;
+                y.y += v.x * x.y + v.y * x.x;
+            });
             y.x += d.x * pr.x - d.y * pr.y;
             y.y += d.x * pr.y + d.y * pr.x;
             ax += pr.x * y.x + pr.y * y.y;  // conj(pr) * y
@@ -249,11 +372,6 @@ __global__ void __launch_bounds__(kEvBlock, 1) k_expval(RowGen rg, int64_t n, co
         const double2 t = block_sum2(ax, ay, red);
         if (threadIdx.x == 0) part[(size_t)sg * gridDim.x + blockIdx.x] = t;
     }
-    double nn = 0.0;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += stride)
-        nn += Sc<V>::abs2(psi[r]);
-    const double2 t = block_sum2(nn, 0.0, red);
-    if (threadIdx.x == 0) npart[blockIdx.x] = t.x;
 }
 
 // Fixed-order sum of the block partials of every segment (one block each).
@@ -270,185 +388,154 @@ __global__ void __launch_bounds__(kEvBlock) k_expval_sum(const double2* __restri
     if (threadIdx.x == 0) seg_out[blockIdx.x] = t;
 }
 
-bool is_diagonal(const std::vector<uint16_t>& key) {
-    for (uint16_t w : key)
-        if ((w >> 8) != QMB_OP_SZ) return false;
-    return true;
-}
-
+// The values of the classes: val[c] = sum_r conj(psi_r) (Tbar_c psi)_r, and
+// <psi|psi>.
 template <class V>
-void run_expval(qmb_ham_s* h, const V* psi, const std::vector<AvgTerms>& ops, double* out) {
+void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cplx>& val, double* norm2) {
     RowGen rg = h->row_gen();
     const size_t gbytes = align16(group_smem_bytes(rg.g));
+    int sms = 148, max_smem = 0;
+    QMB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    QMB_CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    const size_t smem_cap = std::min(kEvSmemCap, (size_t)max_smem);
+    QMB_REQUIRE(gbytes + 64 < smem_cap, QMB_ERR_INVALID, "expval: group tables leave no shared memory");
+    val.assign(cls.n, cplx(0.0, 0.0));
+    const int64_t n = h->n;
+    size_t off = 0;
+    auto place = [&](size_t bytes) {
+        const size_t o = off;
+        off = align16(off + bytes);
+        return o;
+    };
+
+    // products of Sz, and the norm
+    {
+        const int nm = (int)cls.masks.size(), groups = (nm + kEvMasks - 1) / kEvMasks;
+        const bool small = cls.s->L <= 32;
+        // rows in slabs, which bounds the scratch (12 or 16 bytes a row); about
+        // 48 warps an SM, chunks of at least 256 rows
+        const int64_t slab = std::min<int64_t>(n, nm ? kEvSlab : n);
+        const int64_t want = groups ? std::max<int64_t>(1, (int64_t)sms * 48 / groups) : 1;
+        const int chunks = (int)std::min<int64_t>(want, (slab + 255) / 256);
+        const int64_t chunk = ((slab + chunks - 1) / chunks + 31) / 32 * 32;
+        const int nblk = (int)std::min<int64_t>((slab + kEvBlock - 1) / kEvBlock, (int64_t)sms * 4);
+        const size_t us = small ? 4 : 8;
+        off = 0;
+        const size_t o_mask = place(us * nm), o_q = place(sizeof(double) * nm), o_norm = place(sizeof(double) * nblk),
+                     o_p = place(nm ? sizeof(double) * slab : 0), o_down = place(nm ? us * slab : 0),
+                     o_part = place(sizeof(double) * (size_t)nm * chunks);
+        DevBuf<unsigned char> blk(off);
+        unsigned char* b = blk.p;
+        double* q = reinterpret_cast<double*>(b + o_q);
+        double* npart = reinterpret_cast<double*>(b + o_norm);
+        double* p2 = nm ? reinterpret_cast<double*>(b + o_p) : nullptr;
+        uint32_t* d32 = small ? reinterpret_cast<uint32_t*>(b + o_down) : nullptr;
+        uint64_t* d64 = reinterpret_cast<uint64_t*>(b + o_down);
+        double* part = reinterpret_cast<double*>(b + o_part);
+        std::vector<uint32_t> m32;
+        const void* hm = cls.masks.data();
+        if (small) {
+            m32.assign(cls.masks.begin(), cls.masks.end());
+            hm = m32.data();
+        }
+        if (nm) QMB_CUDA_TRY(cudaMemcpyAsync(b + o_mask, hm, us * nm, cudaMemcpyHostToDevice, 0));
+        QMB_CUDA_TRY(cudaMemsetAsync(b + o_q, 0, o_norm + sizeof(double) * nblk - o_q, 0));
+        set_group_smem_attr((const void*)k_ev_rows<V>, gbytes);
+        for (int64_t r0 = 0; r0 < n; r0 += slab) {
+            const int64_t rows = std::min(slab, n - r0);
+            k_ev_rows<V><<<nblk, kEvBlock, gbytes>>>(rg, r0, rows, psi, d64, d32, p2, npart);
+            check_launch("k_ev_rows");
+            if (!nm) continue;
+            const int grid = (groups * chunks + kEvBlock / 32 - 1) / (kEvBlock / 32);
+            if (small)
+                k_ev_diag<uint32_t><<<grid, kEvBlock>>>(rows, d32, p2, reinterpret_cast<const uint32_t*>(b + o_mask), nm,
+                                                        groups, chunks, chunk, part);
+            else
+                k_ev_diag<uint64_t><<<grid, kEvBlock>>>(rows, d64, p2, reinterpret_cast<const uint64_t*>(b + o_mask), nm,
+                                                        groups, chunks, chunk, part);
+            check_launch("k_ev_diag");
+            k_ev_diag_sum<<<(nm + 31) / 32, 32>>>(part, nm, chunks, q);
+            check_launch("k_ev_diag_sum");
+        }
+        std::vector<unsigned char> res(o_norm + sizeof(double) * nblk - o_q);
+        QMB_CUDA_TRY(cudaMemcpy(res.data(), b + o_q, res.size(), cudaMemcpyDeviceToHost));
+        blk.mark_idle();
+        const double* hq = reinterpret_cast<const double*>(res.data());
+        const double* hn = reinterpret_cast<const double*>(res.data() + (o_norm - o_q));
+        for (int k = 0; k < nm; ++k) val[cls.mask_class[k]] += cls.mask_w[k] * hq[k];
+        *norm2 = 0.0;
+        for (int k = 0; k < nblk; ++k) *norm2 += hn[k];
+    }
+
+    // the other terms, as many as fit in shared memory at a time
+    const size_t n_gen = cls.gen_key.size();
+    if (!n_gen) return;
     DevBuf<int> err(1);
     err.zero();
     rg.err = err.p;
-
-    // items of operator k back to back, its diagonal terms first
-    struct Item {
-        int op;
-        const std::vector<uint16_t>* key;
-        std::complex<double> sc;
-        bool diag;
-    };
-    std::vector<Item> items;
-    for (size_t k = 0; k < ops.size(); ++k) {
-        for (size_t i = 0; i < ops[k].keys.size(); ++i)
-            if (is_diagonal(ops[k].keys[i])) items.push_back({(int)k, &ops[k].keys[i], ops[k].sc[i], true});
-        for (size_t i = 0; i < ops[k].keys.size(); ++i)
-            if (!is_diagonal(ops[k].keys[i])) items.push_back({(int)k, &ops[k].keys[i], ops[k].sc[i], false});
-    }
-
-    const int dev = h->device;
-    int sms = 148, max_smem = 0;
-    QMB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    QMB_CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t smem_cap = std::min(kEvSmemCap, (size_t)max_smem);
-    QMB_REQUIRE(gbytes + 64 < smem_cap, QMB_ERR_INVALID, "expval: group tables leave no shared memory");
-    auto chunk_bytes = [&](size_t n_gen, int n_col, size_t n_diag) {
-        return gbytes + ((20 + 2 * (size_t)n_col) * n_gen + 15) / 16 * 16 + 24 * n_diag;
-    };
-
-    std::vector<double2> seg_sum;
-    std::vector<int> seg_op;
-    double norm2 = 0.0;
-    bool have_norm = false;
-    size_t pos = 0;
-    do {
-        // chunk: as many items as fit in shared memory
-        struct Seg {
-            int op;
-            int4 r;
-        };
-        std::vector<Seg> segs;
-        std::vector<std::vector<uint16_t>> gkeys;
-        std::vector<double2> gsc, dsc;
-        std::vector<uint64_t> dmask;
+    for (size_t pos = 0; pos < n_gen;) {
+        std::vector<int2> seg;
+        std::vector<int> seg_class, nops;
+        std::vector<double2> sc;
         int n_col = 1;
         size_t end = pos;
-        for (; end < items.size(); ++end) {
-            const Item& it = items[end];
-            const size_t ng = gkeys.size() + (it.diag ? 0 : 1), nd = dmask.size() + (it.diag ? 1 : 0);
-            const int c = it.diag ? n_col : std::max(n_col, (int)it.key->size());
-            if (chunk_bytes(ng, c, nd) > smem_cap || ng > (size_t)kMaxTerms) break;
+        for (; end < n_gen; ++end) {
+            const size_t ng = end - pos + 1;
+            const int c = std::max(n_col, cls.gen_key[end].n);
+            if (gbytes + ((20 + 2 * (size_t)c) * ng + 15) / 16 * 16 > smem_cap || ng > (size_t)kMaxTerms) break;
             n_col = c;
-            if (segs.empty() || segs.back().op != it.op) {
-                const int nd0 = (int)dmask.size(), ng0 = (int)gkeys.size();
-                segs.push_back({it.op, make_int4(nd0, nd0, ng0, ng0)});
+            if (seg.empty() || seg_class.back() != cls.gen_class[end]) {
+                seg.push_back(make_int2((int)ng - 1, (int)ng - 1));
+                seg_class.push_back(cls.gen_class[end]);
             }
-            if (it.diag) {
-                uint64_t m = 0;
-                double f = 1.0;
-                for (uint16_t w : *it.key) {
-                    m ^= 1ull << (w & 0xff);
-                    f *= 0.5;
-                }
-                dmask.push_back(m);
-                dsc.push_back(make_double2(it.sc.real() * f, it.sc.imag() * f));
-                segs.back().r.y += 1;
-            } else {
-                gkeys.push_back(*it.key);
-                gsc.push_back(make_double2(it.sc.real(), it.sc.imag()));
-                segs.back().r.w += 1;
-            }
+            seg.back().y += 1;
+            nops.push_back(cls.gen_key[end].n);
+            sc.push_back(make_double2(cls.gen_w[end], 0.0));
         }
-        QMB_REQUIRE(end > pos || items.empty(), QMB_ERR_INVALID, "expval: a term does not fit");
-        const int ng = (int)gkeys.size(), nd = (int)dmask.size();
-        std::vector<int> nops(std::max(ng, 1), 0);
-        std::vector<uint16_t> opw((size_t)std::max(ng, 1) * n_col, 0);
-        for (int i = 0; i < ng; ++i) {
-            nops[i] = (int)gkeys[i].size();
-            std::copy(gkeys[i].begin(), gkeys[i].end(), opw.begin() + (size_t)i * n_col);
-        }
-        if (gsc.empty()) gsc.push_back(make_double2(0.0, 0.0));
-        if (dsc.empty()) {
-            dsc.push_back(make_double2(0.0, 0.0));
-            dmask.push_back(0);
-        }
-        const int n_seg = (int)segs.size();
-        std::vector<int4> seg_h(std::max(n_seg, 1), make_int4(0, 0, 0, 0));
-        for (int i = 0; i < n_seg; ++i) seg_h[i] = segs[i].r;
-
+        QMB_REQUIRE(end > pos, QMB_ERR_INVALID, "expval: a term does not fit");
+        const int ng = (int)(end - pos), n_seg = (int)seg.size();
+        std::vector<uint16_t> opw((size_t)ng * n_col, 0);
+        for (int i = 0; i < ng; ++i) key_words(cls.gen_key[pos + i], opw.data() + (size_t)i * n_col);
         rg.terms.n_terms = ng;
         rg.terms.n_col = n_col;
-        const size_t smem = gbytes + terms_smem_bytes(rg.terms) + 24 * (size_t)nd;
-        const void* kf = (const void*)k_expval<V>;
-        set_group_smem_attr(kf, smem);
+        const size_t smem = gbytes + terms_smem_bytes(rg.terms);
+        set_group_smem_attr((const void*)k_expval<V>, smem);
         int per_sm = 0;
         QMB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_expval<V>, kEvBlock, smem));
-        const int64_t want = (h->n + kEvBlock - 1) / kEvBlock;
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * std::max(1, per_sm)));
-
-        // one device block per chunk: the inputs staged and copied at once,
-        // then the per-segment results with the norm partials, then the
-        // block partials
-        size_t off = 0;
-        auto place = [&](size_t bytes) {
-            const size_t o = off;
-            off = align16(off + bytes);
-            return o;
-        };
-        const size_t o_nops = place(sizeof(int) * nops.size()), o_ops = place(sizeof(uint16_t) * opw.size()),
-                     o_sc = place(sizeof(double2) * gsc.size()), o_dsc = place(sizeof(double2) * dsc.size()),
-                     o_mask = place(sizeof(uint64_t) * dmask.size()), o_seg = place(sizeof(int4) * seg_h.size());
+        const int grid = (int)std::max<int64_t>(
+            1, std::min<int64_t>((n + kEvBlock - 1) / kEvBlock, (int64_t)sms * std::max(1, per_sm)));
+        off = 0;
+        const size_t o_nops = place(sizeof(int) * ng), o_ops = place(sizeof(uint16_t) * opw.size()),
+                     o_sc = place(sizeof(double2) * ng), o_seg = place(sizeof(int2) * n_seg);
         const size_t in_bytes = off;
-        const size_t res_bytes = sizeof(double2) * seg_h.size() + sizeof(double) * grid;
-        const size_t o_res = place(res_bytes);
-        const size_t o_part = place(sizeof(double2) * seg_h.size() * grid);
+        const size_t o_res = place(sizeof(double2) * n_seg), o_part = place(sizeof(double2) * (size_t)n_seg * grid);
         std::vector<unsigned char> stage(in_bytes);
-        std::memcpy(stage.data() + o_nops, nops.data(), sizeof(int) * nops.size());
+        std::memcpy(stage.data() + o_nops, nops.data(), sizeof(int) * ng);
         std::memcpy(stage.data() + o_ops, opw.data(), sizeof(uint16_t) * opw.size());
-        std::memcpy(stage.data() + o_sc, gsc.data(), sizeof(double2) * gsc.size());
-        std::memcpy(stage.data() + o_dsc, dsc.data(), sizeof(double2) * dsc.size());
-        std::memcpy(stage.data() + o_mask, dmask.data(), sizeof(uint64_t) * dmask.size());
-        std::memcpy(stage.data() + o_seg, seg_h.data(), sizeof(int4) * seg_h.size());
+        std::memcpy(stage.data() + o_sc, sc.data(), sizeof(double2) * ng);
+        std::memcpy(stage.data() + o_seg, seg.data(), sizeof(int2) * n_seg);
         DevBuf<unsigned char> blk(off);
         QMB_CUDA_TRY(cudaMemcpy(blk.p, stage.data(), in_bytes, cudaMemcpyHostToDevice));
         unsigned char* b = blk.p;
         rg.terms.n_ops = reinterpret_cast<const int*>(b + o_nops);
         rg.terms.ops = reinterpret_cast<const uint16_t*>(b + o_ops);
         rg.terms.scalar = reinterpret_cast<const double2*>(b + o_sc);
-        double2* seg_d = reinterpret_cast<double2*>(b + o_res);
-        double* npart = reinterpret_cast<double*>(seg_d + seg_h.size());
+        double2* res_d = reinterpret_cast<double2*>(b + o_res);
         double2* part = reinterpret_cast<double2*>(b + o_part);
-        k_expval<V><<<grid, kEvBlock, smem>>>(rg, h->n, psi, n_seg, reinterpret_cast<const int4*>(b + o_seg), nd,
-                                               reinterpret_cast<const uint64_t*>(b + o_mask),
-                                               reinterpret_cast<const double2*>(b + o_dsc), part, npart);
+        k_expval<V><<<grid, kEvBlock, smem>>>(rg, n, psi, n_seg, reinterpret_cast<const int2*>(b + o_seg), part);
         check_launch("k_expval");
-        if (n_seg) {
-            k_expval_sum<<<n_seg, kEvBlock>>>(part, grid, seg_d);
-            check_launch("k_expval_sum");
-        }
-        std::vector<unsigned char> res(res_bytes);
-        QMB_CUDA_TRY(cudaMemcpy(res.data(), seg_d, res_bytes, cudaMemcpyDeviceToHost));
+        k_expval_sum<<<n_seg, kEvBlock>>>(part, grid, res_d);
+        check_launch("k_expval_sum");
+        std::vector<double2> res(n_seg);
+        QMB_CUDA_TRY(cudaMemcpy(res.data(), res_d, sizeof(double2) * n_seg, cudaMemcpyDeviceToHost));
         blk.mark_idle();
-        const double2* hs = reinterpret_cast<const double2*>(res.data());
-        const double* hn = reinterpret_cast<const double*>(hs + seg_h.size());
-        for (int i = 0; i < n_seg; ++i) {
-            seg_sum.push_back(hs[i]);
-            seg_op.push_back(segs[i].op);
-        }
-        if (!have_norm) {
-            for (int i = 0; i < grid; ++i) norm2 += hn[i];
-            have_norm = true;
-        }
+        for (int i = 0; i < n_seg; ++i) val[seg_class[i]] += cplx(res[i].x, res[i].y);
         pos = end;
-    } while (pos < items.size());
+    }
     int herr = 0;
     QMB_CUDA_TRY(cudaMemcpy(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost));
     err.mark_idle();
     QMB_REQUIRE(herr == 0, QMB_ERR_INVALID, "expval: a term left the sector's representative table");
-    QMB_REQUIRE(norm2 > 0.0, QMB_ERR_INVALID, "expval: psi is zero");
-    for (size_t k = 0; k < ops.size(); ++k) out[2 * k] = out[2 * k + 1] = 0.0;
-    for (size_t i = 0; i < seg_sum.size(); ++i) {
-        out[2 * seg_op[i]] += seg_sum[i].x;
-        out[2 * seg_op[i] + 1] += seg_sum[i].y;
-    }
-    // conj(s) / <psi|psi>
-    for (size_t k = 0; k < ops.size(); ++k) {
-        out[2 * k] /= norm2;
-        out[2 * k + 1] = -out[2 * k + 1] / norm2;
-    }
 }
 
 }  // namespace
@@ -473,33 +560,29 @@ extern "C" qmb_status qmb_expval(qmb_ham h, int n_ops, const qmb_terms* ops, con
         if (n_ops == 0) return;
         DeviceGuard dg(h->device);
         const auto t0 = std::chrono::steady_clock::now();
-        // operators average independently: spread them over host threads
-        std::vector<AvgTerms> avg(n_ops);
-        const int nth = std::max(1, std::min<int>(n_ops, (int)std::min(16u, std::thread::hardware_concurrency())));
-        std::vector<std::exception_ptr> errs(nth);
-        std::atomic<int> next{0};
-        auto work = [&](int tid) {
-            try {
-                for (int k = next++; k < n_ops; k = next++) average_terms(h->sector, ops[k], avg[k]);
-            } catch (...) {
-                errs[tid] = std::current_exception();
-            }
-        };
-        std::vector<std::thread> pool;
-        for (int t = 1; t < nth; ++t) pool.emplace_back(work, t);
-        work(0);
-        for (auto& th : pool) th.join();
-        for (auto& e : errs)
-            if (e) std::rethrow_exception(e);
+        Classes cls(h->sector);
+        std::vector<std::vector<std::pair<int, cplx>>> terms(n_ops);
+        std::vector<int> last_op;
+        std::vector<size_t> last_at;
+        for (int k = 0; k < n_ops; ++k) sort_terms(ops[k], cls, last_op, last_at, k, terms[k]);
         const auto t1 = std::chrono::steady_clock::now();
-        if (h->cplx) run_expval<double2>(h, (const double2*)psi, avg, out);
-        else run_expval<double>(h, (const double*)psi, avg, out);
+        std::vector<cplx> val;
+        double norm2 = 0.0;
+        if (h->cplx) class_values<double2>(h, (const double2*)psi, cls, val, &norm2);
+        else class_values<double>(h, (const double*)psi, cls, val, &norm2);
+        QMB_REQUIRE(norm2 > 0.0, QMB_ERR_INVALID, "expval: psi is zero");
+        for (int k = 0; k < n_ops; ++k) {
+            cplx sum(0.0, 0.0);
+            for (const auto& t : terms[k]) sum += t.second * val[t.first];
+            out[2 * k] = sum.real() / norm2;  // conj(s) / <psi|psi>
+            out[2 * k + 1] = -sum.imag() / norm2;
+        }
         if (trace_on()) {
             size_t nt = 0;
-            for (const auto& a : avg) nt += a.keys.size();
+            for (int k = 0; k < n_ops; ++k) nt += (size_t)ops[k].n_terms;
             const auto t2 = std::chrono::steady_clock::now();
-            std::fprintf(stderr, "[qmb expval] %d operators, %zu averaged terms: averaging %.3f ms, kernels %.3f ms\n",
-                         n_ops, nt, std::chrono::duration<double, std::milli>(t1 - t0).count(),
+            std::fprintf(stderr, "[qmb expval] %d operators, %zu terms in %d classes: sorting %.3f ms, values %.3f ms\n",
+                         n_ops, nt, cls.n, std::chrono::duration<double, std::milli>(t1 - t0).count(),
                          std::chrono::duration<double, std::milli>(t2 - t1).count());
         }
     });
