@@ -47,8 +47,8 @@ typedef int qmb_status;
 #define QMB_ERR_NOMEM 3         /* device or host allocation failed               */
 #define QMB_ERR_ELL_OVERFLOW 4  /* a row needs more slots than the given width    */
 #define QMB_ERR_NOT_CONVERGED 5 /* Lanczos stopped at max_iter above tolerance    */
-#define QMB_ERR_TIMEOUT 6       /* reserved: no entry point of this version spins on
-                                 * the device, so none returns it                 */
+#define QMB_ERR_TIMEOUT 6       /* a wait on the device (the grid barrier of a Lanczos
+                                 * solve, a few seconds) gave up                  */
 #define QMB_ERR_UNSUPPORTED 7   /* valid request outside what this build handles  */
 #define QMB_ERR_NO_DEVICE 8     /* no CUDA device is visible                      */
 #define QMB_ERR_IO 9            /* a table file could not be opened, read or written */

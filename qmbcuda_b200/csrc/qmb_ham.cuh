@@ -185,6 +185,13 @@ __device__ __forceinline__ double2 gen_row(const RowGen& rg, const GroupSmem& gs
     return gen_row_range(rg, gs, ts, 0, ts.n_terms, src, ns, static_cast<Emit&&>(emit));
 }
 
+// An element of x: through the read-only path, or from L2 in a kernel that
+// writes the next x itself (LIVE).
+template <bool LIVE, class V>
+__device__ __forceinline__ V load_x(const V* p) {
+    return LIVE ? __ldcg(p) : __ldg(p);
+}
+
 // --------------------------------------------------------- stored operator
 // Sliced ELL: 32-row slices, slot j of row r at off[r/32] + j*32 + r%32.
 template <class M>
@@ -201,14 +208,14 @@ struct SellOp {
     void pre(const V*, const int*, cudaStream_t) const {}
     // Part p of S of (H x)_r: the slots j = p, p + S, ..., four loads of a
     // column, a value and an x element in flight; part 0 holds the diagonal.
-    template <int S, class V>
+    template <int S, bool LIVE = false, class V>
     __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
         const int64_t s = r >> 5;
         const int lane = (int)(r & 31);
         const int w = width[s];
         const uint32_t* c = col + off[s] + lane + (int64_t)p * 32;
         const M* v = val + off[s] + lane + (int64_t)p * 32;
-        V acc = p == 0 ? Sc<V>::mul(cvt<V>(diag[r]), x[r]) : Sc<V>::zero();
+        V acc = p == 0 ? Sc<V>::mul(cvt<V>(diag[r]), load_x<LIVE>(x + r)) : Sc<V>::zero();
         int j = p;
         for (; j + 3 * S < w; j += 4 * S) {
             uint32_t cc[4];
@@ -220,7 +227,7 @@ struct SellOp {
                 vv[u] = __ldg(v + u * S * 32);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) xx[u] = __ldg(x + cc[u]);
+            for (int u = 0; u < 4; ++u) xx[u] = load_x<LIVE>(x + cc[u]);
 #pragma unroll
             for (int u = 0; u < 4; ++u) acc = Sc<V>::fma(cvt<V>(vv[u]), xx[u], acc);
             c += 4 * S * 32;
@@ -237,7 +244,7 @@ struct SellOp {
             }
 #pragma unroll
         for (int u = 0; u < 3; ++u)
-            if (j + u * S < w) acc = Sc<V>::fma(cvt<V>(vv[u]), __ldg(x + cc[u]), acc);
+            if (j + u * S < w) acc = Sc<V>::fma(cvt<V>(vv[u]), load_x<LIVE>(x + cc[u]), acc);
         return acc;
     }
 };
@@ -303,7 +310,7 @@ struct CbSellOp {
     }
     // the last pass: (H x)_r from the partial sums of the earlier passes (rows
     // are not split: the layout serves matrices of millions of rows)
-    template <int S, class V>
+    template <int S, bool LIVE = false, class V>
     __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int) const {
         static_assert(S == 1, "coded rows are not split");
         const V acc = nb > 1 ? reinterpret_cast<const V*>(ytmp)[r] : Sc<V>::mul(cvt<V>(diag[r]), x[r]);
@@ -353,7 +360,7 @@ struct RefEllOp {
     void pre(const V*, const int*, cudaStream_t) const {}
     // Part p of S of (H x)_r: S neighbouring lanes read neighbouring slots of
     // the row-major table, two slots each in flight.
-    template <int S, class V>
+    template <int S, bool LIVE = false, class V>
     __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
         V acc = Sc<V>::zero();
         const int nt = track[r];
@@ -363,7 +370,7 @@ struct RefEllOp {
             const bool two = i + S < nt;
             const uint32_t c0 = __ldg(c + i), c1 = two ? __ldg(c + i + S) : 0u;
             const M v0 = __ldg(v + i), v1 = two ? __ldg(v + i + S) : Sc<M>::zero();
-            const V x0 = x[c0], x1 = two ? x[c1] : Sc<V>::zero();
+            const V x0 = load_x<LIVE>(x + c0), x1 = two ? load_x<LIVE>(x + c1) : Sc<V>::zero();
             acc = Sc<V>::fma(cvt<V>(v0), x0, acc);
             if (two) acc = Sc<V>::fma(cvt<V>(v1), x1, acc);
         }
@@ -742,7 +749,7 @@ struct MfOp {
     }
     // Part p of S of (H x)_r: the hops (or a range of the general terms) p of S;
     // with a hop table part 0 holds the diagonal.
-    template <int S, class V>
+    template <int S, bool LIVE = false, class V>
     __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
         const uint64_t rep = look.reps32 ? (uint64_t)look.reps32[r] : look.reps64[r];
         const uint64_t src = apply_elem(rg.g, gs, 0, rep);
@@ -817,49 +824,69 @@ inline void with_split(const Op& op, F&& f, bool whole = false) {
     const int S = whole ? 1 : OpSplit<Op>::of(op);
     if constexpr (OpSplit<Op>::lanes) {
         f(std::integral_constant<int, top>{});
-        return;
+    } else {
+        if constexpr (top >= 8)
+            if (S == 8) return f(std::integral_constant<int, 8>{});
+        if constexpr (top >= 4)
+            if (S == 4) return f(std::integral_constant<int, 4>{});
+        if constexpr (top >= 2)
+            if (S == 2) return f(std::integral_constant<int, 2>{});
+        f(std::integral_constant<int, 1>{});
     }
-    if constexpr (top >= 8)
-        if (S == 8) return f(std::integral_constant<int, 8>{});
-    if constexpr (top >= 4)
-        if (S == 4) return f(std::integral_constant<int, 4>{});
-    if constexpr (top >= 2)
-        if (S == 2) return f(std::integral_constant<int, 2>{});
-    f(std::integral_constant<int, 1>{});
 }
 
 // f(r, (H x)_r, x_r) for every row, by one thread of the row's S.  Every thread
 // of a block of 256 calls it.
+// The 256 / S rows from base on: f(r, (H x)_r, x_r, pre(r)) by one thread a row,
+// with x_r and pre(r) loaded ahead of the row's entries.
+template <int S, bool LIVE, class Op, class V, class Pre, class F>
+__device__ __forceinline__ void row_block(const Op& op, const V* __restrict__ x, int64_t base, V* sh, Pre&& pre, F&& f) {
+    const int64_t n = op.n;
+    if constexpr (S == 1) {
+        const int64_t r = base + threadIdx.x;
+        if (r < n) {
+            const V xr = load_x<LIVE>(x + r);
+            const auto e = pre(r);
+            f(r, op.template part<1, LIVE>(r, x, 0), xr, e);
+        }
+    } else if constexpr (OpSplit<Op>::lanes) {
+        const int p = threadIdx.x % S;
+        const int64_t r = base + threadIdx.x / S;
+        const int64_t rr = r < n ? r : n - 1;
+        const V xr = load_x<LIVE>(x + rr);
+        const auto e = pre(rr);
+        V a = r < n ? op.template part<S, LIVE>(r, x, p) : Sc<V>::zero();
+#pragma unroll
+        for (int o = S / 2; o; o >>= 1) a = Sc<V>::add(a, Sc<V>::shfl_xor(a, o));
+        if (r < n && p == 0) f(r, a, xr, e);
+    } else {
+        const int warp = threadIdx.x >> 5, p = warp % S;
+        const int64_t r = base + (warp / S) * 32 + (threadIdx.x & 31);
+        const int64_t rr = r < n ? r : n - 1;
+        const V xr = load_x<LIVE>(x + rr);
+        const auto e = pre(rr);
+        if (r < n) sh[threadIdx.x] = op.template part<S, LIVE>(r, x, p);
+        __syncthreads();
+        if (r < n && p == 0) {
+            V a = sh[threadIdx.x];
+#pragma unroll
+            for (int q = 1; q < S; ++q) a = Sc<V>::add(a, sh[threadIdx.x + 32 * q]);
+            f(r, a, xr, e);
+        }
+        __syncthreads();
+    }
+}
+
 template <int S, class Op, class V, class F>
 __device__ __forceinline__ void for_rows(const Op& op, const V* __restrict__ x, F&& f) {
     const int64_t n = op.n;
     if constexpr (S == 1) {
         for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-            f(r, op.template part<1, V>(r, x, 0), x[r]);
-    } else if constexpr (OpSplit<Op>::lanes) {
-        const int p = threadIdx.x % S;
-        for (int64_t base = blockIdx.x * (int64_t)(256 / S); base < n; base += (int64_t)gridDim.x * (256 / S)) {
-            const int64_t r = base + threadIdx.x / S;
-            V a = r < n ? op.template part<S, V>(r, x, p) : Sc<V>::zero();
-#pragma unroll
-            for (int o = S / 2; o; o >>= 1) a = Sc<V>::add(a, Sc<V>::shfl_xor(a, o));
-            if (r < n && p == 0) f(r, a, x[r]);
-        }
+            f(r, op.template part<1>(r, x, 0), x[r]);
     } else {
-        __shared__ V part[256];
-        const int warp = threadIdx.x >> 5, p = warp % S;
-        for (int64_t base = blockIdx.x * (int64_t)(256 / S); base < n; base += (int64_t)gridDim.x * (256 / S)) {
-            const int64_t r = base + (warp / S) * 32 + (threadIdx.x & 31);
-            if (r < n) part[threadIdx.x] = op.template part<S, V>(r, x, p);
-            __syncthreads();
-            if (r < n && p == 0) {
-                V a = part[threadIdx.x];
-#pragma unroll
-                for (int q = 1; q < S; ++q) a = Sc<V>::add(a, part[threadIdx.x + 32 * q]);
-                f(r, a, x[r]);
-            }
-            __syncthreads();
-        }
+        __shared__ V sh[256];
+        for (int64_t base = blockIdx.x * (int64_t)(256 / S); base < n; base += (int64_t)gridDim.x * (256 / S))
+            row_block<S, false>(op, x, base, sh, [](int64_t) { return 0; }, [&](int64_t r, V hx, V xr, int) { f(r, hx, xr); });
     }
 }
 

@@ -40,6 +40,10 @@ struct LzDev {
     double2* coefs;     // [cap + 1]
     double* cpart;      // [2 * max_blocks * (cap + 1)]
     double* scratch;    // [4]
+    // the resident kernel (k_lz_run)
+    double* wsum;       // [rows / 32] warp sums of the reorthogonalised norm
+    unsigned* chunk_ctr;  // [vector chunks]
+    struct GridBar* bar;
 };
 
 __host__ __device__ inline uint64_t splitmix64(uint64_t z) {
@@ -332,7 +336,331 @@ __global__ void __launch_bounds__(kLzBlock) k_residual(Op op, const P* __restric
     if (lb && threadIdx.x == 0) d.scratch[1] = tb;
 }
 
+// ------------------------------------------------- resident Lanczos kernel
+// Up to some 10^5 rows a step's kernels take 3 to 6 us each and their launches
+// and dependencies as much again (six of them with reorthogonalisation, whose
+// dot kernel walked the basis 16 vectors at a time in 51 blocks: 47 us a pass on
+// 12,870 rows).  k_lz_run stays on the chip for all steps up to the next
+// convergence test: one cooperative launch, with a grid barrier where a step
+// needs a sum from all blocks.  What bounds it is the chain of L2 round trips (about
+// ten a step, 9 us; five barriers and 30 us with reorthogonalisation).  Measured:
+// 150 reorthogonalised steps of 12,870 rows 10.4 -> 5.2 ms, 100 plain steps of 9,252
+// rows 1.42 -> 0.91 ms, an L=24 solve of 56,450 rows 1.45 -> 1.15 ms.
+//
+// All sums are those of the kernels above, in the same order (a row block of 256
+// threads as a block there, block partials in block order, warps' and lanes'
+// trees), so that with whole rows (S = 1) the coefficients are the same bits.
+
+// Grid barrier of a cooperative launch.  The wait is bounded: a block that
+// gives up sets err, which ends the others' waits, and the kernel returns.
+struct GridBar {
+    unsigned arrived, gen;
+    int err;
+};
+// Rows up to which the resident kernel runs the steps.  A step of 2,704, 112,720
+// and 208,012 rows takes 9.1, 17 and 22 us against 12.9, 21 and 26 with a graph of
+// two launches; beyond, the vectors leave L2 and the launches no longer count.
+constexpr int64_t kRunMaxRows = 262144;
+constexpr int kRunParts = 2048;  // row blocks at most
+constexpr unsigned kBarSpins = 1u << 23;  // polls of about 0.5 us
+
+// All threads' writes lie before a __syncthreads that thread 0 has passed.
+__device__ __forceinline__ bool grid_wait(GridBar* b, unsigned& gen) {
+    __shared__ int ok;
+    if (threadIdx.x == 0) {
+        int good = 1;
+        if (gridDim.x > 1) {
+            __threadfence();
+            if (atomicAdd(&b->arrived, 1u) == gridDim.x - 1) {
+                *(volatile unsigned*)&b->arrived = 0;
+                __threadfence();
+                *(volatile unsigned*)&b->gen = gen + 1;
+            } else {
+                for (unsigned it = 0; *(volatile unsigned*)&b->gen == gen; ++it)
+                    if (it > kBarSpins || ((it & 255u) == 255u && *(volatile int*)&b->err)) {
+                        atomicExch(&b->err, 1);
+                        good = 0;
+                        break;
+                    }
+            }
+            __threadfence();
+        }
+        ok = good;
+    }
+    __syncthreads();
+    ++gen;
+    return ok != 0;
+}
+
+// Sum over i < n of part(i) in the order of grid_reduce, to every thread: thread
+// t sums parts t, t + 256, ..., the eight warps' trees are added as block_sum
+// does.  (Every warp reading all partials for itself saves the barrier but
+// queues 8 times the reads on the same L2 lines: 12,870 rows 10 -> 16 us a step.)
+template <class F>
+__device__ __forceinline__ double sum_parts(int n, double* red8, F&& part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += kLzBlock) s += part(i);
+    if (warp * 32 < n)
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) red8[warp] = s;
+    __syncthreads();
+    return ((red8[0] + red8[4]) + (red8[2] + red8[6])) + ((red8[1] + red8[5]) + (red8[3] + red8[7]));
+}
+
+template <class V> struct ReorthShape {
+    static constexpr int chunk = 8;                         // basis vectors of one dot unit (16: 3 % slower)
+    static constexpr int lanes = 4;                         // lanes a row of the update
+    static constexpr int rows = kLzBlock / lanes;           // rows of one update unit
+    static constexpr int deep = sizeof(V) >= 16 ? 8 : 16;   // loads in flight a lane
+};
+
+template <class Op, class V, class P, int S>
+__global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring, int K, LzDev d, int steps, int reorth,
+                                                        int selective, const double* __restrict__ ritz, P* psi) {
+    __shared__ V sh[256];
+    __shared__ double red[32];
+    __shared__ double red8[3][8];
+    __shared__ double dred[2 * ReorthShape<V>::chunk * (kLzBlock / 32)];
+    __shared__ bool last;
+    extern __shared__ __align__(16) unsigned char smem_run[];
+    double2* cf = reinterpret_cast<double2*>(smem_run);  // [basis size] with reorthogonalisation
+    const int64_t n = op.n;
+    constexpr int RB = 256 / S;  // rows of a row block
+    const int n_rb = (int)((n + RB - 1) / RB);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool one = n_rb <= (int)gridDim.x;
+    double* pa = d.partials;
+    double* pb = d.partials + kRunParts;
+    unsigned gen = *(volatile unsigned*)&d.bar->gen;
+    const int j0 = *(volatile int*)d.iter;
+    double bj = __ldcg(d.beta + j0);
+    for (int j = j0; j < j0 + steps; ++j) {
+        const V* X = wbuf + (int64_t)(j & 1) * n;
+        V* Y = wbuf + (int64_t)((j + 1) & 1) * n;
+        V* Vc = vring + (int64_t)(j % K) * n;
+        const V* Vp = vring + (int64_t)((j + K - 1) % K) * n;
+        const double inv = 1.0 / bj;
+        const double c = ritz ? ritz[j] : 0.0;
+        // K1 on this block's row blocks; with one row block a block, y and v_j stay
+        // in the registers of the thread that owns the row until K2
+        int64_t own = -1;
+        V y_own = Sc<V>::zero(), v_own = Sc<V>::zero();
+        for (int rb = blockIdx.x; rb < n_rb; rb += gridDim.x) {
+            double acc = 0.0;
+            auto prev = [&](int64_t r) { return j > 0 ? __ldcg(Vp + r) : Sc<V>::zero(); };
+            row_block<S, true>(op, X, (int64_t)rb * RB, sh, prev, [&](int64_t r, V hx, V xr, V vp) {
+                const V vj = Sc<V>::scale(xr, inv);
+                V y = Sc<V>::scale(hx, inv);
+                if (j > 0) y = Sc<V>::sub(y, Sc<V>::scale(vp, bj));
+                Vc[r] = vj;
+                if (one) {
+                    own = r;
+                    y_own = y;
+                    v_own = vj;
+                } else {
+                    Y[r] = y;
+                }
+                acc += Sc<V>::re_conj_mul(vj, y);
+                if (psi) psi[r] = Sc<P>::add(psi[r], Sc<P>::scale(cvt<P>(vj), c));
+            });
+            const double t = block_sum(acc, red);
+            if (threadIdx.x == 0) pa[rb] = t;
+        }
+        if (!grid_wait(d.bar, gen)) return;
+        const double alpha = sum_parts(n_rb, red8[0], [&](int i) { return __ldcg(pa + i); });
+        if (blockIdx.x == 0 && threadIdx.x == 0) d.alpha[j] = alpha;
+        // K2 on the same rows
+        for (int rb = blockIdx.x; rb < n_rb; rb += gridDim.x) {
+            double acc = 0.0;
+            if (!one) {
+                own = threadIdx.x < RB && (int64_t)rb * RB + threadIdx.x < n ? (int64_t)rb * RB + threadIdx.x : -1;
+                if (own >= 0) {
+                    y_own = __ldcg(Y + own);
+                    v_own = __ldcg(Vc + own);
+                }
+            }
+            if (own >= 0) {
+                const V y = Sc<V>::sub(y_own, Sc<V>::scale(v_own, alpha));
+                Y[own] = y;
+                acc += Sc<V>::abs2(y);
+            }
+            const double t = block_sum(acc, red);
+            if (threadIdx.x == 0) pb[rb] = t;
+        }
+        if (!grid_wait(d.bar, gen)) return;
+        double b = sqrt(sum_parts(n_rb, red8[1], [&](int i) { return __ldcg(pb + i); }));
+        if constexpr (S == 1) {
+            using R = ReorthShape<V>;
+            const double b_pre = b;
+            const int n_ch = (j + R::chunk) / R::chunk;  // chunks of the basis v_0 .. v_j
+            for (int pass = 0; pass < reorth; ++pass) {
+                // the second pass when the first removed enough (Kahan-Parlett)
+                if (pass == 1 && selective && !(b < kReorthEta * b_pre)) break;
+                // dots: a unit is a row block x a chunk of basis vectors
+                for (int u = blockIdx.x; u < n_rb * n_ch; u += gridDim.x) {
+                    const int rb = u % n_rb, i0 = (u / n_rb) * R::chunk, cnt = min(R::chunk, j + 1 - i0);
+                    const int64_t r = (int64_t)rb * RB + threadIdx.x;
+                    double re[R::chunk], im[Sc<V>::cplx ? R::chunk : 1];
+                    const V y = r < n ? __ldcg(Y + r) : Sc<V>::zero();
+                    V v[R::chunk];
+#pragma unroll
+                    for (int k = 0; k < R::chunk; ++k)
+                        v[k] = k < cnt && r < n ? __ldcg(vring + (int64_t)(i0 + k) * n + r) : Sc<V>::zero();
+#pragma unroll
+                    for (int k = 0; k < R::chunk; ++k) {
+                        re[k] = r < n && k < cnt ? 0.0 + Sc<V>::re_conj_mul(v[k], y) : 0.0;
+                        if constexpr (Sc<V>::cplx) im[k] = r < n && k < cnt ? 0.0 + Sc<V>::im_conj_mul(v[k], y) : 0.0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < R::chunk; ++k)
+                        for (int o = 16; o > 0; o >>= 1) {
+                            re[k] += __shfl_xor_sync(0xffffffffu, re[k], o);
+                            if constexpr (Sc<V>::cplx) im[k] += __shfl_xor_sync(0xffffffffu, im[k], o);
+                        }
+                    if (lane == 0)
+#pragma unroll
+                        for (int k = 0; k < R::chunk; ++k) {
+                            dred[2 * (warp * R::chunk + k)] = re[k];
+                            dred[2 * (warp * R::chunk + k) + 1] = Sc<V>::cplx ? im[Sc<V>::cplx ? k : 0] : 0.0;
+                        }
+                    __syncthreads();
+                    if (threadIdx.x < cnt) {
+                        double bre = 0.0, bim = 0.0;
+                        for (int w = 0; w < kLzBlock / 32; ++w) {
+                            bre += dred[2 * (w * R::chunk + threadIdx.x)];
+                            bim += dred[2 * (w * R::chunk + threadIdx.x) + 1];
+                        }
+                        const int64_t at = 2 * ((int64_t)(i0 + threadIdx.x) * n_rb + rb);
+                        d.cpart[at] = bre;
+                        d.cpart[at + 1] = bim;
+                    }
+                    // the chunk's last unit adds up its coefficients
+                    __threadfence();
+                    __syncthreads();
+                    if (threadIdx.x == 0) last = atomicAdd(d.chunk_ctr + i0 / R::chunk, 1u) == (unsigned)n_rb - 1u;
+                    __syncthreads();
+                    if (last) {
+                        __threadfence();
+                        for (int i = i0 + warp; i < i0 + cnt; i += kLzBlock / 32) {
+                            double sr = 0.0, si = 0.0;
+                            for (int q = lane; q < n_rb; q += 32) {
+                                sr += __ldcg(d.cpart + 2 * ((int64_t)i * n_rb + q));
+                                si += __ldcg(d.cpart + 2 * ((int64_t)i * n_rb + q) + 1);
+                            }
+                            for (int o = 16; o > 0; o >>= 1) {
+                                sr += __shfl_xor_sync(0xffffffffu, sr, o);
+                                si += __shfl_xor_sync(0xffffffffu, si, o);
+                            }
+                            if (lane == 0) d.coefs[i] = make_double2(sr, si);
+                        }
+                        if (threadIdx.x == 0) d.chunk_ctr[i0 / R::chunk] = 0u;
+                    }
+                    __syncthreads();
+                }
+                if (!grid_wait(d.bar, gen)) return;
+                // update: four lanes a row load the basis, 64 vectors in flight,
+                // and run the same subtractions in basis order
+                for (int i = threadIdx.x; i <= j; i += blockDim.x) cf[i] = __ldcg(d.coefs + i);
+                __syncthreads();
+                const int n_u = (int)((n + R::rows - 1) / R::rows);
+                for (int u = blockIdx.x; u < n_u; u += gridDim.x) {
+                    const int q = threadIdx.x % R::lanes, row = threadIdx.x / R::lanes;
+                    const int64_t r = (int64_t)u * R::rows + row;
+                    const int64_t rr = min(r, n - 1);
+                    V y = __ldcg(Y + rr);
+                    for (int i0 = 0; i0 <= j; i0 += R::lanes * R::deep) {
+                        V v[R::deep];
+#pragma unroll
+                        for (int k = 0; k < R::deep; ++k) {
+                            const int i = i0 + k * R::lanes + q;
+                            v[k] = i <= j ? __ldcg(vring + (int64_t)i * n + rr) : Sc<V>::zero();
+                        }
+#pragma unroll
+                        for (int k = 0; k < R::deep; ++k)
+#pragma unroll
+                            for (int l = 0; l < R::lanes; ++l) {
+                                const V w = Sc<V>::shfl(v[k], l, R::lanes);
+                                const int i = i0 + k * R::lanes + l;
+                                if (i <= j) y = Sc<V>::sub(y, Sc<V>::mul(Sc<V>::from(cf[i]), w));
+                            }
+                    }
+                    if (q == 0) {
+                        if (r < n) Y[r] = y;
+                        dred[row] = r < n ? 0.0 + Sc<V>::abs2(y) : 0.0;
+                    }
+                    __syncthreads();
+                    if (warp < R::rows / 32) {
+                        double v = dred[warp * 32 + lane];
+                        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                        if (lane == 0) d.wsum[(int64_t)u * (R::rows / 32) + warp] = v;
+                    }
+                    __syncthreads();
+                }
+                if (!grid_wait(d.bar, gen)) return;
+                // norm: the row blocks' partials from their eight warps, then as above
+                const int n_w = (int)((n + 31) / 32);
+                b = sqrt(sum_parts(n_rb, red8[2], [&](int rb) {
+                    double q[8];
+#pragma unroll
+                    for (int m = 0; m < 8; ++m) q[m] = rb * 8 + m < n_w ? __ldcg(d.wsum + rb * 8 + m) : 0.0;
+                    return ((q[0] + q[4]) + (q[2] + q[6])) + ((q[1] + q[5]) + (q[3] + q[7]));
+                }));
+            }
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) d.beta[j + 1] = b;
+        bj = b;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d.iter = j0 + steps;
+}
+
 // ------------------------------------------------------------------- host
+template <class Op> struct RunsResident { static constexpr bool value = false; };
+template <class M> struct RunsResident<SellOp<M>> { static constexpr bool value = true; };
+template <class M> struct RunsResident<RefEllOp<M>> { static constexpr bool value = true; };
+template <class Op>
+inline bool runs_resident(const Op& op) {
+    // row blocks of 256 / S rows, each with its place in the two partial arrays
+    return RunsResident<Op>::value && op.n <= kRunMaxRows && (op.n * OpSplit<Op>::of(op) + 255) / 256 <= kRunParts;
+}
+
+// `steps` Lanczos steps from *d.iter in one cooperative launch.
+template <class Op, class V, class P>
+void launch_lz_run(const Op& op, V* wbuf, V* vring, int K, const LzDev& d, int steps, int cap, int reorth, int selective,
+                   const double* ritz, P* psi, cudaStream_t s) {
+    if constexpr (RunsResident<Op>::value) {
+        with_split(op, [&](auto sp) {
+            constexpr int S = decltype(sp)::value;
+            auto kern = k_lz_run<Op, V, P, S>;
+            const size_t smem = reorth ? sizeof(double2) * (size_t)(cap + 2) : 0;
+            if (smem > 0)
+                QMB_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            int dev = 0, sms = 148, per_sm = 0;
+            QMB_CUDA_TRY(cudaGetDevice(&dev));
+            QMB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            QMB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLzBlock, smem));
+            QMB_REQUIRE(per_sm >= 1, QMB_ERR_CUDA, "the resident Lanczos kernel does not fit an SM");
+            const int n_rb = (int)((op.n + 256 / S - 1) / (256 / S));
+            QMB_REQUIRE(n_rb <= kRunParts && op.n <= kRunMaxRows, QMB_ERR_INVALID, "internal: too many rows for the resident kernel");
+            // reorthogonalisation has units for more blocks than there are row blocks
+            const int want = reorth ? std::max(n_rb, std::min(8 * n_rb, 2 * sms)) : n_rb;
+            const int grid = std::min(want, std::min(per_sm, 4) * sms);
+            Op o = op;
+            LzDev dd = d;
+            void* args[] = {&o, &wbuf, &vring, &K, &dd, &steps, &reorth, &selective, &ritz, &psi};
+            QMB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kLzBlock), args, smem, s));
+        }, reorth > 0);
+    }
+}
+
+// Throws when a grid barrier gave up (after the stream was waited for).
+inline void check_run(const LzDev& d, cudaStream_t s) {
+    int err = 0;
+    QMB_CUDA_TRY(cudaMemcpyAsync(&err, &d.bar->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    QMB_CUDA_TRY(cudaStreamSynchronize(s));
+    QMB_REQUIRE(err == 0, QMB_ERR_TIMEOUT, "a grid barrier of the resident Lanczos kernel gave up");
+}
+
 // K1 and the residual with the operator's row split.
 template <class Op, class V, class P>
 void launch_lz_hv(const Op& op, size_t smem, int nb, V* wbuf, V* vring, int K, const LzDev& d, const double* ritz,
@@ -374,9 +702,10 @@ int lz_blocks() {
 struct LzState {
     int cap = 0;
     int nb = 0;
-    DevBuf<double> alpha, beta, partials, cpart, scratch;
+    DevBuf<double> alpha, beta, partials, cpart, scratch, wsum;
     DevBuf<int> iter;
-    DevBuf<unsigned> counter;
+    DevBuf<unsigned> counter, chunk_ctr;
+    DevBuf<GridBar> bar;
     DevBuf<double2> coefs;
     LzDev d{};
     void init(int cap_, int nb_, bool reorth) {
@@ -384,7 +713,12 @@ struct LzState {
         nb = nb_;
         alpha.alloc(cap + 1);
         beta.alloc(cap + 2);
-        partials.alloc(2 * (size_t)nb);
+        partials.alloc(std::max<size_t>(2 * (size_t)nb, 2 * kRunParts));
+        bar.alloc(1);
+        bar.zero();
+        wsum.alloc(reorth ? kRunMaxRows / 32 + 8 : 1);
+        chunk_ctr.alloc(reorth ? (size_t)cap / 8 + 2 : 1);
+        chunk_ctr.zero();
         scratch.alloc(4);
         scratch.zero();
         iter.alloc(1);
@@ -392,7 +726,8 @@ struct LzState {
         counter.zero();
         iter.zero();
         coefs.alloc(reorth ? cap + 2 : 1);
-        cpart.alloc(reorth ? 2 * (size_t)nb * (cap + 2) : 1);
+        // a partial a block (or, resident, a row block of 256 rows) and basis vector
+        cpart.alloc(reorth ? 2 * std::max<size_t>(nb, kRunMaxRows / 256) * (cap + 2) : 1);
         d.alpha = alpha.p;
         d.beta = beta.p;
         d.iter = iter.p;
@@ -401,9 +736,12 @@ struct LzState {
         d.coefs = coefs.p;
         d.cpart = cpart.p;
         d.scratch = scratch.p;
+        d.wsum = wsum.p;
+        d.chunk_ctr = chunk_ctr.p;
+        d.bar = bar.p;
     }
     // after the wait that ends a solve
-    void mark_idle() { qmb::mark_idle(alpha, beta, partials, cpart, scratch, iter, counter, coefs); }
+    void mark_idle() { qmb::mark_idle(alpha, beta, partials, cpart, scratch, wsum, iter, counter, chunk_ctr, bar, coefs); }
 };
 
 struct PhaseOut {
@@ -489,7 +827,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
         const size_t avail = vring.bytes->n + free_bytes();
         const int K_fit = avail > reserve ? (int)std::min<size_t>((avail - reserve) / slot, (size_t)K_full) : 0;
         K = std::min(K, K_fit);
-        if (K < 2 + every_steps) {  // not even one block of steps: regenerate instead
+        if (K < std::min(K_full, 2 + every_steps)) {  // not even one block of steps: regenerate instead
             store = false;
             K = 2;
         }
@@ -526,7 +864,9 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
 
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
+    const bool resident = runs_resident(op);
     auto capture = [&]() {
+        if (resident) return;
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         exec = nullptr;
@@ -570,11 +910,17 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
                 capture();
             }
         }
-        for (int t = 0; t < todo; ++t) {
-            if (exec) QMB_CUDA_TRY(cudaGraphLaunch(exec, s));
-            else step(s);
+        if (resident) {
+            launch_lz_run<Op, V, P>(op, wbuf.p, vring.p, K, st.d, todo, cap, po.reorth, reorth_selective() ? 1 : 0,
+                                    nullptr, nullptr, s);
+            g_lz_kernels += 1;
+        } else {
+            for (int t = 0; t < todo; ++t) {
+                if (exec) QMB_CUDA_TRY(cudaGraphLaunch(exec, s));
+                else step(s);
+            }
+            g_lz_kernels += (double)todo * (2 + 2 * po.reorth);
         }
-        g_lz_kernels += (double)todo * (2 + 2 * po.reorth);
         check_launch("lanczos step");
         done += todo;
         out.n_hv += todo;
@@ -583,6 +929,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
         QMB_CUDA_TRY(cudaMemcpyAsync(hb.data(), st.beta.p, sizeof(double) * (done + 1),
                                      cudaMemcpyDeviceToHost, s));
         QMB_CUDA_TRY(cudaStreamSynchronize(s));
+        if (resident) check_run(st.d, s);
         // a (near) zero beta ends the Krylov space: keep the steps up to it
         bool breakdown = false;
         for (int i = done - todo; i < done; ++i) {
@@ -682,8 +1029,17 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
     // regenerate v_0..v_{m-1} with the same start; kernels are deterministic
     QMB_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(P) * n, s));
     const int nb = st.nb;
-    g_lz_kernels += 2 * ph.m;  // start, m products, m - 1 updates
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, start_mode, seed, from, wbuf.p, st.d);
+    if (runs_resident(op)) {  // as the phase ran
+        launch_lz_run<Op, V, P>(op, wbuf.p, vring.p, K, st.d, ph.m, ph.m, 0, 0, ritz.p, psi, s);
+        g_lz_kernels += 2;
+        n_hv += ph.m;
+        QMB_CUDA_TRY(cudaStreamSynchronize(s));
+        check_run(st.d, s);
+        ritz.mark_idle();
+        return;
+    }
+    g_lz_kernels += 2 * ph.m;  // start, m products, m - 1 updates
     for (int j = 0; j < ph.m; ++j) {
         op.pre((const V*)wbuf.p, st.d.iter, s);
         launch_lz_hv<Op, V, P>(op, op_smem, nb, wbuf.p, vring.p, K, st.d, ritz.p, psi, s);
@@ -719,7 +1075,8 @@ bool fits_device(size_t bytes) {
 //   V32/V64: vector types of the low / high phase, Op32/Op64 the operators.
 template <class Op32, class Op64, class V32, class V64>
 void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t sm64,
-           const qmb_lanczos_opts& o, qmb_lanczos_result* res, double* coeffs, int64_t n_coeffs) {
+           const qmb_lanczos_opts& o, qmb_lanczos_result* res, double* coeffs, int64_t n_coeffs,
+           bool energy_only = false) {
     cudaStream_t s;
     QMB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
@@ -742,7 +1099,7 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
     po.check_every = o.check_every > 0 ? o.check_every : 10;
     const int cap = std::max(1, o.max_iter);
     int n_hv = 0;
-    DevBuf<unsigned char> psi_bytes(sizeof(V64) * n);
+    DevBuf<unsigned char> psi_bytes(energy_only ? 1 : sizeof(V64) * n);
     struct { V64* p; } psi{reinterpret_cast<V64*>(psi_bytes.p)};
     double theta = 0.0;
     int iters = 0;
@@ -782,7 +1139,8 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
                 p1.stall_tol = 2e-7;
             }
         }
-        bool store = o.reorth > 0 ? fits_device(sizeof(V32) * (size_t)(cap + 3) * n) : true;
+        // energy_only (FP32 mode): no Ritz vector, so no stored basis and no residual
+        bool store = o.reorth > 0 ? fits_device(sizeof(V32) * (size_t)(cap + 3) * n) : !energy_only;
         QMB_REQUIRE(o.reorth == 0 || store, QMB_ERR_NOMEM, "Krylov basis does not fit for reorthogonalisation");
         PhaseOut ph1;
         {
@@ -790,7 +1148,7 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
             int K;
             ph1 = run_phase<Op32, V32, V64>(op32, sm32, p1, o.start, o.seed, nullptr, store, vr, K, wb, st, s);
             n_hv += ph1.n_hv;
-            ritz_vector<Op32, V32, V64>(op32, sm32, ph1, o.start, o.seed, nullptr, ph1.stored, vr, K, wb,
+            if (!energy_only) ritz_vector<Op32, V32, V64>(op32, sm32, ph1, o.start, o.seed, nullptr, ph1.stored, vr, K, wb,
                                         st, psi.p, n_hv, s, o.mode == QMB_MODE_MIXED);
         }
         res->E0_low = ph1.theta;
@@ -825,8 +1183,10 @@ void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t
         }
     }
     double pn2 = 0;
-    res->residual = residual_norm<Op64, V64>(op64, sm64, psi.p, theta, st, s, &pn2);
-    ++n_hv;
+    if (!energy_only) {
+        res->residual = residual_norm<Op64, V64>(op64, sm64, psi.p, theta, st, s, &pn2);
+        ++n_hv;
+    }
     if (o.mode == QMB_MODE_MIXED && o.tol > 0) {
         // A restart whose Krylov residual estimate is far below the true FP64
         // residual has stagnated (its start vector lacked the ground state,
@@ -1033,12 +1393,15 @@ extern "C" qmb_status qmb_lanczos_ref_ell(float* E, int n_iter, int nobv, int ma
         o.check_every = o.max_iter;
         qmb_lanczos_result r;
         std::vector<double> cf(o.max_iter);
+        const bool energy_only = !(residual && check_eig_state);
         if (is_complex) {
             RefEllOp<float2> op{nobv, max_terms, ind_dev, (const float2*)val_dev, track_dev};
-            solve<RefEllOp<float2>, RefEllOp<float2>, float2, double2>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter);
+            solve<RefEllOp<float2>, RefEllOp<float2>, float2, double2>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter,
+                                                                       energy_only);
         } else {
             RefEllOp<float> op{nobv, max_terms, ind_dev, (const float*)val_dev, track_dev};
-            solve<RefEllOp<float>, RefEllOp<float>, float, double>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter);
+            solve<RefEllOp<float>, RefEllOp<float>, float, double>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter,
+                                                                   energy_only);
         }
         mark_idle(dummy.lz_ring, dummy.lz_wbuf);  // the solve ended with a wait
         *E = (float)r.E0;
@@ -1063,10 +1426,10 @@ constexpr int kNaMaxIter = 1024;        // n_iter limit
 constexpr int kNaMaxBlocks = 1024;      // reduction partials per grid
 // vectors: 2 work + 2 basis vectors in FP32 and the FP64 Ritz vector, complex
 constexpr size_t kNaVecBytes = (size_t)kNaMaxRows * (4 * sizeof(float2) + sizeof(double2));
-// scalars: alpha, beta, Ritz coefficients, partials (2 grids), scratch, step, counters
+// scalars: alpha, beta, Ritz coefficients, partials, scratch, step, counters, barrier
 constexpr size_t kNaScalarBytes = 64 * 1024;
 constexpr size_t kNaScratchBytes = kNaVecBytes + kNaScalarBytes;  // 12 MiB + 64 KiB
-static_assert(sizeof(double) * ((kNaMaxIter + 1) + (kNaMaxIter + 2) + kNaMaxIter + 2 * kNaMaxBlocks + 4) +
+static_assert(sizeof(double) * ((kNaMaxIter + 1) + (kNaMaxIter + 2) + kNaMaxIter + 2 * kRunParts + 4) +
                       64 <= kNaScalarBytes,
               "scalar region too small");
 
@@ -1114,18 +1477,24 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
     d.beta = d.alpha + (kNaMaxIter + 1);
     double* ritz = d.beta + (kNaMaxIter + 2);
     d.partials = ritz + kNaMaxIter;
-    d.scratch = d.partials + 2 * kNaMaxBlocks;
+    d.scratch = d.partials + 2 * kRunParts;
     d.iter = reinterpret_cast<int*>(d.scratch + 4);
     d.counter = reinterpret_cast<unsigned*>(d.iter + 4);
     d.coefs = nullptr;
     d.cpart = nullptr;
+    d.wsum = nullptr;
+    d.chunk_ctr = nullptr;
+    d.bar = reinterpret_cast<GridBar*>(d.counter + 4);
     const int K = 2;
+    const bool resident = runs_resident(op);
     // the reduction counters must start at zero (an interrupted earlier call
     // may have left them set)
-    QMB_CUDA_TRY(cudaMemsetAsync(d.counter, 0, 2 * sizeof(unsigned), s));
+    QMB_CUDA_TRY(cudaMemsetAsync(d.counter, 0, 4 * sizeof(unsigned) + sizeof(GridBar), s));
 
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, 1, seed, (const P*)nullptr, wbuf, d);
-    for (int j = 0; j < n_iter; ++j) {
+    if (resident)
+        launch_lz_run<RefEllOp<V>, V, P>(op, wbuf, vring, K, d, n_iter, n_iter, 0, 0, nullptr, nullptr, s);
+    for (int j = 0; j < n_iter && !resident; ++j) {
         launch_lz_hv<RefEllOp<V>, V, P>(op, 0, nb, wbuf, vring, K, d, nullptr, nullptr, s);
         k_lz_update<V><<<nb, kLzBlock, 0, s>>>(n, wbuf, vring, K, d, 1);
     }
@@ -1135,6 +1504,7 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
     QMB_CUDA_TRY(cudaMemcpyAsync(ha, d.alpha, sizeof(double) * n_iter, cudaMemcpyDeviceToHost, s));
     QMB_CUDA_TRY(cudaMemcpyAsync(hb, d.beta, sizeof(double) * (n_iter + 1), cudaMemcpyDeviceToHost, s));
     QMB_CUDA_TRY(cudaStreamSynchronize(s));
+    if (resident) check_run(d, s);
     int m = n_iter;
     for (int i = 0; i < n_iter; ++i) {
         QMB_REQUIRE(std::isfinite(ha[i]) && std::isfinite(hb[i + 1]), QMB_ERR_INVALID,
@@ -1155,7 +1525,8 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
     QMB_CUDA_TRY(cudaMemcpyAsync(ritz, sv, sizeof(double) * m, cudaMemcpyHostToDevice, s));
     QMB_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(P) * n, s));
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, 1, seed, (const P*)nullptr, wbuf, d);
-    for (int j = 0; j < m; ++j) {
+    if (resident) launch_lz_run<RefEllOp<V>, V, P>(op, wbuf, vring, K, d, m, m, 0, 0, ritz, psi, s);
+    for (int j = 0; j < m && !resident; ++j) {
         launch_lz_hv<RefEllOp<V>, V, P>(op, 0, nb, wbuf, vring, K, d, ritz, psi, s);
         if (j + 1 < m) k_lz_update<V><<<nb, kLzBlock, 0, s>>>(n, wbuf, vring, K, d, 1);
     }

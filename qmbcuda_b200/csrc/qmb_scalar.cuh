@@ -15,6 +15,7 @@ template <> struct Sc<double> {
     __host__ __device__ static double mul(double a, double b) { return a * b; }
     __host__ __device__ static double add(double a, double b) { return a + b; }
     __device__ static double shfl_xor(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+    __device__ static double shfl(double a, int l, int w) { return __shfl_sync(0xffffffffu, a, l, w); }
     __host__ __device__ static double sub(double a, double b) { return a - b; }
     __host__ __device__ static double scale(double a, double s) { return a * s; }
     __host__ __device__ static double fma(double a, double b, double c) { return ::fma(a, b, c); }
@@ -32,6 +33,7 @@ template <> struct Sc<float> {
     __host__ __device__ static float mul(float a, float b) { return a * b; }
     __host__ __device__ static float add(float a, float b) { return a + b; }
     __device__ static float shfl_xor(float a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+    __device__ static float shfl(float a, int l, int w) { return __shfl_sync(0xffffffffu, a, l, w); }
     __host__ __device__ static float sub(float a, float b) { return a - b; }
     __host__ __device__ static float scale(float a, double s) { return (float)(a * s); }
     // a float factor: the product of two floats is exact in double, so the
@@ -51,6 +53,9 @@ template <> struct Sc<double2> {
     __host__ __device__ static double2 to2(double2 v) { return v; }
     __host__ __device__ static double2 mul(double2 a, double2 b) {
         return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    }
+    __device__ static double2 shfl(double2 a, int l, int w) {
+        return make_double2(__shfl_sync(0xffffffffu, a.x, l, w), __shfl_sync(0xffffffffu, a.y, l, w));
     }
     __device__ static double2 shfl_xor(double2 a, int o) {
         return make_double2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
@@ -85,6 +90,9 @@ template <> struct Sc<float2> {
     __host__ __device__ static double2 to2(float2 v) { return make_double2(v.x, v.y); }
     __host__ __device__ static float2 mul(float2 a, float2 b) {
         return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    }
+    __device__ static float2 shfl(float2 a, int l, int w) {
+        return make_float2(__shfl_sync(0xffffffffu, a.x, l, w), __shfl_sync(0xffffffffu, a.y, l, w));
     }
     __device__ static float2 shfl_xor(float2 a, int o) {
         return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
