@@ -111,6 +111,7 @@ struct BLz {
     int* iter;
     int n_prob;
     unsigned* sec_ctr;       // [n_sectors] tiles finished in the current kernel
+    unsigned* step_ctr;      // blocks of the update that are done
     const int* sec_tile0;    // [n_sectors]
     const int* sec_ntiles;   // [n_sectors]
     double gap_cap = kRestartGapCap;  // restart gap cap relative to |theta| (with a phase-1 gap)
@@ -145,7 +146,13 @@ __device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz
 }
 
 // Batched H*v, and with `lanczos` the Lanczos step K1:
-//   y = H w_j / beta_j - beta_j v_{j-1};  v_j = w_j / beta_j;  alpha partials per (tile, set)
+//   y = H w_j / beta_j - (beta_j / beta_{j-1}) w_{j-1},  alpha_j = <w_j, y> / beta_j
+// (partials per (tile, set)).  The ring keeps the unnormalised vectors w_j: slot
+// j % K is gathered from, slot (j + 1) % K receives y, and v_j = w_j / beta_j is
+// never written.  That is one vector pass of seven less a step and one rounding
+// less (20 momenta of L = 20, 128 sets: the FP32 phase's 80 steps 20.2 -> 18.1 ms
+// with the update below).  With K = 2 y replaces w_{j-1} in place, each row read by the
+// thread that writes it.
 // Thread layout: a row is handled by TPR = nsp/SPL threads (whole warps),
 // thread t owns sets t*SPL .. t*SPL+SPL-1, so every gather of x[col] is one
 // 16-byte access per thread and a contiguous nsp-element run per row.  The
@@ -155,7 +162,7 @@ __device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz
 // keeps the gathered x resident in L2.  ctr[0] is the queue head, ctr[1]
 // counts retired blocks; the last block resets both.
 //
-// HOIST: the row's own x[r] and v_{j-1}[r] are loaded before its gathers
+// HOIST: the row's own x[r] and w_{j-1}[r] are loaded before its gathers
 // instead of after them, so they travel with the first batch of gathers
 // rather than adding a dependent round trip per row; the per-set constants of
 // the tile (couplings, beta_j, 1/beta_j) and the alpha partials live in
@@ -164,7 +171,7 @@ __device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz
 template <class V, int SPL, int UNR, int MINB, bool HOIST = false>
 __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tiles, unsigned* __restrict__ ctr,
                                                    const V* __restrict__ X0, V* __restrict__ Y0,
-                                                   V* __restrict__ vring, int K, BLz lz,
+                                                   V* ring, int K, BLz lz,
                                                    const double* __restrict__ ritz, void* psi_v,
                                                    int lanczos) {
     using M = V;
@@ -188,7 +195,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
     const M* dz = reinterpret_cast<const M*>(a.dz);
     using R = typename Sc<V>::real;
     R cx[SPL], cz[SPL];
-    __shared__ R s_cst[HOIST ? 4 * 256 : 1];  // HOIST: cx, cz, beta_j, 1/beta_j per set (nsp <= 256)
+    __shared__ R s_cst[HOIST ? 4 * 256 : 1];  // HOIST: cx, cz, beta_j/beta_{j-1}, 1/beta_j per set (nsp <= 256)
     for (;;) {
         if (threadIdx.x == 0) s_tile = (int)atomicAdd(ctr, 1u);
         __syncthreads();
@@ -206,10 +213,9 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
         }
         const int64_t nrows = a.sec_nrows[s];
         const int64_t eo = a.sec_elem[s];
-        const V* X = X0 + (lanczos ? (int64_t)(j & 1) * tot : 0) + eo;
-        V* Y = Y0 + (lanczos ? (int64_t)((j + 1) & 1) * tot : 0) + eo;
-        V* Vc = lanczos ? vring + (int64_t)(j % K) * tot + eo : nullptr;
-        const V* Vp = lanczos ? vring + (int64_t)((j + K - 1) % K) * tot + eo : nullptr;
+        const V* X = (lanczos ? ring + (int64_t)(j % K) * tot : X0) + eo;
+        V* Y = (lanczos ? ring + (int64_t)((j + 1) % K) * tot : Y0) + eo;
+        const V* Vp = lanczos ? ring + (int64_t)((j + K - 1) % K) * tot + eo : nullptr;
         const int prob0 = s * nsp + set0;
         R bj[SPL], inv[SPL];
         double apar[SPL];
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
                 const double b = lanczos ? lz.beta[(int64_t)j * lz.n_prob + s * nsp + i] : 1.0;
                 s_cst[i] = (R)a.cxy[(int64_t)s * a.c_stride + i];
                 s_cst[256 + i] = (R)a.cz[(int64_t)s * a.c_stride + i];
-                s_cst[512 + i] = (R)b;
+                s_cst[512 + i] = lanczos && j > 0 ? (R)(b / lz.beta[(int64_t)(j - 1) * lz.n_prob + s * nsp + i]) : (R)0;
                 s_cst[768 + i] = (R)(1.0 / b);
             }
 #pragma unroll
@@ -227,7 +233,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
 #pragma unroll
             for (int q = 0; q < SPL; ++q) {
                 const double b = lanczos ? lz.beta[(int64_t)j * lz.n_prob + prob0 + q] : 1.0;
-                bj[q] = (R)b;
+                bj[q] = lanczos && j > 0 ? (R)(b / lz.beta[(int64_t)(j - 1) * lz.n_prob + prob0 + q]) : (R)0;
                 inv[q] = (R)(1.0 / b);
                 apar[q] = 0.0;
             }
@@ -257,7 +263,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
 #pragma unroll
             for (int q = 0; q < SPL; ++q) acc[q] = Sc<V>::zero();
             const int p0 = s_rp[r - r0], p1 = s_rp[r - r0 + 1];
-            PK xr, vp, vo, yo;
+            PK xr, vp, yo;
             if constexpr (HOIST) {
                 xr = *reinterpret_cast<const PK*>(X + r * nsp + set0);
                 if (lanczos && j > 0) vp = *reinterpret_cast<const PK*>(Vp + r * nsp + set0);
@@ -301,28 +307,25 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
                     yo.v[q] = hx;
                     continue;
                 }
-                V vj = Sc<V>::scale(xr.v[q], invq);
                 V y = Sc<V>::scale(hx, invq);
                 if (j > 0) y = Sc<V>::sub(y, Sc<V>::scale(vp.v[q], bjq));
-                vo.v[q] = vj;
                 yo.v[q] = y;
-                if constexpr (HOIST) red[rg * nsp + set0 + q] += Sc<V>::re_conj_mul(vj, y);
-                else apar[q] += Sc<V>::re_conj_mul(vj, y);
+                if constexpr (HOIST) red[rg * nsp + set0 + q] += Sc<V>::re_conj_mul(xr.v[q], y);
+                else apar[q] += Sc<V>::re_conj_mul(xr.v[q], y);
                 const double crq = (psi_v && ritz) ? ritz[(int64_t)j * lz.n_prob + prob0 + q] : 0.0;
                 if (crq != 0.0) {
                     const int64_t e = eo + r * nsp + set0 + q;
                     if constexpr (Sc<V>::cplx) {
                         double2* p2 = reinterpret_cast<double2*>(psi_v) + e;
-                        double2 tv = cvt<double2>(vj);
+                        double2 tv = cvt<double2>(xr.v[q]);
                         p2->x += crq * tv.x;
                         p2->y += crq * tv.y;
                     } else {
-                        reinterpret_cast<double*>(psi_v)[e] += crq * (double)vj;
+                        reinterpret_cast<double*>(psi_v)[e] += crq * (double)xr.v[q];
                     }
                 }
             }
             *reinterpret_cast<PK*>(Y + r * nsp + set0) = yo;
-            if (lanczos) *reinterpret_cast<PK*>(Vc + r * nsp + set0) = vo;
         }
         if (lanczos) {
             if constexpr (!HOIST) {
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
             for (int i = threadIdx.x; i < nsp; i += blockDim.x) {
                 double tt = 0.0;
                 for (int g = 0; g < RG; ++g) tt += red[g * nsp + i];
-                lz.partials[(int64_t)tile * nsp + i] = tt;
+                lz.partials[(int64_t)tile * nsp + i] = tt / lz.beta[(int64_t)j * lz.n_prob + s * nsp + i];
             }
             sector_tail_reduce(a, lz, s, lz.alpha + (int64_t)j * lz.n_prob, false);
         } else {
@@ -351,35 +354,68 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
     }
 }
 
-// K2 (batched): w_{j+1} = y - alpha_j v_j; ||w_{j+1}||^2 partials.  One
-// block per work item, thread t = set t (coalesced [row][set] runs).
-template <class V>
-__global__ void k_bupdate(BatchArgs a, int n_tiles, V* __restrict__ W0, const V* __restrict__ vring,
-                          int K, BLz lz) {
+// K2 (batched): w_{j+1} = y - (alpha_j / beta_j) w_j; ||w_{j+1}||^2 partials, and
+// the step index advances when the last block is done.  One block per work item;
+// a row's sets are read in 16-byte slices by TPR threads, 256 / TPR rows at a time
+// with four rows of a thread in flight.
+template <class V, int SPL>
+__global__ void __launch_bounds__(kBThreads) k_bupdate(BatchArgs a, int n_tiles, V* ring, int K, BLz lz) {
+    using PK = Pack<V, SPL>;
+    __shared__ double red[kBThreads * SPL];
     const int tile = blockIdx.x;
-    const int set = threadIdx.x;
-    if (tile >= n_tiles) return;
+    const int nsp = a.nsp, TPR = nsp / SPL, RG = kBThreads / TPR;
+    const int rg = threadIdx.x / TPR, set0 = (threadIdx.x % TPR) * SPL;
     const int s = a.tile_sector[tile];
-    if (!a.active[s]) return;
-    const int nsp = a.nsp;
     const int j = *lz.iter;
-    const int64_t tot = a.sec_elem[a.n_sectors];
-    const int64_t eo = a.sec_elem[s];
-    V* Y = W0 + (int64_t)((j + 1) & 1) * tot + eo;
-    const V* Vc = vring + (int64_t)(j % K) * tot + eo;
-    if (set < nsp) {
-        const double al = lz.alpha[(int64_t)j * lz.n_prob + s * nsp + set];
-        double acc = 0.0;
-        const int64_t r_end = min(a.sec_nrows[s], (int64_t)a.tile_row0[tile] + kBTile);
-        for (int64_t r = a.tile_row0[tile]; r < r_end; ++r) {
-            const int64_t e = r * nsp + set;
-            V y = Sc<V>::sub(Y[e], Sc<V>::scale(Vc[e], al));
-            Y[e] = y;
-            acc += Sc<V>::abs2(y);
+    if (a.active[s]) {
+        const int64_t tot = a.sec_elem[a.n_sectors];
+        const int64_t eo = a.sec_elem[s];
+        V* Y = ring + (int64_t)((j + 1) % K) * tot + eo + set0;
+        const V* X = ring + (int64_t)(j % K) * tot + eo + set0;
+        double al[SPL], acc[SPL];
+#pragma unroll
+        for (int q = 0; q < SPL; ++q) {
+            const int64_t p = (int64_t)j * lz.n_prob + s * nsp + set0 + q;
+            al[q] = lz.alpha[p] / lz.beta[p];
+            acc[q] = 0.0;
         }
-        lz.partials[(int64_t)tile * nsp + set] = acc;
+        const int64_t r0 = a.tile_row0[tile], r_end = min(a.sec_nrows[s], r0 + kBTile);
+        for (int64_t r = r0 + rg; r < r_end; r += 4 * RG) {
+            PK y[4], x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (r + u * RG < r_end) {
+                    y[u] = *reinterpret_cast<const PK*>(Y + (r + u * RG) * nsp);
+                    x[u] = *reinterpret_cast<const PK*>(X + (r + u * RG) * nsp);
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (r + u * RG < r_end) {
+#pragma unroll
+                    for (int q = 0; q < SPL; ++q) {
+                        y[u].v[q] = Sc<V>::sub(y[u].v[q], Sc<V>::scale(x[u].v[q], al[q]));
+                        acc[q] += Sc<V>::abs2(y[u].v[q]);
+                    }
+                    *reinterpret_cast<PK*>(Y + (r + u * RG) * nsp) = y[u];
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < SPL; ++q) red[rg * nsp + set0 + q] = acc[q];
+        __syncthreads();
+        for (int i = threadIdx.x; i < nsp; i += kBThreads) {
+            double t = 0.0;
+            for (int g = 0; g < RG; ++g) t += red[g * nsp + i];
+            lz.partials[(int64_t)tile * nsp + i] = t;
+        }
+        sector_tail_reduce(a, lz, s, lz.beta + (int64_t)(j + 1) * lz.n_prob, true);
     }
-    sector_tail_reduce(a, lz, s, lz.beta + (int64_t)(j + 1) * lz.n_prob, true);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(lz.step_ctr, 1u) == gridDim.x - 1) {
+            *lz.step_ctr = 0u;
+            *lz.iter = j + 1;
+        }
+    }
 }
 
 // ||w0||^2 partials per (tile, set).
@@ -395,10 +431,6 @@ __global__ void k_bnorm0(BatchArgs a, int n_tiles, const V* __restrict__ W0, BLz
     const int64_t r_end = min(a.sec_nrows[s], (int64_t)a.tile_row0[tile] + kBTile);
     for (int64_t r = a.tile_row0[tile]; r < r_end; ++r) acc += Sc<V>::abs2(X[r * nsp + set]);
     lz.partials[(int64_t)tile * nsp + set] = acc;
-}
-
-__global__ void k_badvance(BLz lz) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *lz.iter += 1;
 }
 
 // Start vectors (splitmix uniform(-1,1) or a copy) and beta_0 per problem.
@@ -890,7 +922,7 @@ __device__ void add_ritz_vector(const BLz& lz, int p, int m, double th, double* 
     for (int i = 0; i < m; ++i) out[(int64_t)i * np + p] += x[(int64_t)i * np + p];
 }
 
-// Ritz coefficients of every problem: the lowest Ritz vector plus the Ritz
+// Ritz coefficients of every problem over the stored vectors w_i: the lowest Ritz vector plus the Ritz
 // vectors of up to three further Ritz values within 1e-4 |theta| of it
 // (ghost copies, within 1e-10, excluded).  A partner level that close may
 // swap order with the ground state under FP32 rounding; starting the FP64
@@ -928,6 +960,8 @@ __global__ void k_britz(BLz lz, const int* __restrict__ msteps, const double* __
             if (tk - th > 1e-4 * sc) break;
             if (tk - th > 1e-10 * sc) add_ritz_vector(lz, p, m, tk, L, D, x, ritz);
         }
+        // the stored basis is w_i = beta_i v_i
+        for (int i = 0; i < m; ++i) ritz[(int64_t)i * np + p] /= lz.beta[(int64_t)i * np + p];
     }
 }
 
@@ -986,7 +1020,7 @@ __global__ void k_bscatter_state(int n_prob_c, const int* __restrict__ slot_src,
     }
 }
 
-// psi = sum_{i < m_p} ritz[i][p] v_i over the stored basis (FP64 result).
+// psi = sum_{i < m_p} ritz[i][p] w_i over the stored basis (FP64 result).
 template <class V>
 __global__ void k_bpsi(BatchArgs a, int64_t tot, const V* __restrict__ vring, int maxm,
                        const int* __restrict__ msteps, const double* __restrict__ ritz, int n_prob,
@@ -1113,11 +1147,11 @@ struct BKind {
     std::vector<int64_t> sec_elem;     // [n_all+1]
     std::vector<int> tile_sector, tile_row0, sec_tile0, sec_ntiles;
     DevBuf<int> d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active;
-    DevBuf<unsigned> d_ctr;      // work queue head + retired blocks
+    DevBuf<unsigned> d_ctr;      // work queue head, retired blocks, update blocks done
     DevBuf<unsigned> d_sec_ctr;  // per-sector finished tiles
     int variant[2] = {-1, -1};    // tuned k_bhv variant per precision (FP32, FP64)
     int ring_hint = 0;            // Krylov ring slots the phases on this handle needed
-    DevBuf<unsigned char> ws_ring, ws_w;  // Lanczos workspace kept between solves
+    DevBuf<unsigned char> ws_ring;  // Lanczos vectors kept between solves
     std::unique_ptr<BKind> compact;        // descriptor of the last compacted sub-batch
     float tune_ms[2][8] = {};  // tuner timings per precision and variant
     DevBuf<int64_t> d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0;
@@ -1131,7 +1165,7 @@ struct BKind {
 
     void mark_idle() {
         qmb::mark_idle(d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active, d_ctr, d_sec_ctr, ws_ring,
-                       ws_w, d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0, d_col, val64, val32, dxy64, dxy32, dz64,
+                       d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0, d_col, val64, val32, dxy64, dxy32, dz64,
                        dz32);
         if (compact) compact->mark_idle();
     }
@@ -1185,7 +1219,7 @@ static BatchArgs make_args(const qmb_batch_s* b, const BKind& k) {
 
 // Kernel variants the tuner chooses from: gathers in flight per thread
 // (UNR), the register budget (MINB resident blocks per SM), whether a row's
-// own x[r] and v_{j-1}[r] loads are hoisted ahead of its gathers, and the
+// own x[r] and w_{j-1}[r] loads are hoisted ahead of its gathers, and the
 // slices per thread: one 16-byte slice of each gathered row (variants 0-2),
 // two (3-5) or four (6-7).  Wider slices mean fewer threads per row, so more
 // rows of a tile are in flight per block, and an entry's index and value
@@ -1285,13 +1319,12 @@ static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneEntry> g_tune_cache;
 
 template <class V>
-static void bupdate_any(const BatchArgs& a, const BKind& k, V* w, const V* vring, int K, BLz lz, cudaStream_t st);
+static void bupdate_any(const BatchArgs& a, V* ring, int K, BLz lz, cudaStream_t st);
 template <class V>
 static void bnorm0_any(const BatchArgs& a, const BKind& k, const V* w, BLz lz, cudaStream_t st);
 
 // The variants are timed in the form the solve runs, K1 of a Lanczos step
-// (the product with the epilogue that reads v_{j-1}, writes v_j and y and
-// sums alpha), at step 1 of a seeded start on scratch vectors; the plain
+// (the product with the epilogue that reads w_{j-1}, writes y and sums alpha), at step 1 of a seeded start on scratch vectors; the plain
 // product (qmb_batch_hv) uses the same choice.
 template <class V>
 static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st) {
@@ -1324,7 +1357,7 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     }
     const int64_t tot = k.sec_elem[k.n_sectors];
     const int n_prob = k.n_sectors * a.nsp;
-    DevBuf<V> w(2 * (size_t)tot), ring(2 * (size_t)tot);
+    DevBuf<V> ring(3 * (size_t)tot);  // so that repeating step 1 reads and writes the same slots
     DevBuf<double> alpha(4 * (size_t)n_prob), beta(5 * (size_t)n_prob),
         partials((size_t)std::max(1, k.n_tiles) * a.nsp);
     DevBuf<int> iter(1), act(k.n_sectors);
@@ -1335,14 +1368,13 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     at.n_sectors = k.n_sectors;
     at.n_tiles = k.n_tiles;
     at.active = act.p;  // every sector, whatever the caller's phase has active
-    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_sec_tile0.p, k.d_sec_ntiles.p};
-    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(at, tot, 0, 2212456ull, nullptr, w.p);
-    bnorm0_any<V>(at, k, w.p, lz, st);
+    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
+    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(at, tot, 0, 2212456ull, nullptr, ring.p);
+    bnorm0_any<V>(at, k, ring.p, lz, st);
     k_bbeta0<<<(n_prob + 255) / 256, 256, 0, st>>>(at, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
-    // one step, so that the timed launches run at step 1 (v_0 read, v_1 written)
-    bhv_variant<V>(0, at, k, w.p, w.p, ring.p, 2, lz, nullptr, nullptr, 1, st);
-    bupdate_any<V>(at, k, w.p, ring.p, 2, lz, st);
-    k_badvance<<<1, 32, 0, st>>>(lz);
+    // one step, so that the timed launches run at step 1 (w_0 and w_1 read, y written)
+    bhv_variant<V>(0, at, k, nullptr, nullptr, ring.p, 3, lz, nullptr, nullptr, 1, st);
+    bupdate_any<V>(at, ring.p, 3, lz, st);
     cudaEvent_t e0, e1;
     QMB_CUDA_TRY(cudaEventCreate(&e0));
     QMB_CUDA_TRY(cudaEventCreate(&e1));
@@ -1354,13 +1386,13 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     for (int c = 0; c < kBVariants; ++c) {
         tmin[c] = 1e30f;
         fits[c] = bhv_variant_ok<V>(c, a.nsp, spl_for<V>(a.nsp));
-        if (fits[c]) bhv_variant<V>(c, at, k, w.p, w.p, ring.p, 2, lz, nullptr, nullptr, 1, st);  // warm
+        if (fits[c]) bhv_variant<V>(c, at, k, nullptr, nullptr, ring.p, 3, lz, nullptr, nullptr, 1, st);  // warm
     }
     for (int r = 0; r < 5; ++r)
         for (int c = 0; c < kBVariants; ++c) {
             if (!fits[c]) continue;
             cudaEventRecord(e0, st);
-            bhv_variant<V>(c, at, k, w.p, w.p, ring.p, 2, lz, nullptr, nullptr, 1, st);
+            bhv_variant<V>(c, at, k, nullptr, nullptr, ring.p, 3, lz, nullptr, nullptr, 1, st);
             cudaEventRecord(e1, st);
             cudaEventSynchronize(e1);
             float ms = 0.f;
@@ -1399,11 +1431,15 @@ static void bhv_any(const BatchArgs& a, BKind& k, const V* x, V* y, V* vring, in
 }
 
 template <class V>
-static void bupdate_any(const BatchArgs& a, const BKind& k, V* w, const V* vring, int K, BLz lz,
-                        cudaStream_t st) {
-    if (k.n_tiles == 0) return;
+static void bupdate_any(const BatchArgs& a, V* ring, int K, BLz lz, cudaStream_t st) {
+    if (a.n_tiles == 0) return;
     g_kernels += 1;
-    k_bupdate<V><<<k.n_tiles, a.nsp, 0, st>>>(a, k.n_tiles, w, vring, K, lz);
+    const int spl = spl_for<V>(a.nsp);
+    if constexpr (sizeof(V) <= 4)
+        if (spl == 4) return k_bupdate<V, 4><<<a.n_tiles, kBThreads, 0, st>>>(a, a.n_tiles, ring, K, lz);
+    if constexpr (sizeof(V) <= 8)
+        if (spl == 2) return k_bupdate<V, 2><<<a.n_tiles, kBThreads, 0, st>>>(a, a.n_tiles, ring, K, lz);
+    k_bupdate<V, 1><<<a.n_tiles, kBThreads, 0, st>>>(a, a.n_tiles, ring, K, lz);
 }
 
 template <class V>
@@ -1620,7 +1656,7 @@ struct CSrc {
 // Continues the Lanczos recurrences of the unconverged problems of a phase
 // (K = 2 ring, no Ritz vector wanted) in a compacted sub-batch of 32 slots
 // per virtual sector, from step j up to step cap.  src describes the layout
-// they come from (w_j and v_{j-1} at w_src and v_src) and conv_h its
+// they come from (w_j and w_{j-1} at w_src and v_src) and conv_h its
 // convergence flags after step j.  When the unconverged problems of the
 // sub-batch again fill few enough slots, they move on into a smaller one (up
 // to kCompactDepth levels).  Results (theta, steps, flags) go back into the
@@ -1713,7 +1749,7 @@ static int run_compacted(qmb_batch_s* b, BKind& k, std::unique_ptr<BKind>& holde
     up_l(ck.d_row0, r0);
     std::vector<int> ones(nv, 1);
     up_i(ck.d_active, ones);
-    if (ck.d_ctr.n < 2) ck.d_ctr.alloc(2);
+    if (ck.d_ctr.n < 3) ck.d_ctr.alloc(3);
     ck.d_ctr.zero(st);
     if (ck.d_sec_ctr.n < (size_t)nv) ck.d_sec_ctr.alloc(nv);
     ck.d_sec_ctr.zero(st);
@@ -1743,14 +1779,14 @@ static int run_compacted(qmb_batch_s* b, BKind& k, std::unique_ptr<BKind>& holde
     ac.cz = d_cz.p;
     ac.c_stride = NC;
     ac.active = ck.d_active.p;
-    // recurrence state: w_j, v_{j-1}, alpha/beta history, test state
-    Buf<V> wc = ws_take<V>(2 * (size_t)tot_c), vc = ws_take<V>(2 * (size_t)tot_c);
+    // recurrence state: w_j, w_{j-1}, alpha/beta history, test state
+    Buf<V> wc = ws_take<V>(2 * (size_t)tot_c);  // w_j and w_{j-1}
     g_kernels += 1;
     k_bgather_vec<V><<<ck.n_tiles, 256, 0, st>>>(ac, d_slot_src.p, src.d_sec_elem, src.nsp, w_src,
                                                  wc.p + (int64_t)(j & 1) * tot_c);
     g_kernels += 1;
     k_bgather_vec<V><<<ck.n_tiles, 256, 0, st>>>(ac, d_slot_src.p, src.d_sec_elem, src.nsp, v_src,
-                                                 vc.p + (int64_t)((j + 1) & 1) * tot_c);
+                                                 wc.p + (int64_t)((j + 1) & 1) * tot_c);
     Buf<double> alpha = ws_take<double>((size_t)(cap + 1) * n_prob_c),
         beta = ws_take<double>((size_t)(cap + 2) * n_prob_c),
         partials = ws_take<double>((size_t)ck.n_tiles * NC),
@@ -1767,13 +1803,11 @@ static int run_compacted(qmb_batch_s* b, BKind& k, std::unique_ptr<BKind>& holde
         src.gap, alpha.p, beta.p, theta_prev.p, msteps.p, gap.p, conv.p);
     iter.upload(&j, 1, st);
     check_launch("compaction");
-    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob_c, ck.d_sec_ctr.p, ck.d_sec_tile0.p, ck.d_sec_ntiles.p};
+    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob_c, ck.d_sec_ctr.p, ck.d_ctr.p + 2, ck.d_sec_tile0.p, ck.d_sec_ntiles.p};
     lz.gap_cap = restart_gap_cap();
     auto step = [&](cudaStream_t ss) {
-        bhv_any<V>(ac, ck, wc.p, wc.p, vc.p, 2, lz, nullptr, nullptr, 1, ss);
-        bupdate_any<V>(ac, ck, wc.p, vc.p, 2, lz, ss);
-        g_kernels += 1;
-        k_badvance<<<1, 32, 0, ss>>>(lz);
+        bhv_any<V>(ac, ck, nullptr, nullptr, wc.p, 2, lz, nullptr, nullptr, 1, ss);
+        bupdate_any<V>(ac, wc.p, 2, lz, ss);
     };
     const double* gap_c = src.gap ? gap.p : nullptr;
     int done = j;
@@ -1813,7 +1847,7 @@ static int run_compacted(qmb_batch_s* b, BKind& k, std::unique_ptr<BKind>& holde
             conv.download(hc.data(), n_prob_c, st);
             QMB_CUDA_TRY(cudaStreamSynchronize(st));
             done = run_compacted<V>(b, k, ck.compact, f64, a_base, me, wc.p + (int64_t)(done & 1) * tot_c,
-                                    vc.p + (int64_t)((done + 1) & 1) * tot_c, done, cap, stall, res_tol, e_tol,
+                                    wc.p + (int64_t)((done + 1) & 1) * tot_c, done, cap, stall, res_tol, e_tol,
                                     check, hc, depth + 1, products, n_hv, st);
         } else if (lo.reason != 1 && done < cap) {
             std::vector<int> act(nv);
@@ -1871,9 +1905,8 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             buf.alloc(bytes);
         }
     };
-    grow(k.ws_w, 2 * (size_t)tot * sizeof(V));
     grow(k.ws_ring, (size_t)K * vec_bytes);
-    struct View { V* p; } wbuf{reinterpret_cast<V*>(k.ws_w.p)}, vring{reinterpret_cast<V*>(k.ws_ring.p)};
+    struct View { V* p; } vring{reinterpret_cast<V*>(k.ws_ring.p)};
     Buf<double> alpha = ws_take<double>((size_t)(cap + 1) * n_prob),
         beta = ws_take<double>((size_t)(cap + 2) * n_prob),
         partials = ws_take<double>((size_t)std::max(1, k.n_tiles) * b->nsp),
@@ -1903,21 +1936,19 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
     a.val = f64 ? k.val64.p : k.val32.p;
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
-    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_sec_tile0.p, k.d_sec_ntiles.p};
+    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
     lz.gap_cap = restart_gap_cap();
     const int rb = 256, rg = (n_prob + rb - 1) / rb;
     tuned_variant<V>(a, k, f64, st);
     g_kernels += 1;
-    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, wbuf.p);
-    bnorm0_any<V>(a, k, wbuf.p, lz, st);
+    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, vring.p);
+    bnorm0_any<V>(a, k, vring.p, lz, st);
     g_kernels += 1;
     k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
     check_launch("batch start");
     auto step = [&](cudaStream_t ss) {
-        bhv_any<V>(a, k, wbuf.p, wbuf.p, vring.p, K, lz, nullptr, nullptr, 1, ss);
-        bupdate_any<V>(a, k, wbuf.p, vring.p, K, lz, ss);
-        g_kernels += 1;
-        k_badvance<<<1, 32, 0, ss>>>(lz);
+        bhv_any<V>(a, k, nullptr, nullptr, vring.p, K, lz, nullptr, nullptr, 1, ss);
+        bupdate_any<V>(a, vring.p, K, lz, ss);
     };
     int done = 0;
     if (trace_on()) {
@@ -1941,7 +1972,8 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             j0 = lo.done;
             if (lo.reason != 2 || cap_run >= cap) break;
             // the ring is full: continue in one twice as large, the filled
-            // slots copied over (slot i holds v_i while no slot was reused);
+            // slots copied over (slot i holds w_i, up to the current w_{j0}, while
+            // no slot was reused);
             // without the memory the ring stays and wraps from here on
             const int K2 = std::min(K_full, 2 * K);
             DevBuf<unsigned char> grown;
@@ -1953,7 +1985,7 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
                 K_full = K;
                 continue;
             }
-            QMB_CUDA_TRY(cudaMemcpyAsync(grown.p, vring.p, (size_t)j0 * vec_bytes, cudaMemcpyDeviceToDevice, st));
+            QMB_CUDA_TRY(cudaMemcpyAsync(grown.p, vring.p, (size_t)(j0 + 1) * vec_bytes, cudaMemcpyDeviceToDevice, st));
             QMB_CUDA_TRY(cudaStreamSynchronize(st));
             k.ws_ring.swap(grown);
             grown.release();
@@ -1996,7 +2028,7 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             base.gap = gap_in;
             base.msteps = msteps.p;
             base.conv = conv.p;
-            done = run_compacted<V>(b, k, k.compact, f64, a, base, wbuf.p + (int64_t)(done & 1) * tot,
+            done = run_compacted<V>(b, k, k.compact, f64, a, base, vring.p + (int64_t)(done & 1) * tot,
                                     vring.p + (int64_t)((done + 1) & 1) * tot, done, cap, stall, res_tol, e_tol,
                                     check, hc, 0, out.products, n_hv, st);
         } else if (lo.reason != 1 && done < cap) {
@@ -2059,17 +2091,15 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             std::vector<int> all(k.n_sectors, 1);
             k.d_active.upload(all.data(), k.n_sectors, st);
             g_kernels += 1;
-            k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, wbuf.p);
-            bnorm0_any<V>(a, k, wbuf.p, lz, st);
+            k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, vring.p);
+            bnorm0_any<V>(a, k, vring.p, lz, st);
             g_kernels += 1;
             k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
             // regeneration runs every problem to the longest m; coefficients
             // beyond a problem's own m are zero (k_britz wrote m entries)
             for (int j = 0; j < done; ++j) {
-                bhv_any<V>(a, k, wbuf.p, wbuf.p, vring.p, K, lz, ritz.p, psi_out, 1, st);
-                bupdate_any<V>(a, k, wbuf.p, vring.p, K, lz, st);
-                g_kernels += 1;
-                k_badvance<<<1, 32, 0, st>>>(lz);
+                bhv_any<V>(a, k, nullptr, nullptr, vring.p, K, lz, ritz.p, psi_out, 1, st);
+                bupdate_any<V>(a, vring.p, K, lz, st);
                 ++n_hv;
                 out.products += (double)k.n_sectors * b->n_sets;
             }
@@ -2385,7 +2415,7 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             up_i(K.d_sec_ntiles, K.sec_ntiles);
             up_i(K.d_tiles, tiles);
             K.d_active.alloc(K.n_all);
-            K.d_ctr.alloc(2);
+            K.d_ctr.alloc(3);
             K.d_ctr.zero();
             K.d_sec_ctr.alloc(K.n_all);
             K.d_sec_ctr.zero();
@@ -2516,7 +2546,7 @@ static void batch_hv_kind(qmb_batch_s* b, BKind& k, bool f64, const V* x, V* y, 
     a.val = f64 ? k.val64.p : k.val32.p;
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
-    BLz lz{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr};
+    BLz lz{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr};
     int v = tuned_variant<V>(a, k, f64, st);
     // the multi-slice variants read 32- or 64-byte runs: caller vectors that
     // are only 16-byte aligned take a one-slice variant
@@ -2560,7 +2590,7 @@ static double k1_kind_ms(qmb_batch_s* b, BKind& k, bool f64, int reps, cudaStrea
     const int64_t tot = k.sec_elem[k.n_sectors];
     const int n_prob = k.n_sectors * b->nsp;
     const int cap = reps + 2;
-    DevBuf<V> w(2 * (size_t)tot), ring(2 * (size_t)tot);
+    DevBuf<V> ring(2 * (size_t)tot);
     DevBuf<double> alpha((size_t)(cap + 1) * n_prob), beta((size_t)(cap + 2) * n_prob),
         partials((size_t)k.n_tiles * b->nsp);
     DevBuf<int> iter(1);
@@ -2571,11 +2601,11 @@ static double k1_kind_ms(qmb_batch_s* b, BKind& k, bool f64, int reps, cudaStrea
     a.val = f64 ? k.val64.p : k.val32.p;
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
-    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_sec_tile0.p, k.d_sec_ntiles.p};
+    BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
     const int rb = 256, rg = (n_prob + rb - 1) / rb;
     tuned_variant<V>(a, k, f64, st);
-    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, 0, 2212456ull, nullptr, w.p);
-    bnorm0_any<V>(a, k, w.p, lz, st);
+    k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, 0, 2212456ull, nullptr, ring.p);
+    bnorm0_any<V>(a, k, ring.p, lz, st);
     k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
     std::vector<cudaEvent_t> ev(2 * (size_t)(reps + 1));
     for (auto& e : ev) QMB_CUDA_TRY(cudaEventCreate(&e));
@@ -2585,10 +2615,9 @@ static double k1_kind_ms(qmb_batch_s* b, BKind& k, bool f64, int reps, cudaStrea
     } evg{ev};
     for (int j = 0; j <= reps; ++j) {  // step 0 warms up
         QMB_CUDA_TRY(cudaEventRecord(ev[2 * j], st));
-        bhv_any<V>(a, k, w.p, w.p, ring.p, 2, lz, nullptr, nullptr, 1, st);
+        bhv_any<V>(a, k, nullptr, nullptr, ring.p, 2, lz, nullptr, nullptr, 1, st);
         QMB_CUDA_TRY(cudaEventRecord(ev[2 * j + 1], st));
-        bupdate_any<V>(a, k, w.p, ring.p, 2, lz, st);
-        k_badvance<<<1, 32, 0, st>>>(lz);
+        bupdate_any<V>(a, ring.p, 2, lz, st);
     }
     check_launch("k1 timing");
     QMB_CUDA_TRY(cudaStreamSynchronize(st));
@@ -2620,10 +2649,10 @@ extern "C" qmb_status qmb_batch_k1_time(qmb_batch b, int prec, int reps, double*
             t += k1_kind_ms<float>(b, b->kind[0], false, reps, st);
             t += k1_kind_ms<float2>(b, b->kind[1], false, reps, st);
         }
-        // the product's bytes, plus v_{j-1} read and v_j written per (row, set)
+        // the product's bytes, plus w_{j-1} read per (row, set)
         double extra = 0.0;
         for (int kd = 0; kd < 2; ++kd)
-            extra += 2.0 * (double)b->kind[kd].rows_solve * b->n_sets * (f64 ? 8.0 : 4.0) * (kd ? 2 : 1);
+            extra += (double)b->kind[kd].rows_solve * b->n_sets * (f64 ? 8.0 : 4.0) * (kd ? 2 : 1);
         *ms = t;
         *bytes = batch_bytes(b, f64, true) + extra;
     });
@@ -2741,7 +2770,7 @@ extern "C" qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const dou
                             sums = ws_take<double>(2 * (size_t)n_prob),
                             Eq = ws_take<double>(n_prob),
                             r2 = ws_take<double>(2 * (size_t)n_prob);
-                        BLz lz0{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr};
+                        BLz lz0{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr};
                         std::vector<int> ones(k.n_sectors, 1);
                         k.d_active.upload(ones.data(), k.n_sectors, st);
                         const int rb2 = 256, rg2 = (n_prob + 255) / 256;
