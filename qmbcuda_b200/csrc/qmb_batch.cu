@@ -117,13 +117,38 @@ struct BLz {
     double gap_cap = kRestartGapCap;  // restart gap cap relative to |theta| (with a phase-1 gap)
 };
 
+// Sums over the nt tiles of a sector, part[k * nsp + set] for k < nt, by a block
+// of 256 threads: f(set, sum) by one thread a set.  256 / nsp threads share a
+// set's tiles with 16 loads in flight each and are added in a fixed order.  (A
+// thread a set walking all tiles took 20 to 36 us for the 290 tiles of an L = 20
+// sector, at the end of every K1 and K2.)  sm: 256 doubles.
+template <class F>
+__device__ __forceinline__ void sum_tiles(const double* part, int nt, int nsp, double* sm, F&& f) {
+    const int G = kBThreads / nsp, g = threadIdx.x / nsp, set = threadIdx.x % nsp;
+    double t = 0.0;
+    for (int k = g; k < nt; k += 16 * G) {
+        double v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = k + u * G < nt ? __ldcg(part + (int64_t)(k + u * G) * nsp + set) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) t += v[u];
+    }
+    sm[threadIdx.x] = t;
+    __syncthreads();
+    if (g == 0) {
+        for (int q = 1; q < G; ++q) t += sm[q * nsp + set];
+        f(set, t);
+    }
+    __syncthreads();
+}
+
 // Called by every thread of a block after it wrote the partials of one tile
 // of sector s.  The block that finishes the sector's last tile sums the
-// sector's partials in tile order (deterministic) into out[s*nsp + set],
-// optionally as a square root, and resets the sector counter.  Other blocks
-// keep working on later sectors meanwhile.
-__device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz& lz, int s,
-                                                   double* __restrict__ out, bool take_sqrt) {
+// sector's partials (deterministic) into out[s*nsp + set], optionally as a
+// square root, and resets the sector counter.  Other blocks keep working on
+// later sectors meanwhile.
+__device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz& lz, int s, double* __restrict__ out,
+                                                   bool take_sqrt, double* sm) {
     __shared__ bool last;
     __threadfence();
     __syncthreads();
@@ -134,12 +159,8 @@ __device__ __forceinline__ void sector_tail_reduce(const BatchArgs& a, const BLz
     __syncthreads();
     if (last) {
         __threadfence();
-        const int nsp = a.nsp, t0 = lz.sec_tile0[s], nt = lz.sec_ntiles[s];
-        for (int set = threadIdx.x; set < nsp; set += blockDim.x) {
-            double t = 0.0;
-            for (int k = 0; k < nt; ++k) t += __ldcg(lz.partials + (int64_t)(t0 + k) * nsp + set);
-            out[(int64_t)s * nsp + set] = take_sqrt ? sqrt(t) : t;
-        }
+        sum_tiles(lz.partials + (int64_t)lz.sec_tile0[s] * a.nsp, lz.sec_ntiles[s], a.nsp, sm,
+                  [&](int set, double t) { out[(int64_t)s * a.nsp + set] = take_sqrt ? sqrt(t) : t; });
         if (threadIdx.x == 0) lz.sec_ctr[s] = 0u;
     }
     __syncthreads();
@@ -338,7 +359,7 @@ __global__ void __launch_bounds__(kBThreads, MINB) k_bhv(BatchArgs a, int n_tile
                 for (int g = 0; g < RG; ++g) tt += red[g * nsp + i];
                 lz.partials[(int64_t)tile * nsp + i] = tt / lz.beta[(int64_t)j * lz.n_prob + s * nsp + i];
             }
-            sector_tail_reduce(a, lz, s, lz.alpha + (int64_t)j * lz.n_prob, false);
+            sector_tail_reduce(a, lz, s, lz.alpha + (int64_t)j * lz.n_prob, false, red);
         } else {
             __syncthreads();
         }
@@ -407,7 +428,7 @@ __global__ void __launch_bounds__(kBThreads) k_bupdate(BatchArgs a, int n_tiles,
             for (int g = 0; g < RG; ++g) t += red[g * nsp + i];
             lz.partials[(int64_t)tile * nsp + i] = t;
         }
-        sector_tail_reduce(a, lz, s, lz.beta + (int64_t)(j + 1) * lz.n_prob, true);
+        sector_tail_reduce(a, lz, s, lz.beta + (int64_t)(j + 1) * lz.n_prob, true, red);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -463,19 +484,15 @@ __global__ void k_bdot(BatchArgs a, int n_tiles, const V* __restrict__ u, const 
     part[(nt + tile) * nsp + set] = p1;
 }
 
-// Sums the tile partials of every problem in tile order: out[k][p] for k < n_arr.
-__global__ void k_bsum(BatchArgs a, int n_tiles, const int* __restrict__ sec_tile0,
-                       const int* __restrict__ sec_ntiles, const double* __restrict__ part, int n_arr,
-                       int n_prob, double* __restrict__ out) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_prob; p += gridDim.x * blockDim.x) {
-        int s = p / a.nsp, set = p % a.nsp;
-        for (int k = 0; k < n_arr; ++k) {
-            double t = 0.0;
-            for (int i = 0; i < sec_ntiles[s]; ++i)
-                t += part[((int64_t)k * n_tiles + sec_tile0[s] + i) * a.nsp + set];
-            out[(int64_t)k * n_prob + p] = t;
-        }
-    }
+// Sums the tile partials of every problem: out[k][p], a block for sector
+// blockIdx.x of array k = blockIdx.y.
+__global__ void __launch_bounds__(kBThreads) k_bsum(BatchArgs a, int n_tiles, const int* __restrict__ sec_tile0,
+                                                    const int* __restrict__ sec_ntiles, const double* __restrict__ part,
+                                                    int n_prob, double* __restrict__ out) {
+    __shared__ double sm[kBThreads];
+    const int s = blockIdx.x, k = blockIdx.y;
+    sum_tiles(part + ((int64_t)k * n_tiles + sec_tile0[s]) * a.nsp, sec_ntiles[s], a.nsp, sm,
+              [&](int set, double t) { out[(int64_t)k * n_prob + s * a.nsp + set] = t; });
 }
 
 // Rayleigh quotient of psi (E = <psi,H psi>/<psi,psi>) from s1, s2 in out.
@@ -527,89 +544,14 @@ __global__ void k_bstart(BatchArgs a, int64_t tot, int mode, uint64_t seed, cons
     }
 }
 
-__global__ void k_bbeta0(BatchArgs a, const int* __restrict__ sec_tile0,
-                         const int* __restrict__ sec_ntiles, BLz lz) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < lz.n_prob; p += gridDim.x * blockDim.x) {
-        int s = p / a.nsp, set = p % a.nsp;
-        double t = 0.0;
-        int t0 = sec_tile0[s], nt = sec_ntiles[s];
-        for (int k = 0; k < nt; ++k) t += lz.partials[(int64_t)(t0 + k) * a.nsp + set];
-        lz.beta[p] = sqrt(t);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *lz.iter = 0;
-}
-
-// Lowest Ritz value of every problem by Sturm bisection on its tridiagonal
-// (m_p steps).  Marks converged problems and deactivates finished sectors.
-__device__ double bis_kth(const double* al, const double* be, int n_prob, int p, int m, int kth) {
-    double lo = al[p], hi = al[p];
-    for (int i = 0; i < m; ++i) {
-        double a = al[(int64_t)i * n_prob + p];
-        double r = (i > 0 ? fabs(be[(int64_t)i * n_prob + p]) : 0.0) +
-                   (i < m - 1 ? fabs(be[(int64_t)(i + 1) * n_prob + p]) : 0.0);
-        lo = fmin(lo, a - r);
-        hi = fmax(hi, a + r);
-    }
-    double span = fmax(fabs(lo), fabs(hi));
-    lo -= 1e-12 * span + 1e-300;
-    hi += 1e-12 * span + 1e-300;
-    for (int it = 0; it < 200; ++it) {
-        double x = 0.5 * (lo + hi);
-        if (x <= lo || x >= hi) break;
-        int cnt = 0;
-        double d = al[p] - x;
-        if (d < 0) ++cnt;
-        for (int i = 1; i < m; ++i) {
-            if (fabs(d) < 1e-290) d = d < 0 ? -1e-290 : 1e-290;
-            double e = be[(int64_t)i * n_prob + p];
-            d = al[(int64_t)i * n_prob + p] - x - e * e / d;
-            if (d < 0) ++cnt;
-        }
-        if (cnt >= kth + 1) hi = x;
-        else lo = x;
-        if (hi - lo <= 4.5e-16 * fmax(fabs(lo), fabs(hi))) break;
-    }
-    return 0.5 * (lo + hi);
-}
-
-__device__ double bis_min(const double* al, const double* be, int n_prob, int p, int m) {
-    return bis_kth(al, be, n_prob, p, m, 0);
-}
-
-// Last component of the unit eigenvector of T_m for eigenvalue th: inverse
-// iteration with LDL^T of T - th I (tiny pivots replaced), scratch [i][p].
-__device__ double last_ritz_component(const BLz& lz, int p, int m, double th, double* L,
-                                      double* D, double* x) {
-    const int np = lz.n_prob;
-    double scale = 0.0;
-    for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(lz.alpha[(int64_t)i * np + p] - th));
-    double tiny = 1e-15 * fmax(scale, 1e-300);
-    double d = lz.alpha[p] - th;
-    for (int i = 0; i < m; ++i) {
-        if (i > 0) {
-            double e = lz.beta[(int64_t)i * np + p];
-            double l = e / D[(int64_t)(i - 1) * np + p];
-            L[(int64_t)(i - 1) * np + p] = l;
-            d = lz.alpha[(int64_t)i * np + p] - th - l * e;
-        }
-        if (fabs(d) < tiny) d = d < 0 ? -tiny : tiny;
-        D[(int64_t)i * np + p] = d;
-    }
-    for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] = 1.0;
-    double last = 0.0;
-    for (int it = 0; it < 2; ++it) {
-        for (int i = 1; i < m; ++i)
-            x[(int64_t)i * np + p] -= L[(int64_t)(i - 1) * np + p] * x[(int64_t)(i - 1) * np + p];
-        for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] /= D[(int64_t)i * np + p];
-        for (int i = m - 2; i >= 0; --i)
-            x[(int64_t)i * np + p] -= L[(int64_t)i * np + p] * x[(int64_t)(i + 1) * np + p];
-        double nrm = 0.0;
-        for (int i = 0; i < m; ++i) nrm += x[(int64_t)i * np + p] * x[(int64_t)i * np + p];
-        nrm = sqrt(nrm);
-        for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] /= nrm;
-        last = x[(int64_t)(m - 1) * np + p];
-    }
-    return last;
+// beta_0 of every problem, a block a sector; resets the step index.
+__global__ void __launch_bounds__(kBThreads) k_bbeta0(BatchArgs a, const int* __restrict__ sec_tile0,
+                                                      const int* __restrict__ sec_ntiles, BLz lz) {
+    __shared__ double sm[kBThreads];
+    const int s = blockIdx.x;
+    sum_tiles(lz.partials + (int64_t)sec_tile0[s] * a.nsp, sec_ntiles[s], a.nsp, sm,
+              [&](int set, double t) { lz.beta[s * a.nsp + set] = sqrt(t); });
+    if (s == 0 && threadIdx.x == 0) *lz.iter = 0;
 }
 
 // Number of eigenvalues of the m x m tridiagonal (a, b) below x: sign
@@ -666,6 +608,76 @@ __device__ double warp_kth_eig(const double* a, const double* b2, int m, int k, 
     return 0.5 * (lo + hi);
 }
 
+// Unit eigenvector of T_m (a, b in shared memory) for eigenvalue th into x, by a
+// warp: inverse iteration with LDL^T of T - th I (tiny pivots replaced), two
+// solves.  The recurrences run on lane 0, divisions and norms over the lanes.
+__device__ void warp_ritz_vector(const double* a, const double* b, int m, double th, double* L, double* D, double* x) {
+    const int lane = threadIdx.x & 31;
+    double scale = 0.0;
+    for (int i = lane; i < m; i += 32) {
+        scale = fmax(scale, fabs(a[i] - th));
+        x[i] = 1.0;
+    }
+    for (int o = 16; o; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
+    const double tiny = 1e-15 * fmax(scale, 1e-300);
+    if (lane == 0) {
+        double d = a[0] - th;
+        for (int i = 0; i < m; ++i) {
+            if (i > 0) {
+                const double l = b[i] / D[i - 1];
+                L[i - 1] = l;
+                d = a[i] - th - l * b[i];
+            }
+            if (fabs(d) < tiny) d = d < 0 ? -tiny : tiny;
+            D[i] = d;
+        }
+    }
+    __syncwarp();
+    for (int it = 0; it < 2; ++it) {
+        if (lane == 0) {
+            double c = x[0];
+            for (int i = 1; i < m; ++i) {
+                c = x[i] - L[i - 1] * c;
+                x[i] = c;
+            }
+        }
+        __syncwarp();
+        for (int i = lane; i < m; i += 32) x[i] /= D[i];
+        __syncwarp();
+        if (lane == 0) {
+            double c = x[m - 1];
+            for (int i = m - 2; i >= 0; --i) {
+                c = x[i] - L[i] * c;
+                x[i] = c;
+            }
+        }
+        __syncwarp();
+        double nrm = 0.0;
+        for (int i = lane; i < m; i += 32) nrm += x[i] * x[i];
+        for (int o = 16; o; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+        nrm = sqrt(nrm);
+        for (int i = lane; i < m; i += 32) x[i] /= nrm;
+        __syncwarp();
+    }
+}
+
+// Gershgorin bracket of T_m's eigenvalues, a little widened.
+__device__ __forceinline__ void warp_bracket(const double* a, const double* b, int m, double* lo, double* hi) {
+    double glo = 1e300, ghi = -1e300;
+    for (int i = threadIdx.x & 31; i < m; i += 32) {
+        const double r = (i > 0 ? fabs(b[i]) : 0.0) + (i < m - 1 ? fabs(b[i + 1]) : 0.0);
+        glo = fmin(glo, a[i] - r);
+        ghi = fmax(ghi, a[i] + r);
+    }
+    for (int o = 16; o; o >>= 1) {
+        glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
+        ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
+    }
+    const double span = fmax(fabs(glo), fabs(ghi));
+    *lo = glo - (1e-12 * span + 1e-300);
+    *hi = ghi + (1e-12 * span + 1e-300);
+}
+
 // Lowest Ritz value of every active problem and its convergence test.  With
 // est = beta_m |s_{m-1}| (residual norm of the Ritz pair) and gap = second
 // minus lowest Ritz value (or gap_in from an earlier phase), a problem has
@@ -720,20 +732,8 @@ __global__ void k_bcheck(BatchArgs a, BLz lz, int nsets, double stall, double re
         }
         const bool brk = me < m || (me == m && !(sb[m] > 1e-13 * (fabs(sa[m - 1]) + 1e-300)));
         const bool first = msteps[p] == 0;
-        // Gershgorin bracket of T_me
-        double glo = 1e300, ghi = -1e300;
-        for (int i = lane; i < me; i += 32) {
-            const double r = (i > 0 ? fabs(sb[i]) : 0.0) + (i < me - 1 ? fabs(sb[i + 1]) : 0.0);
-            glo = fmin(glo, sa[i] - r);
-            ghi = fmax(ghi, sa[i] + r);
-        }
-        for (int o = 16; o; o >>= 1) {
-            glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
-            ghi = fmax(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
-        }
-        const double span = fmax(fabs(glo), fabs(ghi));
-        glo -= 1e-12 * span + 1e-300;
-        ghi += 1e-12 * span + 1e-300;
+        double glo, ghi;
+        warp_bracket(sa, sb, me, &glo, &ghi);
         // theta can only decrease as the Krylov space grows: try a narrow
         // bracket below the previous value first
         const double prev = theta_prev[p];
@@ -752,38 +752,8 @@ __global__ void k_bcheck(BatchArgs a, BLz lz, int nsets, double stall, double re
         bool done = brk;
         double own_gap = -1.0;
         if (!done) {
-            double est = 0.0;
-            if (lane == 0) {
-                // last component of the unit eigenvector of T_me for th:
-                // inverse iteration with LDL^T of T - th I (tiny pivots replaced)
-                double scale = 0.0;
-                for (int i = 0; i < me; ++i) scale = fmax(scale, fabs(sa[i] - th));
-                const double tiny = 1e-15 * fmax(scale, 1e-300);
-                double d = sa[0] - th;
-                for (int i = 0; i < me; ++i) {
-                    if (i > 0) {
-                        const double l = sb[i] / sD[i - 1];
-                        sL[i - 1] = l;
-                        d = sa[i] - th - l * sb[i];
-                    }
-                    if (fabs(d) < tiny) d = d < 0 ? -tiny : tiny;
-                    sD[i] = d;
-                }
-                for (int i = 0; i < me; ++i) sx[i] = 1.0;
-                double last = 0.0;
-                for (int it = 0; it < 2; ++it) {
-                    for (int i = 1; i < me; ++i) sx[i] -= sL[i - 1] * sx[i - 1];
-                    for (int i = 0; i < me; ++i) sx[i] /= sD[i];
-                    for (int i = me - 2; i >= 0; --i) sx[i] -= sL[i] * sx[i + 1];
-                    double nrm = 0.0;
-                    for (int i = 0; i < me; ++i) nrm += sx[i] * sx[i];
-                    nrm = sqrt(nrm);
-                    for (int i = 0; i < me; ++i) sx[i] /= nrm;
-                    last = sx[me - 1];
-                }
-                est = sb[me] * fabs(last);
-            }
-            est = __shfl_sync(0xffffffffu, est, 0);
+            warp_ritz_vector(sa, sb, me, th, sL, sD, sx);
+            const double est = sb[me] * fabs(sx[me - 1]);
             if (res_tol > 0 && est <= res_tol * sc) done = true;
             // the gap (to the next Ritz value that is not a ghost copy of theta)
             // only matters once the residual is small
@@ -887,81 +857,65 @@ __global__ void k_bloop_ctl(cudaGraphConditionalHandle h, int in_graph, int n_se
     }
 }
 
-// Inverse iteration on T_m - th I (LDL^T without pivoting, tiny pivots
-// replaced) for problem p; adds the unit eigenvector to out[i][p].
-__device__ void add_ritz_vector(const BLz& lz, int p, int m, double th, double* L, double* D,
-                                double* x, double* out) {
-    const int np = lz.n_prob;
-    double scale = 0.0;
-    for (int i = 0; i < m; ++i) scale = fmax(scale, fabs(lz.alpha[(int64_t)i * np + p] - th));
-    double tiny = 1e-15 * fmax(scale, 1e-300);
-    double d = lz.alpha[p] - th;
-    for (int i = 0; i < m; ++i) {
-        if (i > 0) {
-            double e = lz.beta[(int64_t)i * np + p];
-            double l = e / D[(int64_t)(i - 1) * np + p];
-            L[(int64_t)(i - 1) * np + p] = l;
-            d = lz.alpha[(int64_t)i * np + p] - th - l * e;
-        }
-        if (fabs(d) < tiny) d = d < 0 ? -tiny : tiny;
-        D[(int64_t)i * np + p] = d;
-    }
-    for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] = 1.0;
-    for (int it = 0; it < 2; ++it) {
-        for (int i = 1; i < m; ++i)
-            x[(int64_t)i * np + p] -= L[(int64_t)(i - 1) * np + p] * x[(int64_t)(i - 1) * np + p];
-        for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] /= D[(int64_t)i * np + p];
-        for (int i = m - 2; i >= 0; --i)
-            x[(int64_t)i * np + p] -= L[(int64_t)i * np + p] * x[(int64_t)(i + 1) * np + p];
-        double nrm = 0.0;
-        for (int i = 0; i < m; ++i) nrm += x[(int64_t)i * np + p] * x[(int64_t)i * np + p];
-        nrm = sqrt(nrm);
-        double sg = x[p] < 0 ? -1.0 : 1.0;
-        for (int i = 0; i < m; ++i) x[(int64_t)i * np + p] *= sg / nrm;
-    }
-    for (int i = 0; i < m; ++i) out[(int64_t)i * np + p] += x[(int64_t)i * np + p];
-}
-
-// Ritz coefficients of every problem over the stored vectors w_i: the lowest Ritz vector plus the Ritz
-// vectors of up to three further Ritz values within 1e-4 |theta| of it
-// (ghost copies, within 1e-10, excluded).  A partner level that close may
-// swap order with the ground state under FP32 rounding; starting the FP64
-// restart from the sum keeps both in its Krylov space.  Scratch arrays [i][p].
-__global__ void k_britz(BLz lz, const int* __restrict__ msteps, const double* __restrict__ theta,
-                        double* __restrict__ L, double* __restrict__ D, double* __restrict__ x,
+// Ritz coefficients of every problem over the stored vectors w_i: the lowest Ritz
+// vector plus the Ritz vectors of up to three further Ritz values within
+// 1e-4 |theta| of it (ghost copies, within 1e-10, excluded).  A partner level that
+// close may swap order with the ground state under FP32 rounding; starting the
+// FP64 restart from the sum keeps both in its Krylov space.  One warp a problem
+// with its tridiagonal in shared memory (kRitzArrays arrays of stride m_max + 2):
+// 1,408 problems of up to 80 steps take 160 us, a thread a problem with its arrays
+// in global memory took 1,050 us.
+constexpr int kRitzArrays = 7;
+__global__ void k_britz(BLz lz, int m_max, const int* __restrict__ msteps, const double* __restrict__ theta,
                         double* __restrict__ ritz, double* __restrict__ gap_out) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < lz.n_prob; p += gridDim.x * blockDim.x) {
-        const int np = lz.n_prob;
+    extern __shared__ __align__(16) unsigned char s_rz[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int stride = m_max + 2, np = lz.n_prob;
+    double* sa = reinterpret_cast<double*>(s_rz) + (size_t)wib * kRitzArrays * stride;
+    double *sb = sa + stride, *sb2 = sb + stride, *sL = sb2 + stride, *sD = sL + stride, *sx = sD + stride,
+           *so = sx + stride;
+    for (int p = blockIdx.x * wpb + wib; p < np; p += gridDim.x * wpb) {
         const int m = msteps[p];
+        if (m < 1) continue;
         const double th = theta[p];
         const double sc = fmax(fabs(th), 1e-300);
-        for (int i = 0; i < m; ++i) ritz[(int64_t)i * np + p] = 0.0;
-        add_ritz_vector(lz, p, m, th, L, D, x, ritz);
-        // Ritz values 1..4, each found by bisection at most once
-        double tks[5];
-        int known = 1;
-        auto kth_value = [&](int kth) {
-            while (known <= kth) {
-                tks[known] = bis_kth(lz.alpha, lz.beta, np, p, m, known);
-                ++known;
-            }
-            return tks[kth];
+        for (int i = lane; i < m; i += 32) {
+            sa[i] = lz.alpha[(int64_t)i * np + p];
+            const double bb = lz.beta[(int64_t)i * np + p];
+            sb[i] = bb;
+            sb2[i] = bb * bb;
+            so[i] = 0.0;
+        }
+        if (lane == 0) sb[m] = sb2[m] = 0.0;
+        __syncwarp();
+        double glo, ghi;
+        warp_bracket(sa, sb, m, &glo, &ghi);
+        auto add_vector = [&](double e) {
+            warp_ritz_vector(sa, sb, m, e, sL, sD, sx);
+            const double sg = sx[0] < 0 ? -1.0 : 1.0;
+            for (int i = lane; i < m; i += 32) so[i] += sg * sx[i];
+            __syncwarp();
         };
-        if (gap_out) {  // gap to the next Ritz value that is not a ghost copy
-            double g = 1e-10 * sc;
-            for (int kth = 1; kth < min(m, 5); ++kth) {
-                double tk = kth_value(kth);
-                if (tk - th > 1e-10 * sc) { g = tk - th; break; }
+        add_vector(th);
+        // Ritz values 1, 2, ... as far as the gap or a partner needs them
+        double gap = 1e-10 * sc;
+        bool have_gap = !gap_out;
+        for (int kth = 1; kth < min(m, 5); ++kth) {
+            const double tk = warp_kth_eig(sa, sb2, m, kth, glo, ghi, 4.5e-16, 0.0);
+            const double dist = tk - th;
+            if (!have_gap && dist > 1e-10 * sc) {
+                gap = dist;
+                have_gap = true;
             }
-            gap_out[p] = g;
+            if (dist > 1e-4 * sc || kth >= 4) {
+                if (have_gap) break;
+                continue;
+            }
+            if (kth < 4 && dist > 1e-10 * sc) add_vector(tk);
         }
-        for (int kth = 1; kth < min(m, 4); ++kth) {
-            const double tk = kth_value(kth);
-            if (tk - th > 1e-4 * sc) break;
-            if (tk - th > 1e-10 * sc) add_ritz_vector(lz, p, m, tk, L, D, x, ritz);
-        }
-        // the stored basis is w_i = beta_i v_i
-        for (int i = 0; i < m; ++i) ritz[(int64_t)i * np + p] /= lz.beta[(int64_t)i * np + p];
+        if (gap_out && lane == 0) gap_out[p] = gap;
+        for (int i = lane; i < m; i += 32) ritz[(int64_t)i * np + p] = so[i] / sb[i];  // the basis is w_i = beta_i v_i
+        __syncwarp();
     }
 }
 
@@ -1371,7 +1325,7 @@ static int tuned_variant(const BatchArgs& a, BKind& k, bool f64, cudaStream_t st
     BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
     k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(at, tot, 0, 2212456ull, nullptr, ring.p);
     bnorm0_any<V>(at, k, ring.p, lz, st);
-    k_bbeta0<<<(n_prob + 255) / 256, 256, 0, st>>>(at, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
+    k_bbeta0<<<k.n_sectors, kBThreads, 0, st>>>(at, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
     // one step, so that the timed launches run at step 1 (w_0 and w_1 read, y written)
     bhv_variant<V>(0, at, k, nullptr, nullptr, ring.p, 3, lz, nullptr, nullptr, 1, st);
     bupdate_any<V>(at, ring.p, 3, lz, st);
@@ -1912,9 +1866,7 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
         partials = ws_take<double>((size_t)std::max(1, k.n_tiles) * b->nsp),
         theta = ws_take<double>(n_prob),
         theta_prev = ws_take<double>(n_prob),
-        ritz = ws_take<double>((size_t)(cap + 1) * n_prob),
-        Ls = ws_take<double>((size_t)(cap + 1) * n_prob),
-        Ds = ws_take<double>((size_t)(cap + 1) * n_prob);
+        ritz = ws_take<double>((size_t)(cap + 1) * n_prob);
     Buf<int> iter = ws_take<int>(1),
         msteps = ws_take<int>(n_prob),
         conv = ws_take<int>(n_prob),
@@ -1938,13 +1890,12 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
     a.dz = f64 ? k.dz64.p : k.dz32.p;
     BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
     lz.gap_cap = restart_gap_cap();
-    const int rb = 256, rg = (n_prob + rb - 1) / rb;
     tuned_variant<V>(a, k, f64, st);
     g_kernels += 1;
     k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, vring.p);
     bnorm0_any<V>(a, k, vring.p, lz, st);
     g_kernels += 1;
-    k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
+    k_bbeta0<<<k.n_sectors, kBThreads, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
     check_launch("batch start");
     auto step = [&](cudaStream_t ss) {
         bhv_any<V>(a, k, nullptr, nullptr, vring.p, K, lz, nullptr, nullptr, 1, ss);
@@ -2060,7 +2011,6 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
     }
     // Ritz vectors (FP64) for the next phase or the caller
     if (psi_out) {
-        Buf<double> xs = ws_take<double>((size_t)(cap + 1) * n_prob);
         cudaEvent_t te[3] = {nullptr, nullptr, nullptr};
         if (trace_on())
             for (auto& e : te) {
@@ -2068,9 +2018,14 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             }
         if (te[0]) QMB_CUDA_TRY(cudaEventRecord(te[0], st));
         g_kernels += 1;
-        // one thread per problem, long serial loops: 32-thread blocks spread
-        // the problems over every SM (5,120 problems are 20 blocks of 256)
-        k_britz<<<(n_prob + 31) / 32, 32, 0, st>>>(lz, msteps.p, theta.p, Ls.p, Ds.p, xs.p, ritz.p, gap_out);
+        {
+            const size_t per_warp = sizeof(double) * kRitzArrays * (size_t)(done + 2);
+            const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (96u << 10) / per_warp));
+            const size_t smem = per_warp * wpb;
+            if (smem > (48u << 10))
+                QMB_CUDA_TRY(cudaFuncSetAttribute(k_britz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            k_britz<<<(n_prob + wpb - 1) / wpb, 32 * wpb, smem, st>>>(lz, done, msteps.p, theta.p, ritz.p, gap_out);
+        }
         if (te[1]) QMB_CUDA_TRY(cudaEventRecord(te[1], st));
         if (K > 2 && done < K) {
             g_kernels += 1;
@@ -2094,7 +2049,7 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, start, seed, psi_in, vring.p);
             bnorm0_any<V>(a, k, vring.p, lz, st);
             g_kernels += 1;
-            k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
+            k_bbeta0<<<k.n_sectors, kBThreads, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
             // regeneration runs every problem to the longest m; coefficients
             // beyond a problem's own m are zero (k_britz wrote m entries)
             for (int j = 0; j < done; ++j) {
@@ -2602,11 +2557,10 @@ static double k1_kind_ms(qmb_batch_s* b, BKind& k, bool f64, int reps, cudaStrea
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
     BLz lz{alpha.p, beta.p, partials.p, iter.p, n_prob, k.d_sec_ctr.p, k.d_ctr.p + 2, k.d_sec_tile0.p, k.d_sec_ntiles.p};
-    const int rb = 256, rg = (n_prob + rb - 1) / rb;
     tuned_variant<V>(a, k, f64, st);
     k_bstart<V><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, 0, 2212456ull, nullptr, ring.p);
     bnorm0_any<V>(a, k, ring.p, lz, st);
-    k_bbeta0<<<rg, rb, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
+    k_bbeta0<<<k.n_sectors, kBThreads, 0, st>>>(a, k.d_sec_tile0.p, k.d_sec_ntiles.p, lz);
     std::vector<cudaEvent_t> ev(2 * (size_t)(reps + 1));
     for (auto& e : ev) QMB_CUDA_TRY(cudaEventCreate(&e));
     struct EvG {
@@ -2786,14 +2740,14 @@ extern "C" qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const dou
                             k_bdot<double><<<k.n_tiles, b->nsp, 0, st>>>(a, k.n_tiles, (const double*)psi.p, (const double*)hy.p, nullptr, part.p);
                         }
                         g_kernels += 1;
-                        k_bsum<<<rg2, rb2, 0, st>>>(a, k.n_tiles, k.d_sec_tile0.p, k.d_sec_ntiles.p, part.p, 2, n_prob, sums.p);
+                        k_bsum<<<dim3(k.n_sectors, 2), kBThreads, 0, st>>>(a, k.n_tiles, k.d_sec_tile0.p, k.d_sec_ntiles.p, part.p, n_prob, sums.p);
                         g_kernels += 1;
                         k_brq_energy<<<rg2, rb2, 0, st>>>(n_prob, sums.p, Eq.p);
                         g_kernels += 1;
                         if (kd) k_bdot<double2><<<k.n_tiles, b->nsp, 0, st>>>(a, k.n_tiles, (const double2*)psi.p, (const double2*)hy.p, Eq.p, part.p);
                         else k_bdot<double><<<k.n_tiles, b->nsp, 0, st>>>(a, k.n_tiles, (const double*)psi.p, (const double*)hy.p, Eq.p, part.p);
                         g_kernels += 1;
-                        k_bsum<<<rg2, rb2, 0, st>>>(a, k.n_tiles, k.d_sec_tile0.p, k.d_sec_ntiles.p, part.p, 1, n_prob, r2.p);
+                        k_bsum<<<dim3(k.n_sectors, 1), kBThreads, 0, st>>>(a, k.n_tiles, k.d_sec_tile0.p, k.d_sec_ntiles.p, part.p, n_prob, r2.p);
                         act_d.zero(st);
                         g_kernels += 1;
                         k_brq_accept<<<rg2, rb2, 0, st>>>(a, n_prob, b->n_sets, Eq.p, r2.p, sums.p + n_prob, gapb.p, tol64,
