@@ -134,7 +134,11 @@ uint64_t host_binom(int n, int k);
 __host__ __device__ __forceinline__ uint64_t next_comb(uint64_t s) {
     uint64_t c = s & (~s + 1);
     uint64_t r = s + c;
+#ifdef __CUDA_ARCH__
+    return (((r ^ s) >> 2) >> (__ffsll((long long)c) - 1)) | r;  // c is a power of two
+#else
     return (((r ^ s) >> 2) / c) | r;
+#endif
 }
 
 // ----------------------------------------------------------- group elements

@@ -133,6 +133,7 @@ __device__ __forceinline__ uint32_t apply_site_map32(const GroupArgs& g, const G
     return rot32_rows(rot32_bits(s, (int)e.rr, g.L, (uint32_t)g.mask), (int)e.ri, g.W, (uint32_t)e.lo);
 }
 
+template <bool ELEM = true>
 __device__ __forceinline__ uint32_t chain_orbit_min(const GroupArgs& g, const GroupSmem& sm, uint32_t x,
                                                     int* elem);
 __device__ __forceinline__ uint64_t torus_orbit_min(const GroupArgs& g, const GroupSmem& sm, uint64_t t,
@@ -141,8 +142,11 @@ __device__ __forceinline__ uint64_t torus_orbit_min(const GroupArgs& g, const Gr
 // True iff no element maps s below s (s is its orbit's minimum).
 __device__ __forceinline__ bool is_rep(const GroupArgs& g, const GroupSmem& sm, uint64_t s) {
     if (g.full_rot) {
+        // a minimum under all rotations ends in a one and starts with a zero,
+        // unless the string is constant: three of four strings stop here
+        if (!(s & 1ull) ? s != 0ull : ((s >> (g.L - 1)) & 1ull) && s != g.mask) return false;
         int e;
-        return chain_orbit_min(g, sm, (uint32_t)s, &e) == (uint32_t)s;
+        return chain_orbit_min<false>(g, sm, (uint32_t)s, &e) == (uint32_t)s;
     }
     if (g.full_torus) {
         int e;
@@ -184,6 +188,8 @@ __device__ __forceinline__ uint32_t rotl_chain(uint32_t v, int r, int L, uint32_
     return L == 32 ? __funnelshift_l(v, v, r) : (r ? (((v << r) | (v >> (L - r))) & m) : v);
 }
 
+// Without ELEM only the minimum is formed (*elem is 0).
+template <bool ELEM>
 __device__ __forceinline__ uint32_t chain_orbit_min(const GroupArgs& g, const GroupSmem& sm, uint32_t x,
                                                     int* elem) {
     const int L = g.L;
@@ -231,6 +237,10 @@ __device__ __forceinline__ uint32_t chain_orbit_min(const GroupArgs& g, const Gr
             c &= c - 1;
             const int r = L - 1 - p;
             const uint32_t y = rotl_chain(v, r, L, m);
+            if constexpr (!ELEM) {
+                best = min(best, y);
+                continue;
+            }
             const int gi = sm.gofr[r];
             if (y < best || (y == best && (gi < bg || (gi == bg && z < bz)))) {
                 best = y;

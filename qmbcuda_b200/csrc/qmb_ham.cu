@@ -1046,6 +1046,19 @@ __global__ void k_mf_bucket(const K* __restrict__ reps, int64_t n, int shift, ui
     }
 }
 
+// The windows over the rows' 32-bit representatives (zeroed before): one bit a
+// key, the base written by a window's first row.
+__global__ void k_mf_window(const uint32_t* __restrict__ reps, int64_t n, int odd, MfWindow* __restrict__ win) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t key = reps[i] >> odd, w = key >> 6;
+        atomicOr(&win[w].bits, 1ull << (key & 63u));
+        if (i == 0 || ((reps[i - 1] >> odd) >> 6) != w) win[w].base = (uint32_t)i;
+    }
+}
+// Windows up to this size are built: 179 MB at the 32-site chain (of which the
+// populated part stays in L2); a 4x8 torus would take 1 GB.
+constexpr double kMfWindowMaxBytes = 256.0 * 1024 * 1024;
+
 // Fills the matrix-free hash table: row i under its representative.
 __global__ void k_mf_hash(const uint64_t* __restrict__ reps, int64_t n, uint64_t* __restrict__ tab, uint64_t mask,
                           int hidx) {
@@ -1078,6 +1091,20 @@ __global__ void k_mf_diag(RowGen rg, int64_t n, D* __restrict__ diag) {
     }
 }
 
+// The bucket table over the rows' representatives, where a lookup needs it.
+void mf_bucket_table(qmb_ham_s* h) {
+    if (h->mf_bucket.p) return;
+    const bool all = h->sector->n_active == h->sector->R;
+    h->mf_bucket.alloc(h->mf_nb + 1);
+    const int g = grid_for((int64_t)h->mf_nb + 1, 256);
+    if (h->mf_reps32.p)
+        k_mf_bucket<uint32_t><<<g, 256>>>(h->mf_reps32.p, h->n, h->mf_shift, h->mf_nb, h->mf_bucket.p);
+    else
+        k_mf_bucket<uint64_t><<<g, 256>>>(all ? h->sector->reps.p : h->mf_reps64.p, h->n, h->mf_shift, h->mf_nb,
+                                          h->mf_bucket.p);
+    check_launch("k_mf_bucket");
+}
+
 // The matrix-free operator's tables.  The rows' representatives in row
 // order (32-bit up to 32 sites; beyond, the sector's table when every orbit
 // is active), the bucket table over them on the top 24 bits of the largest
@@ -1102,12 +1129,28 @@ void mf_tables(qmb_ham_s* h) {
     while (bits < 64 && (top >> bits)) ++bits;
     h->mf_shift = std::max(0, bits - 24);
     h->mf_nb = (top >> h->mf_shift) + 1;
-    h->mf_bucket.alloc(h->mf_nb + 1);
-    const int g = grid_for((int64_t)h->mf_nb + 1, 256);
-    if (r32) k_mf_bucket<uint32_t><<<g, 256>>>(h->mf_reps32.p, n, h->mf_shift, h->mf_nb, h->mf_bucket.p);
-    else k_mf_bucket<uint64_t><<<g, 256>>>(all ? s->reps.p : h->mf_reps64.p, n, h->mf_shift, h->mf_nb,
-                                              h->mf_bucket.p);
-    check_launch("k_mf_bucket");
+    h->mf_trivial = 1;
+    for (const auto& c : s->chars)
+        if (c != std::complex<double>(1.0, 0.0)) h->mf_trivial = 0;
+    if (r32) {
+        // minima under all rotations of a chain end in a one (unless there is none)
+        const int odd = s->full_rot && s->n_up > 0 ? 1 : 0;
+        const uint64_t n_win = (top >> odd >> 6) + 1;
+        const size_t bytes = n_win * sizeof(MfWindow);
+        size_t fr = 0, tot = 0;
+        if (bytes > ((size_t)64 << 20)) dev_mem_info(&fr, &tot);
+        const char* we = std::getenv("QMB_MF_WINDOW");  // 0: the bucket search (tests)
+        if ((double)bytes <= kMfWindowMaxBytes && (bytes <= ((size_t)64 << 20) || bytes <= fr / 4) &&
+            !(we && we[0] == '0')) {
+            h->mf_win.alloc(n_win);
+            QMB_CUDA_TRY(cudaMemset(h->mf_win.p, 0, bytes));
+            k_mf_window<<<grid_for(n, 256), 256>>>(h->mf_reps32.p, n, odd, h->mf_win.p);
+            check_launch("k_mf_window");
+            h->mf_nwin = (uint32_t)n_win;
+            h->mf_odd = odd;
+        }
+    }
+    if (!h->mf_nwin) mf_bucket_table(h);
     // beyond 32 sites with a representative table well beyond L2: the hash
     // table, when a representative and a row index fit one word (top bit 0);
     // QMB_MF_HASH=1 builds it at any size (tests)
@@ -1280,10 +1323,15 @@ void hv_dispatch(const qmb_ham_s* h, int prec, const void* x, void* y, cudaStrea
         // QMB_MF_LOOKUP=warp: the warp-cooperative lookup over the bucket table
         const char* le = std::getenv("QMB_MF_LOOKUP");
         if (le && std::strcmp(le, "warp") == 0 && h->n_hops) {
+            if (!h->mf_bucket.p) {
+                mf_bucket_table(const_cast<qmb_ham_s*>(h));  // (the caller's handle, in use by this thread alone)
+                QMB_CUDA_TRY(cudaDeviceSynchronize());
+            }
             auto run = [&](auto op, auto* xv, auto* yv) {
                 using V = std::remove_const_t<std::remove_pointer_t<decltype(xv)>>;
                 using MT = typename decltype(op)::scalar;
                 op.look.hash = nullptr;
+                op.look.bucket = h->mf_bucket.p;
                 const size_t sm = op.smem_bytes();
                 set_group_smem_attr((const void*)k_hv_mfw<MT, V>, sm);
                 op.pre(xv, (const int*)nullptr, st);

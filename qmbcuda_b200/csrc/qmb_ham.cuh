@@ -392,7 +392,19 @@ __host__ __device__ __forceinline__ uint64_t mf_hash_slot(uint64_t r, uint64_t m
 }
 constexpr uint64_t kMfHashEmpty = ~0ull;
 
+// Up to 32 sites: 64 consecutive keys (representatives, or their halves when all
+// are odd, as the minima of a rotation group are) as one bit each, and the row of
+// the first.  A lookup is one 16-byte load and a population count; the bucket
+// table and its binary search took about six dependent loads.
+struct __align__(16) MfWindow {
+    unsigned long long bits;
+    uint32_t base, pad;
+};
+
 struct ActiveLookup {
+    const MfWindow* win;     // [n_win] or null
+    uint32_t n_win;
+    int odd;                 // 1: keys are r >> 1
     const uint32_t* reps32;  // [n] or null
     const uint64_t* reps64;  // [n] when reps32 is null
     const uint32_t* bucket;  // [n_b + 1]: rows of bucket b (top bits r >> shift == b)
@@ -408,7 +420,27 @@ struct ActiveLookup {
     const uint64_t* hash;    // [hmask + 1] or null
     uint64_t hmask;
     int hidx;                // bits of the row index in a word
+    // row of r through the windows; false when r is no representative of a row
+    __device__ __forceinline__ bool window(uint32_t r, uint32_t* row) const {
+        const uint32_t key = r >> odd, w = key >> 6;
+        if (w >= n_win || (r & (uint32_t)odd) != (uint32_t)odd) return false;
+        const uint4 e = __ldg(reinterpret_cast<const uint4*>(win) + w);
+        const unsigned long long bits = ((unsigned long long)e.y << 32) | e.x;
+        const int k = (int)(key & 63u);
+        *row = e.z + (uint32_t)__popcll(bits & ((1ull << k) - 1ull));
+        return (bits >> k) & 1ull;
+    }
     __device__ __forceinline__ int find(const RowGen& rg, uint64_t r, int64_t* idx, double* f) const {
+        if (win) {
+            uint32_t row;
+            if (window((uint32_t)r, &row)) {
+                *idx = row;
+                *f = 1.0;
+                return 1;
+            }
+            if (all_active) return -1;
+            return find_rep(rg.rt, r) < 0 ? -1 : 0;  // a null orbit, or outside the sector
+        }
         if (hash) {
             uint64_t slot = mf_hash_slot(r, hmask);
             for (uint64_t it = 0; it <= hmask; ++it) {
@@ -505,6 +537,12 @@ struct ActiveLookup {
     // lockstep, so each step has two independent loads in flight
     __device__ __forceinline__ void find32x2(const RowGen& rg, uint32_t r1, uint32_t r2, uint32_t* i1,
                                              uint32_t* i2, int* f1, int* f2) const {
+        if (win) {
+            const bool h1 = window(r1, i1), h2 = window(r2, i2);
+            *f1 = h1 ? 1 : (all_active ? -1 : (find_rep(rg.rt, r1) < 0 ? -1 : 0));
+            *f2 = h2 ? 1 : (all_active ? -1 : (find_rep(rg.rt, r2) < 0 ? -1 : 0));
+            return;
+        }
         const uint32_t b1 = r1 >> shift, b2 = r2 >> shift;
         uint32_t lo1 = 0, hi1 = 0, lo2 = 0, hi2 = 0;
         if (b1 < (uint32_t)n_b) {
@@ -580,6 +618,7 @@ struct MfOp {
     void* xs;            // [n] scaled x in the product's vector type
     int n_hops;
     int hop_one_way;     // some hop has a zero coefficient in one direction
+    int trivial;         // every character is 1: an entry's element is not needed
     const Hop* hops;     // [n_hops]
     const double2* hop_c;  // [2 n_hops]: coefficient for bit i = 0, bit j = 1; then the reverse
     const void* diag;    // [n] the diagonal (double2 for complex handles, else double)
@@ -665,12 +704,16 @@ struct MfOp {
                 const uint32_t p1 = s_pair32[b1], p2 = s_pair32[b2];
                 const double2 cf1 = s_hop_c[2 * b1 + ((src & p1 & (0u - p1)) ? 1 : 0)];
                 const double2 cf2 = s_hop_c[2 * b2 + ((src & p2 & (0u - p2)) ? 1 : 0)];
-                int e1, e2;
+                int e1 = 0, e2 = 0;
                 const uint32_t t1 = src ^ p1, t2 = src ^ p2;
-                const uint32_t r1 = rg.g.full_rot ? chain_orbit_min(rg.g, gs, t1, &e1)
-                                                  : (uint32_t)orbit_min(rg.g, gs, t1, &e1);
-                const uint32_t r2 = rg.g.full_rot ? chain_orbit_min(rg.g, gs, t2, &e2)
-                                                  : (uint32_t)orbit_min(rg.g, gs, t2, &e2);
+                uint32_t r1, r2;
+                if (rg.g.full_rot && trivial) {
+                    r1 = chain_orbit_min<false>(rg.g, gs, t1, &e1);
+                    r2 = chain_orbit_min<false>(rg.g, gs, t2, &e2);
+                } else {
+                    r1 = rg.g.full_rot ? chain_orbit_min(rg.g, gs, t1, &e1) : (uint32_t)orbit_min(rg.g, gs, t1, &e1);
+                    r2 = rg.g.full_rot ? chain_orbit_min(rg.g, gs, t2, &e2) : (uint32_t)orbit_min(rg.g, gs, t2, &e2);
+                }
                 uint32_t c1, c2;
                 int f1, f2;
                 look.find32x2(rg, r1, r2, &c1, &c2, &f1, &f2);
@@ -683,12 +726,12 @@ struct MfOp {
                 const V x1 = u1 ? __ldg(xsv + c1) : Sc<V>::zero();
                 const V x2 = u2 ? __ldg(xsv + c2) : Sc<V>::zero();
                 if (u1) {
-                    const double2 ch = rg.g.chars[e1];
+                    const double2 ch = trivial ? make_double2(1.0, 0.0) : rg.g.chars[e1];
                     acc = Sc<V>::fma(Sc<V>::from(make_double2(cf1.x * ch.x + cf1.y * ch.y, cf1.y * ch.x - cf1.x * ch.y)),
                                      x1, acc);
                 }
                 if (u2) {
-                    const double2 ch = rg.g.chars[e2];
+                    const double2 ch = trivial ? make_double2(1.0, 0.0) : rg.g.chars[e2];
                     acc = Sc<V>::fma(Sc<V>::from(make_double2(cf2.x * ch.x + cf2.y * ch.y, cf2.y * ch.x - cf2.x * ch.y)),
                                      x2, acc);
                 }
@@ -945,6 +988,10 @@ struct qmb_ham_s {
     qmb::DevBuf<uint32_t> mf_reps32;   // [n] active representatives, L <= 32
     qmb::DevBuf<uint64_t> mf_reps64;   // [n] L > 32 with null orbits (else the sector's table)
     qmb::DevBuf<uint32_t> mf_bucket;   // [mf_nb + 1]
+    qmb::DevBuf<qmb::MfWindow> mf_win; // up to 32 sites, where it is small enough
+    uint32_t mf_nwin = 0;
+    int mf_odd = 0;
+    int mf_trivial = 0;                // every character of the irrep is 1
     qmb::DevBuf<uint64_t> mf_hash;     // rows by representative, beyond 32 sites when the table exceeds L2
     uint64_t mf_hmask = 0;
     int mf_hidx = 0;
@@ -965,7 +1012,7 @@ struct qmb_ham_s {
         if (!err.p) return;
         err.release();
         qmb::mark_idle(slice_off, slice_w, col, val64, val32, diag64, diag32, t_nops, t_ops, t_scalar, hops, hop_c,
-                       mf_reps32, mf_reps64, mf_bucket, mf_hash, mf_norm, mf_diag, mf_xs, lz_ring, lz_wbuf, psi);
+                       mf_reps32, mf_reps64, mf_bucket, mf_win, mf_hash, mf_norm, mf_diag, mf_xs, lz_ring, lz_wbuf, psi);
         for (qmb::CbLayout* L : {&cb32, &cb64}) qmb::mark_idle(L->off, L->width, L->packed, L->dict, L->ytmp);
     }
 
@@ -1024,6 +1071,10 @@ struct qmb_ham_s {
         qmb::MfOp<M> op;
         op.n = n;
         op.rg = row_gen();
+        op.look.win = mf_win.p;
+        op.look.n_win = mf_nwin;
+        op.look.odd = mf_odd;
+        op.trivial = mf_trivial;
         op.look.reps32 = mf_reps32.p;
         op.look.reps64 = mf_reps32.p ? nullptr : (mf_reps64.p ? mf_reps64.p : sector->reps.p);
         op.look.bucket = mf_bucket.p;
