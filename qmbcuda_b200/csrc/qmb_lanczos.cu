@@ -1278,11 +1278,12 @@ extern "C" qmb_status qmb_lanczos(qmb_ham h, const qmb_lanczos_opts* opts, qmb_l
                 solve<A, B, R, D>(h, a, sa, b, sb, o, res, krylov_coeffs, n_coeffs);
             };
             auto op32 = [&](auto&& k) {
-                if (h->cb32.nb > 0) k(h->cb<R>(), CbSellOp<R>::smem_bytes());
+                // (up to kRunMaxRows the resident kernel with the plain entries is faster)
+                if (h->cb32.nb > 0 && (h->cb32.nb > 1 || h->n > kRunMaxRows)) k(h->cb<R>(), CbSellOp<R>::smem_bytes());
                 else k(h->sell<R>(false), (size_t)0);
             };
             auto op64 = [&](auto&& k) {
-                if (h->cb64.nb > 0) {
+                if (h->cb64.nb > 0 && (h->cb64.nb > 1 || h->n > kRunMaxRows)) {
                     k(h->cb<D>(), CbSellOp<D>::smem_bytes());
                     return;
                 }
