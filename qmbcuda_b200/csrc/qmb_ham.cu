@@ -232,7 +232,17 @@ __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off
 constexpr int kPackMaxTerms = 1024;  // mobile terms (7 bytes of shared memory a warp each)
 constexpr int kPackWarps = 4;        // warps a block
 
+// A term whose operators sit on distinct sites, as word operations: it applies to
+// strings with (src & care) == val, its image is src ^ flip and its coefficient sc
+// times (-1)^(down spins among zmask), powers of 1/2 included (the same bits as
+// the operators applied one by one).
+struct __align__(16) QuickTerm {
+    unsigned long long care, val, flip, zmask;
+    double2 sc;
+};
+
 struct PackArgs {
+    const QuickTerm* quick;  // [n_terms], or null when a term meets a site twice
     const int16_t* midx;  // [n_terms] position among the mobile terms, or -1
     const uint16_t* mob;  // [n_mob] their term indices
     int n_mob;
@@ -262,7 +272,18 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_ell_masks(RowGen rg, PackAr
         for (int hi = 0; hi < ts.n_terms; ++hi) {
             uint64_t t = src;
             double2 coef;
-            const bool some = act && apply_term(ts, hi, src, &t, &coef);
+            bool some;
+            if (pk.quick) {
+                const QuickTerm& q = pk.quick[hi];
+                some = act && (src & q.care) == q.val;
+                t = src ^ q.flip;
+                if (q.flip == 0) {
+                    const double f = (__popcll(~src & q.zmask) & 1) ? -1.0 : 1.0;
+                    coef = make_double2(f * q.sc.x, f * q.sc.y);
+                }
+            } else {
+                some = act && apply_term(ts, hi, src, &t, &coef);
+            }
             bool live = some && t != src;
             if (some && !live) {
                 d.x += coef.x;
@@ -375,13 +396,29 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_ell_pack(RowGen rg, PackArg
                     }
                 }
                 ++j;
-                gen_row_range(rg, gs, ts, hi, hi + 1, src, ns, [&](int64_t ot, double2 v) {
+                auto put = [&](int64_t ot, double2 v) {
                     const int64_t p = base + (int64_t)at * 32;
-                    col[p] = (uint32_t)rg.row_of_orbit[ot];
+                    col[p] = (uint32_t)(pk.exact ? ot : rg.row_of_orbit[ot]);  // (all active: orbits are rows)
                     const M64 v64 = Sc<M64>::from(v);
                     if (val64) val64[p] = v64;
                     if (val32) val32[p] = cvt<M32>(v64);
-                });
+                };
+                if (pk.quick) {
+                    // gen_row_range() of one term, without walking its operators
+                    const QuickTerm& q = pk.quick[hi];
+                    int e;
+                    const int64_t ot = find_rep(rg.rt, orbit_min(rg.g, gs, src ^ q.flip, &e));
+                    if (ot < 0) {
+                        *rg.err = 2;
+                        continue;
+                    }
+                    const double sg = (__popcll(~src & q.zmask) & 1) ? -1.0 : 1.0;
+                    const double2 cf = make_double2(sg * q.sc.x, sg * q.sc.y), ch = rg.g.chars[e];
+                    const double f = rg.norms[ot] / ns;
+                    put(ot, make_double2((cf.x * ch.x + cf.y * ch.y) * f, (cf.y * ch.x - cf.x * ch.y) * f));
+                } else {
+                    gen_row_range(rg, gs, ts, hi, hi + 1, src, ns, put);
+                }
             }
             if (!place)
                 for (; j < w; ++j) {
@@ -509,7 +546,33 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
         dev_mem_info(&fr, &tot);
         packed = mask_bytes <= fr / 8;
     }
-    PackArgs pk{nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0,
+    // word forms of the terms
+    std::vector<QuickTerm> quick(std::max(1, t->n_terms));
+    bool all_quick = t->n_terms > 0;
+    for (int i = 0; i < t->n_terms && all_quick; ++i) {
+        QuickTerm q{};
+        double f = 1.0;
+        uint64_t seen = 0;
+        for (int j = 0; j < t->n_ops[i]; ++j) {
+            const int c = t->op_code[i * t->n_col + j];
+            const uint64_t bit = 1ull << t->op_site[i * t->n_col + j];
+            if (c != QMB_OP_SZ && c != QMB_OP_SP && c != QMB_OP_SM) continue;
+            if (seen & bit) all_quick = false;
+            seen |= bit;
+            if (c == QMB_OP_SZ) {
+                q.zmask |= bit;
+                f *= 0.5;
+                continue;
+            }
+            q.care |= bit;
+            q.flip |= bit;
+            if (c == QMB_OP_SM) q.val |= bit;
+        }
+        q.sc = make_double2(f * t->scalar[2 * i], f * t->scalar[2 * i + 1]);
+        quick[i] = q;
+    }
+    DevBuf<QuickTerm> d_quick;
+    PackArgs pk{nullptr, nullptr, nullptr, (int)mob.size(), h->sector->n_active == h->sector->R ? 1 : 0,
                 h->sector->n_ext > 1 ? 1 : 0, nullptr};
     DevBuf<int16_t> d_midx;
     DevBuf<uint32_t> masks;
@@ -525,6 +588,11 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
         d_midx.alloc(both.size());
         d_midx.upload(both.data(), both.size());
         masks.alloc(mask_bytes / sizeof(uint32_t));
+        if (all_quick) {
+            d_quick.alloc(quick.size());
+            d_quick.upload(quick.data(), quick.size());
+            pk.quick = d_quick.p;
+        }
         pk.midx = d_midx.p;
         pk.mob = reinterpret_cast<const uint16_t*>(d_midx.p + midx.size());
         pk.masks = masks.p;
@@ -587,7 +655,7 @@ void build_sell(qmb_ham_s* h, const qmb_terms* t) {
     });
     check_launch("k_ell_fill");
     check_err();  // waits for the fill
-    mark_idle(slots, stats, d_midx, masks, cnt, tmp);
+    mark_idle(slots, stats, d_quick, d_midx, masks, cnt, tmp);
 }
 
 // ------------------------------------------ column-blocked coded layout
@@ -772,7 +840,9 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
     // dictionary from a strided sample of the values, reduced to its distinct
     // nonzero keys on the device (copying the 2^20 samples out and sorting them
     // on the host was most of a 28-site matrix's build: 28.4 -> 12.8 ms with the fill below)
-    const int64_t n_samp = std::min<int64_t>(h->padded, (int64_t)1 << 20);
+    // (a value that the sample misses costs a second fill: up to 2^25 slots all are
+    // looked at)
+    const int64_t n_samp = std::min<int64_t>(h->padded, (int64_t)1 << 25);
     const int64_t stride = std::max<int64_t>(1, h->padded / std::max<int64_t>(1, n_samp));
     std::vector<uint64_t> keys;
     DevBuf<int> miss(2);

