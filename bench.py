@@ -157,7 +157,7 @@ def build_batched(q, L=20, n_sets=256):
 
 def time_k1(q, b, prec, reps=20):
     """The Lanczos step's product kernel as the solve runs it (K1: H x with
-    the epilogue that reads v_{j-1} and writes v_j), CUDA events around each
+    the epilogue that reads w_{j-1}), CUDA events around each
     launch inside the library: (ms per step, algorithmic bytes)."""
     ms, byt = q._capi.C.c_double(), q._capi.C.c_double()
     q.check(q.lib().qmb_batch_k1_time(b.h, prec, reps, q._capi.C.byref(ms), q._capi.C.byref(byt)))
@@ -713,10 +713,9 @@ def run_batched(args, torch, q, rank, world):
                 e2e_value=float(np.mean(hv_count)) / e2e_s,
                 h2d=2 * n_sets * 8, d2h=n_sets * L * 8, roof_bytes=k1_32_bytes, roof_ms=k1_32_ms,
                 launches=launches,
-                kernel="k_bhv in the Lanczos step form (K1: y = H w/beta - beta v_{j-1}, v_j stored, alpha "
-                       "summed), FP32, one launch per step over all 20 sectors x 256 sets (the real momenta "
-                       "k=0, 10 are solved in the complex kind); bytes: the product's plus v_{j-1} read and "
-                       "v_j written",
+                kernel="k_bhv in the Lanczos step form (K1: y = H w_j/beta_j - (beta_j/beta_{j-1}) w_{j-1}, alpha "
+                       "summed), FP32, one launch per step over the 11 momenta a solve runs (of 20: the others "
+                       "are conjugates) x 256 sets; bytes: the product's over those sectors plus w_{j-1} read",
                 dtype="f32+f64")
 
 

@@ -329,12 +329,17 @@ __global__ void __launch_bounds__(kEvBlock) k_ev_diag(int64_t n, const U* __rest
     }
 }
 
-// q[m] += the chunks' part[chunk][m], added up in chunk order.
+// q[m] += the chunks' part[chunk][m], added up in chunk order with the rounding of
+// each addition carried along (Neumaier 1974).
 __global__ void k_ev_diag_sum(const double* __restrict__ part, int n_mask, int n_chunks, double* __restrict__ q) {
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n_mask; m += gridDim.x * blockDim.x) {
-        double t = 0.0;
-        for (int c = 0; c < n_chunks; ++c) t += part[(int64_t)c * n_mask + m];
-        q[m] += t;
+        double t = q[m], low = 0.0;
+        for (int c = 0; c < n_chunks; ++c) {
+            const double v = part[(int64_t)c * n_mask + m], s = __dadd_rn(t, v);
+            low += fabs(t) >= fabs(v) ? __dadd_rn(__dadd_rn(t, -s), v) : __dadd_rn(__dadd_rn(v, -s), t);
+            t = s;
+        }
+        q[m] = t + low;
     }
 }
 
@@ -462,7 +467,9 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
         blk.mark_idle();
         const double* hq = reinterpret_cast<const double*>(res.data());
         const double* hn = reinterpret_cast<const double*>(res.data() + (o_norm - o_q));
-        for (int k = 0; k < nm; ++k) val[cls.mask_class[k]] += cls.mask_w[k] * hq[k];
+        std::vector<long double> sum(cls.n, 0.0L);
+        for (int k = 0; k < nm; ++k) sum[cls.mask_class[k]] += (long double)cls.mask_w[k] * hq[k];
+        for (int c = 0; c < cls.n; ++c) val[c] = (double)sum[c];
         *norm2 = 0.0;
         for (int k = 0; k < nblk; ++k) *norm2 += hn[k];
     }
@@ -572,10 +579,12 @@ extern "C" qmb_status qmb_expval(qmb_ham h, int n_ops, const qmb_terms* ops, con
         else class_values<double>(h, (const double*)psi, cls, val, &norm2);
         QMB_REQUIRE(norm2 > 0.0, QMB_ERR_INVALID, "expval: psi is zero");
         for (int k = 0; k < n_ops; ++k) {
-            cplx sum(0.0, 0.0);
-            for (const auto& t : terms[k]) sum += t.second * val[t.first];
-            out[2 * k] = sum.real() / norm2;  // conj(s) / <psi|psi>
-            out[2 * k + 1] = -sum.imag() / norm2;
+            // (operators such as S(q) cancel among their classes)
+            std::complex<long double> sum(0.0L, 0.0L);
+            for (const auto& t : terms[k])
+                sum += std::complex<long double>(t.second) * std::complex<long double>(val[t.first]);
+            out[2 * k] = (double)(sum.real() / norm2);  // conj(s) / <psi|psi>
+            out[2 * k + 1] = (double)(-sum.imag() / norm2);
         }
         if (trace_on()) {
             size_t nt = 0;

@@ -644,11 +644,20 @@ void launch_lz_run(const Op& op, V* wbuf, V* vring, int K, const LzDev& d, int s
             QMB_REQUIRE(n_rb <= kRunParts && op.n <= kRunMaxRows, QMB_ERR_INVALID, "internal: too many rows for the resident kernel");
             // reorthogonalisation has units for more blocks than there are row blocks
             const int want = reorth ? std::max(n_rb, std::min(8 * n_rb, 2 * sms)) : n_rb;
-            const int grid = std::min(want, std::min(per_sm, 4) * sms);
+            int grid = std::min(want, std::min(per_sm, 4) * sms);
             Op o = op;
             LzDev dd = d;
             void* args[] = {&o, &wbuf, &vring, &K, &dd, &steps, &reorth, &selective, &ritz, &psi};
-            QMB_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kLzBlock), args, smem, s));
+            // any grid does the work; a process that may use fewer SMs than the device
+            // has (a service's limit) gets fewer blocks
+            cudaError_t e;
+            while ((e = cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kLzBlock), args, smem, s)) ==
+                       cudaErrorCooperativeLaunchTooLarge &&
+                   grid > 1) {
+                (void)cudaGetLastError();
+                grid /= 2;
+            }
+            QMB_CUDA_TRY(e);
         }, reorth > 0);
     }
 }
@@ -708,23 +717,25 @@ struct LzState {
     DevBuf<GridBar> bar;
     DevBuf<double2> coefs;
     LzDev d{};
-    void init(int cap_, int nb_, bool reorth) {
+    // zeroed on the solve's own stream: the legacy stream may have other threads'
+    // work queued, and its memset would then land in the middle of the solve
+    void init(int cap_, int nb_, bool reorth, cudaStream_t s) {
         cap = cap_;
         nb = nb_;
         alpha.alloc(cap + 1);
         beta.alloc(cap + 2);
         partials.alloc(std::max<size_t>(2 * (size_t)nb, 2 * kRunParts));
         bar.alloc(1);
-        bar.zero();
+        bar.zero(s);
         wsum.alloc(reorth ? kRunMaxRows / 32 + 8 : 1);
         chunk_ctr.alloc(reorth ? (size_t)cap / 8 + 2 : 1);
-        chunk_ctr.zero();
+        chunk_ctr.zero(s);
         scratch.alloc(4);
-        scratch.zero();
+        scratch.zero(s);
         iter.alloc(1);
         counter.alloc(2);
-        counter.zero();
-        iter.zero();
+        counter.zero(s);
+        iter.zero(s);
         coefs.alloc(reorth ? cap + 2 : 1);
         // a partial a block (or, resident, a row block of 256 rows) and basis vector
         cpart.alloc(reorth ? 2 * std::max<size_t>(nb, kRunMaxRows / 256) * (cap + 2) : 1);
@@ -839,7 +850,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
     bool wrapped = false;
     vring.alloc((size_t)K * n);
     wbuf.alloc(2 * (size_t)n);
-    st.init(cap, lz_blocks(), po.reorth > 0);
+    st.init(cap, lz_blocks(), po.reorth > 0, s);
     const int nb = st.nb;
     QMB_REQUIRE(po.reorth == 0 || store, QMB_ERR_INVALID, "reorthogonalisation needs the stored basis");
 
@@ -1355,7 +1366,7 @@ extern "C" qmb_status qmb_eigvec_from_seed_ref(long long seed, void* psi_dev, co
         ph.m = m;
         ph.s.assign(krylov, krylov + m);
         LzState st;
-        st.init(m, lz_blocks(), false);
+        st.init(m, lz_blocks(), false, s);
         int n_hv = 0;
         if (is_complex) {
             RefEllOp<float2> op{nobv, max_terms, ind_dev, (const float2*)val_dev, track_dev};
