@@ -86,7 +86,7 @@ struct Classes {
     std::unordered_map<uint64_t, int> of_mask;
     std::vector<int> pair_class;                // [L][L] classes of masks of one or two sites, -1: not seen
     std::vector<uint64_t> masks;                // images of all diagonal classes
-    std::vector<double> mask_w;                 // their weights
+    std::vector<double> mask_w;                 // elements reaching them (weight = that / G)
     std::vector<int> mask_class;
     // other terms
     struct At {
@@ -95,7 +95,7 @@ struct Classes {
     };
     std::unordered_map<TermKey, At, TermKeyHash> of_key;
     std::vector<TermKey> gen_key;               // averaged terms, class by class
-    std::vector<double> gen_w;
+    std::vector<double> gen_w;                  // signed elements reaching them (weight = that / n_ext)
     std::vector<int> gen_class;
 
     explicit Classes(const qmb_sector_s* sec) : s(sec), pair_class(sec->L * sec->L, -1) {}
@@ -114,11 +114,11 @@ struct Classes {
             if (of_mask.emplace(y, c).second) {
                 if (zero) continue;
                 masks.push_back(y);
-                mask_w.push_back(1.0 / s->G);
+                mask_w.push_back(1.0);
                 mask_class.push_back(c);
             } else if (!zero) {
                 for (size_t k = first; k < masks.size(); ++k)
-                    if (masks[k] == y) mask_w[k] += 1.0 / s->G;
+                    if (masks[k] == y) mask_w[k] += 1.0;
             }
         }
         of_mask.emplace(m, c);  // (among its images already when the group has the identity)
@@ -159,11 +159,11 @@ struct Classes {
             const double sign = (e >= s->G && (n_z & 1)) ? -1.0 : 1.0;
             if (of_key.emplace(k, At{c, sign}).second) {
                 gen_key.push_back(k);
-                gen_w.push_back(sign / s->n_ext);
+                gen_w.push_back(sign);
                 gen_class.push_back(c);
             } else {
                 for (size_t q = first; q < gen_key.size(); ++q)
-                    if (gen_key[q] == k) gen_w[q] += sign / s->n_ext;
+                    if (gen_key[q] == k) gen_w[q] += sign;
             }
         }
         return of_key.find(k0)->second;
@@ -469,9 +469,10 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
         const double* hn = reinterpret_cast<const double*>(res.data() + (o_norm - o_q));
         std::vector<long double> sum(cls.n, 0.0L);
         for (int k = 0; k < nm; ++k) sum[cls.mask_class[k]] += (long double)cls.mask_w[k] * hq[k];
-        for (int c = 0; c < cls.n; ++c) val[c] = (double)sum[c];
-        *norm2 = 0.0;
-        for (int k = 0; k < nblk; ++k) *norm2 += hn[k];
+        for (int c = 0; c < cls.n; ++c) val[c] = (double)(sum[c] / cls.s->G);
+        long double nn = 0.0L;
+        for (int k = 0; k < nblk; ++k) nn += hn[k];
+        *norm2 = (double)nn;
     }
 
     // the other terms, as many as fit in shared memory at a time
@@ -497,7 +498,7 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
             }
             seg.back().y += 1;
             nops.push_back(cls.gen_key[end].n);
-            sc.push_back(make_double2(cls.gen_w[end], 0.0));
+            sc.push_back(make_double2(cls.gen_w[end] / cls.s->n_ext, 0.0));
         }
         QMB_REQUIRE(end > pos, QMB_ERR_INVALID, "expval: a term does not fit");
         const int ng = (int)(end - pos), n_seg = (int)seg.size();
