@@ -10,7 +10,7 @@
 // every load is coalesced and the matrix entries are warp-uniform broadcasts.
 // A warp owns a row; lane l owns sets l*SPL .. l*SPL+SPL-1.  The Lanczos
 // scalars are per (sector, set); the convergence test and the Ritz
-// coefficients are computed on the device, one thread per problem.  Sectors
+// coefficients are computed on the device, one warp per problem.  Sectors
 // whose problems have all converged leave the work list (their tiles return
 // at once), and every step is a replayable CUDA graph.
 #include <algorithm>

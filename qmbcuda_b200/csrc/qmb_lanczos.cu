@@ -9,7 +9,8 @@
 // with FP64 scalars kept on the device (deterministic last-block reductions)
 // and the step index read from device memory, so a step is a replayable CUDA
 // graph.  Optional full reorthogonalisation runs classical Gram-Schmidt
-// passes against the stored Krylov basis.  The tridiagonal eigenproblem is
+// passes against the stored Krylov basis.  Sectors of up to 262,144 rows run all
+// steps up to the next convergence test in one resident kernel (k_lz_run).  The tridiagonal eigenproblem is
 // solved on the host in FP64 every `check_every` steps.
 #include <curand_kernel.h>
 
