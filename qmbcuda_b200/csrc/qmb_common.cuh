@@ -49,9 +49,13 @@ qmb_status guarded(F&& f) {
 
 // ------------------------------------------------------------ device memory
 // qmb_mem.cu: device memory, with freed idle buffers kept for reuse.
-void* dev_alloc(size_t bytes, size_t* got, int* dev);
-void dev_free(void* p, size_t bytes, int dev, bool idle);
-void dev_trim();  // frees what is kept on the current device
+struct DevPlace {
+    int dev = -1;
+    unsigned long long ctx = 0;  // identifier of the context (0: unknown)
+};
+void* dev_alloc(size_t bytes, size_t* got, DevPlace* at);
+void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle);
+void dev_trim();  // frees what is kept in the current context
 bool dev_mem_info(size_t* free_bytes, size_t* total);  // cudaMemGetInfo, kept buffers counted as free
 
 template <class T>
@@ -71,11 +75,11 @@ struct DevBuf {
     void alloc(size_t count) {
         release();
         if (count == 0) count = 1;
-        p = static_cast<T*>(dev_alloc(count * sizeof(T), &bytes_, &dev_));
+        p = static_cast<T*>(dev_alloc(count * sizeof(T), &bytes_, &at_));
         n = count;
     }
     void release() {
-        dev_free(p, bytes_, dev_, idle_);
+        dev_free(p, bytes_, at_, idle_);
         p = nullptr;
         n = 0;
         idle_ = false;
@@ -86,7 +90,7 @@ struct DevBuf {
         std::swap(p, o.p);
         std::swap(n, o.n);
         std::swap(bytes_, o.bytes_);
-        std::swap(dev_, o.dev_);
+        std::swap(at_, o.at_);
         std::swap(idle_, o.idle_);
     }
     void zero(cudaStream_t st = 0) { QMB_CUDA_TRY(cudaMemsetAsync(p, 0, n * sizeof(T), st)); }
@@ -99,7 +103,7 @@ struct DevBuf {
 
 private:
     size_t bytes_ = 0;   // as allocated
-    int dev_ = -1;
+    DevPlace at_;
     bool idle_ = false;
 };
 // mark_idle() on several buffers

@@ -4,7 +4,7 @@
 // cudaMalloc and cudaFree cost 0.1 to 0.3 ms each for the larger ones: at 28
 // sites they were 9 of the 13 ms of building a sector and its matrix (its
 // kernels take 2.5 ms).  Freed buffers of up to kMaxBlock bytes are therefore
-// kept, at most kMaxTotal bytes a device, and handed out again.
+// kept, at most kMaxTotal bytes a context, and handed out again.
 //
 // Rules.  A buffer comes here only idle: no work on any stream may still use
 // it.  DevBuf::mark_idle() says so, and is called after the wait that ends a
@@ -14,9 +14,13 @@
 // holds one lock.  The oldest buffers are freed when the total passes the bound
 // and all of them when an allocation fails (which is then tried again);
 // dev_mem_info() counts them as free memory.  A buffer is larger than the request
-// by at most an eighth.  A device reset by the application leaves dangling
-// addresses: the context's identifier is compared on every access and buffers of
-// an earlier context are forgotten.
+// by at most an eighth.
+//
+// A buffer belongs to the context in which it was allocated (DevBuf keeps its
+// identifier, unique in the process) and is kept and handed out in that context
+// alone.  One released while another context is current is freed, or forgotten
+// when its own context is gone: after a device reset its address may belong to a
+// live buffer of the new context.
 #include <cuda.h>
 
 #include <iterator>
@@ -31,61 +35,55 @@ namespace {
 
 constexpr size_t kMaxBlock = (size_t)128 << 20;
 constexpr size_t kMaxTotal = (size_t)512 << 20;
-constexpr int kMaxDevices = 64;
 
 struct Kept {
     void* p;
     size_t bytes;
 };
 using KeptList = std::list<Kept>;
-struct DeviceCache {
+struct Cache {
     KeptList kept;                                      // oldest first
     std::multimap<size_t, KeptList::iterator> by_size;  // newest last among equals
     size_t total = 0;
-    unsigned long long ctx = 0;
 };
 
 std::mutex g_mu;
-// never destroyed: handles may be released while the process exits
-DeviceCache* caches() {
-    static DeviceCache* c = new DeviceCache[kMaxDevices];
-    return c;
+// by context; never destroyed: handles may be released while the process exits
+std::map<unsigned long long, Cache>& caches() {
+    static auto* c = new std::map<unsigned long long, Cache>;
+    return *c;
 }
 
-// Identifier of the current context, unique in the process (0: unknown).
-unsigned long long context_id() {
-    using Fn = CUresult (*)(CUcontext, unsigned long long*);
-    static Fn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            (void)cudaGetLastError();
-            f = nullptr;
-        }
-        return reinterpret_cast<Fn>(f);
-    }();
+// A driver function by name, or null.
+template <class Fn>
+Fn driver_fn(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        f = nullptr;
+    }
+    return reinterpret_cast<Fn>(f);
+}
+
+// Identifier of a context (null: the current one), 0 when unknown.
+unsigned long long context_id(CUcontext c = nullptr) {
+    static const auto fn = driver_fn<CUresult (*)(CUcontext, unsigned long long*)>("cuCtxGetId");
     unsigned long long id = 0;
-    if (!fn || fn(nullptr, &id) != CUDA_SUCCESS) return 0;
+    if (!fn || fn(c, &id) != CUDA_SUCCESS) return 0;
     return id;
 }
 
-// The current device's cache, or null where nothing may be kept.
-DeviceCache* current(int dev) {
-    if (dev < 0 || dev >= kMaxDevices) return nullptr;
-    const unsigned long long id = context_id();
-    if (id == 0) return nullptr;
-    DeviceCache& c = caches()[dev];
-    if (c.ctx != id) {
-        c.kept.clear();
-        c.by_size.clear();
-        c.total = 0;
-        c.ctx = id;
-    }
-    return &c;
+// Identifier of the context that the memory at p belongs to now, 0 for none.
+unsigned long long owner_id(void* p) {
+    static const auto fn =
+        driver_fn<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>("cuPointerGetAttribute");
+    CUcontext c = nullptr;
+    if (!fn || fn(&c, CU_POINTER_ATTRIBUTE_CONTEXT, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS || !c) return 0;
+    return context_id(c);
 }
 
-void* take(DeviceCache& c, std::multimap<size_t, KeptList::iterator>::iterator at) {
+void* take(Cache& c, std::multimap<size_t, KeptList::iterator>::iterator at) {
     void* p = at->second->p;
     c.total -= at->first;
     c.kept.erase(at->second);
@@ -93,7 +91,7 @@ void* take(DeviceCache& c, std::multimap<size_t, KeptList::iterator>::iterator a
     return p;
 }
 
-void drop(DeviceCache& c, size_t keep) {
+void drop(Cache& c, size_t keep) {
     while (c.total > keep && !c.kept.empty()) {
         auto range = c.by_size.equal_range(c.kept.front().bytes);
         for (auto it = range.first; it != range.second; ++it)
@@ -111,20 +109,18 @@ size_t rounded(size_t bytes) {
 
 }  // namespace
 
-void* dev_alloc(size_t bytes, size_t* got, int* dev_out) {
-    int dev = -1;
-    QMB_CUDA_TRY(cudaGetDevice(&dev));
-    *dev_out = dev;
+void* dev_alloc(size_t bytes, size_t* got, DevPlace* at) {
+    QMB_CUDA_TRY(cudaGetDevice(&at->dev));
+    at->ctx = context_id();
     const size_t want = rounded(bytes);
     *got = want;
-    {
+    if (want <= kMaxBlock && at->ctx) {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (DeviceCache* c = want <= kMaxBlock ? current(dev) : nullptr) {
-            auto it = c->by_size.lower_bound(want);
-            if (it != c->by_size.end() && it->first <= want + want / 8) {
-                *got = it->first;
-                return take(*c, it);
-            }
+        Cache& c = caches()[at->ctx];
+        auto it = c.by_size.lower_bound(want);
+        if (it != c.by_size.end() && it->first <= want + want / 8) {
+            *got = it->first;
+            return take(c, it);
         }
     }
     void* p = nullptr;
@@ -137,30 +133,34 @@ void* dev_alloc(size_t bytes, size_t* got, int* dev_out) {
     if (e != cudaSuccess)
         throw Error{e == cudaErrorMemoryAllocation ? QMB_ERR_NOMEM : QMB_ERR_CUDA,
                     std::string("cudaMalloc of ") + std::to_string(want) + " bytes: " + cudaGetErrorString(e)};
+    if (!at->ctx) at->ctx = context_id();  // (the first allocation of a process makes the context)
     return p;
 }
 
-void dev_free(void* p, size_t bytes, int dev, bool idle) {
+void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle) {
     if (!p) return;
-    int cur = -1;
-    if (idle && bytes <= kMaxBlock && cudaGetDevice(&cur) == cudaSuccess && cur == dev) {
+    const unsigned long long id = at.ctx ? context_id() : 0;
+    if (at.ctx && id != at.ctx) {
+        if (owner_id(p) == at.ctx) cudaFree(p);
+        return;
+    }
+    if (idle && bytes <= kMaxBlock && id) {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (DeviceCache* c = current(dev)) {
-            c->kept.push_back(Kept{p, bytes});
-            c->by_size.emplace(bytes, std::prev(c->kept.end()));
-            c->total += bytes;
-            drop(*c, kMaxTotal);
-            return;
-        }
+        Cache& c = caches()[id];
+        c.kept.push_back(Kept{p, bytes});
+        c.by_size.emplace(bytes, std::prev(c.kept.end()));
+        c.total += bytes;
+        drop(c, kMaxTotal);
+        return;
     }
     cudaFree(p);
 }
 
 void dev_trim() {
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    const unsigned long long id = context_id();
     std::lock_guard<std::mutex> lock(g_mu);
-    if (DeviceCache* c = current(dev)) drop(*c, 0);
+    const auto it = caches().find(id);
+    if (it != caches().end()) drop(it->second, 0);
 }
 
 bool dev_mem_info(size_t* free_bytes, size_t* total) {
@@ -169,10 +169,10 @@ bool dev_mem_info(size_t* free_bytes, size_t* total) {
         *free_bytes = *total = 0;
         return false;
     }
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return true;
+    const unsigned long long id = context_id();
     std::lock_guard<std::mutex> lock(g_mu);
-    if (DeviceCache* c = current(dev)) *free_bytes += c->total;
+    const auto it = caches().find(id);
+    if (it != caches().end()) *free_bytes += it->second.total;
     return true;
 }
 
