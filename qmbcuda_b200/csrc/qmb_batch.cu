@@ -1134,11 +1134,8 @@ struct qmb_batch_s {
     std::vector<int> alias;  // caller sector whose solve gives this sector's energies (itself, or its conjugate)
     DevBuf<double> cxy, cz;
 
-    // freeing cxy waits for the device; the rest is idle then
     ~qmb_batch_s() {
-        if (!cxy.p) return;
-        cxy.release();
-        cz.mark_idle();
+        if (!qmb::mark_idle_after_wait(cxy, cz)) return;
         for (BKind& k : kind) k.mark_idle();
         for (auto& b : ws.bufs) b->mark_idle();
     }

@@ -55,6 +55,7 @@ struct DevPlace {
 };
 void* dev_alloc(size_t bytes, size_t* got, DevPlace* at);
 void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle);
+bool dev_wait(const DevPlace& at);  // waits for the device; false when that was refused or at is of another context
 void dev_trim();  // frees what is kept in the current context
 bool dev_mem_info(size_t* free_bytes, size_t* total);  // cudaMemGetInfo, kept buffers counted as free
 
@@ -84,6 +85,7 @@ struct DevBuf {
         n = 0;
         idle_ = false;
     }
+    bool wait() const { return dev_wait(at_); }
     // No work on any stream uses the buffer any more: release() may keep it.
     void mark_idle() { idle_ = p != nullptr; }
     void swap(DevBuf& o) noexcept {
@@ -109,7 +111,16 @@ private:
 // mark_idle() on several buffers
 template <class... B>
 void mark_idle(B&... b) { (b.mark_idle(), ...); }
-
+// A handle's buffers when it goes: idle once the device has been waited for.  The
+// wait is refused while a thread captures a graph in global mode; the buffers are
+// then freed as if no pool were there.
+template <class T, class... B>
+bool mark_idle_after_wait(DevBuf<T>& first, B&... rest) {
+    if (!first.p || !first.wait()) return false;
+    first.mark_idle();
+    mark_idle(rest...);
+    return true;
+}
 
 struct DeviceGuard {
     int prev = -1;

@@ -1007,12 +1007,11 @@ struct qmb_ham_s {
     qmb::DevBuf<unsigned char> psi;
     int64_t psi_n = 0;
 
-    // freeing the error flag waits for the device; the rest is idle then
     ~qmb_ham_s() {
-        if (!err.p) return;
-        err.release();
-        qmb::mark_idle(slice_off, slice_w, col, val64, val32, diag64, diag32, t_nops, t_ops, t_scalar, hops, hop_c,
-                       mf_reps32, mf_reps64, mf_bucket, mf_win, mf_hash, mf_norm, mf_diag, mf_xs, lz_ring, lz_wbuf, psi);
+        const bool idle = qmb::mark_idle_after_wait(
+            err, slice_off, slice_w, col, val64, val32, diag64, diag32, t_nops, t_ops, t_scalar, hops, hop_c, mf_reps32,
+            mf_reps64, mf_bucket, mf_win, mf_hash, mf_norm, mf_diag, mf_xs, lz_ring, lz_wbuf, psi);
+        if (!idle) return;
         for (qmb::CbLayout* L : {&cb32, &cb64}) qmb::mark_idle(L->off, L->width, L->packed, L->dict, L->ytmp);
     }
 

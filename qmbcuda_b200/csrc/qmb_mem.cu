@@ -8,8 +8,8 @@
 //
 // Rules.  A buffer comes here only idle: no work on any stream may still use
 // it.  DevBuf::mark_idle() says so, and is called after the wait that ends a
-// solve or a build, or on a handle's buffers once the first of them went through
-// cudaFree, which waits for the device; every other buffer is freed as before.
+// solve or a build, or on a handle's buffers after a wait for the device that was
+// not refused (mark_idle_after_wait); every other buffer is freed.
 // A buffer taken from here can thus be used on any stream at once.  Every access
 // holds one lock.  The oldest buffers are freed when the total passes the bound
 // and all of them when an allocation fails (which is then tried again);
@@ -154,6 +154,13 @@ void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle) {
         return;
     }
     cudaFree(p);
+}
+
+bool dev_wait(const DevPlace& at) {
+    if (!at.ctx || context_id() != at.ctx) return false;
+    if (cudaDeviceSynchronize() == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 void dev_trim() {

@@ -35,11 +35,8 @@ struct qmb_sector_s {
     qmb::DevBuf<int64_t> row_of_orbit;        // [R], -1 for null orbits
     qmb::DevBuf<int64_t> orbit_of_row;        // [n_active]
 
-    // freeing the group tables waits for the device; the rest is idle then
     ~qmb_sector_s() {
-        if (!tables.p) return;
-        tables.release();
-        qmb::mark_idle(rot, reps, bucket, chars_dev, norms, row_of_orbit, orbit_of_row);
+        qmb::mark_idle_after_wait(tables, rot, reps, bucket, chars_dev, norms, row_of_orbit, orbit_of_row);
     }
 
     qmb::GroupArgs group_args() const {

@@ -1,5 +1,6 @@
 // The pool of device buffers (qmb_mem.cu) over a stand-in for the CUDA calls that
-// it makes: contexts that are reset or changed.  Host code only.  Prints one
+// it makes: contexts that are reset or changed, waits
+// that are refused.  Host code only.  Prints one
 // line "<case> ok" or "<case> FAILED <condition>" per case.
 #include <cstdio>
 #include <map>
@@ -15,6 +16,7 @@ std::set<unsigned long long> live_ctx = {1};
 std::map<uintptr_t, unsigned long long> owner;  // live allocations
 uintptr_t base = 0x10000000;                    // the first address tried
 int mallocs = 0, frees = 0, bad_frees = 0;
+bool refuse = false;                            // as while a thread captures a graph
 
 // a reset: the context and its memory are gone, the next one starts at the same addresses
 void reset() {
@@ -54,6 +56,7 @@ cudaError_t cudaMalloc(void** p, size_t bytes) {
     return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
+    if (fake::refuse) return cudaErrorStreamCaptureUnsupported;
     if (!fake::owner.erase((uintptr_t)p)) {
         ++fake::bad_frees;
         return cudaErrorInvalidValue;
@@ -61,6 +64,7 @@ cudaError_t cudaFree(void* p) {
     ++fake::frees;
     return cudaSuccess;
 }
+cudaError_t cudaDeviceSynchronize() { return fake::refuse ? cudaErrorStreamCaptureUnsupported : cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
     *f = *t = (size_t)1 << 30;
     return cudaSuccess;
@@ -165,6 +169,29 @@ static void two_contexts() {
     EXPECT(fake::bad_frees == 0);
 }
 
+// the shape of the library's handles
+struct Handle {
+    Buf a{900}, b{90000};
+    ~Handle() { qmb::mark_idle_after_wait(a, b); }
+};
+
+// a handle's buffers are handed out again only when the device was waited for
+static void refused_wait() {
+    std::set<void*> first;
+    {
+        Handle h;
+        first = {h.a.p, h.b.p};
+    }
+    {
+        Handle h;
+        EXPECT(first.count(h.a.p) && first.count(h.b.p));
+        fake::refuse = true;
+    }
+    fake::refuse = false;
+    Handle h;
+    EXPECT(!first.count(h.a.p) && !first.count(h.b.p));
+}
+
 int main() {
     const struct {
         const char* name;
@@ -172,7 +199,8 @@ int main() {
     } cases[] = {{"reuse", reuse},
                  {"released_after_reset", released_after_reset},
                  {"kept_before_reset", kept_before_reset},
-                 {"two_contexts", two_contexts}};
+                 {"two_contexts", two_contexts},
+                 {"refused_wait", refused_wait}};
     for (const auto& c : cases) {
         g_case = c.name;
         g_ok = true;
