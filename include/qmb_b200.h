@@ -66,6 +66,12 @@ QMB_API const char* qmb_last_error(void);
 QMB_API const char* qmb_status_string(qmb_status s);
 /* Number of visible CUDA devices (0 on a host without a GPU). */
 QMB_API int qmb_device_count(void);
+/* Gives the device's memory that the library keeps for reuse back to the
+ * driver.  Closed handles and finished calls leave up to 512 MB of idle buffers
+ * with the library (a later allocation of the library takes them, and one that
+ * fails frees them all and tries again); another allocator in the process that
+ * runs short of device memory does not see them.  Open handles keep theirs. */
+QMB_API qmb_status qmb_trim(int device);
 
 /* Measurement entry point, no counterpart in the reference: the current
  * device's bandwidth (GB/s) for gathering whole rows of row_bytes bytes at

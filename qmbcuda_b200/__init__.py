@@ -9,7 +9,7 @@ from . import _capi
 from ._capi import QMBError, check, lib
 from .engine import (Batch, Hamiltonian, Sector, TermTable, chain_bonds, export_nosym,
                      export_ref, fourier_terms, geometry, load_ref_ell, multiply_terms, operator_terms,
-                     reciprocal_basis, save_ref_ell, square_bonds, translation_group,
+                     reciprocal_basis, save_ref_ell, square_bonds, translation_group, trim,
                      with_spin_flip, xxz_terms)
 
 lib()
@@ -17,4 +17,4 @@ lib()
 __all__ = ["Batch", "Hamiltonian", "QMBError", "Sector", "TermTable", "chain_bonds", "check",
            "export_nosym", "export_ref", "fourier_terms", "geometry", "lib", "load_ref_ell", "multiply_terms",
            "operator_terms", "reciprocal_basis", "save_ref_ell", "square_bonds", "translation_group",
-           "with_spin_flip", "xxz_terms"]
+           "trim", "with_spin_flip", "xxz_terms"]

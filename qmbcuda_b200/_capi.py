@@ -107,6 +107,7 @@ SIGNATURES = {
     "qmb_last_error": (C.c_char_p, []),
     "qmb_status_string": (C.c_char_p, [i32]),
     "qmb_device_count": (i32, []),
+    "qmb_trim": (i32, [i32]),
     "qmb_l2_gather_probe": (i32, [i64, i32, i64, P(dbl), P(dbl)]),
     "qmb_geometry_sites": (i32, [P(Geometry), vp, vp]),
     "qmb_tstandard_pairs": (i32, [P(Geometry), i32, vp, vp, i32, i32, i32, vp, vp, vp, P(i32)]),

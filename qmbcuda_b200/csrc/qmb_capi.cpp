@@ -3,7 +3,7 @@
 
 #include <string>
 
-#include "qmb_b200.h"
+#include "qmb_common.cuh"
 
 namespace qmb {
 
@@ -37,6 +37,13 @@ extern "C" const char* qmb_status_string(qmb_status s) {
         case QMB_ERR_CORRUPT: return "corrupt table file";
         default: return "unknown status";
     }
+}
+
+extern "C" qmb_status qmb_trim(int device) {
+    return qmb::guarded([&] {
+        qmb::DeviceGuard dg(device);
+        qmb::dev_trim();
+    });
 }
 
 extern "C" int qmb_device_count(void) {

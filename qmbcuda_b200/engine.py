@@ -257,6 +257,12 @@ class Sector:
         return o, e
 
 
+def trim(device: int = 0) -> None:
+    """Gives the idle device memory that the library keeps for reuse (at most
+    512 MB) back to the driver; open handles keep theirs."""
+    check(lib().qmb_trim(device))
+
+
 def export_ref(sector: Sector, terms: TermTable, W: int):
     R = sector.info.n_orbits
     ind = np.zeros(R * W, np.uint32)

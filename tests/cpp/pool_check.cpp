@@ -192,6 +192,21 @@ static void refused_wait() {
     EXPECT(!first.count(h.a.p) && !first.count(h.b.p));
 }
 
+// what is kept goes back to the driver, what is in use stays
+static void trim() {
+    Buf used(100), a(100), b(1 << 20);
+    void *pa = a.p, *pb = b.p;
+    qmb::mark_idle(a, b);
+    a.release();
+    b.release();
+    EXPECT(fake::owner_of(pa) && fake::owner_of(pb));
+    qmb::dev_trim();
+    EXPECT(!fake::owner_of(pa) && !fake::owner_of(pb) && fake::owner_of(used.p));
+    size_t f = 0, t = 0;
+    qmb::dev_mem_info(&f, &t);
+    EXPECT(f == t);
+}
+
 int main() {
     const struct {
         const char* name;
@@ -200,7 +215,8 @@ int main() {
                  {"released_after_reset", released_after_reset},
                  {"kept_before_reset", kept_before_reset},
                  {"two_contexts", two_contexts},
-                 {"refused_wait", refused_wait}};
+                 {"refused_wait", refused_wait},
+                 {"trim", trim}};
     for (const auto& c : cases) {
         g_case = c.name;
         g_ok = true;

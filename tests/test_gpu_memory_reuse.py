@@ -83,3 +83,21 @@ def test_kept_memory_is_bounded():
         _product(L)
     # 512 MB are kept at most; two allocation granules of slack for each buffer size
     assert free0 - torch.cuda.mem_get_info()[0] <= (512 + 64) << 20
+
+
+def test_trim_gives_kept_memory_back():
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    s = _sector(24)
+    q.trim()
+    free0 = torch.cuda.mem_get_info()[0]
+    h = q.Hamiltonian(s, q.xxz_terms(q.chain_bonds(24), 1.0, 0.8))
+    h.lanczos(tol=1e-10)
+    h.close()
+    assert torch.cuda.mem_get_info()[0] < free0  # kept for reuse
+    q.trim()
+    # (kernels loaded meanwhile may hold a few allocation granules)
+    assert free0 - torch.cuda.mem_get_info()[0] <= 8 << 20
+    with pytest.raises(q.QMBError):
+        q.trim(99)
