@@ -54,8 +54,9 @@ struct DevPlace {
     unsigned long long ctx = 0;  // identifier of the context (0: unknown)
 };
 void* dev_alloc(size_t bytes, size_t* got, DevPlace* at);
-void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle);
-bool dev_wait(const DevPlace& at);  // waits for the device; false when that was refused or at is of another context
+// True when the memory went through cudaFree without an error, which waits for
+// the device first (measured on 256 bytes with work on a non-blocking stream).
+bool dev_free(void* p, size_t bytes, const DevPlace& at, bool idle);
 void dev_trim();  // frees what is kept in the current context
 bool dev_mem_info(size_t* free_bytes, size_t* total);  // cudaMemGetInfo, kept buffers counted as free
 
@@ -79,13 +80,13 @@ struct DevBuf {
         p = static_cast<T*>(dev_alloc(count * sizeof(T), &bytes_, &at_));
         n = count;
     }
-    void release() {
-        dev_free(p, bytes_, at_, idle_);
+    bool release() {  // as dev_free
+        const bool freed = dev_free(p, bytes_, at_, idle_);
         p = nullptr;
         n = 0;
         idle_ = false;
+        return freed;
     }
-    bool wait() const { return dev_wait(at_); }
     // No work on any stream uses the buffer any more: release() may keep it.
     void mark_idle() { idle_ = p != nullptr; }
     void swap(DevBuf& o) noexcept {
@@ -111,13 +112,14 @@ private:
 // mark_idle() on several buffers
 template <class... B>
 void mark_idle(B&... b) { (b.mark_idle(), ...); }
-// A handle's buffers when it goes: idle once the device has been waited for.  The
-// wait is refused while a thread captures a graph in global mode; the buffers are
-// then freed as if no pool were there.
+// A handle's buffers when it goes: the first is freed, which waits for the device,
+// and the others are idle then.  A free is refused while a thread captures a graph
+// in global mode; nothing was waited for and the others are freed as if no pool
+// were there.  (cudaDeviceSynchronize() would break a capture of any mode in
+// another thread.)
 template <class T, class... B>
 bool mark_idle_after_wait(DevBuf<T>& first, B&... rest) {
-    if (!first.p || !first.wait()) return false;
-    first.mark_idle();
+    if (!first.release()) return false;
     mark_idle(rest...);
     return true;
 }

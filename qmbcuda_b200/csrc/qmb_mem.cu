@@ -8,8 +8,9 @@
 //
 // Rules.  A buffer comes here only idle: no work on any stream may still use
 // it.  DevBuf::mark_idle() says so, and is called after the wait that ends a
-// solve or a build, or on a handle's buffers after a wait for the device that was
-// not refused (mark_idle_after_wait); every other buffer is freed.
+// solve or a build, or on a handle's buffers once the first of them went through
+// cudaFree, which waits for the device, and was not refused
+// (mark_idle_after_wait); every other buffer is freed.
 // A buffer taken from here can thus be used on any stream at once.  Every access
 // holds one lock.  The oldest buffers are freed when the total passes the bound
 // and all of them when an allocation fails (which is then tried again);
@@ -137,12 +138,12 @@ void* dev_alloc(size_t bytes, size_t* got, DevPlace* at) {
     return p;
 }
 
-void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle) {
-    if (!p) return;
+bool dev_free(void* p, size_t bytes, const DevPlace& at, bool idle) {
+    if (!p) return false;
     const unsigned long long id = at.ctx ? context_id() : 0;
     if (at.ctx && id != at.ctx) {
         if (owner_id(p) == at.ctx) cudaFree(p);
-        return;
+        return false;
     }
     if (idle && bytes <= kMaxBlock && id) {
         std::lock_guard<std::mutex> lock(g_mu);
@@ -151,14 +152,9 @@ void dev_free(void* p, size_t bytes, const DevPlace& at, bool idle) {
         c.by_size.emplace(bytes, std::prev(c.kept.end()));
         c.total += bytes;
         drop(c, kMaxTotal);
-        return;
+        return false;
     }
-    cudaFree(p);
-}
-
-bool dev_wait(const DevPlace& at) {
-    if (!at.ctx || context_id() != at.ctx) return false;
-    if (cudaDeviceSynchronize() == cudaSuccess) return true;
+    if (cudaFree(p) == cudaSuccess) return true;
     (void)cudaGetLastError();
     return false;
 }

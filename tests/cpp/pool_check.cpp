@@ -1,5 +1,5 @@
 // The pool of device buffers (qmb_mem.cu) over a stand-in for the CUDA calls that
-// it makes: contexts that are reset or changed, waits
+// it makes: contexts that are reset or changed, frees
 // that are refused.  Host code only.  Prints one
 // line "<case> ok" or "<case> FAILED <condition>" per case.
 #include <cstdio>
@@ -64,7 +64,6 @@ cudaError_t cudaFree(void* p) {
     ++fake::frees;
     return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { return fake::refuse ? cudaErrorStreamCaptureUnsupported : cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
     *f = *t = (size_t)1 << 30;
     return cudaSuccess;
@@ -171,12 +170,12 @@ static void two_contexts() {
 
 // the shape of the library's handles
 struct Handle {
-    Buf a{900}, b{90000};
-    ~Handle() { qmb::mark_idle_after_wait(a, b); }
+    Buf flag{900}, a{9000}, b{90000};
+    ~Handle() { qmb::mark_idle_after_wait(flag, a, b); }
 };
 
 // a handle's buffers are handed out again only when the device was waited for
-static void refused_wait() {
+static void refused_free() {
     std::set<void*> first;
     {
         Handle h;
@@ -215,7 +214,7 @@ int main() {
                  {"released_after_reset", released_after_reset},
                  {"kept_before_reset", kept_before_reset},
                  {"two_contexts", two_contexts},
-                 {"refused_wait", refused_wait},
+                 {"refused_free", refused_free},
                  {"trim", trim}};
     for (const auto& c : cases) {
         g_case = c.name;

@@ -20,6 +20,6 @@ def results(tmp_path_factory):
     return dict(line.split(" ", 1) for line in out.splitlines())
 
 
-@pytest.mark.parametrize("case", ["reuse", "released_after_reset", "kept_before_reset", "two_contexts", "refused_wait", "trim"])
+@pytest.mark.parametrize("case", ["reuse", "released_after_reset", "kept_before_reset", "two_contexts", "refused_free", "trim"])
 def test_pool(results, case):
     assert results[case] == "ok"
