@@ -341,7 +341,9 @@ QMB_API qmb_status qmb_set_ground_state(qmb_ham h, const void* psi /* host */, i
  * NIter steps, no reorthogonalization, cuRAND start vector from seed;
  * FP64 reductions and an FP64 tridiagonal eigensolve.  Writes E[0], the
  * Ritz coefficients (if krylov_out) and returns the residual
- * ||H psi - E psi|| / nobv through *residual (checkEigState path). */
+ * ||H psi - E psi|| / nobv through *residual (checkEigState path).
+ * The call runs after work queued on the default stream; arrays that another,
+ * non-blocking stream fills have to be ready before it. */
 QMB_API qmb_status qmb_lanczos_ref_ell(float* E, int n_iter, int nobv, int max_terms, long long seed,
                                const uint32_t* ind_dev, const void* val_dev, const int16_t* track_dev,
                                int is_complex, float* krylov_out, int check_eig_state,
@@ -379,7 +381,8 @@ QMB_API qmb_status qmb_lanczos_ref_ell_noalloc(float* E, int n_iter, int nobv, i
  * Lanczos vectors are bit-identical to the solve's (same start, same
  * kernels); psi_dev receives nobv floats (complex: interleaved pairs).
  * krylov is the host array the solve wrote to krylov_out; trailing zeros
- * (a solve that broke down early) shorten the regeneration. */
+ * (a solve that broke down early) shorten the regeneration.  Ordered after the
+ * default stream as qmb_lanczos_ref_ell is. */
 QMB_API qmb_status qmb_eigvec_from_seed_ref(long long seed, void* psi_dev, const float* krylov, int n_iter,
                                     int nobv, int max_terms, const uint32_t* ind_dev,
                                     const void* val_dev, const int16_t* track_dev, int is_complex);
@@ -432,6 +435,8 @@ QMB_API qmb_status qmb_ref_ell_load(const char* path, int64_t* n_rows, int* widt
  * complex), or NULL for the ground state kept on the handle (qmb_lanczos with
  * want_vector, or qmb_set_ground_state).  Terms whose S+ and S- counts differ
  * change Sz and contribute zero.  Other operator codes are QMB_ERR_INVALID.
+ * Runs on the default stream: psi_dev filled by another, non-blocking stream has
+ * to be ready before the call.
  * All operators are evaluated in one pass of one kernel per shared-memory
  * chunk of terms; sums are FP64 and deterministic. */
 QMB_API qmb_status qmb_expval(qmb_ham h, int n_ops, const qmb_terms* ops, const void* psi_dev, double* out);

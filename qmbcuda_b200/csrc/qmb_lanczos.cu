@@ -1083,15 +1083,27 @@ bool fits_device(size_t bytes) {
     return bytes < fr * 0.6;
 }
 
+// Orders s after what the caller queued on the default stream: entry points on
+// caller-owned device arrays that take no stream run on one of their own.  (An
+// allocation that happened to wait for the device did this at times.)
+void after_default_stream(cudaStream_t s) {
+    cudaEvent_t e;
+    QMB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    struct EG { cudaEvent_t e; ~EG() { cudaEventDestroy(e); } } eg{e};
+    QMB_CUDA_TRY(cudaEventRecord(e, cudaStreamLegacy));
+    QMB_CUDA_TRY(cudaStreamWaitEvent(s, e, 0));
+}
+
 // Full solve for one storage / precision combination.
 //   V32/V64: vector types of the low / high phase, Op32/Op64 the operators.
 template <class Op32, class Op64, class V32, class V64>
 void solve(qmb_ham_s* h, const Op32& op32, size_t sm32, const Op64& op64, size_t sm64,
            const qmb_lanczos_opts& o, qmb_lanczos_result* res, double* coeffs, int64_t n_coeffs,
-           bool energy_only = false) {
+           bool energy_only = false, bool caller_arrays = false) {
     cudaStream_t s;
     QMB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
+    if (caller_arrays) after_default_stream(s);
     cudaEvent_t e0, e1;
     QMB_CUDA_TRY(cudaEventCreate(&e0));
     QMB_CUDA_TRY(cudaEventCreate(&e1));
@@ -1357,6 +1369,7 @@ extern "C" qmb_status qmb_eigvec_from_seed_ref(long long seed, void* psi_dev, co
         cudaStream_t s;
         QMB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
+        after_default_stream(s);
         const size_t es = is_complex ? sizeof(float2) : sizeof(float);
         QMB_CUDA_TRY(cudaMemsetAsync(psi_dev, 0, es * (size_t)nobv, s));
         if (m == 0) {
@@ -1410,11 +1423,11 @@ extern "C" qmb_status qmb_lanczos_ref_ell(float* E, int n_iter, int nobv, int ma
         if (is_complex) {
             RefEllOp<float2> op{nobv, max_terms, ind_dev, (const float2*)val_dev, track_dev};
             solve<RefEllOp<float2>, RefEllOp<float2>, float2, double2>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter,
-                                                                       energy_only);
+                                                                       energy_only, true);
         } else {
             RefEllOp<float> op{nobv, max_terms, ind_dev, (const float*)val_dev, track_dev};
             solve<RefEllOp<float>, RefEllOp<float>, float, double>(&dummy, op, 0, op, 0, o, &r, cf.data(), o.max_iter,
-                                                                   energy_only);
+                                                                   energy_only, true);
         }
         mark_idle(dummy.lz_ring, dummy.lz_wbuf);  // the solve ended with a wait
         *E = (float)r.E0;
