@@ -784,7 +784,12 @@ __global__ void k_cb_fill(SellOp<M> a, int shift, int nb, const int64_t* __restr
         for (int j = 0; j < w; ++j) {
             const int64_t k = a.off[s] + (int64_t)j * 32 + lane;
             const M v = a.val[k];
-            if (val_zero(v)) continue;
+            if (val_zero(v)) {
+                // one block: zeros keep their column, so that padding gathers the row's
+                // own x as the plain entries do (code 0 is the value 0)
+                if (nb == 1) packed[k] = a.col[k];
+                continue;
+            }
             const uint64_t key = val_key(v);
             int lo = 0, hi = n_keys;  // first key >= key
             while (lo < hi) {
