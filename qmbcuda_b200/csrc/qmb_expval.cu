@@ -26,15 +26,16 @@
 // sign of an odd number of Sz under inversion), so the terms of all operators
 // are sorted into classes, one value per class is computed on the device, and an
 // operator is the sum of its scalars times its classes' values.  The structure
-// factor at all 24 momenta of a 24-site chain with the 24 correlators has 27,672
+// factor at all 24 momenta of a 24-site chain with the 24 correlators has 13,848
 // terms in 13 classes.  Terms that change Sz are dropped (zero expectation in a
 // fixed-Sz sector).
 //
 // Products of Sz are signs: a class's value is a sum over its distinct images m
 // of Q(m) = sum_r |psi_r|^2 (-1)^popc(m & down_r), and k_ev_diag computes all Q
 // in one launch.  Other classes go through the Hamiltonian's row rule, their
-// averaged terms back to back in shared memory, one segment per class, each
-// reduced separately.
+// averaged terms back to back in shared memory, in segments that are reduced
+// separately: one per class that several operators hold, and one per operator for
+// the classes that it alone holds (gen_terms).
 #include <algorithm>
 #include <chrono>
 #include <complex>
@@ -96,7 +97,7 @@ struct Classes {
     std::unordered_map<TermKey, At, TermKeyHash> of_key;
     std::vector<TermKey> gen_key;               // averaged terms, class by class
     std::vector<double> gen_w;                  // signed elements reaching them (weight = that / n_ext)
-    std::vector<int> gen_class;
+    std::unordered_map<int, std::pair<size_t, size_t>> gen_range;  // class -> its terms
 
     explicit Classes(const qmb_sector_s* sec) : s(sec), pair_class(sec->L * sec->L, -1) {}
 
@@ -160,15 +161,48 @@ struct Classes {
             if (of_key.emplace(k, At{c, sign}).second) {
                 gen_key.push_back(k);
                 gen_w.push_back(sign);
-                gen_class.push_back(c);
             } else {
                 for (size_t q = first; q < gen_key.size(); ++q)
                     if (gen_key[q] == k) gen_w[q] += sign;
             }
         }
+        gen_range.emplace(c, std::make_pair(first, gen_key.size()));
         return of_key.find(k0)->second;
     }
 };
+
+// An averaged term of the general kernel and the value that its sum goes to.
+struct GenTerm {
+    int target;  // a class, or cls.n + operator
+    size_t key;
+    cplx sc;
+};
+
+// What the general kernel evaluates: a class that one operator alone holds goes, with
+// the operator's scalar, into the one sum of that operator, so that a row's data are
+// read once for all of them; a class that several operators hold is a sum of its
+// own, evaluated once.  Without a group (184,756 rows) the 80 classes of a J1-J2
+// Hamiltonian take 0.30 ms, as sums of their own 0.40; eight operators of 300 distinct
+// four-site terms 7.9 against 12.1.
+std::vector<GenTerm> gen_terms(const Classes& cls, const std::vector<std::vector<std::pair<int, cplx>>>& terms) {
+    std::vector<GenTerm> out;
+    if (cls.gen_key.empty()) return out;
+    std::vector<int> users(cls.n, 0);
+    for (const auto& op : terms)
+        for (const auto& t : op) ++users[t.first];
+    out.reserve(cls.gen_key.size());
+    auto add = [&](int target, int c, cplx s) {
+        const auto& r = cls.gen_range.at(c);
+        for (size_t i = r.first; i < r.second; ++i)
+            if (cls.gen_w[i] != 0.0) out.push_back(GenTerm{target, i, s * (cls.gen_w[i] / cls.s->n_ext)});
+    };
+    for (size_t k = 0; k < terms.size(); ++k)
+        for (const auto& t : terms[k])
+            if (users[t.first] == 1 && cls.gen_range.count(t.first)) add(cls.n + (int)k, t.first, t.second);
+    for (int c = 0; c < cls.n; ++c)
+        if (users[c] > 1 && cls.gen_range.count(c)) add(c, c, 1.0);
+    return out;
+}
 
 // Adds the terms of one operator: (class, scalar) pairs, one per class.
 void sort_terms(const qmb_terms& A, Classes& cls, std::vector<int>& last_op, std::vector<size_t>& last_at, int op,
@@ -403,10 +437,11 @@ __global__ void __launch_bounds__(kEvBlock) k_expval_sum(const double2* __restri
     if (threadIdx.x == 0) seg_out[blockIdx.x] = t;
 }
 
-// The values of the classes: val[c] = sum_r conj(psi_r) (Tbar_c psi)_r, and
-// <psi|psi>.
+// The values of the classes, val[c] = sum_r conj(psi_r) (Tbar_c psi)_r, behind them
+// the operators' own sums of general terms (gen_terms), and <psi|psi>.
 template <class V>
-void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cplx>& val, double* norm2) {
+void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, const std::vector<GenTerm>& gen, int n_ops,
+                  std::vector<cplx>& val, double* norm2) {
     RowGen rg = h->row_gen();
     const size_t gbytes = align16(group_smem_bytes(rg.g));
     int sms = 148, max_smem = 0;
@@ -414,7 +449,7 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
     QMB_CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
     const size_t smem_cap = std::min(kEvSmemCap, (size_t)max_smem);
     QMB_REQUIRE(gbytes + 64 < smem_cap, QMB_ERR_INVALID, "expval: group tables leave no shared memory");
-    val.assign(cls.n, cplx(0.0, 0.0));
+    val.assign(cls.n + n_ops, cplx(0.0, 0.0));
     const int64_t n = h->n;
     size_t off = 0;
     auto place = [&](size_t bytes) {
@@ -486,34 +521,35 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
     }
 
     // the other terms, as many as fit in shared memory at a time
-    const size_t n_gen = cls.gen_key.size();
+    const size_t n_gen = gen.size();
     if (!n_gen) return;
     DevBuf<int> err(1);
     err.zero();
     rg.err = err.p;
     for (size_t pos = 0; pos < n_gen;) {
         std::vector<int2> seg;
-        std::vector<int> seg_class, nops;
+        std::vector<int> seg_target, nops;
         std::vector<double2> sc;
         int n_col = 1;
         size_t end = pos;
         for (; end < n_gen; ++end) {
             const size_t ng = end - pos + 1;
-            const int c = std::max(n_col, cls.gen_key[end].n);
+            const TermKey& key = cls.gen_key[gen[end].key];
+            const int c = std::max(n_col, key.n);
             if (gbytes + ((20 + 2 * (size_t)c) * ng + 15) / 16 * 16 > smem_cap || ng > (size_t)kMaxTerms) break;
             n_col = c;
-            if (seg.empty() || seg_class.back() != cls.gen_class[end]) {
+            if (seg.empty() || seg_target.back() != gen[end].target) {
                 seg.push_back(make_int2((int)ng - 1, (int)ng - 1));
-                seg_class.push_back(cls.gen_class[end]);
+                seg_target.push_back(gen[end].target);
             }
             seg.back().y += 1;
-            nops.push_back(cls.gen_key[end].n);
-            sc.push_back(make_double2(cls.gen_w[end] / cls.s->n_ext, 0.0));
+            nops.push_back(key.n);
+            sc.push_back(make_double2(gen[end].sc.real(), gen[end].sc.imag()));
         }
         QMB_REQUIRE(end > pos, QMB_ERR_INVALID, "expval: a term does not fit");
         const int ng = (int)(end - pos), n_seg = (int)seg.size();
         std::vector<uint16_t> opw((size_t)ng * n_col, 0);
-        for (int i = 0; i < ng; ++i) key_words(cls.gen_key[pos + i], opw.data() + (size_t)i * n_col);
+        for (int i = 0; i < ng; ++i) key_words(cls.gen_key[gen[pos + i].key], opw.data() + (size_t)i * n_col);
         rg.terms.n_terms = ng;
         rg.terms.n_col = n_col;
         const size_t smem = gbytes + terms_smem_bytes(rg.terms);
@@ -547,7 +583,7 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, std::vector<cp
         std::vector<double2> res(n_seg);
         QMB_CUDA_TRY(cudaMemcpy(res.data(), res_d, sizeof(double2) * n_seg, cudaMemcpyDeviceToHost));
         blk.mark_idle();
-        for (int i = 0; i < n_seg; ++i) val[seg_class[i]] += cplx(res[i].x, res[i].y);
+        for (int i = 0; i < n_seg; ++i) val[seg_target[i]] += cplx(res[i].x, res[i].y);
         pos = end;
     }
     int herr = 0;
@@ -586,12 +622,13 @@ extern "C" qmb_status qmb_expval(qmb_ham h, int n_ops, const qmb_terms* ops, con
         const auto t1 = std::chrono::steady_clock::now();
         std::vector<cplx> val;
         double norm2 = 0.0;
-        if (h->cplx) class_values<double2>(h, (const double2*)psi, cls, val, &norm2);
-        else class_values<double>(h, (const double*)psi, cls, val, &norm2);
+        const std::vector<GenTerm> gen = gen_terms(cls, terms);
+        if (h->cplx) class_values<double2>(h, (const double2*)psi, cls, gen, n_ops, val, &norm2);
+        else class_values<double>(h, (const double*)psi, cls, gen, n_ops, val, &norm2);
         QMB_REQUIRE(norm2 > 0.0, QMB_ERR_INVALID, "expval: psi is zero");
         for (int k = 0; k < n_ops; ++k) {
             // (operators such as S(q) cancel among their classes)
-            std::complex<long double> sum(0.0L, 0.0L);
+            std::complex<long double> sum(val[cls.n + k]);
             for (const auto& t : terms[k])
                 sum += std::complex<long double>(t.second) * std::complex<long double>(val[t.first]);
             out[2 * k] = (double)(sum.real() / norm2);  // conj(s) / <psi|psi>
