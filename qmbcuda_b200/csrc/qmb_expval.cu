@@ -53,7 +53,8 @@ namespace {
 
 constexpr int kEvBlock = 256;
 constexpr size_t kEvSmemCap = 200 * 1024;  // dynamic shared memory per block
-constexpr int64_t kEvSlab = (int64_t)1 << 23;  // rows of one pass of the sign sums
+constexpr int64_t kEvSlab = (int64_t)1 << 23;     // rows of one pass of the sign sums
+constexpr int64_t kEvSlabMin = (int64_t)1 << 16;  // the fewest, where memory is short
 
 using cplx = std::complex<double>;
 
@@ -462,19 +463,34 @@ void class_values(qmb_ham_s* h, const V* psi, const Classes& cls, const std::vec
     {
         const int nm = (int)cls.masks.size(), groups = (nm + kEvMasks - 1) / kEvMasks;
         const bool small = cls.s->L <= 32;
-        // rows in slabs, which bounds the scratch (12 or 16 bytes a row); about
-        // 48 warps an SM, chunks of at least 256 rows
-        const int64_t slab = std::min<int64_t>(n, nm ? kEvSlab : n);
-        const int64_t want = groups ? std::max<int64_t>(1, (int64_t)sms * 48 / groups) : 1;
-        const int chunks = (int)std::min<int64_t>(want, (slab + 255) / 256);
-        const int64_t chunk = ((slab + chunks - 1) / chunks + 31) / 32 * 32;
-        const int nblk = (int)std::min<int64_t>((slab + kEvBlock - 1) / kEvBlock, (int64_t)sms * 4);
+        // rows in slabs, which bounds the scratch (12 or 16 bytes a row; smaller ones
+        // where the memory is short); about 48 warps an SM, chunks of at least 256 rows
+        int64_t slab = std::min<int64_t>(n, nm ? kEvSlab : n), chunk = 0;
+        int chunks = 0, nblk = 0;
         const size_t us = small ? 4 : 8;
-        off = 0;
-        const size_t o_mask = place(us * nm), o_q = place(sizeof(double) * nm), o_norm = place(sizeof(double) * nblk),
-                     o_p = place(nm ? sizeof(double) * slab : 0), o_down = place(nm ? us * slab : 0),
-                     o_part = place(sizeof(double) * (size_t)nm * chunks);
-        DevBuf<unsigned char> blk(off);
+        size_t o_mask, o_q, o_norm, o_p, o_down, o_part;
+        DevBuf<unsigned char> blk;
+        for (;;) {
+            const int64_t want = groups ? std::max<int64_t>(1, (int64_t)sms * 48 / groups) : 1;
+            chunks = (int)std::min<int64_t>(want, (slab + 255) / 256);
+            chunk = ((slab + chunks - 1) / chunks + 31) / 32 * 32;
+            nblk = (int)std::min<int64_t>((slab + kEvBlock - 1) / kEvBlock, (int64_t)sms * 4);
+            off = 0;
+            o_mask = place(us * nm);
+            o_q = place(sizeof(double) * nm);
+            o_norm = place(sizeof(double) * nblk);
+            o_p = place(nm ? sizeof(double) * slab : 0);
+            o_down = place(nm ? us * slab : 0);
+            o_part = place(sizeof(double) * (size_t)nm * chunks);
+            try {
+                blk.alloc(off);
+                break;
+            } catch (const Error& e) {
+                if (e.code != QMB_ERR_NOMEM || slab <= kEvSlabMin) throw;
+                (void)cudaGetLastError();
+                slab = std::max(kEvSlabMin, slab / 2);
+            }
+        }
         unsigned char* b = blk.p;
         double* q = reinterpret_cast<double*>(b + o_q);
         double* npart = reinterpret_cast<double*>(b + o_norm);

@@ -101,3 +101,27 @@ def test_trim_gives_kept_memory_back():
     assert free0 - torch.cuda.mem_get_info()[0] <= 8 << 20
     with pytest.raises(q.QMBError):
         q.trim(99)
+
+
+def test_observables_where_memory_is_short():
+    """9,657,700 rows with 48 MB of device memory left: the sign sums' scratch
+    (100 MB with memory to spare) shrinks, and the values stay."""
+    import torch
+    L, n_up = 26, 12
+    s = q.Sector(L, n_up, np.arange(L, dtype=np.uint32)[None, :]).set_irrep([1.0])
+    h = q.Hamiltonian(s, q.xxz_terms([(0, 1)], 1.0, 0.5), prec=A.PREC_FP32)
+    h.set_ground_state(np.ones(h.info.n_rows))
+    ops = [q.operator_terms([(1.0, [("Sz", 0), ("Sz", j)])]) for j in (1, 13, 25)]
+    want = h.expval(ops)
+    q.trim()
+    torch.cuda.empty_cache()
+    rest = torch.cuda.mem_get_info()[0] - (48 << 20)
+    hog = torch.empty(rest, dtype=torch.uint8, device="cuda")
+    try:
+        got = h.expval(ops)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    m = 2 * n_up - L
+    assert np.abs(got - want).max() <= 1e-14
+    assert np.abs(got - (m * m - L) / (4.0 * L * (L - 1))).max() <= 1e-14
