@@ -2084,9 +2084,10 @@ struct BatchPart {
 };
 
 // Weighted sums of a sector's values, with weights in [1, 2) hashed from the
-// entry's place and column: out[0] = sum w Re, out[1] = sum w Im, out[2] =
-// sum w |v|, over the off-diagonal entries and both diagonals.  Two conjugate
-// matrices have equal out[0] and opposite out[1].
+// entry's place and column: out[0] = sum w Re, out[1] = sum w Im, out[2] = sum w |v|
+// over the hopping part (off-diagonal entries and their diagonal), out[3..5] the
+// same over the diagonal part.  Two conjugate matrices have equal out[0] and out[3]
+// and opposite out[1] and out[4].
 __device__ __forceinline__ double hash_weight(uint64_t k) {
     return 1.0 + (double)(mf_hash_slot(k + 0x9E3779B97F4A7C15ull, ~0ull) >> 11) * 0x1p-53;
 }
@@ -2094,45 +2095,41 @@ __global__ void k_part_print(int64_t n, int64_t nnz, const uint32_t* __restrict_
                              const double2* __restrict__ val, const double2* __restrict__ dxy,
                              const double2* __restrict__ dz, double* __restrict__ out) {
     __shared__ double red[32];
-    double re = 0.0, im = 0.0, ab = 0.0;
-    auto add = [&](double w, double2 v) {
-        re += w * v.x;
-        im += w * v.y;
-        ab += w * (fabs(v.x) + fabs(v.y));
+    double sum[6] = {};
+    auto add = [&](double w, double2 v, int part) {
+        sum[3 * part] += w * v.x;
+        sum[3 * part + 1] += w * v.y;
+        sum[3 * part + 2] += w * (fabs(v.x) + fabs(v.y));
     };
     const int64_t m = n > nnz ? n : nnz;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        if (i < nnz) add(hash_weight(((uint64_t)i << 24) ^ col[i]), val[i]);
+        if (i < nnz) add(hash_weight(((uint64_t)i << 24) ^ col[i]), val[i], 0);
         if (i < n) {
-            add(hash_weight(~(uint64_t)(2 * i)), dxy[i]);
-            add(hash_weight(~(uint64_t)(2 * i + 1)), dz[i]);
+            add(hash_weight(~(uint64_t)(2 * i)), dxy[i], 0);
+            add(hash_weight(~(uint64_t)(2 * i + 1)), dz[i], 1);
         }
     }
-    re = block_sum(re, red);
-    im = block_sum(im, red);
-    ab = block_sum(ab, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(out, re);
-        atomicAdd(out + 1, im);
-        atomicAdd(out + 2, ab);
+    for (int q = 0; q < 6; ++q) {
+        const double t = block_sum(sum[q], red);
+        if (threadIdx.x == 0) atomicAdd(out + q, t);
     }
 }
 
 // Clears *same unless the two sectors' entries have equal places and values
-// conjugate to within tol.
+// conjugate to within tol (hopping part) and tol_z (diagonal part).
 __global__ void k_part_conj(int64_t n, int64_t nnz, const int64_t* __restrict__ rp1, const int64_t* __restrict__ rp2,
                             const uint32_t* __restrict__ col1, const uint32_t* __restrict__ col2,
                             const double2* __restrict__ v1, const double2* __restrict__ v2,
                             const double2* __restrict__ x1, const double2* __restrict__ x2,
                             const double2* __restrict__ z1, const double2* __restrict__ z2, double tol,
-                            int* __restrict__ same) {
-    auto conj_eq = [&](double2 a, double2 b) { return fabs(a.x - b.x) <= tol && fabs(a.y + b.y) <= tol; };
+                            double tol_z, int* __restrict__ same) {
+    auto conj_eq = [](double2 a, double2 b, double t) { return fabs(a.x - b.x) <= t && fabs(a.y + b.y) <= t; };
     bool ok = true;
     const int64_t m = n + 1 > nnz ? n + 1 : nnz;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         if (i <= n) ok = ok && rp1[i] == rp2[i];
-        if (i < nnz) ok = ok && col1[i] == col2[i] && conj_eq(v1[i], v2[i]);
-        if (i < n) ok = ok && conj_eq(x1[i], x2[i]) && conj_eq(z1[i], z2[i]);
+        if (i < nnz) ok = ok && col1[i] == col2[i] && conj_eq(v1[i], v2[i], tol);
+        if (i < n) ok = ok && conj_eq(x1[i], x2[i], tol) && conj_eq(z1[i], z2[i], tol_z);
     }
     if (!ok) *same = 0;
 }
@@ -2142,7 +2139,8 @@ __global__ void k_part_conj(int64_t n, int64_t nnz, const int64_t* __restrict__ 
 // one of the two: alias[s] is the sector that is solved for s.  A rotation's
 // characters are rounded at about 5e-16 times their phase, 2e-14 at 20 sites
 // and 5e-14 at 48, which moves an energy far less than the solves' tolerance;
-// 2.5e-13 of the mean entry is accepted.  The L=20 batch of all 20 momenta
+// 2.5e-13 of the mean entry is accepted, of the hopping part for its entries and of
+// the diagonal part for its (the coupling sets scale the two apart).  The L=20 batch of all 20 momenta
 // solves 11 sectors (128 sets, mixed: 55.8 -> 35.6 ms a solve).
 constexpr double kConjTol = 2.5e-13;
 static void find_conjugates(const std::vector<BatchPart>& parts, const std::vector<int>& kind,
@@ -2153,16 +2151,16 @@ static void find_conjugates(const std::vector<BatchPart>& parts, const std::vect
     if (S < 2) return;
     auto rows = [&](int s) { return (int64_t)parts[s].row_ptr.size() - 1; };
     auto ents = [&](int s) { return parts[s].row_ptr.back(); };
-    DevBuf<double> pr(3 * (size_t)S);
+    DevBuf<double> pr(6 * (size_t)S);
     pr.zero();
     for (int s = 0; s < S; ++s) {
         const BatchPart& P = parts[s];
         if (rows(s) == 0) continue;
         k_part_print<<<std::min(grid_for(std::max(rows(s), ents(s)), 256), 592), 256>>>(
-            rows(s), ents(s), P.col.p, P.val.p, P.dxy.p, P.dz.p, pr.p + 3 * s);
+            rows(s), ents(s), P.col.p, P.val.p, P.dxy.p, P.dz.p, pr.p + 6 * s);
     }
     check_launch("k_part_print");
-    std::vector<double> h(3 * (size_t)S);
+    std::vector<double> h(6 * (size_t)S);
     pr.download(h.data(), h.size());
     QMB_CUDA_TRY(cudaStreamSynchronize(0));
     // candidates: the first earlier sector with equal sizes and matching sums
@@ -2175,20 +2173,22 @@ static void find_conjugates(const std::vector<BatchPart>& parts, const std::vect
         auto range = by_size.equal_range(key);
         for (auto it = range.first; it != range.second && cand[s] < 0; ++it) {
             const int t = it->second;
-            const double tol = 1e-11 * std::max(h[3 * s + 2], h[3 * t + 2]);
-            if (kind[s] == kind[t] && rows(s) > 0 && std::fabs(h[3 * s] - h[3 * t]) <= tol &&
-                std::fabs(h[3 * s + 1] + h[3 * t + 1]) <= tol)
-                cand[s] = t;
+            const double *a = &h[6 * s], *b = &h[6 * t];
+            auto near = [&](int q) {  // sums q .. q + 2
+                const double tol = 1e-11 * std::max(a[q + 2], b[q + 2]);
+                return std::fabs(a[q] - b[q]) <= tol && std::fabs(a[q + 1] + b[q + 1]) <= tol;
+            };
+            if (kind[s] == kind[t] && rows(s) > 0 && near(0) && near(3)) cand[s] = t;
         }
         if (cand[s] < 0) {
             by_size.emplace(key, s);
             continue;
         }
         const BatchPart &P = parts[cand[s]], &Q = parts[s];
-        const double mean = h[3 * s + 2] / std::max<double>(1.0, 1.5 * (double)(ents(s) + 2 * rows(s)));
+        const double mean = h[6 * s + 2] / (1.5 * (double)(ents(s) + rows(s))), mean_z = h[6 * s + 5] / (1.5 * (double)rows(s));
         k_part_conj<<<grid_for(std::max(rows(s) + 1, ents(s)), 256), 256>>>(
             rows(s), ents(s), P.rp.p, Q.rp.p, P.col.p, Q.col.p, P.val.p, Q.val.p, P.dxy.p, Q.dxy.p, P.dz.p, Q.dz.p,
-            kConjTol * mean, same.p + s);
+            kConjTol * mean, kConjTol * mean_z, same.p + s);
     }
     check_launch("k_part_conj");
     std::vector<int> hs(S);
