@@ -1187,8 +1187,7 @@ static void launch_bhv_v(const BatchArgs& a, BKind& k, const V* x, V* y, V* vrin
     int dev = 0;
     cudaGetDevice(&dev);
     int& g = grid[dev & 63];
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    set_group_smem_attr((const void*)kern, smem);
     if (g == 0) {
         int per_sm = 0, sms = 148;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, smem);
@@ -1475,8 +1474,7 @@ static void launch_check(const BatchArgs& a, const BLz& lz, int nsets, double st
     const size_t per_warp = sizeof(double) * kCheckArrays * (size_t)(m + 2);
     const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (96u << 10) / per_warp));
     const size_t smem = per_warp * wpb;
-    if (smem > (48u << 10))
-        cudaFuncSetAttribute(k_bcheck, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    set_group_smem_attr((const void*)k_bcheck, smem);
     const int nblk = (lz.n_prob + wpb - 1) / wpb;
     g_kernels += 1;
     k_bcheck<<<nblk, 32 * wpb, smem, st>>>(a, lz, nsets, stall, res_tol, e_tol, gap_in, gap_out, theta,
@@ -2019,8 +2017,7 @@ static BPhase run_bphase(qmb_batch_s* b, BKind& k, bool f64, int max_iter, doubl
             const size_t per_warp = sizeof(double) * kRitzArrays * (size_t)(done + 2);
             const int wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (96u << 10) / per_warp));
             const size_t smem = per_warp * wpb;
-            if (smem > (48u << 10))
-                QMB_CUDA_TRY(cudaFuncSetAttribute(k_britz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            set_group_smem_attr((const void*)k_britz, smem);
             k_britz<<<(n_prob + wpb - 1) / wpb, 32 * wpb, smem, st>>>(lz, done, msteps.p, theta.p, ritz.p, gap_out);
         }
         if (te[1]) QMB_CUDA_TRY(cudaEventRecord(te[1], st));

@@ -634,8 +634,7 @@ void launch_lz_run(const Op& op, V* wbuf, V* vring, int K, const LzDev& d, int s
             constexpr int S = decltype(sp)::value;
             auto kern = k_lz_run<Op, V, P, S>;
             const size_t smem = reorth ? sizeof(double2) * (size_t)(cap + 2) : 0;
-            if (smem > 0)
-                QMB_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            set_group_smem_attr((const void*)kern, smem);
             int dev = 0, sms = 148, per_sm = 0;
             QMB_CUDA_TRY(cudaGetDevice(&dev));
             QMB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

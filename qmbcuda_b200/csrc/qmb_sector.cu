@@ -224,10 +224,16 @@ int grid_for(int64_t n, int block) {
     return (int)g;
 }
 
+// The limit belongs to the kernel, not to the launch: it is only ever raised, so that
+// a thread that needs less does not take it from under another's launch.
 void set_group_smem_attr(const void* kernel, size_t bytes) {
-    if (bytes > 48 * 1024)
-        QMB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)bytes));
+    if (bytes <= 48 * 1024) return;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes a;
+    QMB_CUDA_TRY(cudaFuncGetAttributes(&a, kernel));
+    if ((size_t)a.maxDynamicSharedSizeBytes < bytes)
+        QMB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
 // Detects whether every site map is a torus translation with rows of W bits.
