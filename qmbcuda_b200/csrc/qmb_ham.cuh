@@ -866,6 +866,7 @@ inline void with_split(const Op& op, F&& f, bool whole = false) {
     constexpr int top = OpMaxSplit<Op>::value;
     const int S = whole ? 1 : OpSplit<Op>::of(op);
     if constexpr (OpSplit<Op>::lanes) {
+        if (whole) return f(std::integral_constant<int, 1>{});
         f(std::integral_constant<int, top>{});
     } else {
         if constexpr (top >= 8)
