@@ -507,7 +507,7 @@ void launch_hv(const Op& op, const V* x, V* y, cudaStream_t st, size_t smem) {
         constexpr int S = decltype(sp)::value;
         set_group_smem_attr((const void*)k_hv<Op, V, S>, smem);
         k_hv<Op, V, S><<<grid_for(op.n, 256 / S), 256, smem, st>>>(op, x, y);
-    });
+    }, smem > kSplitSmemMax);
     check_launch("k_hv");
 }
 

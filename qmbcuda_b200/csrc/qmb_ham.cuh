@@ -859,6 +859,11 @@ template <class M> struct OpMaxSplit<SellOp<M>> { static constexpr int value = 4
 template <class M> struct OpMaxSplit<MfOp<M>> { static constexpr int value = 8; };
 template <class M> struct OpMaxSplit<RefEllOp<M>> { static constexpr int value = 4; };
 
+// Dynamic shared memory up to which a kernel may split rows: the sums of the split
+// take up to 4 KB beside it, and a block has 227 KB.  (Term and group tables reach
+// this with some 3,600 terms of 8 factors and 96 KB of group tables.)
+constexpr size_t kSplitSmemMax = 220 * 1024;
+
 // f(std::integral_constant<int, S>) for the split of op's rows; S = 1 when the
 // caller wants the rows whole.
 template <class Op, class F>

@@ -678,7 +678,7 @@ void launch_lz_hv(const Op& op, size_t smem, int nb, V* wbuf, V* vring, int K, c
         constexpr int S = decltype(sp)::value;
         set_group_smem_attr((const void*)k_lz_hv<Op, V, P, S>, smem);
         k_lz_hv<Op, V, P, S><<<nb, kLzBlock, smem, s>>>(op, wbuf, vring, K, d, ritz, psi);
-    }, whole);
+    }, whole || smem > kSplitSmemMax);
 }
 template <class Op, class P>
 void launch_residual(const Op& op, size_t smem, int nb, const P* psi, double theta, const LzDev& d, cudaStream_t s) {
@@ -686,7 +686,7 @@ void launch_residual(const Op& op, size_t smem, int nb, const P* psi, double the
         constexpr int S = decltype(sp)::value;
         set_group_smem_attr((const void*)k_residual<Op, P, S>, smem);
         k_residual<Op, P, S><<<nb, kLzBlock, smem, s>>>(op, psi, theta, d);
-    });
+    }, smem > kSplitSmemMax);
 }
 
 // QMB_REORTH_ALWAYS=1: with two passes requested, always run the second one
