@@ -363,10 +363,10 @@ struct GridBar {
 // two launches; beyond, the vectors leave L2 and the launches no longer count.
 constexpr int64_t kRunMaxRows = 262144;
 constexpr int kRunParts = 2048;  // row blocks at most
-constexpr unsigned kBarSpins = 1u << 23;  // polls of about 0.5 us
+constexpr unsigned kBarSpins = 1u << 23;  // polls of about 0.5 us (QMB_LZ_BAR_SPINS=n: n, tests of the give-up)
 
 // All threads' writes lie before a __syncthreads that thread 0 has passed.
-__device__ __forceinline__ bool grid_wait(GridBar* b, unsigned& gen) {
+__device__ __forceinline__ bool grid_wait(GridBar* b, unsigned& gen, unsigned spins) {
     __shared__ int ok;
     if (threadIdx.x == 0) {
         int good = 1;
@@ -378,7 +378,7 @@ __device__ __forceinline__ bool grid_wait(GridBar* b, unsigned& gen) {
                 *(volatile unsigned*)&b->gen = gen + 1;
             } else {
                 for (unsigned it = 0; *(volatile unsigned*)&b->gen == gen; ++it)
-                    if (it > kBarSpins || ((it & 255u) == 255u && *(volatile int*)&b->err)) {
+                    if (it > spins || ((it & 255u) == 255u && *(volatile int*)&b->err)) {
                         atomicExch(&b->err, 1);
                         good = 0;
                         break;
@@ -418,7 +418,7 @@ template <class V> struct ReorthShape {
 
 template <class Op, class V, class P, int S>
 __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring, int K, LzDev d, int steps, int reorth,
-                                                        int selective, const double* __restrict__ ritz, P* psi) {
+                                                        int selective, unsigned spins, const double* __restrict__ ritz, P* psi) {
     __shared__ V sh[256];
     __shared__ double red[32];
     __shared__ double red8[3][8];
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring
             const double t = block_sum(acc, red);
             if (threadIdx.x == 0) pa[rb] = t;
         }
-        if (!grid_wait(d.bar, gen)) return;
+        if (!grid_wait(d.bar, gen, spins)) return;
         const double alpha = sum_parts(n_rb, red8[0], [&](int i) { return __ldcg(pa + i); });
         if (blockIdx.x == 0 && threadIdx.x == 0) d.alpha[j] = alpha;
         // K2 on the same rows
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring
             const double t = block_sum(acc, red);
             if (threadIdx.x == 0) pb[rb] = t;
         }
-        if (!grid_wait(d.bar, gen)) return;
+        if (!grid_wait(d.bar, gen, spins)) return;
         double b = sqrt(sum_parts(n_rb, red8[1], [&](int i) { return __ldcg(pb + i); }));
         if constexpr (S == 1) {
             using R = ReorthShape<V>;
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring
                     }
                     __syncthreads();
                 }
-                if (!grid_wait(d.bar, gen)) return;
+                if (!grid_wait(d.bar, gen, spins)) return;
                 // update: four lanes a row load the basis, 64 vectors in flight,
                 // and run the same subtractions in basis order
                 for (int i = threadIdx.x; i <= j; i += blockDim.x) cf[i] = __ldcg(d.coefs + i);
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring
                     }
                     __syncthreads();
                 }
-                if (!grid_wait(d.bar, gen)) return;
+                if (!grid_wait(d.bar, gen, spins)) return;
                 // norm: the row blocks' partials from their eight warps, then as above
                 const int n_w = (int)((n + 31) / 32);
                 b = sqrt(sum_parts(n_rb, red8[2], [&](int rb) {
@@ -647,7 +647,9 @@ void launch_lz_run(const Op& op, V* wbuf, V* vring, int K, const LzDev& d, int s
             int grid = std::min(want, std::min(per_sm, 4) * sms);
             Op o = op;
             LzDev dd = d;
-            void* args[] = {&o, &wbuf, &vring, &K, &dd, &steps, &reorth, &selective, &ritz, &psi};
+            const char* be = std::getenv("QMB_LZ_BAR_SPINS");
+            unsigned spins = be ? (unsigned)std::strtoul(be, nullptr, 10) : kBarSpins;
+            void* args[] = {&o, &wbuf, &vring, &K, &dd, &steps, &reorth, &selective, &spins, &ritz, &psi};
             // any grid does the work; a process that may use fewer SMs than the device
             // has (a service's limit) gets fewer blocks
             cudaError_t e;
