@@ -2232,13 +2232,15 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             qmb_sector sec = d->sectors[s];
             QMB_REQUIRE(sec && sec->has_irrep, QMB_ERR_INVALID, "every sector needs a selected irrep");
             QMB_REQUIRE(sec->device == d->device, QMB_ERR_INVALID, "sectors must live on the batch device");
-            qmb_ham hx = nullptr, hz = nullptr;
-            qmb_status st = qmb_ham_create(sec, d->terms_xy, QMB_PREC_FP64, &hx);
-            if (st != QMB_OK) throw Error{st, std::string("terms_xy: ") + qmb_last_error()};
-            std::unique_ptr<qmb_ham_s> ox(hx);
-            st = qmb_ham_create(sec, d->terms_z, QMB_PREC_FP64, &hz);
-            if (st != QMB_OK) throw Error{st, std::string("terms_z: ") + qmb_last_error()};
-            std::unique_ptr<qmb_ham_s> oz(hz);
+            auto build = [&](const qmb_terms* t, const char* name) {
+                try {
+                    return ham_create(sec, t, QMB_PREC_FP64, false);  // only the plain entries are read
+                } catch (const Error& e) {
+                    throw Error{e.code, std::string(name) + ": " + e.msg};
+                }
+            };
+            const std::unique_ptr<qmb_ham_s> ox = build(d->terms_xy, "terms_xy"), oz = build(d->terms_z, "terms_z");
+            const qmb_ham hx = ox.get(), hz = oz.get();
             QMB_REQUIRE(hz->nnz == 0, QMB_ERR_INVALID, "terms_z must be diagonal");
             ms_build += ms_since(t_part);
             t_part = std::chrono::steady_clock::now();

@@ -1281,30 +1281,36 @@ static bool terms_complex(const qmb_terms* t) {
     return false;
 }
 
+namespace qmb {
+std::unique_ptr<qmb_ham_s> ham_create(qmb_sector s, const qmb_terms* terms, int prec, bool coded) {
+    QMB_REQUIRE(s->has_irrep, QMB_ERR_INVALID, "select an irrep before building H");
+    QMB_REQUIRE((prec & (QMB_PREC_FP64 | QMB_PREC_FP32)) != 0, QMB_ERR_INVALID,
+                "prec must include QMB_PREC_FP64 and/or QMB_PREC_FP32");
+    QMB_REQUIRE(s->n_active > 0, QMB_ERR_INVALID, "the selected irrep has no active orbit");
+    QMB_REQUIRE(s->n_active < (1ll << 32), QMB_ERR_UNSUPPORTED, "more than 2^32 rows");
+    DeviceGuard dg(s->device);
+    auto h = std::make_unique<qmb_ham_s>();
+    h->sector = s;
+    h->device = s->device;
+    h->n = s->n_active;
+    h->irrep_gen = s->irrep_gen;
+    h->prec = prec;
+    h->cplx = !s->is_real || terms_complex(terms);
+    upload_terms(h.get(), terms, s->L);
+    h->err.alloc(1);
+    h->err.zero();
+    build_sell(h.get(), terms);
+    if (coded) build_cb(h.get());
+    return h;
+}
+}  // namespace qmb
+
 extern "C" qmb_status qmb_ham_create(qmb_sector s, const qmb_terms* terms, int prec,
                                      qmb_ham* out) {
     return guarded([&] {
         QMB_REQUIRE(s && terms && out, QMB_ERR_INVALID, "null argument");
         *out = nullptr;
-        QMB_REQUIRE(s->has_irrep, QMB_ERR_INVALID, "select an irrep before building H");
-        QMB_REQUIRE((prec & (QMB_PREC_FP64 | QMB_PREC_FP32)) != 0, QMB_ERR_INVALID,
-                    "prec must include QMB_PREC_FP64 and/or QMB_PREC_FP32");
-        QMB_REQUIRE(s->n_active > 0, QMB_ERR_INVALID, "the selected irrep has no active orbit");
-        QMB_REQUIRE(s->n_active < (1ll << 32), QMB_ERR_UNSUPPORTED, "more than 2^32 rows");
-        DeviceGuard dg(s->device);
-        auto h = std::make_unique<qmb_ham_s>();
-        h->sector = s;
-        h->device = s->device;
-        h->n = s->n_active;
-        h->irrep_gen = s->irrep_gen;
-        h->prec = prec;
-        h->cplx = !s->is_real || terms_complex(terms);
-        upload_terms(h.get(), terms, s->L);
-        h->err.alloc(1);
-        h->err.zero();
-        build_sell(h.get(), terms);
-        build_cb(h.get());
-        *out = h.release();
+        *out = ham_create(s, terms, prec, true).release();
     });
 }
 

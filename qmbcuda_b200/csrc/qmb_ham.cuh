@@ -1,6 +1,7 @@
 // qmb_ham.cuh -- Hamiltonian storage and the row operators used by H*v.
 #pragma once
 #include <cstdlib>
+#include <memory>
 #include <type_traits>
 
 #include "qmb_scalar.cuh"
@@ -1115,6 +1116,8 @@ void mf_tables(qmb_ham_s* h);
 void hop_form(qmb_ham_s* h, const qmb_terms* t);
 // The coded FP32 layout of a built matrix, when it pays (CbSellOp).
 void build_cb(qmb_ham_s* h);
+// qmb_ham_create() without a status; coded: with the coded layouts of products.
+std::unique_ptr<qmb_ham_s> ham_create(qmb_sector s, const qmb_terms* terms, int prec, bool coded);
 // Upload operator tables (validated) into the handle's term buffers.
 void upload_terms(qmb_ham_s* h, const qmb_terms* t, int L);
 int grid_for(int64_t n, int block);
