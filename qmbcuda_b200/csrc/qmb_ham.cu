@@ -475,7 +475,7 @@ __global__ void k_ell_ref(RowGen rg, int64_t R, int W, uint32_t* __restrict__ in
 }
 
 template <class Op, class V, int S>
-__global__ void __launch_bounds__(256, OpMinBlocks<Op>::value) k_hv(Op op, const V* __restrict__ x, V* __restrict__ y) {
+__global__ void __launch_bounds__(256, OpMinBlocks<Op, S>::value) k_hv(Op op, const V* __restrict__ x, V* __restrict__ y) {
     extern __shared__ __align__(16) unsigned char smem_hv[];
     op.init(smem_hv);
     for_rows<S>(op, x, [&](int64_t r, V hx, V) { y[r] = hx; });
@@ -1432,13 +1432,19 @@ void hv_dispatch(const qmb_ham_s* h, int prec, const void* x, void* y, cudaStrea
             }
             return;
         }
-        if (h->cplx) {
-            if (f64) { auto op = h->mf<double2>(); launch_hv(op, (const double2*)x, (double2*)y, st, op.smem_bytes()); }
-            else { auto op = h->mf<float2>(); launch_hv(op, (const float2*)x, (float2*)y, st, op.smem_bytes()); }
-        } else {
-            if (f64) { auto op = h->mf<double>(); launch_hv(op, (const double*)x, (double*)y, st, op.smem_bytes()); }
-            else { auto op = h->mf<float>(); launch_hv(op, (const float*)x, (float*)y, st, op.smem_bytes()); }
-        }
+        auto run = [&](auto wide) {
+            constexpr bool W = decltype(wide)::value;
+            auto go = [&](const auto& op, const auto* xv, auto* yv) { launch_hv(op, xv, yv, st, op.smem_bytes()); };
+            if (h->cplx) {
+                if (f64) go(h->mf<double2, W>(), (const double2*)x, (double2*)y);
+                else go(h->mf<float2, W>(), (const float2*)x, (float2*)y);
+            } else {
+                if (f64) go(h->mf<double, W>(), (const double*)x, (double*)y);
+                else go(h->mf<float, W>(), (const float*)x, (float*)y);
+            }
+        };
+        if (h->sector->L > 32) run(std::true_type{});
+        else run(std::false_type{});
         return;
     }
     QMB_REQUIRE(f64 ? h->val64.p != nullptr : h->val32.p != nullptr, QMB_ERR_INVALID,

@@ -442,6 +442,10 @@ struct ActiveLookup {
             if (all_active) return -1;
             return find_rep(rg.rt, r) < 0 ? -1 : 0;  // a null orbit, or outside the sector
         }
+        return find_table(rg, r, idx, f);
+    }
+    // the same without windows
+    __device__ __forceinline__ int find_table(const RowGen& rg, uint64_t r, int64_t* idx, double* f) const {
         if (hash) {
             uint64_t slot = mf_hash_slot(r, hmask);
             for (uint64_t it = 0; it <= hmask; ++it) {
@@ -576,6 +580,14 @@ struct ActiveLookup {
     }
 };
 
+// ActiveLookup without its windows, for gen_row_look().
+struct TableLookup {
+    const ActiveLookup& look;
+    __device__ __forceinline__ int find(const RowGen& rg, uint64_t r, int64_t* idx, double* f) const {
+        return look.find_table(rg, r, idx, f);
+    }
+};
+
 // Two-site exchange ("hop") form of a term table, for the matrix-free
 // operator: every off-diagonal term is c S+_i S-_j at two distinct sites and
 // every other term is diagonal (SZ and identity operators only).  Hops on the
@@ -609,7 +621,12 @@ struct CbLayout {
 // set bits are walked, so the threads of a warp run the orbit search and the
 // lookup together instead of at the term where each finds an entry.  Up to
 // 32 sites the strings, masks, representatives and row indices are 32-bit.
-template <class M>
+//
+// Wide is for strings beyond 32 sites.  The two forms are kernels of their own: with
+// both in one, the registers of the window lookup cost the wide form spills (6x6
+// lattice 183.0 -> 187.6 ms a product, 34-site chain 101.9 -> 105.9, 4x9 18.4 -> 19.1;
+// apart 181, 95.5 and 17.4, and the 32-site chain 3.42 -> 3.39).
+template <class M, bool Wide = false>
 struct MfOp {
     using scalar = M;
     int64_t n;
@@ -674,7 +691,7 @@ struct MfOp {
                 const uint64_t rr = orbit_min(rg.g, gs, src ^ pair, &e);
                 int64_t c;
                 double f;
-                const int found = look.find(rg, rr, &c, &f);
+                const int found = look.find_table(rg, rr, &c, &f);
                 if (found <= 0) {
                     if (found < 0) *rg.err = 2;
                     continue;
@@ -795,20 +812,25 @@ struct MfOp {
     // with a hop table part 0 holds the diagonal.
     template <int S, bool LIVE = false, class V>
     __device__ __forceinline__ V part(int64_t r, const V* __restrict__ x, int p) const {
-        const uint64_t rep = look.reps32 ? (uint64_t)look.reps32[r] : look.reps64[r];
+        uint64_t rep;
+        if constexpr (Wide) rep = look.reps64[r];
+        else rep = look.reps32[r];
         const uint64_t src = apply_elem(rg.g, gs, 0, rep);
         const V* __restrict__ xsv = reinterpret_cast<const V*>(xs);
         V acc;
         double2 d = make_double2(0.0, 0.0);
         if (n_hops) {
-            acc = look.reps32 ? hop_sum32x2<S, V>((uint32_t)src, xsv, p) : hop_sum64<S, V>(src, xsv, p);
+            if constexpr (Wide) acc = hop_sum64<S, V>(src, xsv, p);
+            else acc = hop_sum32x2<S, V>((uint32_t)src, xsv, p);
             if (p == 0)
                 d = cplx ? reinterpret_cast<const double2*>(diag)[r]
                          : make_double2(reinterpret_cast<const double*>(diag)[r], 0.0);
         } else {
             acc = Sc<V>::zero();
-            d = gen_row_look(rg, gs, ts, ts.n_terms * p / S, ts.n_terms * (p + 1) / S, src, look,
-                             [&](int64_t c, double2 v) { acc = Sc<V>::fma(Sc<V>::from(v), __ldg(xsv + c), acc); });
+            auto add = [&](int64_t c, double2 v) { acc = Sc<V>::fma(Sc<V>::from(v), __ldg(xsv + c), acc); };
+            const int h0 = ts.n_terms * p / S, h1 = ts.n_terms * (p + 1) / S;
+            if constexpr (Wide) d = gen_row_look(rg, gs, ts, h0, h1, src, TableLookup{look}, add);
+            else d = gen_row_look(rg, gs, ts, h0, h1, src, look, add);
         }
         acc = Sc<V>::scale(acc, 1.0 / nrow[r]);
         if (n_hops && p) return acc;
@@ -817,15 +839,18 @@ struct MfOp {
 };
 
 // Minimum resident blocks of 256 threads a product kernel over Op is compiled
-// for: the matrix-free operator is issue- and latency-bound and runs best at
-// five (at most 48 registers a thread).
-template <class Op> struct OpMinBlocks { static constexpr int value = 1; };
-template <class M> struct OpMinBlocks<MfOp<M>> { static constexpr int value = 5; };
+// for, S threads a row: the matrix-free operator is issue- and latency-bound and runs
+// best at five (at most 48 registers a thread), beyond 32 sites with whole rows at
+// six, where the random reads of tables larger than L2 bound it (6x6: 201 ms at four
+// blocks, 185.4 at five, 181 at six; 34-site chain 95.6 / 95.4 and 4x9 17.3 / 17.35 at
+// five / six; split rows, 16,451 of 4x10: 0.105 / 0.110).
+template <class Op, int S> struct OpMinBlocks { static constexpr int value = 1; };
+template <class M, bool W, int S> struct OpMinBlocks<MfOp<M, W>, S> { static constexpr int value = W && S == 1 ? 6 : 5; };
 // The coded operator hides its gathers' latency with warps: six blocks (40
 // registers) against four take the L=30 J1-J2 FP64 product from 216 to 188 us
 // and leave the FP32 one (L=32: 318 against 322 us) as it is.  Deeper unrolling
 // or loading the next entries ahead changed neither.
-template <class M> struct OpMinBlocks<CbSellOp<M>> { static constexpr int value = 6; };
+template <class M, int S> struct OpMinBlocks<CbSellOp<M>, S> { static constexpr int value = 6; };
 
 // How a product's rows are spread over threads.  One thread a row leaves most
 // of the chip idle below some 10^5 rows, and each thread then walks its row's
@@ -847,9 +872,9 @@ template <class M> struct OpSplit<SellOp<M>> {
     static constexpr bool lanes = false;
     static int of(const SellOp<M>& op) { return op.n < 16384 ? 4 : op.n < (sizeof(M) == 16 ? 640000 : 300000) ? 2 : 1; }
 };
-template <class M> struct OpSplit<MfOp<M>> {
+template <class M, bool W> struct OpSplit<MfOp<M, W>> {
     static constexpr bool lanes = false;
-    static int of(const MfOp<M>& op) { return op.n < 16384 ? 8 : op.n < 131072 ? 4 : op.n < 400000 ? 2 : 1; }
+    static int of(const MfOp<M, W>& op) { return op.n < 16384 ? 8 : op.n < 131072 ? 4 : op.n < 400000 ? 2 : 1; }
 };
 template <class M> struct OpSplit<RefEllOp<M>> {
     static constexpr bool lanes = true;
@@ -857,7 +882,7 @@ template <class M> struct OpSplit<RefEllOp<M>> {
 };
 template <class Op> struct OpMaxSplit { static constexpr int value = 1; };
 template <class M> struct OpMaxSplit<SellOp<M>> { static constexpr int value = 4; };
-template <class M> struct OpMaxSplit<MfOp<M>> { static constexpr int value = 8; };
+template <class M, bool W> struct OpMaxSplit<MfOp<M, W>> { static constexpr int value = 8; };
 template <class M> struct OpMaxSplit<RefEllOp<M>> { static constexpr int value = 4; };
 
 // Dynamic shared memory up to which a kernel may split rows: the sums of the split
@@ -951,9 +976,9 @@ __global__ void __launch_bounds__(256) k_mf_scale(int64_t n, const double* __res
         xs[r] = Sc<V>::scale(x[r], nrow[r]);
 }
 
-template <class M>
+template <class M, bool Wide>
 template <class V>
-void MfOp<M>::pre(const V* x0, const int* iter, cudaStream_t s) const {
+void MfOp<M, Wide>::pre(const V* x0, const int* iter, cudaStream_t s) const {
     k_mf_scale<V><<<grid_for(n, 256), 256, 0, s>>>(n, nrow, x0, iter, reinterpret_cast<V*>(xs));
 }
 
@@ -1073,8 +1098,8 @@ struct qmb_ham_s {
         return op;
     }
     // the matrix-free operator (mf_tables() must have run)
-    template <class M> qmb::MfOp<M> mf() const {
-        qmb::MfOp<M> op;
+    template <class M, bool Wide = false> qmb::MfOp<M, Wide> mf() const {
+        qmb::MfOp<M, Wide> op;
         op.n = n;
         op.rg = row_gen();
         op.look.win = mf_win.p;

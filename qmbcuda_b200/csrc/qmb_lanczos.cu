@@ -104,7 +104,7 @@ __global__ void k_lz_start(int64_t n, int mode, uint64_t seed, const P* __restri
 // K1: y = H w_j / beta_j - beta_j v_{j-1}; v_j = w_j / beta_j; alpha_j = Re <v_j, y>.
 // Optionally psi += c_j v_j (eigenvector regeneration).
 template <class Op, class V, class P, int S>
-__global__ void __launch_bounds__(kLzBlock, OpMinBlocks<Op>::value) k_lz_hv(Op op, V* __restrict__ wbuf, V* __restrict__ vring,
+__global__ void __launch_bounds__(kLzBlock, OpMinBlocks<Op, S>::value) k_lz_hv(Op op, V* __restrict__ wbuf, V* __restrict__ vring,
                                                     int K, LzDev d, const double* __restrict__ ritz,
                                                     P* __restrict__ psi) {
     extern __shared__ __align__(16) unsigned char smem_lz[];
@@ -1315,9 +1315,9 @@ extern "C" qmb_status qmb_lanczos(qmb_ham h, const qmb_lanczos_opts* opts, qmb_l
                 k(h->sell<D>(true), (size_t)0);
             };
             if (mf) {
-                auto a = h->mf<R>();
-                auto b = h->mf<D>();
-                run(a, a.smem_bytes(), b, b.smem_bytes());
+                auto both = [&](const auto& a, const auto& b) { run(a, a.smem_bytes(), b, b.smem_bytes()); };
+                if (h->sector->L > 32) both(h->mf<R, true>(), h->mf<D, true>());
+                else both(h->mf<R>(), h->mf<D>());
             } else if (!need32) {
                 op64([&](const auto& b, size_t sb) { run(b, sb, b, sb); });
             } else if (!need64) {
