@@ -358,10 +358,15 @@ struct GridBar {
     unsigned arrived, gen;
     int err;
 };
-// Rows up to which the resident kernel runs the steps.  A step of 2,704, 112,720
-// and 208,012 rows takes 9.1, 17 and 22 us against 12.9, 21 and 26 with a graph of
-// two launches; beyond, the vectors leave L2 and the launches no longer count.
+// Rows up to which the resident kernel runs the steps: 50 steps of 12,870, 112,720 and
+// 208,012 rows take 1.00, 1.35 and 1.86 ms against 1.23, 1.54 and 2.11 with a graph of
+// two launches; its two partial arrays end at this many.  With reorthogonalisation
+// it walks the basis in 256-row units, which pays while those are few: 60 steps of
+// 43,263 (complex), 48,620, 65,780, 112,720 and 184,756 rows take 3.44, 3.15, 3.81,
+// 4.65 and 6.71 ms against 4.20, 3.37, 3.54, 3.81 and 4.34 with launches, 112,632
+// complex rows 5.87 against 5.34.
 constexpr int64_t kRunMaxRows = 262144;
+constexpr int64_t kRunMaxRowsReorth = 57344, kRunMaxRowsReorthCplx = 81920;
 constexpr int kRunParts = 2048;  // row blocks at most
 constexpr unsigned kBarSpins = 1u << 23;  // polls of about 0.5 us (QMB_LZ_BAR_SPINS=n: n, tests of the give-up)
 
@@ -619,10 +624,12 @@ __global__ void __launch_bounds__(kLzBlock, 4) k_lz_run(Op op, V* wbuf, V* vring
 template <class Op> struct RunsResident { static constexpr bool value = false; };
 template <class M> struct RunsResident<SellOp<M>> { static constexpr bool value = true; };
 template <class M> struct RunsResident<RefEllOp<M>> { static constexpr bool value = true; };
-template <class Op>
-inline bool runs_resident(const Op& op) {
+template <class V, class Op>
+inline bool runs_resident(const Op& op, int reorth) {
+    if (!RunsResident<Op>::value) return false;
+    if (reorth) return op.n <= (Sc<V>::cplx ? kRunMaxRowsReorthCplx : kRunMaxRowsReorth);
     // row blocks of 256 / S rows, each with its place in the two partial arrays
-    return RunsResident<Op>::value && op.n <= kRunMaxRows && (op.n * OpSplit<Op>::of(op) + 255) / 256 <= kRunParts;
+    return op.n <= kRunMaxRows && (op.n * OpSplit<Op>::of(op) + 255) / 256 <= kRunParts;
 }
 
 // `steps` Lanczos steps from *d.iter in one cooperative launch.
@@ -729,7 +736,7 @@ struct LzState {
         partials.alloc(std::max<size_t>(2 * (size_t)nb, 2 * kRunParts));
         bar.alloc(1);
         bar.zero(s);
-        wsum.alloc(reorth ? kRunMaxRows / 32 + 8 : 1);
+        wsum.alloc(reorth ? kRunMaxRowsReorthCplx / 32 + 8 : 1);
         chunk_ctr.alloc(reorth ? (size_t)cap / 8 + 2 : 1);
         chunk_ctr.zero(s);
         scratch.alloc(4);
@@ -740,7 +747,7 @@ struct LzState {
         iter.zero(s);
         coefs.alloc(reorth ? cap + 2 : 1);
         // a partial a block (or, resident, a row block of 256 rows) and basis vector
-        cpart.alloc(reorth ? 2 * std::max<size_t>(nb, kRunMaxRows / 256) * (cap + 2) : 1);
+        cpart.alloc(reorth ? 2 * std::max<size_t>(nb, kRunMaxRowsReorthCplx / 256) * (cap + 2) : 1);
         d.alpha = alpha.p;
         d.beta = beta.p;
         d.iter = iter.p;
@@ -758,6 +765,7 @@ struct LzState {
 };
 
 struct PhaseOut {
+    bool resident = false;  // the steps ran in the resident kernel
     int m = 0;            // Lanczos vectors used (tridiagonal size)
     double theta = 0.0;
     double est = 0.0;     // residual estimate beta_m |s_{m-1}|
@@ -877,7 +885,8 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
 
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
-    const bool resident = runs_resident(op);
+    const bool resident = runs_resident<V>(op, po.reorth);
+    out.resident = resident;
     auto capture = [&]() {
         if (resident) return;
         if (exec) cudaGraphExecDestroy(exec);
@@ -1043,7 +1052,7 @@ void ritz_vector(const Op& op, size_t op_smem, const PhaseOut& ph, int start_mod
     QMB_CUDA_TRY(cudaMemsetAsync(psi, 0, sizeof(P) * n, s));
     const int nb = st.nb;
     k_lz_start<V, P><<<nb, kLzBlock, 0, s>>>(n, start_mode, seed, from, wbuf.p, st.d);
-    if (runs_resident(op)) {  // as the phase ran
+    if (ph.resident) {
         launch_lz_run<Op, V, P>(op, wbuf.p, vring.p, K, st.d, ph.m, ph.m, 0, 0, ritz.p, psi, s);
         g_lz_kernels += 2;
         n_hv += ph.m;
@@ -1386,11 +1395,13 @@ extern "C" qmb_status qmb_eigvec_from_seed_ref(long long seed, void* psi_dev, co
         if (is_complex) {
             RefEllOp<float2> op{nobv, max_terms, ind_dev, (const float2*)val_dev, track_dev};
             DevBuf<float2> vr(2 * (size_t)nobv), wb(2 * (size_t)nobv);
+            ph.resident = runs_resident<float2>(op, 0);
             ritz_vector<RefEllOp<float2>, float2, float2>(op, 0, ph, QMB_START_CURAND, (uint64_t)seed, nullptr,
                                                           false, vr, 2, wb, st, (float2*)psi_dev, n_hv, s);
         } else {
             RefEllOp<float> op{nobv, max_terms, ind_dev, (const float*)val_dev, track_dev};
             DevBuf<float> vr(2 * (size_t)nobv), wb(2 * (size_t)nobv);
+            ph.resident = runs_resident<float>(op, 0);
             ritz_vector<RefEllOp<float>, float, float>(op, 0, ph, QMB_START_CURAND, (uint64_t)seed, nullptr,
                                                        false, vr, 2, wb, st, (float*)psi_dev, n_hv, s);
         }
@@ -1513,7 +1524,7 @@ void na_solve(unsigned char* base, const RefEllOp<V>& op, int n_iter, uint64_t s
     d.chunk_ctr = nullptr;
     d.bar = reinterpret_cast<GridBar*>(d.counter + 4);
     const int K = 2;
-    const bool resident = runs_resident(op);
+    const bool resident = runs_resident<V>(op, 0);
     // the reduction counters must start at zero (an interrupted earlier call
     // may have left them set)
     QMB_CUDA_TRY(cudaMemsetAsync(d.counter, 0, 4 * sizeof(unsigned) + sizeof(GridBar), s));
