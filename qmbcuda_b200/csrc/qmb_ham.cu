@@ -663,10 +663,12 @@ constexpr int kCbMaxBlocks = 32;                     // column blocks at most
 constexpr size_t kCbBlockBytes = (size_t)64 << 20;   // x bytes of one column block
 constexpr double kCbMinVecBytes = 256.0 * (1 << 20); // vectors from this size on (2x L2)
 // single block: plain entries from this size on.  Below L2's size the coded
-// entries still pay, by three times fewer bytes from L2 (us a product, plain /
-// coded: 40 MB complex FP32 10.3 / 9.4, 115 MB 19.3 / 12.4, 176 MB real FP32 42.7 /
-// 26.7, 320 MB 47.1 / 26.7; at 20 MB both take 8.3).
-constexpr double kCbMinStreamBytes = 32.0 * (1 << 20);
+// entries still pay, by two to three times fewer bytes from L2 (us a product, plain /
+// coded: 40 MB complex FP32 10.3 / 9.4, 115 MB 19.3 / 12.4; real FP64 55 MB 10.5 / 10.4,
+// 76 MB 26.7 / 14.5; at 20 MB both take 8.3).  Real FP32 entries are 8 bytes, and their
+// rows split over two threads in the plain layout only: 36 MB 8.4 / 8.9, 55 MB 10.5 /
+// 12.1, 67 MB 12.6 / 13.5, 74 MB 20.6 / 14.6, 92 MB 26.8 / 16.7, 176 MB 42.7 / 26.7.
+constexpr double kCbMinStreamBytes = 32.0 * (1 << 20), kCbMinStreamBytesReal32 = 70.0 * (1 << 20);
 constexpr double kCbMaxSingleVecBytes = 96.0 * (1 << 20);  // single FP64 block: x bytes up to this (L2 126 MB)
 constexpr int kCbMissCap = 1024;                     // values outside the dictionary kept per pass
 
@@ -1057,8 +1059,9 @@ static void share_cb64_t(qmb_ham_s* h) {
 //
 // The same layout with one block (every column in the 24-bit field) serves a
 // matrix whose vectors fit L2 but whose entry stream is large (the plain FP32
-// entries, 8 or 12 bytes, at least kCbMinStreamBytes): its 32-bit coded entries
-// halve (real) or third (complex) the bytes a product streams.
+// entries, 8 or 12 bytes, at least kCbMinStreamBytesReal32 or kCbMinStreamBytes):
+// its 32-bit coded entries halve (real) or third (complex) the bytes a product
+// streams.
 //
 // QMB_CB_SHIFT=s (10..24) builds the layout with blocks of 2^s rows for any
 // matrix with at least two blocks, whatever its size (small cases exercise
@@ -1073,7 +1076,8 @@ void build_cb(qmb_ham_s* h) {
     }
     const bool blocked = (double)h->n * (h->cplx ? 8 : 4) >= kCbMinVecBytes;
     const bool single = !blocked && h->n <= ((int64_t)1 << 24) &&
-                        (double)h->padded * (h->cplx ? 12 : 8) >= kCbMinStreamBytes;
+                        (h->cplx ? (double)h->padded * 12 >= kCbMinStreamBytes
+                                 : (double)h->padded * 8 >= kCbMinStreamBytesReal32);
     if ((h->prec & QMB_PREC_FP32) && h->val32.p && (forced || blocked || single)) {
         if (h->cplx) build_cb_t<float2>(h, forced, single && !forced, h->cb32);
         else build_cb_t<float>(h, forced, single && !forced, h->cb32);
