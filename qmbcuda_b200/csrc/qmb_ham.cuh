@@ -865,7 +865,9 @@ template <class M, int S> struct OpMinBlocks<CbSellOp<M>, S> { static constexpr 
 // against the split): sliced ELL 9,225 rows 4.6 / 4.5 (S = 4), 112,640 10.3 / 8.2
 // and 208,012 10.3 / 8.2 (S = 2), 400,023 complex FP64 49.2 / 34.3 but FP32 real
 // 22.4 / 23.5; matrix-free 2,703 rows 26.2 / 14.0 (S = 8), 32,065 34.8 / 22.5 and
-// 112,632 112 / 96 (S = 4), 208,012 190 / 162 (S = 2), 716,728 369 / 379; row-major
+// 112,632 112 / 96 (S = 4), 208,012 190 / 162 (S = 2), 716,728 369 / 379; matrix-free
+// without a group, where an entry needs no orbit minimum, 43,758 rows 30.8 / 22.7
+// (S = 2) / 22.6 (S = 4), 92,378 24.8 / 22.7 / 24.9, 167,960 30.9 / 32.9; row-major
 // ELL, 50 steps of 9,252 rows 2.00 / 1.79 ms and of 112,720 rows 2.42 / 2.29 (S = 4).
 template <class Op> struct OpSplit { static constexpr bool lanes = false; static int of(const Op&) { return 1; } };
 template <class M> struct OpSplit<SellOp<M>> {
@@ -874,7 +876,10 @@ template <class M> struct OpSplit<SellOp<M>> {
 };
 template <class M, bool W> struct OpSplit<MfOp<M, W>> {
     static constexpr bool lanes = false;
-    static int of(const MfOp<M, W>& op) { return op.n < 16384 ? 8 : op.n < 131072 ? 4 : op.n < 400000 ? 2 : 1; }
+    static int of(const MfOp<M, W>& op) {
+        if (op.rg.g.n_ext == 1) return op.n < 16384 ? 8 : op.n < 40000 ? 4 : op.n < 131072 ? 2 : 1;
+        return op.n < 16384 ? 8 : op.n < 131072 ? 4 : op.n < 400000 ? 2 : 1;
+    }
 };
 template <class M> struct OpSplit<RefEllOp<M>> {
     static constexpr bool lanes = true;

@@ -19,8 +19,9 @@ def test_split_and_whole_rows(tmp_path):
         name, n, s, whole = line.split()
         assert whole == "1", line
         got[name, int(n)] = int(s)
-    assert len(got) == 55
+    assert len(got) == 78
     for (name, n), s in got.items():
         want = {"sell": 4 if n < 16384 else 2 if n < 300000 else 1, "sell_c64": 4 if n < 16384 else 2 if n < 640000 else 1,
-                "mf": 8 if n < 16384 else 4 if n < 131072 else 2 if n < 400000 else 1, "ref_ell": 4, "coded": 1}[name]
+                "mf": 8 if n < 16384 else 4 if n < 131072 else 2 if n < 400000 else 1,
+                "mf_no_group": 8 if n < 16384 else 4 if n < 40000 else 2 if n < 131072 else 1, "ref_ell": 4, "coded": 1}[name]
         assert s == want, (name, n, s)
