@@ -507,8 +507,8 @@ QMB_API qmb_status qmb_batch_k1_time(qmb_batch b, int prec, int reps, double* ms
  * a quarter of the complex sectors' rows are stored and solved complex, with
  * zero imaginary parts); each sector is [row][set] with set stride
  * info.set_stride.  offsets[s] is the
- * start of caller sector s in scalars (a complex element counts 2; the order of
- * the sectors inside a kind is the library's);
+ * start of caller sector s in scalars (a complex element counts 2), the
+ * sectors of a kind in the caller's order;
  * offsets[n_sectors] is the total. */
 QMB_API qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets /* [n_sectors+1] */,
                             int* is_complex /* [n_sectors] */);

@@ -1098,7 +1098,8 @@ struct BKind {
     int n_sectors = 0, n_all = 0;
     std::vector<int> sec_index;        // [n_all] positions in the caller's sector list
     std::vector<int64_t> nrows;        // [n_all] per sector
-    std::vector<int64_t> sec_elem;     // [n_all+1]
+    std::vector<int64_t> sec_elem;     // [n_all+1] where a solve keeps the sectors' vectors
+    std::vector<int64_t> hv_elem;      // [n_all+1] where the caller's vectors have them (qmb_batch_layout)
     std::vector<int> tile_sector, tile_row0, sec_tile0, sec_ntiles;
     DevBuf<int> d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active;
     DevBuf<unsigned> d_ctr;      // work queue head, retired blocks, update blocks done
@@ -1108,7 +1109,7 @@ struct BKind {
     DevBuf<unsigned char> ws_ring;  // Lanczos vectors kept between solves
     std::unique_ptr<BKind> compact;        // descriptor of the last compacted sub-batch
     float tune_ms[2][8] = {};  // tuner timings per precision and variant
-    DevBuf<int64_t> d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0;
+    DevBuf<int64_t> d_sec_elem, d_hv_elem, d_nrows, d_row_ptr, d_row_base, d_row0;
     std::vector<int64_t> h_row_base, h_row0;  // per sector, as on the device
     DevBuf<uint32_t> d_col;
     DevBuf<unsigned char> val64, val32, dxy64, dxy32, dz64, dz32;
@@ -1119,7 +1120,7 @@ struct BKind {
 
     void mark_idle() {
         qmb::mark_idle(d_tile_sector, d_tile_row0, d_sec_tile0, d_sec_ntiles, d_tiles, d_active, d_ctr, d_sec_ctr, ws_ring,
-                       d_sec_elem, d_nrows, d_row_ptr, d_row_base, d_row0, d_col, val64, val32, dxy64, dxy32, dz64,
+                       d_sec_elem, d_hv_elem, d_nrows, d_row_ptr, d_row_base, d_row0, d_col, val64, val32, dxy64, dxy32, dz64,
                        dz32);
         if (compact) compact->mark_idle();
     }
@@ -2354,6 +2355,14 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
                 if (ks < K.n_sectors) K.n_tiles = (int)K.tile_sector.size();
             }
             if (!K.n_all) continue;
+            // the caller's vectors: sectors in the caller's order
+            K.hv_elem.assign(K.n_all + 1, K.sec_elem.back());
+            int64_t at = 0;
+            for (int s = 0; s < d->n_sectors; ++s)
+                if (b->sector_kind[s] == kd) {
+                    K.hv_elem[b->sector_pos[s]] = at;
+                    at += K.nrows[b->sector_pos[s]] * b->nsp;
+                }
             K.nnz = n_ent;
             K.n_tiles_all = (int)K.tile_sector.size();
             std::vector<int> tiles(K.n_tiles_all);
@@ -2371,6 +2380,7 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
             K.d_sec_ctr.alloc(K.n_all);
             K.d_sec_ctr.zero();
             up_l(K.d_sec_elem, K.sec_elem);
+            up_l(K.d_hv_elem, K.hv_elem);
             up_l(K.d_nrows, K.nrows);
             up_l(K.d_row_base, row_base);
             up_l(K.d_row0, row0);
@@ -2478,7 +2488,7 @@ extern "C" qmb_status qmb_batch_layout(qmb_batch b, int64_t* offsets, int* is_co
             int kd = b->sector_kind[s];
             const BKind& k = b->kind[kd];
             int ks = b->sector_pos[s];
-            offsets[s] = kd ? r_elems + 2 * k.sec_elem[ks] : k.sec_elem[ks];
+            offsets[s] = kd ? r_elems + 2 * k.hv_elem[ks] : k.hv_elem[ks];
             if (is_complex) is_complex[s] = kd;
         }
         if (b->kind[1].n_all) end = r_elems + 2 * b->kind[1].sec_elem[b->kind[1].n_all];
@@ -2498,7 +2508,8 @@ static void batch_hv_kind(qmb_batch_s* b, BKind& k, bool f64, const V* x, V* y, 
     a.dxy = f64 ? k.dxy64.p : k.dxy32.p;
     a.dz = f64 ? k.dz64.p : k.dz32.p;
     BLz lz{nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr};
-    int v = tuned_variant<V>(a, k, f64, st);
+    int v = tuned_variant<V>(a, k, f64, st);  // (on vectors of its own)
+    a.sec_elem = k.d_hv_elem.p;
     // the multi-slice variants read 32- or 64-byte runs: caller vectors that
     // are only 16-byte aligned take a one-slice variant
     if ((((uintptr_t)x | (uintptr_t)y) & 63) && kBSlices[v] > 1) v = 0;
