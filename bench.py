@@ -290,7 +290,7 @@ def observables(torch, q, reps=5):
     """Ground-state expectation values (qmb_expval) on the L=24 Heisenberg
     chain, k=0 (112,720 rows): the structure factor <Sz_q Sz_-q> at all 24 q
     (Fourier operators) and the 24 correlators <Sz_0 Sz_j>, 48 operators in one
-    call.  Time of the whole call (host group averaging, chunk staging and the
+    call.  Time of the whole call (sorting the terms into classes and the
     kernels) from CUDA events on the default stream, where it launches, and
     from the wall clock; work = rows x group-averaged terms.  Beside it the
     reference's member-loop rule (oracle restatement, one host thread) on
@@ -342,7 +342,7 @@ def observables(torch, q, reps=5):
     evals = rows * n_terms
     out = {"workload": "L=24 Heisenberg chain ground state, k=0 (%d rows): S(q) at 24 q + 24 <Sz_0 Sz_j>, "
                        "48 operators, %d group-averaged terms" % (rows, n_terms),
-           "kernel": "k_expval (+ k_expval_sum)", "ms_call": ms, "ms_wall": float(np.median(wall)),
+           "kernel": "k_ev_rows, k_ev_diag, k_ev_diag_sum (the terms' classes, each once)", "ms_call": ms, "ms_wall": float(np.median(wall)),
            "row_term_evals_per_s": evals / (ms * 1e-3),
            "S_pi": float(v[L // 2].real), "SzSz_01": float(corr[1]),
            "SzSz_01_times_3L": float(3 * L * corr[1]),

@@ -213,9 +213,9 @@ __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off
 // each row simply in term order, 32 of them touch 17 sectors of 32 bytes on a
 // 26-site J1-J2 sector (FP32) and 12 lines of 128; packed they touch 12 and 8.5,
 // at the same slice widths.  An SM looks up about one line a cycle, so the 8.5
-// lines of a load bound the L=32 J1-J2 product at 0.30 ms.  Measured: that
-// product 383 -> 360 us (FP32), the L=30 one 256 -> 210 us (FP64, with the coded
-// operator's six blocks an SM).
+// lines of a load bound the L=32 J1-J2 product at 0.30 ms.  Measured (products back
+// to back, with the coded operator's six blocks an SM on both sides): that product
+// 347 -> 318 us in FP32 and 473 -> 393 in FP64, the L=30 one 249 -> 195 in FP64.
 //
 // Two passes, a warp a slice.  k_ell_masks tests every term on the 32 rows and
 // keeps a ballot of the rows in which it has an entry (mobile terms only, those
@@ -226,9 +226,9 @@ __global__ void k_ell_fill(RowGen rg, int64_t n, const int64_t* __restrict__ off
 // nowhere is split over the rows' free slots.  Every lane then walks its own
 // terms, so that the orbit searches of a warp run together instead of at the
 // term where each lane finds an entry.  Slices wider than 64 keep term order, and
-// so do sectors without a group: their levels are often degenerate (momenta k and
-// -k, dimer pairs), and which vector of such a level a long solve returns depends
-// on the rounding of its sums.
+// so do sectors without a group.  (There the order of a row's sum, and with it the
+// vector that a long solve returns from a degenerate level, is what it was; packing
+// them has not been measured.)
 constexpr int kPackMaxTerms = 1024;  // mobile terms (7 bytes of shared memory a warp each)
 constexpr int kPackWarps = 4;        // warps a block
 
@@ -846,7 +846,8 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
     SellOp<M> a = h->sell<M>(f64);
     // dictionary from a strided sample of the values, reduced to its distinct
     // nonzero keys on the device (copying the 2^20 samples out and sorting them
-    // on the host was most of a 28-site matrix's build: 28.4 -> 12.8 ms with the fill below)
+    // on the host was most of a 28-site matrix's build beside the allocations: 28.4 -> 12.8 ms
+    // with the fill below, 2.3 with kept buffers)
     // (a value that the sample misses costs a second fill: up to 2^25 slots all are
     // looked at)
     const int64_t n_samp = std::min<int64_t>(h->padded, (int64_t)1 << 25);

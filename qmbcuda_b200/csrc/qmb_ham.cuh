@@ -847,9 +847,9 @@ struct MfOp {
 template <class Op, int S> struct OpMinBlocks { static constexpr int value = 1; };
 template <class M, bool W, int S> struct OpMinBlocks<MfOp<M, W>, S> { static constexpr int value = W && S == 1 ? 6 : 5; };
 // The coded operator hides its gathers' latency with warps: six blocks (40
-// registers) against four take the L=30 J1-J2 FP64 product from 216 to 188 us
-// and leave the FP32 one (L=32: 318 against 322 us) as it is.  Deeper unrolling
-// or loading the next entries ahead changed neither.
+// registers) against four take the L=32 J1-J2 product from 325 to 318 us in FP32 and
+// from 403 to 393 in FP64, the L=30 one from 197 to 195 in FP64 (products back to
+// back).  Deeper unrolling or loading the next entries ahead changed none.
 template <class M, int S> struct OpMinBlocks<CbSellOp<M>, S> { static constexpr int value = 6; };
 
 // How a product's rows are spread over threads.  One thread a row leaves most
@@ -915,8 +915,6 @@ inline void with_split(const Op& op, F&& f, bool whole = false) {
     }
 }
 
-// f(r, (H x)_r, x_r) for every row, by one thread of the row's S.  Every thread
-// of a block of 256 calls it.
 // The 256 / S rows from base on: f(r, (H x)_r, x_r, pre(r)) by one thread a row,
 // with x_r and pre(r) loaded ahead of the row's entries.
 template <int S, bool LIVE, class Op, class V, class Pre, class F>
@@ -957,6 +955,8 @@ __device__ __forceinline__ void row_block(const Op& op, const V* __restrict__ x,
     }
 }
 
+// f(r, (H x)_r, x_r) for every row, by one thread of the row's S.  Every thread
+// of a block of 256 calls it.
 template <int S, class Op, class V, class F>
 __device__ __forceinline__ void for_rows(const Op& op, const V* __restrict__ x, F&& f) {
     const int64_t n = op.n;

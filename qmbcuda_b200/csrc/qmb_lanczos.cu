@@ -345,8 +345,10 @@ __global__ void __launch_bounds__(kLzBlock) k_residual(Op op, const P* __restric
 // convergence test: one cooperative launch, with a grid barrier where a step
 // needs a sum from all blocks.  What bounds it is the chain of L2 round trips (about
 // ten a step, 9 us; five barriers and 30 us with reorthogonalisation).  Measured:
-// 150 reorthogonalised steps of 12,870 rows 10.4 -> 5.2 ms, 100 plain steps of 9,252
-// rows 1.42 -> 0.91 ms, an L=24 solve of 56,450 rows 1.45 -> 1.15 ms.
+// 150 reorthogonalised steps of 12,870 rows 10.4 -> 5.1 ms, 100 plain steps of 9,252
+// rows 1.42 -> 0.91 ms, an L=24 solve of 56,450 rows (51 steps, by the library's
+// events) 1.26 -> 0.93 ms.  Half of such a solve is host work: on a busy host its times
+// spread by more than this.
 //
 // All sums are those of the kernels above, in the same order (a row block of 256
 // threads as a block there, block partials in block order, warps' and lanes'

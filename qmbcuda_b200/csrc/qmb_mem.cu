@@ -14,8 +14,9 @@
 // A buffer taken from here can thus be used on any stream at once.  Every access
 // holds one lock.  The oldest buffers are freed when the total passes the bound
 // and all of them when an allocation fails (which is then tried again);
-// dev_mem_info() counts them as free memory.  A buffer is larger than the request
-// by at most an eighth.
+// dev_mem_info() counts them as free memory, and qmb_trim() gives them back.  Requests
+// are rounded up to 512 bytes, from 1 MB on to 2 MB; a buffer is larger than the rounded
+// request by at most an eighth.
 //
 // A buffer belongs to the context in which it was allocated (DevBuf keeps its
 // identifier, unique in the process) and is kept and handed out in that context
