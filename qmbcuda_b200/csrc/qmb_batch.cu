@@ -1508,9 +1508,9 @@ static LoopOut device_loop(StepFn&& step, const BatchArgs& a, const BLz& lz, int
     open_cnt.zero(st);
     QMB_CUDA_TRY(cudaMemsetAsync(active_next, 0, sizeof(int) * n_sectors, st));
     const int max_loops = (cap - j0) / check + 1;
-    if (host_loop()) {
-        // the same blocks launched from the host, with the loop control read
-        // back after each (QMB_HOST_LOOP=1: every kernel visible to a profiler)
+    // the same blocks launched from the host, with the loop control read back after
+    // each (QMB_HOST_LOOP=1: every kernel visible to a profiler)
+    auto from_host = [&]() {
         LoopCtl hc{};
         for (;;) {
             for (int t = 0; t < check; ++t) step(st);
@@ -1532,7 +1532,8 @@ static LoopOut device_loop(StepFn&& step, const BatchArgs& a, const BLz& lz, int
         out.reason = hc.reason;
         out.products = hc.products;
         return out;
-    }
+    };
+    if (host_loop()) return from_host();
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ex = nullptr;
     struct GG {
@@ -1558,15 +1559,30 @@ static LoopOut device_loop(StepFn&& step, const BatchArgs& a, const BLz& lz, int
     cudaGraph_t body = np.conditional.phGraph_out[0];
     QMB_CUDA_TRY(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     const double kernels_before = g_kernels;  // capture records kernels; they run once per loop
-    for (int t = 0; t < check; ++t) step(st);
-    launch_check(a, lz, nsets, stall, res_tol, e_tol, gap_in, gap_out, theta, theta_prev, msteps, conv,
-                 active_next, cap, st, open_cnt.p);
-    g_kernels += 1;
-    k_bloop_ctl<<<1, 256, 0, st>>>(h, 1, n_sectors, active, active_next, open_cnt.p, d_nrows, d_weight, a.nsp,
-                                   check, cap, lz.iter, max_loops, compact_ratio, d_group, n_groups, ctl.p);
+    std::unique_ptr<Error> thrown;
+    try {
+        for (int t = 0; t < check; ++t) step(st);
+        launch_check(a, lz, nsets, stall, res_tol, e_tol, gap_in, gap_out, theta, theta_prev, msteps, conv,
+                     active_next, cap, st, open_cnt.p);
+        g_kernels += 1;
+        k_bloop_ctl<<<1, 256, 0, st>>>(h, 1, n_sectors, active, active_next, open_cnt.p, d_nrows, d_weight, a.nsp,
+                                       check, cap, lz.iter, max_loops, compact_ratio, d_group, n_groups, ctl.p);
+    } catch (const Error& e) {
+        thrown.reset(new Error(e));
+    }
     cudaGraph_t captured = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(st, &captured);
-    QMB_CUDA_TRY(ce);
+    if (ce == cudaSuccess && thrown) throw *thrown;
+    if (ce != cudaSuccess) {
+        // Another thread broke the capture (a wait for the whole device does).  Nothing of
+        // it ran: the blocks are launched from the host.  The graph is left alone, as
+        // destroying one whose body was being captured crashes inside the driver.
+        (void)cudaGetLastError();
+        if (trace_on()) std::fprintf(stderr, "[qmb batch] capture broken (%s): host loop\n", cudaGetErrorString(ce));
+        g = nullptr;
+        g_kernels = kernels_before;
+        return from_host();
+    }
     const double body_kernels = g_kernels - kernels_before;
     g_kernels = kernels_before;
     QMB_CUDA_TRY(cudaGraphInstantiate(&ex, g, 0));
@@ -2419,7 +2435,7 @@ extern "C" qmb_status qmb_batch_create(const qmb_batch_desc* d, qmb_batch* out) 
         b->cz.alloc(b->nsp);
         b->cxy.zero();
         b->cz.zero();
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
         for (BatchPart& P : parts) mark_idle(P.rp, P.col, P.val, P.dxy, P.dz);
         mark_idle(scan_tmp, row_cnt);
         if (trace_on())

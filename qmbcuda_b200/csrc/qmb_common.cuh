@@ -124,6 +124,10 @@ bool mark_idle_after_wait(DevBuf<T>& first, B&... rest) {
     return true;
 }
 
+// Waits for the default stream, where builds run.  (A wait for the whole device would
+// break a stream capture in another thread, this library's own among them.)
+inline void wait_default_stream() { QMB_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int dev) {

@@ -954,7 +954,7 @@ static void build_cb_t(qmb_ham_s* h, int forced_shift, bool single, CbLayout& L)
     L.nb = nb;
     L.shift = shift;
     L.n_codes = (int)keys.size();
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    wait_default_stream();
     mark_idle(miss, mkeys);
 }
 
@@ -1035,7 +1035,7 @@ static void share_cb64_t(qmb_ham_s* h) {
         return;
     }
     bits.download(hb.data(), hb.size());
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    wait_default_stream();
     std::vector<M64> dict(256);
     std::memset(dict.data(), 0, sizeof(M64) * 256);
     for (int c = 1; c <= n_keys; ++c)
@@ -1272,7 +1272,7 @@ void mf_tables(qmb_ham_s* h) {
         check_launch("k_mf_diag");
     }
     h->mf_xs.alloc((size_t)n * (h->cplx ? 16 : 8));
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    wait_default_stream();
     h->mf_ready = true;
 }
 
@@ -1381,7 +1381,7 @@ extern "C" qmb_status qmb_ham_export_ref(qmb_sector s, const qmb_terms* terms, i
         di.download(ind, (size_t)R * W);
         dv.download(reinterpret_cast<double2*>(val), (size_t)R * W);
         dt.download(track, R);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
         mark_idle(di, dv, dt, ov);
     });
 }
@@ -1415,7 +1415,7 @@ void hv_dispatch(const qmb_ham_s* h, int prec, const void* x, void* y, cudaStrea
         if (le && std::strcmp(le, "warp") == 0 && h->n_hops) {
             if (!h->mf_bucket.p) {
                 mf_bucket_table(const_cast<qmb_ham_s*>(h));  // (the caller's handle, in use by this thread alone)
-                QMB_CUDA_TRY(cudaDeviceSynchronize());
+                wait_default_stream();
             }
             auto run = [&](auto op, auto* xv, auto* yv) {
                 using V = std::remove_const_t<std::remove_pointer_t<decltype(xv)>>;

@@ -405,7 +405,7 @@ void sector_buckets(qmb_sector_s* s) {
     s->bucket.alloc(n_b + 1);
     k_bucket<<<grid_for((int64_t)n_b + 1, kBucketChunk), 256>>>(s->reps.p, s->R, L - s->T, n_b, s->bucket.p);
     check_launch("k_bucket");
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    wait_default_stream();
 }
 
 }  // namespace qmb
@@ -447,7 +447,7 @@ extern "C" qmb_status qmb_sector_create(const qmb_sector_desc* d, qmb_sector* ou
         k_rep_write<<<grid_for((int64_t)n_words, 256), 256>>>(L, s->n_up, n_words, words.p,
                                                               offsets.p, s->reps.p);
         check_launch("k_rep_write");
-        sector_buckets(s);  // waits for the device
+        sector_buckets(s);  // waits for the default stream
         mark_idle(words, counts, offsets, tmp);
         *out = own.release();
     });
@@ -511,7 +511,7 @@ void sector_select_irrep(qmb_sector_s* s, const double* chars, double tol_norm) 
     k_active_maps<<<grid_for(s->R, 256), 256>>>(s->R, active.p, pos.p, s->row_of_orbit.p,
                                                 s->orbit_of_row.p);
     check_launch("k_active_maps");
-    QMB_CUDA_TRY(cudaDeviceSynchronize());
+    wait_default_stream();
     mark_idle(active, pos, tmp);
     s->has_irrep = true;
     ++s->irrep_gen;
@@ -533,7 +533,7 @@ extern "C" qmb_status qmb_sector_reps(qmb_sector s, uint64_t* reps, int64_t cap)
         QMB_REQUIRE(cap >= s->R, QMB_ERR_INVALID, "capacity below the orbit count");
         DeviceGuard dg(s->device);
         s->reps.download(reps, s->R);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
     });
 }
 
@@ -544,7 +544,7 @@ extern "C" qmb_status qmb_sector_norms(qmb_sector s, double* norms, int64_t cap)
         QMB_REQUIRE(cap >= s->R, QMB_ERR_INVALID, "capacity below the orbit count");
         DeviceGuard dg(s->device);
         s->norms.download(norms, s->R);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
     });
 }
 
@@ -555,7 +555,7 @@ extern "C" qmb_status qmb_sector_active(qmb_sector s, int64_t* orbit_of_row, int
         QMB_REQUIRE(cap >= s->n_active, QMB_ERR_INVALID, "capacity below the active count");
         DeviceGuard dg(s->device);
         if (s->n_active) s->orbit_of_row.download(orbit_of_row, s->n_active);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
     });
 }
 
@@ -572,7 +572,7 @@ extern "C" qmb_status qmb_sector_orbit_map(qmb_sector s, uint32_t* orbit_indices
                                                               s->n_states, out.p);
         check_launch("k_orbit_map");
         out.download(orbit_indices, 2 * s->n_states);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
         out.mark_idle();
     });
 }
@@ -594,7 +594,7 @@ extern "C" qmb_status qmb_sector_lookup(qmb_sector s, const uint64_t* t, int64_t
         check_launch("k_lookup");
         o.download(orbit, n);
         e.download(element, n);
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
         mark_idle(in, o, e);
     });
 }

@@ -461,7 +461,7 @@ extern "C" qmb_status qmb_ham_load(qmb_sector s, const char* path, qmb_ham* out)
         }
         h->err.alloc(1);
         h->err.zero();
-        QMB_CUDA_TRY(cudaDeviceSynchronize());
+        wait_default_stream();
         build_cb(h.get());  // the coded FP32 layout, as qmb_ham_create builds it
         *out = h.release();
     });
