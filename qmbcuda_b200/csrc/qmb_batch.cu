@@ -520,6 +520,32 @@ __global__ void k_brq_accept(BatchArgs a, int n_prob, int nsets, const double* _
     }
 }
 
+// Component i of the seeded start vectors, uniform in (-1, 1) (splitmix64).
+__device__ __forceinline__ double start_component(uint64_t seed, uint64_t i) {
+    uint64_t z = seed + i + 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return (double)(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
+}
+
+// Restart vectors of norm 0 (or NaN) become the seeded start.  An FP32 phase that
+// outlives its Krylov space (sectors of a few rows) fills the basis with copies of the
+// same directions, and the Ritz vector over them can cancel to nothing; a restart from
+// that returned the energy 0.
+template <class V>
+__global__ void k_brestart_fill(BatchArgs a, int64_t tot, uint64_t seed, const double* __restrict__ psi2,
+                                V* __restrict__ psi) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
+        int s = 0;
+        while (a.sec_elem[s + 1] <= i) ++s;
+        const int set = (int)((i - a.sec_elem[s]) % a.nsp);
+        if (psi2[s * a.nsp + set] > 1e-24) continue;
+        if constexpr (Sc<V>::cplx) psi[i] = make_double2(start_component(seed, 2 * i), start_component(seed, 2 * i + 1));
+        else psi[i] = start_component(seed, i);
+    }
+}
+
 template <class V>
 __global__ void k_bstart(BatchArgs a, int64_t tot, int mode, uint64_t seed, const void* from,
                          V* __restrict__ w0) {
@@ -530,15 +556,8 @@ __global__ void k_bstart(BatchArgs a, int64_t tot, int mode, uint64_t seed, cons
             if constexpr (Sc<V>::cplx) v = cvt<V>(reinterpret_cast<const double2*>(from)[i]);
             else v = cvt<V>(reinterpret_cast<const double*>(from)[i]);
         } else {
-            auto u = [&](uint64_t k) {
-                uint64_t z = seed + k + 0x9E3779B97F4A7C15ull;
-                z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-                z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-                z ^= z >> 31;
-                return (double)(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
-            };
-            if constexpr (Sc<V>::cplx) v = Sc<V>::from(make_double2(u(2 * i), u(2 * i + 1)));
-            else v = Sc<V>::from(make_double2(u(i), 0.0));
+            if constexpr (Sc<V>::cplx) v = Sc<V>::from(make_double2(start_component(seed, 2 * i), start_component(seed, 2 * i + 1)));
+            else v = Sc<V>::from(make_double2(start_component(seed, i), 0.0));
         }
         w0[i] = v;
     }
@@ -2775,6 +2794,9 @@ extern "C" qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const dou
                         g_kernels += 1;
                         k_brq_accept<<<rg2, rb2, 0, st>>>(a, n_prob, b->n_sets, Eq.p, r2.p, sums.p + n_prob, gapb.p, tol64,
                                                           restart_gap_cap(), ok.p, act_d.p);
+                        g_kernels += 1;
+                        if (kd) k_brestart_fill<double2><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, o.seed, sums.p + n_prob, (double2*)psi.p);
+                        else k_brestart_fill<double><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, o.seed, sums.p + n_prob, (double*)psi.p);
                         check_launch("rq check");
                         if (trace_on()) {
                             QMB_CUDA_TRY(cudaStreamSynchronize(st));
