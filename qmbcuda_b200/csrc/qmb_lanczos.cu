@@ -860,6 +860,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
     PhaseOut out;
     const double gap_cap = restart_gap_cap();
     int cap = std::max(1, po.max_iter);
+    if (po.reorth) cap = (int)std::min<int64_t>(cap, n);  // no more orthogonal vectors than rows
     const int K_full = store ? cap + 1 : 2;
     const int hint = po.ring_hint ? *po.ring_hint : 0;
     const int every_steps = std::max(1, po.check_every);
@@ -940,6 +941,8 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
     capture();
 
     std::vector<double> ha(cap + 1), hb(cap + 2);
+    const bool fp32_reorth = po.reorth > 0 && sizeof(typename Sc<V>::real) == 4;
+    double h_scale = 0.0;
     int done = 0;
     double theta_prev = 0.0;
     bool have_prev = false;
@@ -984,7 +987,10 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
         bool breakdown = false;
         for (int i = done - todo; i < done; ++i) {
             double sc_i = std::fabs(ha[i]) + (i > 0 ? std::fabs(hb[i]) : 0.0) + 1e-300;
-            if (!(hb[i + 1] > 1e-13 * sc_i)) {
+            h_scale = std::max(h_scale, sc_i);
+            // (what FP32 vectors leave of an exhausted space is their rounding, which
+            // Gram-Schmidt does not make orthogonal: the coefficients grew to 1e35)
+            if (!(hb[i + 1] > 1e-13 * sc_i) || (fp32_reorth && !(hb[i + 1] > 1e-6 * h_scale))) {
                 QMB_REQUIRE(std::isfinite(ha[i]), QMB_ERR_INVALID,
                             "non-finite Lanczos coefficient (check the Hamiltonian)");
                 done = i + 1;
@@ -994,6 +1000,7 @@ PhaseOut run_phase(const Op& op, size_t op_smem, const PhaseOpts& po, int start_
             QMB_REQUIRE(std::isfinite(ha[i]) && std::isfinite(hb[i + 1]), QMB_ERR_INVALID,
                         "non-finite Lanczos coefficient (check the Hamiltonian)");
         }
+        if (po.reorth && done >= n) breakdown = true;  // the basis spans the sector
         // tridiagonal of the first `done` steps
         double theta = tridiag_min_eig(ha.data(), hb.data() + 1, done);
         std::vector<double> sv(done);
