@@ -533,14 +533,14 @@ __device__ __forceinline__ double start_component(uint64_t seed, uint64_t i) {
 // outlives its Krylov space (sectors of a few rows) fills the basis with copies of the
 // same directions, and the Ritz vector over them can cancel to nothing; a restart from
 // that returned the energy 0.
+// A block a tile, a thread a set.
 template <class V>
-__global__ void k_brestart_fill(BatchArgs a, int64_t tot, uint64_t seed, const double* __restrict__ psi2,
-                                V* __restrict__ psi) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-        int s = 0;
-        while (a.sec_elem[s + 1] <= i) ++s;
-        const int set = (int)((i - a.sec_elem[s]) % a.nsp);
-        if (psi2[s * a.nsp + set] > 1e-24) continue;
+__global__ void k_brestart_fill(BatchArgs a, uint64_t seed, const double* __restrict__ psi2, V* __restrict__ psi) {
+    const int s = a.tile_sector[blockIdx.x], set = threadIdx.x;
+    if (psi2[s * a.nsp + set] > 1e-24) return;
+    const int64_t r0 = a.tile_row0[blockIdx.x], r_end = min(a.sec_nrows[s], r0 + kBTile);
+    for (int64_t r = r0; r < r_end; ++r) {
+        const int64_t i = a.sec_elem[s] + r * a.nsp + set;
         if constexpr (Sc<V>::cplx) psi[i] = make_double2(start_component(seed, 2 * i), start_component(seed, 2 * i + 1));
         else psi[i] = start_component(seed, i);
     }
@@ -2795,8 +2795,8 @@ extern "C" qmb_status qmb_batch_solve(qmb_batch b, const double* c_xy, const dou
                         k_brq_accept<<<rg2, rb2, 0, st>>>(a, n_prob, b->n_sets, Eq.p, r2.p, sums.p + n_prob, gapb.p, tol64,
                                                           restart_gap_cap(), ok.p, act_d.p);
                         g_kernels += 1;
-                        if (kd) k_brestart_fill<double2><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, o.seed, sums.p + n_prob, (double2*)psi.p);
-                        else k_brestart_fill<double><<<grid_for(tot, 256), 256, 0, st>>>(a, tot, o.seed, sums.p + n_prob, (double*)psi.p);
+                        if (kd) k_brestart_fill<double2><<<k.n_tiles, b->nsp, 0, st>>>(a, o.seed, sums.p + n_prob, (double2*)psi.p);
+                        else k_brestart_fill<double><<<k.n_tiles, b->nsp, 0, st>>>(a, o.seed, sums.p + n_prob, (double*)psi.p);
                         check_launch("rq check");
                         if (trace_on()) {
                             QMB_CUDA_TRY(cudaStreamSynchronize(st));
